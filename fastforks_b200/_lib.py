@@ -14,6 +14,7 @@ import os
 import re
 import shutil
 import subprocess
+import tempfile
 import threading
 from pathlib import Path
 
@@ -21,8 +22,10 @@ from .errors import KernelUnavailableError
 
 LIBRARY = "b200attn"
 PACKAGE_DIR = Path(__file__).resolve().parent
-SOURCE = PACKAGE_DIR / "csrc" / "b200_attn.cu"
+SOURCES = (PACKAGE_DIR / "csrc" / "b200_attn.cu", PACKAGE_DIR / "csrc" / "b200_linear.cu")
 HEADERS = (
+    PACKAGE_DIR / "csrc" / "host_common.h",
+    PACKAGE_DIR / "csrc" / "linear_host.h",
     PACKAGE_DIR / "csrc" / "sm100_ptx.cuh",
     PACKAGE_DIR / "csrc" / "attn_fwd_sm100.cuh",
     PACKAGE_DIR / "csrc" / "sam_rel_terms.cuh",
@@ -35,7 +38,7 @@ SHARED_OBJECT = PACKAGE_DIR / "libb200attn.so"
 # sm_100a only: the kernels use tcgen05 / TMEM / TMA, which exist in no other target.
 NVCC_FLAGS = (
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17", "--expt-relaxed-constexpr",
-    "-shared", "-Xcompiler", "-fPIC",
+    "-Xcompiler", "-fPIC",
 )  # fmt: skip
 
 # Every symbol include/b200_attn.h declares.
@@ -151,7 +154,7 @@ def source_hash() -> str:
     """Digest of the sources the shared object is compiled from (16 hex digits). The build passes it to the compiler,
     which puts it into the library's version string, so a binary can be matched with the sources beside it."""
     digest = hashlib.sha256()
-    for path in sorted((SOURCE, *HEADERS), key=lambda f: f.name):
+    for path in sorted((*SOURCES, *HEADERS), key=lambda f: f.name):
         digest.update(path.name.encode())
         digest.update(path.read_bytes())
     return digest.hexdigest()[:16]
@@ -174,7 +177,8 @@ def needs_build() -> bool:
 
 
 def build(*, force: bool = False, verbose: bool = False) -> Path:
-    """Compile `csrc/b200_attn.cu` for sm_100a into `libb200attn.so` next to this file (needs nvcc, no GPU).
+    """Compile the sources in `csrc/` for sm_100a (one compiler process each, in parallel) and link them into
+    `libb200attn.so` next to this file (needs nvcc, no GPU).
 
     Raises:
         KernelUnavailableError: nvcc is missing or the compilation failed.
@@ -184,15 +188,21 @@ def build(*, force: bool = False, verbose: bool = False) -> Path:
     nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
     if not Path(nvcc).exists():
         raise KernelUnavailableError(LIBRARY, "nvcc not found: cannot build libb200attn.so")
-    tmp = SHARED_OBJECT.with_suffix(f".{os.getpid()}.tmp.so")
-    cmd = [nvcc, *NVCC_FLAGS, f'-DB200_SOURCE_HASH="{source_hash()}"', *(("-Xptxas", "-v") if verbose else ()),
-           "-o", str(tmp), str(SOURCE)]  # fmt: skip
-    proc = subprocess.run(cmd, capture_output=True, text=True, check=False)
-    if proc.returncode != 0:
-        tmp.unlink(missing_ok=True)
-        raise KernelUnavailableError(LIBRARY, f"nvcc failed:\n{proc.stdout}\n{proc.stderr}")
-    if verbose:
-        print(proc.stderr)
+    flags = [*NVCC_FLAGS, f'-DB200_SOURCE_HASH="{source_hash()}"', *(("-Xptxas", "-v") if verbose else ())]
+    with tempfile.TemporaryDirectory(prefix="b200attn-") as scratch:
+        objects = [Path(scratch) / f"{source.stem}.o" for source in SOURCES]
+        jobs = [subprocess.Popen([nvcc, *flags, "-c", "-o", str(o), str(source)], stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+                for source, o in zip(SOURCES, objects, strict=True)]  # fmt: skip
+        for text, code in [(job.communicate()[0], job.returncode) for job in jobs]:
+            if code != 0:
+                raise KernelUnavailableError(LIBRARY, f"nvcc failed:\n{text}")
+            if verbose:
+                print(text)
+        tmp = SHARED_OBJECT.with_suffix(f".{os.getpid()}.tmp.so")
+        proc = subprocess.run([nvcc, "-shared", *NVCC_FLAGS[:2], "-o", str(tmp), *map(str, objects)], capture_output=True, text=True, check=False)
+        if proc.returncode != 0:
+            tmp.unlink(missing_ok=True)
+            raise KernelUnavailableError(LIBRARY, f"linking failed:\n{proc.stdout}\n{proc.stderr}")
     tmp.replace(SHARED_OBJECT)
     return SHARED_OBJECT
 

@@ -3,21 +3,19 @@
 //   y[p, n] = act((sum_k x[p, k] w[n, k] + bias[n]) * scale[n] + res[p, n])         (bias, scale, res optional)
 //
 // x [M, K] (row stride lda) and w [N, K] (row-major) are fp16 or bf16, accumulation is fp32 in tensor memory, bias
-// and res have the type of x, scale is fp32, y has the type of x and may alias res (a thread reads the residual of
-// the columns it is about to write, nobody else touches them). act: 0 none, 1 relu, 5 gelu (erf), 6 gelu (tanh form).
+// and res have the type of x, scale is fp32, y has the type of x and may alias res (the residual of a piece of the
+// tile is read before that piece is written, by the same warp, and nobody else touches it). act: 0 none, 1 relu,
+// 5 gelu (erf), 6 gelu (tanh form). One more epilogue serves SwiGLU layers: w holds 2 * N rows, the gate's and then
+// the value's, and y[p, n] = silu(gate) * value (see kActSwiGlu).
 //
-// Persistent CTAs, one per SM, walk output tiles of BM rows x BN columns (128 x 128, 128 x 256 or 256 x 256, chosen
-// by the host: the product needs 2 * 64 * (BM + BN) bytes from L2 for every 2 * 64 * BM * BN flops, and without
-// multicast the L2 bandwidth, not the tensor pipe, bounds the narrow tiles):
-//   * a loader thread stages x and w tiles of 64 k-values through a ring of shared-memory stages with TMA
-//     (128-byte swizzle, rows and k-values past the end read as zero, no multicast);
-//   * an MMA thread issues tcgen05.mma (M = 128, N = BN, K = 16, both operands K-major) into accumulators in
-//     tensor memory: two alternating ones for BM = 128, so that the next tile's products run during the epilogue;
-//     for BM = 256 the two accumulators are the upper and the lower 128 rows of one tile (two MMAs per k-step that
-//     share the w tile);
-//   * eight epilogue warps read a finished accumulator 32 columns at a time, turn the chunk through shared memory
-//     (a thread owns a row in tensor memory, but a warp should write whole rows), apply the epilogue and write y
-//     with 16-byte stores that fill their sectors.
+// Two kernels; gemm_plan() in b200_linear.cu chooses:
+//   * gemm_pair_kernel, for problems that fill the GPU: pairs of CTAs (cta_group::2) compute tiles of 256 rows x BN
+//     columns, so that a CTA loads 128 rows of x and only half of the columns of w for a product of M = 256 (no load is
+//     multicast). At BN = 256 that is 32 KB from L2 per 2 * 128 * 256 * 64 flops and SM, half of what two separate
+//     CTAs with 128 x 256 tiles would pull, and the accumulator takes 256 of the 512 tensor-memory columns: two
+//     alternate, and a tile's epilogue runs under the next tile's products.
+//   * gemm_split_kernel, for problems with few tiles: one 128 x 64 tile per cluster of S CTAs, each of which takes
+//     1 / S of the k range; the partial sums meet through distributed shared memory (no atomics, fixed order).
 // Every barrier wait is bounded (sm100_ptx.cuh); a wait that runs out sets the CTA's abort flag and the role bit
 // in the status word, and all warps fall through to the common exit.
 #pragma once
@@ -32,53 +30,28 @@
 namespace b200 {
 
 constexpr int kGemmBK = 64;
-constexpr int kGemmThreads = 320;  // warp 0 loader, warp 1 MMA, warps 2..9 epilogue
-constexpr int kGemmEpiWarp0 = 2;
+constexpr int kGemmTileBytes = 128 * kGemmBK * 2;  // 128 rows of 64 k-values, the 128-byte swizzle
 enum : uint32_t { kStatusGemmLoader = 64, kStatusGemmMma = 128, kStatusGemmEpilogue = 256 };
-enum : int { kActNone = 0, kActRelu = 1, kActGelu = 5, kActGeluTanh = 6 };
+enum : int { kActNone = 0, kActRelu = 1, kActGelu = 5, kActGeluTanh = 6, kActSwiGlu = 100 };
 
 struct GemmParams {
-  int m, n, k;
+  int m, n, k;         // n: columns of y (a SwiGLU layer's w has 2 n rows)
+  int bn;              // pair kernel: columns of w per tile, a multiple of 64 up to 256 (always 256 with SwiGLU)
   int tiles_m, tiles_n;
-  const void* bias;    // [n] or null
+  int group_m;         // pair kernel: row tiles per raster group (item_at)
+  int stages;          // pair kernel: ring stages of 16 KB of x and 64 bn bytes of w
+  int whole_tiles;     // pair kernel: tiles worked on whole; each of the others is tail_parts items of tail_bn columns
+  int tail_parts, tail_bn;
+  const void* bias;    // [n] (SwiGLU: [2 n]) or null
   const float* scale;  // [n] or null
   const void* res;     // [m, lres] or null
   int64_t lres;
   void* y;
   int64_t ldy;
   int act;
+  int early_w;         // w was complete before the kernel in front of this one started: load it without waiting for that one
   uint32_t* status;
 };
-
-template <int BM, int BN>
-struct GemmSmem {
-  static constexpr int kStages = BM == 256 ? 3 : BN == 256 ? 4 : 5;
-  static constexpr int kBytesA = BM * kGemmBK * 2, kBytesB = BN * kGemmBK * 2;
-  alignas(1024) uint8_t a[kStages][kBytesA];
-  alignas(1024) uint8_t b[kStages][kBytesB];
-  alignas(16) float turn[8][32][32];  // per epilogue warp: 32 rows x 32 columns of fp32 on their way from row owners to row writers
-  uint64_t full[kStages], empty[kStages];
-  uint64_t acc_full[2], acc_empty[2];
-  uint32_t tmem_base;
-  uint32_t abort;
-};
-
-__device__ __forceinline__ float gemm_act(float v, int act) {
-  switch (act) {
-    case kActRelu:
-      return fmaxf(v, 0.f);
-    case kActGelu:
-      return 0.5f * v * (1.f + erff(v * 0.70710678118654752f));
-    case kActGeluTanh: {
-      float t;
-      const float u = 0.7978845608028654f * v * (1.f + 0.044715f * v * v);
-      asm("tanh.approx.f32 %0, %1;" : "=f"(t) : "f"(u));
-      return 0.5f * v * (1.f + t);
-    }
-    default:
-      return v;
-  }
-}
 
 template <typename T>
 __device__ __forceinline__ float2 gemm_unpack2(uint32_t v) {
@@ -96,39 +69,444 @@ __device__ __forceinline__ uint32_t gemm_pack2(float lo, float hi) {
   }
 }
 
-__device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* map, uint64_t* bar, int x, int y) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-      :
-      : "r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(x), "r"(y)
-      : "memory");
+// v Phi(v) with Phi the normal distribution, as max(v, 0) - |v| Phi(-|v|): no cancellation on the negative side, where
+// 0.5 v (1 + erf) loses digits. Phi(-x) = exp(-x^2 / 2) t P(t), t = 1 / (1 + 0.3 x), where P is a degree-7 least-maximum
+// fit of 0.5 erfcx(x / sqrt 2) / t on 0 <= x <= 13.5 (relative error 1.3e-7; the whole within 2e-6 of v Phi(v) down to
+// v = -5, where erff gave 1e-3). Two MUFU operations and a dozen multiply-adds: a third of the time of erff, which took
+// longer than the products of a 256 x 256 tile at k = 768.
+__device__ __forceinline__ float gelu_erf(float v) {
+  const float x = fabsf(v);
+  float t, e;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(t) : "f"(fmaf(x, 0.3f, 1.f)));
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(x * x * -0.72134752f));
+  float p = 0.0359317549f;
+  p = fmaf(p, t, -0.158276081f);
+  p = fmaf(p, t, 0.208206728f);
+  p = fmaf(p, t, -0.0553939454f);
+  p = fmaf(p, t, 0.129469246f);
+  p = fmaf(p, t, 0.0996374786f);
+  p = fmaf(p, t, 0.120798357f);
+  p = fmaf(p, t, 0.119626388f);
+  return fmaxf(v, 0.f) - x * (t * p) * e;
 }
 
-template <typename T, int BM, int BN>
-__global__ void __launch_bounds__(kGemmThreads, 1)
-gemm_epilogue_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_w, const GemmParams p) {
-  static_assert((BM == 128 && (BN == 128 || BN == 256)) || (BM == 256 && BN == 256), "tile shapes that are built");
-  using Smem = GemmSmem<BM, BN>;
-  constexpr int kStages = Smem::kStages;
-  constexpr bool kTall = BM == 256;  // both accumulators belong to one tile
+template <int ACT>
+__device__ __forceinline__ float gemm_act(float v) {
+  if constexpr (ACT == kActRelu) return fmaxf(v, 0.f);
+  if constexpr (ACT == kActGelu) return gelu_erf(v);
+  if constexpr (ACT == kActGeluTanh) {
+    float t;
+    const float u = 0.7978845608028654f * v * (1.f + 0.044715f * v * v);
+    asm("tanh.approx.f32 %0, %1;" : "=f"(t) : "f"(u));
+    return 0.5f * v * (1.f + t);
+  }
+  return v;
+}
+// silu(g) * u = g u / (1 + exp(-g))
+__device__ __forceinline__ float gemm_swiglu(float g, float u) { return __fdividef(g, 1.f + __expf(-g)) * u; }
+
+// Runs f(integral_constant<int, ACT>) for the launch's activation: one decision per chunk, not one per value.
+template <typename F>
+__device__ __forceinline__ void for_act(int act, F&& f) {
+  if (act == kActGeluTanh) f(std::integral_constant<int, kActGeluTanh>{});
+  else if (act == kActGelu) f(std::integral_constant<int, kActGelu>{});
+  else if (act == kActRelu) f(std::integral_constant<int, kActRelu>{});
+  else f(std::integral_constant<int, kActNone>{});
+}
+
+// ---- pair kernel ----------------------------------------------------------------------------------------------
+constexpr int kPairThreads = 320;  // warp 0 loader, warp 1 MMA, warps 2..9 epilogue
+constexpr int kPairRingBytes = 160 * 1024, kPairMaxStages = 8;
+constexpr int kPairChunkBytes = 32 * 64 * 2;  // what an epilogue warp stages at a time: its 32 rows, 64 columns
+
+struct PairSmem {
+  alignas(1024) uint8_t ring[kPairRingBytes];          // per stage: 128 rows of x, then bn / 2 rows of w
+  alignas(1024) uint8_t stage[8][2][kPairChunkBytes];  // per epilogue warp, two deep: residual in, result out
+  uint64_t full[kPairMaxStages];   // the leader's: both CTAs' tiles of the stage have landed     (TMA of both CTAs)
+  uint64_t empty[kPairMaxStages];  // the stage has been read by its products                     (MMA commit, both CTAs)
+  uint64_t acc_full[2];         // accumulator finished                                        (MMA commit, both CTAs)
+  uint64_t acc_empty[2];        // the leader's: read by the epilogue warps of both CTAs       (16 warps)
+  uint64_t res_full[8][2];      // per epilogue warp: the residual of a piece has landed       (TMA)
+  uint64_t drain;               // abort path: the leader's products have finished             (MMA commit, both CTAs)
+  uint32_t tmem_base;
+  uint32_t abort;
+};
+static_assert(sizeof(PairSmem) + 1024 <= 227 * 1024, "shared memory of one CTA");
+
+struct GemmItem {
+  int tm;    // row tile
+  int col0;  // first column of y
+  int bn;    // columns of w: p.bn, or p.tail_bn for a part of a tile
+};
+// Items are the tiles in groups of `group_m` row tiles, row tiles fastest inside a group: the pairs that run at the same
+// time then share both w tiles and x tiles, and what they read together stays in L2. The tiles behind the last whole
+// round of the grid come in parts (pair_items() in b200_linear.cu says when), parts of a tile one after another.
+__device__ __forceinline__ GemmItem item_at(const GemmParams& p, int item, int out_cols) {
+  GemmItem t;
+  int tile = item, sub = 0;
+  t.bn = p.bn;
+  if (item >= p.whole_tiles) {
+    const int i = item - p.whole_tiles, behind = i / p.tail_parts;
+    tile = p.whole_tiles + behind;
+    sub = (i - behind * p.tail_parts) * p.tail_bn;
+    t.bn = p.tail_bn;
+  }
+  const int per_group = p.group_m * p.tiles_n;
+  const int g = tile / per_group;
+  const int in = tile - g * per_group;
+  const int rows = min(p.group_m, p.tiles_m - g * p.group_m);
+  const int tn = in / rows;
+  t.tm = g * p.group_m + (in - tn * rows);
+  t.col0 = tn * out_cols + sub;
+  return t;
+}
+
+// Bounded by the L2 -> SM operand traffic and, above about 1.4 PFLOP/s sustained, the power cap. ACT and FULL (there is a
+// scale or a residual) are template parameters: decided at run time, the branches alone cost 400 clocks per piece.
+template <typename T, int ACT, bool FULL>
+__global__ void __launch_bounds__(kPairThreads, 1)
+gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_w,
+                 const __grid_constant__ CUtensorMap tm_w_tail, const __grid_constant__ CUtensorMap tm_y,
+                 const __grid_constant__ CUtensorMap tm_res, const GemmParams p) {
   extern __shared__ uint8_t smem_raw[];
-  Smem& sm = *reinterpret_cast<Smem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  PairSmem& sm = *reinterpret_cast<PairSmem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int rank = static_cast<int>(cluster_cta_rank());  // 0: the leader, rows 0..127 of the tile
+  constexpr bool swiglu = ACT == kActSwiGlu;
 
   if (threadIdx.x == 0) {
-    for (int i = 0; i < kStages; ++i) {
+    for (int i = 0; i < kPairMaxStages; ++i) {
       mbar_init(&sm.full[i], 1);
       mbar_init(&sm.empty[i], 1);
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(&sm.acc_full[i], 1);
-      mbar_init(&sm.acc_empty[i], kTall ? 4 : 8);  // one arrival per epilogue warp that reads the accumulator
+      mbar_init(&sm.acc_empty[i], 16);
     }
+    for (int i = 0; i < 16; ++i) mbar_init(&sm.res_full[0][0] + i, 1);
+    mbar_init(&sm.drain, 1);
     sm.abort = 0;
     mbar_init_fence();
   }
   if (warp == 1) {
-    tmem_alloc(&sm.tmem_base, 512);  // two accumulators of up to 256 fp32 columns
+    tmem_alloc_pair(&sm.tmem_base, 512);
+    tmem_relinquish_pair();
+  }
+  if (warp == 0 && lane == 0) {
+    tma_prefetch_desc(&tm_x);
+    tma_prefetch_desc(&tm_w);
+    tma_prefetch_desc(&tm_y);
+    if (FULL && p.res != nullptr) tma_prefetch_desc(&tm_res);
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  cluster_arrive();  // the other CTA's barriers exist before anything of this one reaches for them
+  cluster_wait();
+  tc_fence_after_sync();
+  const uint32_t tmem = sm.tmem_base;
+  volatile uint32_t* abort_flag = &sm.abort;
+  const int items = p.whole_tiles + (p.tiles_m * p.tiles_n - p.whole_tiles) * p.tail_parts;
+  const int first_tile = blockIdx.x >> 1, tile_step = gridDim.x >> 1;
+  const int k_blocks = (p.k + kGemmBK - 1) / kGemmBK;
+  const int stages = p.stages;
+  const uint32_t stage_size = kGemmTileBytes + static_cast<uint32_t>(p.bn) * kGemmBK;  // of one CTA: 128 rows of x, bn / 2 of w
+  const int out_cols = swiglu ? 128 : p.bn;  // columns of y per tile
+
+  if (warp == 0) {
+    // ======================= loader (the whole warp, one lane issues: see elect_one) ==================
+    bool ok = true;
+    int g = 0, st = 0;  // stage uses so far, ring position
+    uint32_t ph = 1;    // parity of the empty barriers: a ring that was never used is empty
+    // Both CTAs count their bytes on the leader's barrier.
+    auto load_x = [&](int s, const GemmItem& t, int kb) {
+      tma_load_2d_pair(sm.ring + s * stage_size, &tm_x, cluster_map(smem_u32(&sm.full[s]), 0), kb * kGemmBK, t.tm * 256 + rank * 128);
+    };
+    auto load_w = [&](int s, const GemmItem& t, int kb) {
+      // SwiGLU: the leader's half are 128 gate columns, the other CTA's the value columns that belong to them
+      const int row = swiglu ? t.col0 + rank * p.n : t.col0 + rank * (t.bn >> 1);
+      tma_load_2d_pair(sm.ring + s * stage_size + kGemmTileBytes, t.bn == p.bn ? &tm_w : &tm_w_tail, cluster_map(smem_u32(&sm.full[s]), 0), kb * kGemmBK, row);
+    };
+    auto expect = [&](int s, const GemmItem& t) {
+      if (rank == 0) mbar_arrive_expect_tx(&sm.full[s], 2u * (kGemmTileBytes + static_cast<uint32_t>(t.bn) * kGemmBK));
+    };
+    int early = 0;  // stages whose w tile is on its way before the wait for the kernel in front
+    if (p.early_w && first_tile < items) {
+      const GemmItem t = item_at(p, first_tile, out_cols);
+      for (; early < stages && early < k_blocks; ++early) {
+        if (elect_one()) {
+          expect(early, t);
+          load_w(early, t, early);
+        }
+      }
+    }
+    grid_dependency_wait();
+    grid_launch_dependents();
+    for (int tile = first_tile; tile < items && ok; tile += tile_step) {
+      const GemmItem t = item_at(p, tile, out_cols);
+      for (int kb = 0; kb < k_blocks; ++kb, ++g) {
+        if (g < early) {
+          if (elect_one()) load_x(st, t, kb);
+        } else {
+          ok = __all_sync(0xffffffffu, mbar_wait(&sm.empty[st], ph, abort_flag));
+          if (!ok) break;
+          if (elect_one()) {
+            expect(st, t);
+            load_x(st, t, kb);
+            load_w(st, t, kb);
+          }
+        }
+        if (++st == stages) {
+          st = 0;
+          ph ^= 1;
+        }
+      }
+    }
+    if (!ok && lane == 0 && atomicExch(const_cast<uint32_t*>(abort_flag), 1u) == 0) atomicOr(p.status, kStatusGemmLoader);
+    if (__any_sync(0xffffffffu, *abort_flag != 0) && rank == 0) {  // let every copy that was issued land (both CTAs count on the leader's barriers)
+      uint32_t no_abort = 0;
+      for (int j = (g > stages ? g - stages : 0); j < g; ++j) mbar_wait(&sm.full[j % stages], (j / stages) & 1, &no_abort);
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    // ======================= MMA issuer (leader only) =================================================
+    if (rank == 0) {
+      constexpr uint32_t fmt = std::is_same<T, __half>::value ? UMMA_F16 : UMMA_BF16;
+      const uint32_t idesc_whole = umma_idesc_f16(fmt, 256, p.bn, 0, 0), idesc_tail = umma_idesc_f16(fmt, 256, p.tail_bn, 0, 0);
+      const uint64_t a_desc0 = umma_smem_desc_sw128(smem_u32(sm.ring), 1024, 16);
+      const uint64_t b_desc0 = umma_smem_desc_sw128(smem_u32(sm.ring) + kGemmTileBytes, 1024, 16);
+      bool ok = true;
+      int st = 0, it = 0;
+      uint32_t ph = 0;
+      bool landed = false;  // this stage's barrier, tested while the stage before was being issued (a test takes some 100 clocks)
+      for (int tile = first_tile; tile < items && ok; tile += tile_step, ++it) {
+        if (it >= 2) ok = __all_sync(0xffffffffu, mbar_wait(&sm.acc_empty[it & 1], ((it >> 1) - 1) & 1, abort_flag));
+        if (!ok) break;
+        tc_fence_after_sync();
+        const uint32_t acc = tmem + (it & 1) * 256;
+        const uint32_t idesc = tile < p.whole_tiles ? idesc_whole : idesc_tail;
+        for (int kb = 0; kb < k_blocks; ++kb) {
+          ok = __all_sync(0xffffffffu, landed || mbar_wait(&sm.full[st], ph, abort_flag));
+          if (!ok) break;
+          tc_fence_after_sync();
+          const int next = st + 1 == stages ? 0 : st + 1;
+          const uint32_t next_ph = st + 1 == stages ? ph ^ 1 : ph;
+          landed = mbar_test_wait(&sm.full[next], next_ph);
+          const uint64_t a = a_desc0 + static_cast<uint64_t>(st) * (stage_size >> 4);
+          const uint64_t b = b_desc0 + static_cast<uint64_t>(st) * (stage_size >> 4);
+          if (elect_one()) {
+#pragma unroll
+            for (int kk = 0; kk < kGemmBK / 16; ++kk) umma_ss_pair(acc, a + 2 * kk, b + 2 * kk, idesc, (kb | kk) != 0 ? 1u : 0u);
+            umma_commit_pair(&sm.empty[st]);
+            if (kb == k_blocks - 1) umma_commit_pair(&sm.acc_full[it & 1]);
+          }
+          st = next;
+          ph = next_ph;
+        }
+      }
+      if (!ok && lane == 0 && atomicExch(const_cast<uint32_t*>(abort_flag), 1u) == 0) atomicOr(p.status, kStatusGemmMma);
+      if (__any_sync(0xffffffffu, *abort_flag != 0)) {  // no product may be running when tensor memory is freed
+        uint32_t no_abort = 0;
+        if (elect_one()) umma_commit_pair(&sm.drain);
+        mbar_wait(&sm.drain, 0, &no_abort);
+      }
+    }
+    __syncwarp();
+  } else {
+    // ======================= epilogue warps ==========================================================
+    // A warp owns 32 rows (its quarter of the tensor-memory lanes) and every second 64-column piece of the tile. A
+    // piece goes: accumulator -> registers -> epilogue -> the warp's staging area (128-byte swizzle) -> TMA store, which
+    // clips rows and columns past the end; a residual comes the same way in. No other warp is waited for.
+    grid_dependency_wait();
+    const int e = warp - 2, part = e >> 2, quarter = warp & 3;
+    const uint32_t lane_addr = static_cast<uint32_t>(quarter * 32) << 16;
+    const uint32_t acc_empty_at[2] = {cluster_map(smem_u32(&sm.acc_empty[0]), 0), cluster_map(smem_u32(&sm.acc_empty[1]), 0)};
+    const bool has_res = FULL && p.res != nullptr;
+    const uint32_t stage_row = smem_u32(sm.stage[e][0]) + lane * 128;
+    auto row_of = [&](const GemmItem& t) { return t.tm * 256 + rank * 128 + quarter * 32; };
+    auto inside = [&](int row, int col) { return row < p.m && col < p.n; };
+    bool ok = true;
+    int it = 0;
+    uint32_t loads[2] = {0, 0};  // residual loads into either buffer so far (phases of res_full)
+    for (int tile = first_tile; tile < items && ok; tile += tile_step, ++it) {
+      const GemmItem t = item_at(p, tile, out_cols);
+      const int row0 = row_of(t), col0 = t.col0;
+      const int pieces = swiglu ? 2 : t.bn / 64;
+      // What the epilogue needs besides the accumulator is asked for before the wait for it: the residual of this warp's
+      // two pieces, one per buffer, and bias and scale.
+      if (has_res && lane == 0) {
+        tma_store_wait_read<0>();  // the stores of the tile before have read both buffers
+        for (int i = 0; i < 2; ++i) {
+          const int c = part + 2 * i;
+          if (c < pieces && inside(row0, col0 + c * 64)) {
+            mbar_arrive_expect_tx(&sm.res_full[e][i], kPairChunkBytes);
+            tma_load_2d(sm.stage[e][i], &tm_res, &sm.res_full[e][i], col0 + c * 64, row0);
+          }
+        }
+      }
+      // Lane l holds bias and scale of columns 2 l and 2 l + 1 of either piece; the lanes pass them round with shuffles.
+      // (Loads at one address for the whole warp, where a value is needed, took half of the epilogue's time.)
+      uint32_t bias2[2] = {0, 0}, bias_up = 0;
+      float2 scale2[2] = {make_float2(1.f, 1.f), make_float2(1.f, 1.f)};
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const int c = col0 + (part + 2 * i) * 64 + 2 * lane;
+        if (part + 2 * i < pieces && c < p.n) {
+          if (p.bias != nullptr) bias2[i] = __ldg(reinterpret_cast<const uint32_t*>(static_cast<const T*>(p.bias) + c));
+          if (swiglu && p.bias != nullptr) bias_up = __ldg(reinterpret_cast<const uint32_t*>(static_cast<const T*>(p.bias) + p.n + c));
+          if (p.scale != nullptr) scale2[i] = __ldg(reinterpret_cast<const float2*>(p.scale + c));
+        }
+      }
+      if (!__all_sync(0xffffffffu, mbar_wait(&sm.acc_full[it & 1], (it >> 1) & 1, abort_flag))) {
+        ok = false;
+        break;
+      }
+      tc_fence_after_sync();
+      const uint32_t acc = tmem + lane_addr + (it & 1) * 256;
+      if (part >= pieces) {
+        if (lane == 0) mbar_arrive_cluster(acc_empty_at[it & 1]);
+        continue;
+      }
+#pragma unroll 1
+      for (int c = part; c < pieces; c += 2) {
+        const int buf = c >> 1;
+        const int col = col0 + c * 64;
+        const bool here = inside(row0, col);
+        if (has_res) {
+          if (here) {
+            if (!__all_sync(0xffffffffu, mbar_wait(&sm.res_full[e][buf], loads[buf] & 1, abort_flag))) {
+              ok = false;
+              break;
+            }
+            ++loads[buf];
+          }
+        } else {
+          if (lane == 0) {  // the store that used this buffer last has read it
+            if (part + 2 < pieces) tma_store_wait_read<1>();
+            else tma_store_wait_read<0>();
+          }
+        }
+        __syncwarp();
+        if (here) {
+          const uint32_t at = stage_row + buf * kPairChunkBytes;
+          const uint32_t piece_bias = buf == 0 ? bias2[0] : bias2[1];
+          const float2 piece_scale = buf == 0 ? scale2[0] : scale2[1];
+          // one lane's row: eight 16-byte groups of eight columns at the positions of the 128-byte swizzle, in two halves
+#pragma unroll
+          for (int half = 0; half < 2; ++half) {
+            [[maybe_unused]] uint4 r4[FULL ? 4 : 1];
+            if constexpr (FULL) {
+#pragma unroll
+              for (int q = 0; q < 4; ++q) r4[q] = has_res ? ld_shared_v4(at + (((4 * half + q) ^ (lane & 7)) << 4)) : make_uint4(0, 0, 0, 0);
+            }
+            float v[32];
+            [[maybe_unused]] float u[swiglu ? 32 : 1];
+            tmem_ld_x32(acc + c * 64 + half * 32, reinterpret_cast<uint32_t*>(v));
+            if constexpr (swiglu) tmem_ld_x32(acc + 128 + c * 64 + half * 32, reinterpret_cast<uint32_t*>(u));
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              float x[8];
+              const uint32_t spot = at + (((4 * half + q) ^ (lane & 7)) << 4);
+              [[maybe_unused]] uint32_t rw[4] = {0, 0, 0, 0};
+              if constexpr (FULL) { rw[0] = r4[q].x; rw[1] = r4[q].y; rw[2] = r4[q].z; rw[3] = r4[q].w; }
+#pragma unroll
+              for (int i = 0; i < 4; ++i) {
+                const int pair = 16 * half + 4 * q + i, at_v = 8 * q + 2 * i;
+                const float2 b = gemm_unpack2<T>(__shfl_sync(0xffffffffu, piece_bias, pair));
+                if constexpr (swiglu) {
+                  const float2 bu = gemm_unpack2<T>(__shfl_sync(0xffffffffu, bias_up, pair));
+                  x[2 * i] = gemm_swiglu(v[at_v] + b.x, u[at_v] + bu.x);
+                  x[2 * i + 1] = gemm_swiglu(v[at_v + 1] + b.y, u[at_v + 1] + bu.y);
+                } else {
+                  const float2 r = gemm_unpack2<T>(rw[i]);
+                  float2 y = make_float2(v[at_v] + b.x, v[at_v + 1] + b.y);
+                  if constexpr (FULL) {
+                    y.x = fmaf(y.x, __shfl_sync(0xffffffffu, piece_scale.x, pair), r.x);
+                    y.y = fmaf(y.y, __shfl_sync(0xffffffffu, piece_scale.y, pair), r.y);
+                  }
+                  x[2 * i] = gemm_act<ACT>(y.x);
+                  x[2 * i + 1] = gemm_act<ACT>(y.y);
+                }
+              }
+              st_shared_v4(spot, make_uint4(gemm_pack2<T>(x[0], x[1]), gemm_pack2<T>(x[2], x[3]), gemm_pack2<T>(x[4], x[5]), gemm_pack2<T>(x[6], x[7])));
+            }
+          }
+          fence_proxy_async_smem();
+        }
+        if (c + 2 >= pieces) tc_fence_before_sync();  // this warp has read all it needs of the accumulator
+        __syncwarp();
+        if (c + 2 >= pieces && lane == 0) mbar_arrive_cluster(acc_empty_at[it & 1]);
+        if (lane == 0) {
+          if (here) tma_store_2d(&tm_y, sm.stage[e][buf], col, row0);
+          tma_store_commit();
+        }
+      }
+    }
+    if (!ok && lane == 0 && atomicExch(const_cast<uint32_t*>(abort_flag), 1u) == 0) atomicOr(p.status, kStatusGemmEpilogue);
+    if (lane == 0) {
+      tma_store_wait_read<0>();
+      if (*abort_flag != 0 && has_res) {  // a residual still on its way must land before the CTA goes
+        uint32_t no_abort = 0;
+        for (int i = 0; i < 2; ++i) mbar_wait(&sm.res_full[e][i], loads[i] & 1, &no_abort);
+      }
+    }
+    __syncwarp();
+  }
+
+  tc_fence_before_sync();
+  __syncthreads();
+  cluster_arrive();  // neither CTA goes while the other may still signal its barriers or multiply into its tensor memory
+  cluster_wait();
+  if (warp == 1) {
+    tc_fence_after_sync();
+    tmem_dealloc_pair(tmem, 512);
+  }
+}
+
+// ---- split kernel ---------------------------------------------------------------------------------------------
+constexpr int kSplitThreads = 192;  // warp 0 loader, warp 1 MMA, warps 2..5 epilogue
+constexpr int kSplitStages = 6;     // a round trip to L2 covers some four stages
+constexpr int kSplitBN = 64;
+
+template <int S>
+struct SplitSmem {
+  static constexpr int kRows = (128 + S - 1) / S;  // rows of the tile each CTA of the cluster finishes (the last one what is left)
+  static constexpr int kStride = kRows | 1;        // in float4: odd, so that rows and columns are both read without conflicts
+  alignas(1024) uint8_t a[kSplitStages][kGemmTileBytes];
+  alignas(1024) uint8_t b[kSplitStages][kSplitBN * kGemmBK * 2];
+  float4 recv[S][kSplitBN / 4][kStride];     // [from CTA][four columns][row]: partial sums of this CTA's rows
+  uint64_t full[kSplitStages], empty[kSplitStages];
+  uint64_t acc_full;
+  uint32_t tmem_base;
+  uint32_t abort;
+};
+
+// Latency-bound: a few tiles of a small problem. The k range is cut over the S CTAs of a cluster so that more SMs pull
+// operands; every CTA sends each of its 128 rows' partial sums to the CTA that finishes that row, and adds the S parts
+// of its own rows in rank order.
+template <typename T, int S>
+__global__ void __launch_bounds__(kSplitThreads)
+gemm_split_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_w, const GemmParams p) {
+  using Smem = SplitSmem<S>;
+  extern __shared__ uint8_t smem_raw[];
+  Smem& sm = *reinterpret_cast<Smem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int rank = S > 1 ? static_cast<int>(cluster_cta_rank()) : 0;
+  const int tile = blockIdx.x / S;
+  const int tm = tile % p.tiles_m, tn = tile / p.tiles_m;
+  const int k_blocks = (p.k + kGemmBK - 1) / kGemmBK;
+  const int kb0 = k_blocks * rank / S, kb1 = k_blocks * (rank + 1) / S;  // at least one each (gemm_plan)
+
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < kSplitStages; ++i) {
+      mbar_init(&sm.full[i], 1);
+      mbar_init(&sm.empty[i], 1);
+    }
+    mbar_init(&sm.acc_full, 1);
+    sm.abort = 0;
+    mbar_init_fence();
+  }
+  if (warp == 1) {
+    tmem_alloc(&sm.tmem_base, 64);
     tmem_relinquish();
   }
   if (warp == 0 && lane == 0) {
@@ -138,205 +516,151 @@ gemm_epilogue_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_cons
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
-  grid_dependency_wait();  // programmatic stream serialisation: see the attention kernel
+  if constexpr (S > 1) cluster_arrive();  // this CTA runs; waited for before anybody writes into its receive area
   const uint32_t tmem = sm.tmem_base;
   volatile uint32_t* abort_flag = &sm.abort;
-  const int tiles = p.tiles_m * p.tiles_n;
-  const int k_blocks = (p.k + kGemmBK - 1) / kGemmBK;
 
   if (warp == 0) {
-    // ======================= loader ==================================================================
-    if (lane == 0) {
-      bool ok = true;
-      int g = 0;  // stage uses so far
-      for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
-        // m runs fastest: CTAs that work at the same time share a w tile (it meets them in L2)
-        const int tm = tile % p.tiles_m, tn = tile / p.tiles_m;
-        for (int kb = 0; kb < k_blocks; ++kb, ++g) {
-          const int st = g % kStages;
-          ok = mbar_wait_relaxed(&sm.empty[st], ((g / kStages) & 1) ^ 1, abort_flag);
-          if (!ok) break;
-          mbar_arrive_expect_tx(&sm.full[st], Smem::kBytesA + Smem::kBytesB);
-          // a box holds 128 rows: one per 128 rows of either operand
-#pragma unroll
-          for (int h = 0; h < BM / 128; ++h)
-            tma_load_2d(sm.a[st] + h * 128 * kGemmBK * 2, &tm_x, &sm.full[st], kb * kGemmBK, tm * BM + h * 128);
-#pragma unroll
-          for (int h = 0; h < BN / 128; ++h)
-            tma_load_2d(sm.b[st] + h * 128 * kGemmBK * 2, &tm_w, &sm.full[st], kb * kGemmBK, tn * BN + h * 128);
+    bool ok = true;
+    constexpr uint32_t kBytes = kGemmTileBytes + kSplitBN * kGemmBK * 2;
+    int early = 0;
+    if (p.early_w) {
+      for (; early < kSplitStages && kb0 + early < kb1; ++early) {
+        if (elect_one()) {
+          mbar_arrive_expect_tx(&sm.full[early], kBytes);
+          tma_load_2d(sm.b[early], &tm_w, &sm.full[early], (kb0 + early) * kGemmBK, tn * kSplitBN);
         }
       }
-      if (!ok && atomicExch(const_cast<uint32_t*>(abort_flag), 1u) == 0) atomicOr(p.status, kStatusGemmLoader);
-      if (*abort_flag != 0) {  // let every copy that was issued land before the CTA goes
-        uint32_t no_abort = 0;
-        for (int j = (g > kStages ? g - kStages : 0); j < g; ++j) mbar_wait_relaxed(&sm.full[j % kStages], (j / kStages) & 1, &no_abort);
+    }
+    grid_dependency_wait();
+    grid_launch_dependents();
+    int g = 0, st = 0;
+    uint32_t ph = 1;
+    for (int kb = kb0; kb < kb1; ++kb, ++g) {
+      if (g < early) {
+        if (elect_one()) tma_load_2d(sm.a[st], &tm_x, &sm.full[st], kb * kGemmBK, tm * 128);
+      } else {
+        // the first round of the ring needs no wait: nothing has been in it
+        ok = __all_sync(0xffffffffu, g < kSplitStages || mbar_wait(&sm.empty[st], ph, abort_flag));
+        if (!ok) break;
+        if (elect_one()) {
+          mbar_arrive_expect_tx(&sm.full[st], kBytes);
+          tma_load_2d(sm.b[st], &tm_w, &sm.full[st], kb * kGemmBK, tn * kSplitBN);
+          tma_load_2d(sm.a[st], &tm_x, &sm.full[st], kb * kGemmBK, tm * 128);
+        }
       }
+      if (++st == kSplitStages) {
+        st = 0;
+        ph ^= 1;
+      }
+    }
+    if (!ok && lane == 0 && atomicExch(const_cast<uint32_t*>(abort_flag), 1u) == 0) atomicOr(p.status, kStatusGemmLoader);
+    if (__any_sync(0xffffffffu, *abort_flag != 0)) {
+      uint32_t no_abort = 0;
+      for (int j = (g > kSplitStages ? g - kSplitStages : 0); j < g; ++j) mbar_wait(&sm.full[j % kSplitStages], (j / kSplitStages) & 1, &no_abort);
     }
     __syncwarp();
   } else if (warp == 1) {
-    // ======================= MMA issuer ==============================================================
-    if (lane == 0) {
-      constexpr uint32_t fmt = std::is_same<T, __half>::value ? UMMA_F16 : UMMA_BF16;
-      constexpr uint32_t idesc = umma_idesc_f16(fmt, 128, BN, 0, 0);
-      const uint64_t a_desc0 = umma_smem_desc_sw128(smem_u32(sm.a[0]), 1024, 16);
-      const uint64_t b_desc0 = umma_smem_desc_sw128(smem_u32(sm.b[0]), 1024, 16);
-      bool ok = true;
-      int g = 0, it = 0;
-      for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x, ++it) {
-        // The epilogue must have read the accumulator(s) this tile writes: for 128-row tiles the one used two tiles
-        // ago, for 256-row tiles both halves of the tile before.
-        if constexpr (kTall) {
-          if (it >= 1) ok = mbar_wait(&sm.acc_empty[0], (it - 1) & 1, abort_flag) && mbar_wait(&sm.acc_empty[1], (it - 1) & 1, abort_flag);
-        } else {
-          if (it >= 2) ok = mbar_wait(&sm.acc_empty[it & 1], ((it >> 1) - 1) & 1, abort_flag);
-        }
-        if (!ok) break;
-        tc_fence_after_sync();
-        const uint32_t acc = tmem + (kTall ? 0 : (it & 1) * 256);
-        for (int kb = 0; kb < k_blocks; ++kb, ++g) {
-          const int st = g % kStages;
-          ok = mbar_wait(&sm.full[st], (g / kStages) & 1, abort_flag);
-          if (!ok) break;
-          tc_fence_after_sync();
-          const uint64_t a = a_desc0 + static_cast<uint64_t>(st) * (Smem::kBytesA >> 4);
-          const uint64_t b = b_desc0 + static_cast<uint64_t>(st) * (Smem::kBytesB >> 4);
-#pragma unroll
-          for (int h = 0; h < BM / 128; ++h)
-#pragma unroll
-            for (int kk = 0; kk < kGemmBK / 16; ++kk)
-              umma_ss(acc + h * 256, a + h * ((128 * kGemmBK * 2) >> 4) + 2 * kk, b + 2 * kk, idesc, (kb | kk) != 0 ? 1u : 0u);
-          umma_commit(&sm.empty[st]);
-        }
-        if (ok) {
-          if constexpr (kTall) {
-            umma_commit(&sm.acc_full[0]);
-            umma_commit(&sm.acc_full[1]);
-          } else {
-            umma_commit(&sm.acc_full[it & 1]);
-          }
-        }
-      }
-      if (!ok && atomicExch(const_cast<uint32_t*>(abort_flag), 1u) == 0) atomicOr(p.status, kStatusGemmMma);
-    }
-    __syncwarp();
-  } else {
-    // ======================= epilogue warps ==========================================================
-    const int e = warp - kGemmEpiWarp0;          // 0..7
-    const int quarter = warp & 3;                // the tensor-memory lanes this warp may read: 32 * (warp % 4) ..
-    const int part = e >> 2;                     // 128-row tiles: which half of the columns; 256-row tiles: which half of the rows
-    const uint32_t lane_addr = static_cast<uint32_t>(quarter * 32) << 16;
-    constexpr int kCols = kTall ? BN : BN / 2;   // columns per warp
-    float(*turn)[32] = sm.turn[e];
-    bool ok = true;
-    int it = 0;
-    for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x, ++it) {
-      const int tm = tile % p.tiles_m, tn = tile / p.tiles_m;
-      const int buf = kTall ? part : (it & 1);
-      const uint32_t parity = kTall ? (it & 1) : ((it >> 1) & 1);
-      if (!__all_sync(0xffffffffu, mbar_wait(&sm.acc_full[buf], parity, abort_flag))) {
-        ok = false;
-        break;
-      }
+    constexpr uint32_t fmt = std::is_same<T, __half>::value ? UMMA_F16 : UMMA_BF16;
+    constexpr uint32_t idesc = umma_idesc_f16(fmt, 128, kSplitBN, 0, 0);
+    const uint64_t a_desc0 = umma_smem_desc_sw128(smem_u32(sm.a[0]), 1024, 16);
+    const uint64_t b_desc0 = umma_smem_desc_sw128(smem_u32(sm.b[0]), 1024, 16);
+    bool ok = true, landed = false;
+    int st = 0;
+    uint32_t ph = 0;
+    for (int kb = kb0; kb < kb1; ++kb) {
+      ok = __all_sync(0xffffffffu, landed || mbar_wait(&sm.full[st], ph, abort_flag));
+      if (!ok) break;
       tc_fence_after_sync();
-      const int row0 = tm * BM + (kTall ? part * 128 : 0) + quarter * 32;  // first of this warp's 32 rows
-      const int col0 = tn * BN + (kTall ? 0 : part * kCols);
-      const uint32_t acc = tmem + lane_addr + buf * 256 + (kTall ? 0 : part * kCols);
-#pragma unroll 1
-      for (int c = 0; c < kCols; c += 32) {
-        if (col0 + c >= p.n) break;  // warp-uniform: the whole chunk lies past the last column
-        // The residual of the eight columns this lane will write, asked for before anything else of the chunk:
-        // the loads fly while the accumulator is read and turned.
-        const int cg = lane & 3;                  // which eight columns of the chunk
-        const int col = col0 + c + cg * 8;
-        uint4 rv[4];
-        if (p.res != nullptr && col < p.n) {
+      const int next = st + 1 == kSplitStages ? 0 : st + 1;
+      const uint32_t next_ph = st + 1 == kSplitStages ? ph ^ 1 : ph;
+      landed = mbar_test_wait(&sm.full[next], next_ph);
+      const uint64_t a = a_desc0 + static_cast<uint64_t>(st) * (kGemmTileBytes >> 4);
+      const uint64_t b = b_desc0 + static_cast<uint64_t>(st) * ((kSplitBN * kGemmBK * 2) >> 4);
+      if (elect_one()) {
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const int row = row0 + (lane >> 2) + 8 * i;
-            rv[i] = row < p.m ? *reinterpret_cast<const uint4*>(static_cast<const T*>(p.res) + static_cast<int64_t>(row) * p.lres + col)
-                              : make_uint4(0, 0, 0, 0);
-          }
-        }
-        float v[32];
-        tmem_ld_x32(acc + c, reinterpret_cast<uint32_t*>(v));
-        // Row owner -> row writer: thread `lane` holds row `lane`; afterwards lane l holds, for i = 0..3, the eight
-        // columns (l % 4) * 8.. of row l / 4 + 8 i, so that a store instruction of the warp writes eight rows of
-        // 64 contiguous bytes. 16-byte chunks are placed at chunk ^ (row % 8): conflict-free both ways.
-#pragma unroll
-        for (int q = 0; q < 8; ++q)
-          *reinterpret_cast<float4*>(&turn[lane][((q ^ (lane & 7)) << 2)]) = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
-        __syncwarp();
-        if (col < p.n) {                          // n is a multiple of 8: eight columns are inside or outside together
-          float bias8[8], scale8[8];
-#pragma unroll
-          for (int q = 0; q < 8; ++q) {
-            bias8[q] = 0.f;
-            scale8[q] = 1.f;
-          }
-          if (p.bias != nullptr) {
-            const uint4 bv = __ldg(reinterpret_cast<const uint4*>(static_cast<const T*>(p.bias) + col));
-            const uint32_t w4[4] = {bv.x, bv.y, bv.z, bv.w};
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-              const float2 f = gemm_unpack2<T>(w4[q]);
-              bias8[2 * q] = f.x;
-              bias8[2 * q + 1] = f.y;
-            }
-          }
-          if (p.scale != nullptr) {
-            const float4 s0 = __ldg(reinterpret_cast<const float4*>(p.scale + col));
-            const float4 s1 = __ldg(reinterpret_cast<const float4*>(p.scale + col + 4));
-            scale8[0] = s0.x; scale8[1] = s0.y; scale8[2] = s0.z; scale8[3] = s0.w;
-            scale8[4] = s1.x; scale8[5] = s1.y; scale8[6] = s1.z; scale8[7] = s1.w;
-          }
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const int r = (lane >> 2) + 8 * i;
-            const int row = row0 + r;
-            if (row >= p.m) break;
-            const float4 lo = *reinterpret_cast<const float4*>(&turn[r][(((2 * cg) ^ (r & 7)) << 2)]);
-            const float4 hi = *reinterpret_cast<const float4*>(&turn[r][(((2 * cg + 1) ^ (r & 7)) << 2)]);
-            float x[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
-#pragma unroll
-            for (int q = 0; q < 8; ++q) x[q] = (x[q] + bias8[q]) * scale8[q];
-            if (p.res != nullptr) {
-              const uint32_t w4[4] = {rv[i].x, rv[i].y, rv[i].z, rv[i].w};
-#pragma unroll
-              for (int q = 0; q < 4; ++q) {
-                const float2 f = gemm_unpack2<T>(w4[q]);
-                x[2 * q] += f.x;
-                x[2 * q + 1] += f.y;
-              }
-            }
-            if (p.act != kActNone) {
-#pragma unroll
-              for (int q = 0; q < 8; ++q) x[q] = gemm_act(x[q], p.act);
-            }
-            uint4 out;
-            out.x = gemm_pack2<T>(x[0], x[1]);
-            out.y = gemm_pack2<T>(x[2], x[3]);
-            out.z = gemm_pack2<T>(x[4], x[5]);
-            out.w = gemm_pack2<T>(x[6], x[7]);
-            *reinterpret_cast<uint4*>(static_cast<T*>(p.y) + static_cast<int64_t>(row) * p.ldy + col) = out;
-          }
-        }
-        __syncwarp();  // the chunk has been read back before the next one overwrites it
+        for (int kk = 0; kk < kGemmBK / 16; ++kk) umma_ss(tmem, a + 2 * kk, b + 2 * kk, idesc, (kb != kb0 || kk != 0) ? 1u : 0u);
+        umma_commit(&sm.empty[st]);
       }
-      // every column of this warp is in registers or written: the accumulator may be overwritten
-      tc_fence_before_sync();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&sm.acc_empty[buf]);
+      st = next;
+      ph = next_ph;
     }
-    if (!ok && lane == 0) {
-      if (atomicExch(const_cast<uint32_t*>(abort_flag), 1u) == 0) atomicOr(p.status, kStatusGemmEpilogue);
-    }
+    if (!ok && lane == 0 && atomicExch(const_cast<uint32_t*>(abort_flag), 1u) == 0) atomicOr(p.status, kStatusGemmMma);
+    __syncwarp();
+    if (elect_one()) umma_commit(&sm.acc_full);  // also on the abort path: the epilogue's wait then ends when the products in flight have
+    __syncwarp();
   }
 
+  // Epilogue thread: four columns (the same for all its items) of every eighth row. What the epilogue needs besides the
+  // sums is in flight while the products run.
+  constexpr int kItems = (Smem::kRows * (kSplitBN / 4) + 127) / 128;
+  const int et = threadIdx.x - 64, c4 = et & 15;
+  const int first_row = rank * Smem::kRows, end_row = min(min(first_row + Smem::kRows, 128), p.m - tm * 128);  // in the tile
+  const int row0 = tm * 128 + first_row + (et >> 4), row_end = tm * 128 + end_row, col = tn * kSplitBN + c4 * 4;
+  const bool col_in = col < p.n;
+  uint2 bias = make_uint2(0, 0), res[kItems];
+  float4 scale = make_float4(1.f, 1.f, 1.f, 1.f);
+  if (warp >= 2) {
+    grid_dependency_wait();
+    if (p.bias != nullptr && col_in) bias = __ldg(reinterpret_cast<const uint2*>(static_cast<const T*>(p.bias) + col));
+    if (p.scale != nullptr && col_in) scale = __ldg(reinterpret_cast<const float4*>(p.scale + col));
+#pragma unroll
+    for (int i = 0; i < kItems; ++i) {
+      res[i] = make_uint2(0, 0);
+      if (p.res != nullptr && col_in && row0 + 8 * i < row_end)
+        res[i] = *reinterpret_cast<const uint2*>(static_cast<const T*>(p.res) + static_cast<int64_t>(row0 + 8 * i) * p.lres + col);
+    }
+    if (!__all_sync(0xffffffffu, mbar_wait(&sm.acc_full, 0, abort_flag)) && lane == 0 &&
+        atomicExch(const_cast<uint32_t*>(abort_flag), 1u) == 0)
+      atomicOr(p.status, kStatusGemmEpilogue);
+    tc_fence_after_sync();
+  }
+  if constexpr (S > 1) cluster_wait();
+  if (warp >= 2) {
+    const int row = (warp & 3) * 32 + lane;  // this thread's row of the tile
+    float v[kSplitBN];
+    tmem_ld_x64(tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16), reinterpret_cast<uint32_t*>(v));
+    uint32_t dst = smem_u32(&sm.recv[rank][0][row % Smem::kRows]);
+    if constexpr (S > 1) dst = cluster_map(dst, row / Smem::kRows);
+#pragma unroll
+    for (int c4 = 0; c4 < kSplitBN / 4; ++c4)
+      st_cluster_v4(dst + c4 * (Smem::kStride * 16), make_float4(v[4 * c4], v[4 * c4 + 1], v[4 * c4 + 2], v[4 * c4 + 3]));
+  }
   tc_fence_before_sync();
+  if constexpr (S > 1) {
+    cluster_arrive();
+    cluster_wait();
+  } else {
+    __syncthreads();
+  }
+  if (warp >= 2) {
+    const float2 b0 = gemm_unpack2<T>(bias.x), b1 = gemm_unpack2<T>(bias.y);
+    for_act(p.act, [&](auto act_tag) {
+      constexpr int kAct = decltype(act_tag)::value;
+#pragma unroll
+      for (int i = 0; i < kItems; ++i) {
+        const int r = min((et >> 4) + 8 * i, Smem::kRows - 1);  // past the last row: read what is there, write nothing
+        float4 x = sm.recv[0][c4][r];
+#pragma unroll
+        for (int s = 1; s < S; ++s) {
+          const float4 o = sm.recv[s][c4][r];
+          x.x += o.x; x.y += o.y; x.z += o.z; x.w += o.w;
+        }
+        const float2 r0 = gemm_unpack2<T>(res[i].x), r1 = gemm_unpack2<T>(res[i].y);
+        x.x = fmaf(x.x + b0.x, scale.x, r0.x);
+        x.y = fmaf(x.y + b0.y, scale.y, r0.y);
+        x.z = fmaf(x.z + b1.x, scale.z, r1.x);
+        x.w = fmaf(x.w + b1.y, scale.w, r1.y);
+        if (col_in && row0 + 8 * i < row_end)
+          *reinterpret_cast<uint2*>(static_cast<T*>(p.y) + static_cast<int64_t>(row0 + 8 * i) * p.ldy + col) =
+              make_uint2(gemm_pack2<T>(gemm_act<kAct>(x.x), gemm_act<kAct>(x.y)), gemm_pack2<T>(gemm_act<kAct>(x.z), gemm_act<kAct>(x.w)));
+      }
+    });
+  }
   __syncthreads();
   if (warp == 1) {
     tc_fence_after_sync();
-    tmem_dealloc(tmem, 512);
+    tmem_dealloc(tmem, 64);
   }
 }
 

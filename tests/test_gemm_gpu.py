@@ -78,6 +78,19 @@ def test_layerscale_and_in_place_residual(m: int, n: int, k: int, dtype: str) ->
     check(other, x, w, None, None, before, act=ff.ACT_RELU, what="no bias + residual + relu")
 
 
+# One shape for every way a product is cut: the split kernel whole and with 2, 3, 4, 6 and 8 CTAs per cluster (uneven k
+# shares, rows that do not divide, a last tile of one row), pair tiles of 64 to 256 columns, and a last round in parts.
+PLANS = [(100, 72, 8), (197, 2304, 776), (257, 1024, 1544), (129, 776, 1000), (60, 64, 3080), (255, 384, 1536), (1, 8, 4096), (1000, 3000, 72),
+         (1500, 768, 768), (1025, 2056, 136), (5480, 1000, 328), (9500, 2056, 72), (2740, 4096, 200)]  # fmt: skip
+
+
+@pytest.mark.parametrize(("m", "n", "k"), PLANS)
+def test_every_cut_of_a_product(m: int, n: int, k: int) -> None:
+    x, w, bias, scale, res = (t.cuda() for t in operands(m, n, k, torch.bfloat16, seed=m + k))
+    out = torch.full((m, n), float("nan"), dtype=torch.bfloat16, device="cuda")
+    check(ff.gemm(x, w, bias, scale=scale, res=res, act=ff.ACT_GELU, out=out), x, w, bias, scale, res, act=ff.ACT_GELU, what=f"[{m},{n},{k}]")
+
+
 def test_row_strided_views_and_leading_dims() -> None:
     """x, res and out as 2-D views with a row stride (lda, lres, ldy) and x with leading batch dims."""
     gen = torch.Generator().manual_seed(5)
