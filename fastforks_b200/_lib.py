@@ -22,7 +22,7 @@ from .errors import KernelUnavailableError
 
 LIBRARY = "b200attn"
 PACKAGE_DIR = Path(__file__).resolve().parent
-SOURCES = (PACKAGE_DIR / "csrc" / "b200_attn.cu", PACKAGE_DIR / "csrc" / "b200_linear.cu")
+SOURCES = (PACKAGE_DIR / "csrc" / "b200_attn.cu", PACKAGE_DIR / "csrc" / "b200_linear.cu", PACKAGE_DIR / "csrc" / "b200_encoder.cu")
 HEADERS = (
     PACKAGE_DIR / "csrc" / "host_common.h",
     PACKAGE_DIR / "csrc" / "linear_host.h",
@@ -31,7 +31,9 @@ HEADERS = (
     PACKAGE_DIR / "csrc" / "sam_rel_terms.cuh",
     PACKAGE_DIR / "csrc" / "rope_sm100.cuh",
     PACKAGE_DIR / "csrc" / "gemm_sm100.cuh",
+    PACKAGE_DIR / "csrc" / "encoder_kernels.cuh",
     PACKAGE_DIR.parent / "include" / "b200_attn.h",
+    PACKAGE_DIR.parent / "include" / "b200_encoder.h",
 )
 SHARED_OBJECT = PACKAGE_DIR / "libb200attn.so"
 
@@ -46,6 +48,9 @@ EXPORTS = (
     "b200_attn_fwd", "b200_attn_fwd_static", "b200_gemm", "b200_sam_rel_terms", "b200_rope_qk", "b200_attn_query", "b200_attn_plan", "b200_attn_workspace_size", "b200_attn_status",
     "b200_attn_selftest_wait_limit", "b200_attn_last_error", "b200_attn_version",
 )  # fmt: skip
+
+# ... and include/b200_encoder.h.
+ENCODER_EXPORTS = ("b200_encoder_workspace", "b200_encoder_forward")
 
 OK, UNSUPPORTED, BAD_CONFIG, CUDA_ERROR_BASE = 0, 1, -1, 1000
 F16, BF16, F32 = 0, 1, 2
@@ -150,6 +155,83 @@ class B200RopeArgs(ctypes.Structure):
     )
 
 
+class B200EncoderBlock(ctypes.Structure):
+    """Mirror of `struct B200EncoderBlock` (include/b200_encoder.h)."""
+
+    _fields_ = (
+        ("norm1_w", ctypes.c_void_p),
+        ("norm1_b", ctypes.c_void_p),
+        ("qkv_w", ctypes.c_void_p),
+        ("qkv_b", ctypes.c_void_p),
+        ("proj_w", ctypes.c_void_p),
+        ("proj_b", ctypes.c_void_p),
+        ("gamma1", ctypes.c_void_p),
+        ("norm2_w", ctypes.c_void_p),
+        ("norm2_b", ctypes.c_void_p),
+        ("fc1_w", ctypes.c_void_p),
+        ("fc1_b", ctypes.c_void_p),
+        ("fc2_w", ctypes.c_void_p),
+        ("fc2_b", ctypes.c_void_p),
+        ("gamma2", ctypes.c_void_p),
+        ("rel_pos_h", ctypes.c_void_p),
+        ("rel_pos_w", ctypes.c_void_p),
+        ("window", ctypes.c_int32),
+        ("reserved", ctypes.c_int32),
+    )
+
+
+class B200EncoderTap(ctypes.Structure):
+    """Mirror of `struct B200EncoderTap` (include/b200_encoder.h)."""
+
+    _fields_ = (("after", ctypes.c_int32), ("reserved", ctypes.c_int32), ("out", ctypes.c_void_p))
+
+
+class B200EncoderArgs(ctypes.Structure):
+    """Mirror of `struct B200EncoderArgs` (include/b200_encoder.h)."""
+
+    _fields_ = (
+        ("struct_size", ctypes.c_uint32),
+        ("dtype", ctypes.c_uint32),
+        ("batch", ctypes.c_int32),
+        ("grid_h", ctypes.c_int32),
+        ("grid_w", ctypes.c_int32),
+        ("prefix", ctypes.c_int32),
+        ("dim", ctypes.c_int32),
+        ("heads", ctypes.c_int32),
+        ("hidden", ctypes.c_int32),
+        ("ffn", ctypes.c_int32),
+        ("eps", ctypes.c_float),
+        ("n_blocks", ctypes.c_int32),
+        ("blocks", ctypes.c_void_p),
+        ("images", ctypes.c_void_p),
+        ("image_dtype", ctypes.c_uint32),
+        ("height", ctypes.c_int32),
+        ("width", ctypes.c_int32),
+        ("patch", ctypes.c_int32),
+        ("patch_w", ctypes.c_void_p),
+        ("patch_k", ctypes.c_int32),
+        ("n_taps", ctypes.c_int32),
+        ("start", ctypes.c_void_p),
+        ("x", ctypes.c_void_p),
+        ("norm_w", ctypes.c_void_p),
+        ("norm_b", ctypes.c_void_p),
+        ("taps", ctypes.c_void_p),
+        ("workspace", ctypes.c_void_p),
+        ("workspace_bytes", ctypes.c_int64),
+        ("attn_workspace", ctypes.c_void_p),
+        ("attn_workspace_bytes", ctypes.c_int64),
+        ("neck_w0", ctypes.c_void_p),
+        ("neck_n0_w", ctypes.c_void_p),
+        ("neck_n0_b", ctypes.c_void_p),
+        ("neck_w1", ctypes.c_void_p),
+        ("neck_n1_w", ctypes.c_void_p),
+        ("neck_n1_b", ctypes.c_void_p),
+        ("neck_out", ctypes.c_void_p),
+        ("neck_channels", ctypes.c_int32),
+        ("neck_eps", ctypes.c_float),
+    )
+
+
 def source_hash() -> str:
     """Digest of the sources the shared object is compiled from (16 hex digits). The build passes it to the compiler,
     which puts it into the library's version string, so a binary can be matched with the sources beside it."""
@@ -226,7 +308,7 @@ def library() -> ctypes.CDLL:
         lib = ctypes.CDLL(str(SHARED_OBJECT))
     except OSError as e:
         raise KernelUnavailableError(LIBRARY, f"cannot load {SHARED_OBJECT.name}: {e}") from e
-    missing = [name for name in EXPORTS if not hasattr(lib, name)]
+    missing = [name for name in (*EXPORTS, *ENCODER_EXPORTS) if not hasattr(lib, name)]
     if missing:
         raise KernelUnavailableError(LIBRARY, f"{SHARED_OBJECT.name} lacks the symbols {missing}")
     lib.b200_attn_fwd.argtypes = (ctypes.POINTER(B200AttnArgs), ctypes.c_void_p)
@@ -239,6 +321,10 @@ def library() -> ctypes.CDLL:
     lib.b200_sam_rel_terms.restype = ctypes.c_int
     lib.b200_rope_qk.argtypes = (ctypes.POINTER(B200RopeArgs), ctypes.c_void_p)
     lib.b200_rope_qk.restype = ctypes.c_int
+    lib.b200_encoder_workspace.argtypes = (ctypes.POINTER(B200EncoderArgs), ctypes.POINTER(ctypes.c_int64))
+    lib.b200_encoder_workspace.restype = ctypes.c_int
+    lib.b200_encoder_forward.argtypes = (ctypes.POINTER(B200EncoderArgs), ctypes.c_void_p)
+    lib.b200_encoder_forward.restype = ctypes.c_int
     lib.b200_attn_query.argtypes = (ctypes.POINTER(B200AttnArgs), ctypes.POINTER(ctypes.c_int32))
     lib.b200_attn_query.restype = ctypes.c_int
     i32p = ctypes.POINTER(ctypes.c_int32)

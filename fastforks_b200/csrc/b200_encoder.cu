@@ -1,0 +1,276 @@
+// Whole-encoder forwards (include/b200_encoder.h): every kernel of a ViT's or SAM's image encoder launched from one
+// native call. A block is eight to ten launches of a few microseconds; issued one by one from Python, with the checks
+// and allocations of each operator in between, one image took 1.6 ms where the kernels take a fifth of that.
+#include "../../include/b200_encoder.h"
+
+#include <algorithm>
+#include <cstring>
+
+#include "../../include/b200_attn.h"
+#include "encoder_kernels.cuh"
+#include "gemm_sm100.cuh"
+#include "host_common.h"
+#include "linear_host.h"
+
+namespace {
+
+using namespace b200;
+
+int64_t align256(int64_t bytes) { return (bytes + 255) & ~int64_t(255); }
+
+// Buffers of one forward, as offsets into the workspace.
+struct Layout {
+  int64_t x, y, qkv, att, hid, rel_h, rel_w, neck, total;
+  int64_t rows, most_rows;  // tokens of all images; rows of the largest partition into padded windows
+};
+
+int windows_of(int grid, int side) { return (grid + side - 1) / side; }
+
+Layout layout_of(const B200EncoderArgs* a) {
+  Layout l{};
+  const int64_t tokens = a->prefix + static_cast<int64_t>(a->grid_h) * a->grid_w;
+  l.rows = a->batch * tokens;
+  l.most_rows = l.rows;
+  int64_t rel = 0;
+  for (int i = 0; i < a->n_blocks; ++i) {
+    const B200EncoderBlock& k = a->blocks[i];
+    int64_t rows = l.rows, side = a->grid_h;
+    if (k.window > 0) {
+      side = k.window;
+      rows = a->batch * static_cast<int64_t>(windows_of(a->grid_h, k.window)) * windows_of(a->grid_w, k.window) * k.window * k.window;
+      l.most_rows = std::max(l.most_rows, rows);
+    }
+    if (k.rel_pos_h != nullptr) rel = std::max(rel, rows * a->heads * side);
+  }
+  int64_t wide = l.rows * a->hidden;
+  if (a->images != nullptr) wide = std::max(wide, l.rows * a->patch_k);
+  if (a->neck_w0 != nullptr) wide = std::max(wide, l.rows * 9 * a->neck_channels);
+  int64_t at = 0;
+  const auto take = [&](int64_t values) {
+    const int64_t here = at;
+    at += align256(values * 2);
+    return here;
+  };
+  l.x = take(a->x == nullptr ? l.rows * a->dim : 0);
+  l.y = take(l.most_rows * a->dim);
+  l.qkv = take(l.most_rows * 3 * a->dim);
+  l.att = take(l.most_rows * a->dim);
+  l.hid = take(wide);
+  l.rel_h = take(rel);
+  l.rel_w = take(rel);
+  l.neck = take(a->neck_w0 != nullptr ? l.rows * a->neck_channels : 0);
+  l.total = at;
+  return l;
+}
+
+template <typename T>
+const void* norm_kernel(int chunks) {
+  switch (chunks) {
+    case 1: return reinterpret_cast<const void*>(layer_norm_kernel<T, 1>);
+    case 2: return reinterpret_cast<const void*>(layer_norm_kernel<T, 2>);
+    case 3: return reinterpret_cast<const void*>(layer_norm_kernel<T, 3>);
+    case 4: return reinterpret_cast<const void*>(layer_norm_kernel<T, 4>);
+    case 5: return reinterpret_cast<const void*>(layer_norm_kernel<T, 5>);
+    case 6: return reinterpret_cast<const void*>(layer_norm_kernel<T, 6>);
+    case 7: return reinterpret_cast<const void*>(layer_norm_kernel<T, 7>);
+    default: return reinterpret_cast<const void*>(layer_norm_kernel<T, 8>);
+  }
+}
+
+int launch_norm(uint32_t dtype, NormParams prm, cudaStream_t stream) {
+  const int chunks = (prm.dim + 255) / 256;
+  const void* kernel = dtype == B200_ATTN_F16 ? norm_kernel<__half>(chunks) : norm_kernel<__nv_bfloat16>(chunks);
+  void* args[] = {&prm};
+  return launch_kernel(kernel, static_cast<unsigned>((prm.rows + kNormWarps - 1) / kNormWarps), 1, kNormWarps * 32, 0, 1, stream, args, "layer norm launch");
+}
+
+int check(const B200EncoderArgs* a) {
+  if (a == nullptr) return fail(B200_ATTN_BAD_CONFIG, "args is NULL");
+  if (a->struct_size != sizeof(B200EncoderArgs))
+    return fail(B200_ATTN_BAD_CONFIG, "struct_size %u does not match this library's B200EncoderArgs (%zu bytes)", a->struct_size, sizeof(B200EncoderArgs));
+  if (a->dtype != B200_ATTN_F16 && a->dtype != B200_ATTN_BF16) return fail(B200_ATTN_BAD_CONFIG, "dtype %u: fp16 (0) or bf16 (1)", a->dtype);
+  if (a->batch < 1 || a->grid_h < 1 || a->grid_w < 1 || a->prefix < 0 || a->n_blocks < 0 || (a->n_blocks > 0 && a->blocks == nullptr))
+    return fail(B200_ATTN_BAD_CONFIG, "batch %d grid %d x %d prefix %d blocks %d", a->batch, a->grid_h, a->grid_w, a->prefix, a->n_blocks);
+  if (a->heads < 1 || a->dim != a->heads * 64 || a->dim > 2048) return fail(B200_ATTN_UNSUPPORTED, "dim %d: heads (%d) * 64, at most 2048", a->dim, a->heads);
+  if (a->hidden < 8 || a->hidden % 8 != 0) return fail(B200_ATTN_UNSUPPORTED, "hidden %d must be a positive multiple of 8", a->hidden);
+  if (a->ffn < B200_FFN_GELU_TANH || a->ffn > B200_FFN_GELU) return fail(B200_ATTN_BAD_CONFIG, "ffn %d unknown", a->ffn);
+  const int64_t rows = a->batch * (a->prefix + static_cast<int64_t>(a->grid_h) * a->grid_w);
+  if (rows > 0x3fffffff / 9) return fail(B200_ATTN_UNSUPPORTED, "too many tokens for one call");
+  if (a->images != nullptr) {
+    if (a->patch < 2 || a->patch % 2 != 0 || a->patch_k < 3 * a->patch * a->patch || a->patch_k % 8 != 0 || a->width % 2 != 0 ||
+        a->height < a->grid_h * a->patch || a->width < a->grid_w * a->patch || (a->image_dtype != B200_ATTN_F32 && a->image_dtype != a->dtype))
+      return fail(B200_ATTN_UNSUPPORTED, "images %d x %d with patches of %d, patch_k %d, image_dtype %u", a->height, a->width, a->patch, a->patch_k, a->image_dtype);
+    if (a->patch_w == nullptr || a->start == nullptr) return fail(B200_ATTN_BAD_CONFIG, "images need patch_w and start");
+  } else if (a->x == nullptr) {
+    return fail(B200_ATTN_BAD_CONFIG, "neither images nor x");
+  }
+  for (int i = 0; i < a->n_blocks; ++i) {
+    const B200EncoderBlock& k = a->blocks[i];
+    if (k.window < 0 || (k.window > 0 && a->prefix != 0)) return fail(B200_ATTN_BAD_CONFIG, "block %d: window %d with %d prefix tokens", i, k.window, a->prefix);
+    if (k.rel_pos_h != nullptr && k.window == 0 && a->grid_h != a->grid_w) return fail(B200_ATTN_UNSUPPORTED, "block %d: relative positions need a square grid", i);
+  }
+  if (a->neck_w0 != nullptr && (a->prefix != 0 || a->neck_channels < 8 || a->neck_channels % 8 != 0 || a->neck_channels > kNeckChunks * 256 || a->neck_out == nullptr))
+    return fail(B200_ATTN_UNSUPPORTED, "neck of %d channels", a->neck_channels);
+  return B200_ATTN_OK;
+}
+
+// The launches of one forward.
+struct Forward {
+  const B200EncoderArgs* a;
+  Layout l;
+  cudaStream_t stream;
+  char* ws;
+  void* x;
+
+  void* at(int64_t offset) const { return ws + offset; }
+
+  // y = act((x w^T + b) * gamma + res). Every product follows a kernel of this forward, so its weights were complete
+  // before that kernel started and are loaded ahead of it.
+  int linear(const void* in, int m, int k, const void* w, const void* b, int n, void* out, int act, const float* gamma = nullptr, const void* res = nullptr) const {
+    const GemmCall c{a->dtype, m, n, k, act, in, k, w, b, gamma, res, n, out, n, true};
+    return launch_gemm(c, stream);
+  }
+
+  int norm(const void* in, const void* w, const void* b, void* out, int rows, float eps, WindowMap map = WindowMap{}, void* x_out = nullptr, const void* delta = nullptr) const {
+    NormParams p{};
+    p.x = in; p.x_out = x_out; p.delta = delta; p.weight = w; p.bias = b; p.y = out;
+    p.rows = rows; p.dim = a->dim; p.eps = eps; p.map = map;
+    return launch_norm(a->dtype, p, stream);
+  }
+
+  int start_tokens() const {
+    TokensParams p{};
+    p.images = a->images;
+    p.image_f32 = a->image_dtype == B200_ATTN_F32;
+    p.batch = a->batch; p.height = a->height; p.width = a->width; p.patch = a->patch;
+    p.grid_h = a->grid_h; p.grid_w = a->grid_w; p.prefix = a->prefix;
+    p.k = 3 * a->patch * a->patch; p.k_padded = a->patch_k;
+    p.patches = at(l.hid); p.start = a->start; p.x = x; p.dim = a->dim;
+    void* args[] = {&p};
+    const void* kernel = a->dtype == B200_ATTN_F16 ? reinterpret_cast<const void*>(encoder_tokens_kernel<__half>) : reinterpret_cast<const void*>(encoder_tokens_kernel<__nv_bfloat16>);
+    if (int rc = launch_kernel(kernel, static_cast<unsigned>(a->batch * a->grid_h), 4, kTokensThreads, 0, 1, stream, args, "encoder tokens launch")) return rc;
+    return linear(at(l.hid), static_cast<int>(l.rows), a->patch_k, a->patch_w, nullptr, a->dim, x, kActNone, nullptr, x);
+  }
+
+  int attention(const B200EncoderBlock& k, int batch, int tokens, int side) const {
+    const int dim = a->dim;
+    B200AttnArgs t;
+    std::memset(&t, 0, sizeof(t));
+    t.struct_size = sizeof(t);
+    t.dtype = a->dtype;
+    char* qkv = static_cast<char*>(at(l.qkv));
+    t.q = qkv; t.k = qkv + 2 * dim; t.v = qkv + 4 * dim;
+    t.o = at(l.att);
+    for (int64_t* s : {t.q_stride, t.k_stride, t.v_stride}) {
+      s[0] = static_cast<int64_t>(tokens) * 3 * dim;
+      s[1] = 3 * dim;
+      s[2] = 64;
+    }
+    t.o_stride[0] = static_cast<int64_t>(tokens) * dim;
+    t.o_stride[1] = dim;
+    t.o_stride[2] = 64;
+    t.batch = batch; t.heads = a->heads; t.q_tokens = tokens; t.kv_tokens = tokens; t.head_dim = 64;
+    t.scale = 0.125f;
+    t.workspace = a->attn_workspace;
+    t.workspace_bytes = a->attn_workspace_bytes;
+    if (k.rel_pos_h != nullptr) {
+      B200RelTermsArgs r;
+      std::memset(&r, 0, sizeof(r));
+      r.struct_size = sizeof(r);
+      r.dtype = a->dtype;
+      r.q = t.q;
+      std::memcpy(r.q_stride, t.q_stride, sizeof(r.q_stride));
+      r.rel_pos_h = k.rel_pos_h; r.rel_pos_w = k.rel_pos_w;
+      r.rel_h = at(l.rel_h); r.rel_w = at(l.rel_w);
+      r.batch = batch; r.heads = a->heads; r.side = side; r.head_dim = 64;
+      if (int rc = b200_sam_rel_terms(&r, stream)) return rc;
+      t.rel_h = r.rel_h; t.rel_w = r.rel_w;
+      t.rel_dtype = a->dtype;
+      t.rel_kh = t.rel_kw = side;
+      for (int64_t* s : {t.rel_h_stride, t.rel_w_stride}) {
+        s[0] = static_cast<int64_t>(a->heads) * tokens * side;
+        s[1] = static_cast<int64_t>(tokens) * side;
+        s[2] = side;
+      }
+    }
+    return b200_attn_fwd(&t, stream);
+  }
+
+  int block(const B200EncoderBlock& k) const {
+    const int rows = static_cast<int>(l.rows), dim = a->dim;
+    const int tokens = a->prefix + a->grid_h * a->grid_w;
+    if (k.window > 0) {
+      // Windowed attention (SAM): the first norm writes the padded windows, the projection stays in window order, and the
+      // second norm takes it back to token order while it adds it to the residual stream.
+      const WindowMap map{k.window, a->grid_h, a->grid_w, windows_of(a->grid_w, k.window), windows_of(a->grid_h, k.window)};
+      const int windows = a->batch * map.per_row * map.per_col, area = k.window * k.window, wrows = windows * area;
+      if (int rc = norm(x, k.norm1_w, k.norm1_b, at(l.y), wrows, a->eps, map)) return rc;
+      if (int rc = linear(at(l.y), wrows, dim, k.qkv_w, k.qkv_b, 3 * dim, at(l.qkv), kActNone)) return rc;
+      if (int rc = attention(k, windows, area, k.window)) return rc;
+      if (int rc = linear(at(l.att), wrows, dim, k.proj_w, k.proj_b, dim, at(l.y), kActNone, k.gamma1)) return rc;
+      if (int rc = norm(x, k.norm2_w, k.norm2_b, at(l.att), rows, a->eps, map, x, at(l.y))) return rc;
+    } else {
+      if (int rc = norm(x, k.norm1_w, k.norm1_b, at(l.y), rows, a->eps)) return rc;
+      if (int rc = linear(at(l.y), rows, dim, k.qkv_w, k.qkv_b, 3 * dim, at(l.qkv), kActNone)) return rc;
+      if (int rc = attention(k, a->batch, tokens, a->grid_h)) return rc;
+      if (int rc = linear(at(l.att), rows, dim, k.proj_w, k.proj_b, dim, x, kActNone, k.gamma1, x)) return rc;
+      if (int rc = norm(x, k.norm2_w, k.norm2_b, at(l.att), rows, a->eps)) return rc;
+    }
+    const int act = a->ffn == B200_FFN_SWIGLU ? kActSwiGlu : a->ffn == B200_FFN_GELU ? kActGelu : kActGeluTanh;
+    if (int rc = linear(at(l.att), rows, dim, k.fc1_w, k.fc1_b, a->hidden, at(l.hid), act)) return rc;
+    return linear(at(l.hid), rows, a->hidden, k.fc2_w, k.fc2_b, dim, x, kActNone, k.gamma2, x);
+  }
+
+  int neck() const {
+    const int rows = static_cast<int>(l.rows), ch = a->neck_channels;
+    if (int rc = linear(x, rows, a->dim, a->neck_w0, nullptr, ch, at(l.neck), kActNone)) return rc;
+    NeckParams p{};
+    p.x = at(l.neck); p.weight = a->neck_n0_w; p.bias = a->neck_n0_b; p.out = at(l.hid);
+    p.batch = a->batch; p.grid_h = a->grid_h; p.grid_w = a->grid_w; p.channels = ch; p.eps = a->neck_eps;
+    void* args[] = {&p};
+    const bool f16 = a->dtype == B200_ATTN_F16;
+    const void* im2col = f16 ? reinterpret_cast<const void*>(neck_norm_im2col_kernel<__half>) : reinterpret_cast<const void*>(neck_norm_im2col_kernel<__nv_bfloat16>);
+    if (int rc = launch_kernel(im2col, static_cast<unsigned>((rows + kNeckWarps - 1) / kNeckWarps), 1, kNeckWarps * 32, 0, 1, stream, args, "neck norm launch")) return rc;
+    if (int rc = linear(at(l.hid), rows, 9 * ch, a->neck_w1, nullptr, ch, at(l.neck), kActNone)) return rc;
+    p.weight = a->neck_n1_w; p.bias = a->neck_n1_b; p.out = a->neck_out;
+    const void* chw = f16 ? reinterpret_cast<const void*>(neck_norm_chw_kernel<__half>) : reinterpret_cast<const void*>(neck_norm_chw_kernel<__nv_bfloat16>);
+    const int area = a->grid_h * a->grid_w;
+    const unsigned grid = static_cast<unsigned>(a->batch * ((area + kNeckTokens - 1) / kNeckTokens));
+    return launch_kernel(chw, grid, 1, kNeckWarps * 32, static_cast<size_t>(ch) * (kNeckTokens + 2) * 2, 1, stream, args, "neck norm launch");
+  }
+};
+
+}  // namespace
+
+extern "C" {
+
+int b200_encoder_workspace(const B200EncoderArgs* a, int64_t* bytes) {
+  if (int rc = check(a)) return rc;
+  if (bytes == nullptr) return fail(B200_ATTN_BAD_CONFIG, "bytes is NULL");
+  *bytes = layout_of(a).total;
+  return B200_ATTN_OK;
+}
+
+int b200_encoder_forward(const B200EncoderArgs* a, void* stream_ptr) {
+  if (int rc = check(a)) return rc;
+  Forward f{a, layout_of(a), static_cast<cudaStream_t>(stream_ptr), static_cast<char*>(a->workspace), nullptr};
+  if (a->workspace == nullptr || (reinterpret_cast<uintptr_t>(a->workspace) & 255) != 0 || a->workspace_bytes < f.l.total)
+    return fail(B200_ATTN_BAD_CONFIG, "workspace of %lld bytes: %lld, 256-byte aligned, are needed", static_cast<long long>(a->workspace_bytes), static_cast<long long>(f.l.total));
+  f.x = a->x != nullptr ? a->x : f.at(f.l.x);
+  if (a->images != nullptr)
+    if (int rc = f.start_tokens()) return rc;
+  int tap = 0;
+  for (int i = -1; i < a->n_blocks; ++i) {
+    if (i >= 0)
+      if (int rc = f.block(a->blocks[i])) return rc;
+    for (; tap < a->n_taps && a->taps[tap].after == i; ++tap)
+      if (int rc = f.norm(f.x, a->norm_w, a->norm_b, a->taps[tap].out, static_cast<int>(f.l.rows), a->eps)) return rc;
+  }
+  if (tap != a->n_taps) return fail(B200_ATTN_BAD_CONFIG, "tap %d of %d names no block, or the taps are out of order", tap, a->n_taps);
+  if (a->neck_w0 != nullptr)
+    if (int rc = f.neck()) return rc;
+  clear_error();
+  return B200_ATTN_OK;
+}
+
+}  // extern "C"

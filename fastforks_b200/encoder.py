@@ -1,0 +1,98 @@
+"""Host side of the whole-encoder calls (include/b200_encoder.h): one native call per forward.
+
+`NativeEncoder` keeps what a model's forwards share - the table of the blocks' parameter pointers and, per input
+geometry, a filled-in argument description - and launches a forward with two allocations (outputs and one workspace)
+from torch's caching allocator. Nothing here computes.
+"""
+
+from __future__ import annotations
+
+import ctypes
+from typing import TYPE_CHECKING
+
+import torch
+
+from . import _lib
+from .attention import reserve_workspace
+
+if TYPE_CHECKING:
+    from collections.abc import Sequence
+
+FFN_GELU_TANH, FFN_SWIGLU, FFN_GELU = 0, 1, 2
+MAX_DIM = 2048  # a row of the layer norms lives in one warp's registers
+_DTYPES = {torch.float16: _lib.F16, torch.bfloat16: _lib.BF16}
+BLOCK_TENSORS = tuple(name for name, kind in _lib.B200EncoderBlock._fields_ if kind is ctypes.c_void_p)  # noqa: SLF001
+_SPLIT_MIN_KEYS = 257  # shorter sequences never use the attention workspace
+
+
+def supported(dtype: torch.dtype, dim: int, heads: int, hidden: int) -> bool:
+    """Whether the native forward takes an encoder of this shape."""
+    return dtype in _DTYPES and dim == heads * 64 and dim <= MAX_DIM and hidden % 8 == 0
+
+
+class NativeEncoder:
+    """Blocks of one encoder on one device. `blocks[i]` maps the pointer names of `B200EncoderBlock` to tensors (missing
+    names are NULL) and `window` to the window side; the tensors are kept alive here and read in place."""
+
+    def __init__(self, blocks: Sequence[dict], *, dtype: torch.dtype, dim: int, heads: int, hidden: int, ffn: int, eps: float) -> None:  # noqa: PLR0913
+        self.dtype, self.dim, self.heads, self.hidden, self.ffn, self.eps = dtype, dim, heads, hidden, ffn, eps
+        self._keep = [dict(b) for b in blocks]
+        self.blocks = (_lib.B200EncoderBlock * max(1, len(blocks)))()
+        for entry, tensors in zip(self.blocks, blocks):
+            for name in BLOCK_TENSORS:
+                t = tensors.get(name)
+                if t is not None:
+                    if not t.is_contiguous() or t.data_ptr() % 16:
+                        msg = f"encoder: parameter {name} must be contiguous and 16-byte aligned"
+                        raise ValueError(msg)
+                    setattr(entry, name, t.data_ptr())
+            entry.window = tensors.get("window", 0)
+        self._described: dict[tuple, tuple] = {}  # geometry -> (argument description, workspace bytes)
+
+    def describe(self, batch: int, grid: tuple[int, int], prefix: int, first: int, count: int, extra: dict) -> tuple:
+        """The argument description of a geometry and its workspace size; `extra`: further scalar and pointer fields."""
+        key = (batch, grid, prefix, first, count, tuple(sorted(extra.items())))
+        found = self._described.get(key)
+        if found is None:
+            a = _lib.B200EncoderArgs()
+            a.struct_size = ctypes.sizeof(_lib.B200EncoderArgs)
+            a.dtype, a.batch, a.prefix, a.eps = _DTYPES[self.dtype], batch, prefix, self.eps
+            a.grid_h, a.grid_w = grid
+            a.dim, a.heads, a.hidden, a.ffn = self.dim, self.heads, self.hidden, self.ffn
+            a.n_blocks = count
+            a.blocks = ctypes.addressof(self.blocks) + first * ctypes.sizeof(_lib.B200EncoderBlock)
+            for name, value in extra.items():
+                setattr(a, name, value)
+            size = ctypes.c_int64(0)
+            _lib.raise_for_code(_lib.library().b200_encoder_workspace(ctypes.byref(a), ctypes.byref(size)), "encoder")
+            if len(self._described) >= 64:  # noqa: PLR2004
+                self._described.clear()
+            found = self._described[key] = (a, size.value)
+        return found
+
+    def launch(self, described: tuple, device: torch.device, *, x: torch.Tensor | None = None, images: torch.Tensor | None = None,
+               taps: Sequence[tuple[int, torch.Tensor]] = (), neck_out: torch.Tensor | None = None) -> None:  # fmt: skip
+        """Launch a described forward on the current stream of `device`."""
+        template, size = described
+        a = _lib.B200EncoderArgs.from_buffer_copy(template)
+        index = device.index if device.index is not None else torch.cuda.current_device()
+        if index != torch.cuda.current_device():
+            with torch.cuda.device(index):
+                self.launch(described, torch.device("cuda", index), x=x, images=images, taps=taps, neck_out=neck_out)
+            return
+        workspace = torch.empty(max(size, 1), dtype=torch.uint8, device=device)
+        a.workspace, a.workspace_bytes = workspace.data_ptr(), size
+        a.x = None if x is None else x.data_ptr()
+        a.images = None if images is None else images.data_ptr()
+        a.neck_out = None if neck_out is None else neck_out.data_ptr()
+        if taps:
+            table = (_lib.B200EncoderTap * len(taps))()
+            for entry, (after, out) in zip(table, taps):
+                entry.after, entry.out = after, out.data_ptr()
+            a.taps, a.n_taps = ctypes.addressof(table), len(taps)
+        if a.prefix + a.grid_h * a.grid_w >= _SPLIT_MIN_KEYS:
+            scratch = reserve_workspace(index)
+            if scratch is not None:
+                a.attn_workspace, a.attn_workspace_bytes = scratch.data_ptr(), scratch.numel()
+        code = _lib.library().b200_encoder_forward(ctypes.byref(a), torch._C._cuda_getCurrentRawStream(index))  # noqa: SLF001
+        _lib.raise_for_code(code, "encoder")

@@ -20,6 +20,7 @@ from dataclasses import dataclass
 import torch
 import torch.nn.functional as F  # noqa: N812
 
+from . import _lib, encoder
 from .flash64 import Flash64
 from .gemm import ACT_GELU_TANH, ACT_NONE, gemm
 
@@ -140,26 +141,88 @@ class ViTEncoder:
         # this library never uses) a GEMM of its own is bound by the L2 at about 0.8 of the library's rate.
         self.fuse_plain = fuse_plain
         self.scales = {k: v.to(self.device, torch.float32) for k, v in state.items() if k.endswith(".gamma")}
+        # ... and the whole forward is one native call (`encoder`), made from the parameters in `self.w` and `self.scales`.
+        self._native: encoder.NativeEncoder | None = None
+        if self.fused and self.device.type == "cuda" and encoder.supported(dtype, cfg.dim, cfg.heads, cfg.hidden):
+            self._native = self._make_native()
+            self._start: dict[tuple[int, int], torch.Tensor] = {}
+            self._patch_w = self._patch_matrix()
+
+    def _make_native(self) -> encoder.NativeEncoder:
+        w, cfg, blocks = self.w, self.cfg, []
+        fc1, fc2 = ("mlp.w12", "mlp.w3") if cfg.ffn == "swiglu" else ("mlp.fc1", "mlp.fc2")
+        for i in range(cfg.depth):
+            p = f"blocks.{i}."
+            layers = {"norm1": "norm1", "qkv": "attn.qkv", "proj": "attn.proj", "norm2": "norm2", "fc1": fc1, "fc2": fc2}
+            tensors = {f"{short}_{kind[0]}": w[f"{p}{name}.{kind}"] for short, name in layers.items() for kind in ("weight", "bias")}
+            if cfg.layerscale:
+                tensors |= {"gamma1": self.scales[p + "ls1.gamma"], "gamma2": self.scales[p + "ls2.gamma"]}
+            blocks.append(tensors)
+        ffn = encoder.FFN_SWIGLU if cfg.ffn == "swiglu" else encoder.FFN_GELU_TANH
+        return encoder.NativeEncoder(blocks, dtype=self.dtype, dim=cfg.dim, heads=cfg.heads, hidden=cfg.hidden, ffn=ffn, eps=cfg.eps)
+
+    def _patch_matrix(self) -> torch.Tensor:
+        """The patch embedding's kernel as rows of a linear layer, padded with zeros to a multiple of eight inputs."""
+        rows = self.w["patch_embed.proj.weight"].flatten(1)
+        return F.pad(rows, (0, -rows.shape[1] % 8)).contiguous()
+
+    def start_tokens(self, gh: int, gw: int) -> torch.Tensor:
+        """What a `gh x gw` image's patch products are added to, per token: position embedding plus the patch bias, and
+        plus the class token in the first row."""
+        key = (gh, gw)
+        if key not in self._start:
+            pos = self.pos_embed_fp32(gh, gw)[0]
+            cls = self.w["cls_token"].reshape(1, -1).float()
+            bias = self.w["patch_embed.proj.bias"].float()
+            self._start[key] = torch.cat([pos[:1] + cls, pos[1:] + bias]).to(self.dtype).contiguous()
+        return self._start[key]
+
+    def _forward_native(self, images: torch.Tensor, count: int, taps: tuple[int, ...]) -> list[torch.Tensor] | None:
+        """Normalised tokens after the blocks in `taps`, of the first `count` blocks, as one native call; None when the images
+        are not of a form it takes."""
+        ps = self.cfg.patch
+        if self._native is None or images.dim() != 4 or images.shape[1] != 3 or images.device.type != "cuda" or images.numel() == 0:  # noqa: PLR2004
+            return None
+        if images.dtype not in (torch.float32, self.dtype):
+            images = images.to(self.dtype)
+        images = images.contiguous()
+        b, _, height, width = images.shape
+        gh, gw = height // ps, width // ps
+        if width % 2 or gh == 0 or gw == 0 or images.data_ptr() % 16:
+            return None
+        start = self.start_tokens(gh, gw)
+        extra = {  # "images": any address, the description only needs to know that there are images
+            "images": 1, "image_dtype": _lib.F32 if images.dtype == torch.float32 else encoder._DTYPES[self.dtype],  # noqa: SLF001
+            "height": height, "width": width, "patch": ps, "patch_w": self._patch_w.data_ptr(), "patch_k": self._patch_w.shape[1],
+            "start": start.data_ptr(), "norm_w": self.w["norm.weight"].data_ptr(), "norm_b": self.w["norm.bias"].data_ptr(),
+        }  # fmt: skip
+        described = self._native.describe(b, (gh, gw), 1, 0, count, extra)
+        outs = [torch.empty((b, 1 + gh * gw, self.cfg.dim), dtype=self.dtype, device=images.device) for _ in taps]
+        self._native.launch(described, images.device, images=images, taps=list(zip(taps, outs)))
+        return outs
 
     def pos_embed(self, gh: int, gw: int) -> torch.Tensor:
         """Position table for a `gh x gw` patch grid (upstream `interpolate_pos_encoding`, net/dinov2.py:198-237)."""
         key = (gh, gw)
         if key not in self._pos:
-            table = self.pos_table
-            n = table.shape[1] - 1
-            side = int(math.sqrt(n))
-            if gh * gw == n and gh == gw:
-                pos = table
-            else:
-                off = self.cfg.interpolate_offset
-                grid = table[:, 1:].reshape(1, side, side, -1).permute(0, 3, 1, 2)
-                grid = F.interpolate(grid, scale_factor=((gh + off) / side, (gw + off) / side), mode="bicubic")
-                if grid.shape[-2:] != (gh, gw):
-                    msg = f"position grid {tuple(grid.shape[-2:])} != {(gh, gw)}"
-                    raise RuntimeError(msg)
-                pos = torch.cat([table[:, :1], grid.permute(0, 2, 3, 1).reshape(1, gh * gw, -1)], 1)
-            self._pos[key] = pos.to(self.dtype)
+            self._pos[key] = self.pos_embed_fp32(gh, gw).to(self.dtype)
         return self._pos[key]
+
+    def pos_embed_fp32(self, gh: int, gw: int) -> torch.Tensor:
+        table = self.pos_table
+        n = table.shape[1] - 1
+        side = int(math.sqrt(n))
+        if gh * gw == n and gh == gw:
+            pos = table
+        else:
+            off = self.cfg.interpolate_offset
+            grid = table[:, 1:].reshape(1, side, side, -1).permute(0, 3, 1, 2)
+            grid = F.interpolate(grid, scale_factor=((gh + off) / side, (gw + off) / side), mode="bicubic")
+            if grid.shape[-2:] != (gh, gw):
+                msg = f"position grid {tuple(grid.shape[-2:])} != {(gh, gw)}"
+                raise RuntimeError(msg)
+            pos = torch.cat([table[:, :1], grid.permute(0, 2, 3, 1).reshape(1, gh * gw, -1)], 1)
+        return pos
 
     def tokens(self, images: torch.Tensor) -> torch.Tensor:
         """Patch embedding, class token and position embedding (`prepare_tokens_with_masks`, net/dinov2.py:239-258)."""
@@ -196,6 +259,10 @@ class ViTEncoder:
         src/fastforks/shared/timm_blocks/net/vit.py:60-62). q, k, v are strided views of the packed qkv tensor."""
         w, cfg, p = self.w, self.cfg, f"blocks.{i}."
         b, n, c = x.shape
+        native = self._native is not None and not (x.requires_grad and torch.is_grad_enabled())
+        if native and x.is_cuda and x.dtype == self.dtype and x.is_contiguous() and x.numel() > 0 and x.data_ptr() % 16 == 0:
+            self._native.launch(self._native.describe(b, (n, 1), 0, i, 1, {"x": 1}), x.device, x=x)
+            return x
         heads = cfg.heads
         ls1, ls2 = (p + "ls1.gamma", p + "ls2.gamma") if cfg.layerscale else (None, None)
         qkv = self.linear(F.layer_norm(x, (c,), w[p + "norm1.weight"], w[p + "norm1.bias"], cfg.eps), p + "attn.qkv")
@@ -211,7 +278,11 @@ class ViTEncoder:
 
     @torch.no_grad()
     def __call__(self, images: torch.Tensor) -> torch.Tensor:
-        x = self.tokens(images.to(self.device))
+        images = images.to(self.device)
+        native = self._forward_native(images, self.cfg.depth, (self.cfg.depth - 1,))
+        if native is not None:
+            return native[0]
+        x = self.tokens(images)
         for i in range(self.cfg.depth):
             x = self.block(i, x)
         c = x.shape[-1]
@@ -239,7 +310,11 @@ class ViTEncoder:
         """Normalised tokens after the blocks in `layers`: what the depth models hand to their DPT head
         (upstream `get_intermediate_layers(..., norm=True)`, net/dinov2.py:300-336; Depth-Anything-V2-L takes blocks
         4, 11, 17, 23)."""
-        x = self.tokens(images.to(self.device))
+        images = images.to(self.device)
+        native = self._forward_native(images, max(layers) + 1, tuple(i for i in range(max(layers) + 1) if i in layers))
+        if native is not None:
+            return native
+        x = self.tokens(images)
         c = x.shape[-1]
         outs = []
         for i in range(max(layers) + 1):
