@@ -248,6 +248,25 @@ int launch_gemm(const GemmCall& c, cudaStream_t stream) {
   return launch_kernel(kernel, static_cast<unsigned>(prm.tiles_m * prm.tiles_n * s), 1, kSplitThreads, smem, static_cast<unsigned>(s), stream, args, "gemm kernel launch");
 }
 
+namespace {
+
+template <typename T>
+const void* rel_kernel_of(int tiles) {
+  switch (tiles) {
+    case 1: return reinterpret_cast<const void*>(sam_rel_terms_kernel<T, 1>);
+    case 2: return reinterpret_cast<const void*>(sam_rel_terms_kernel<T, 2>);
+    case 3: return reinterpret_cast<const void*>(sam_rel_terms_kernel<T, 3>);
+    case 4: return reinterpret_cast<const void*>(sam_rel_terms_kernel<T, 4>);
+    case 5: return reinterpret_cast<const void*>(sam_rel_terms_kernel<T, 5>);
+    case 6: return reinterpret_cast<const void*>(sam_rel_terms_kernel<T, 6>);
+    case 7: return reinterpret_cast<const void*>(sam_rel_terms_kernel<T, 7>);
+    default: return reinterpret_cast<const void*>(sam_rel_terms_kernel<T, 8>);
+  }
+}
+const void* rel_kernel(bool f16, int tiles) { return f16 ? rel_kernel_of<__half>(tiles) : rel_kernel_of<__nv_bfloat16>(tiles); }
+
+}  // namespace
+
 }  // namespace b200
 
 using namespace b200;
@@ -313,13 +332,20 @@ int b200_sam_rel_terms(const B200RelTermsArgs* a, void* stream_ptr) {
   prm.batch = a->batch;
   prm.heads = a->heads;
   prm.side = a->side;
-  const int rows = a->side * a->heads;
-  const dim3 grid(static_cast<unsigned>(a->batch * a->side), 2, static_cast<unsigned>(std::min(8, (rows + kRelThreads - 1) / kRelThreads)));
-  cudaStream_t stream = static_cast<cudaStream_t>(stream_ptr);
-  if (a->dtype == B200_ATTN_F16) sam_rel_terms_kernel<__half><<<grid, kRelThreads, 0, stream>>>(prm);
-  else sam_rel_terms_kernel<__nv_bfloat16><<<grid, kRelThreads, 0, stream>>>(prm);
-  const cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return cuda_fail(e, "sam_rel_terms kernel launch");
+  DeviceState* dev = nullptr;
+  if (int rc = device_state(&dev)) return rc;
+  prm.tables_wide = aligned16(a->rel_pos_h) && aligned16(a->rel_pos_w);
+  prm.out_wide = aligned16(a->rel_h) && aligned16(a->rel_w);
+  // One CTA per grid row, and several where there are few rows: about four CTAs per SM, a token per warp at least.
+  const long long grid_rows = static_cast<long long>(a->batch) * a->side;
+  prm.parts = static_cast<int>(std::max(1LL, std::min<long long>((4LL * dev->sms + grid_rows - 1) / grid_rows, (a->side + kRelWarps - 1) / kRelWarps)));
+  if (grid_rows * prm.parts > 0x7fffffffLL) return fail(B200_ATTN_UNSUPPORTED, "batch too large for one launch");
+  const void* kernel = rel_kernel(a->dtype == B200_ATTN_F16, (a->side + 7) / 8);
+  void* args[] = {&prm};
+  const size_t smem = static_cast<size_t>(3 * a->side - 1) * 128;
+  if (int rc = launch_kernel(kernel, static_cast<unsigned>(grid_rows * prm.parts), 1, kRelWarps * 32, smem, 1, static_cast<cudaStream_t>(stream_ptr), args,
+                             "sam_rel_terms kernel launch"))
+    return rc;
   clear_error();
   return B200_ATTN_OK;
 }

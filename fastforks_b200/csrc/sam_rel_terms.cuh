@@ -3,16 +3,22 @@
 //   rel_w[b, head, (y, x), k] = q[b, (y, x), head, :] . rel_pos_w[x - k + side - 1, :]      (k = 0 .. side - 1)
 // q is the UNSCALED query of head dim 64, read in place from the packed qkv tensor; the tables are the module's
 // parameters themselves ([2 * side - 1, 64]): the [side, side, 64] gather the upstream code builds first
-// (get_rel_pos) never exists. HBM-bound work on the FMA pipe: q is read once, the results are written once.
+// (get_rel_pos) never exists.
 //
-// One CTA takes the queries that share one coordinate (which = 0: a grid row y, for rel_h; which = 1: a grid column
-// x, for rel_w), because they share the `side` table rows: those are staged in shared memory as fp32, one thread
-// then owns a query row (64 values in registers) and walks the table rows with broadcast 16-byte loads.
+// One query token is a 16 x 64 operand (its heads) against `side` rows of either table: two small products on the same
+// left operand, so q is read once. A warp takes a token, the CTA's tables lie in shared memory. mma.sync fits: the
+// operands are 16 rows high and change their table rows from token to token, and the work is bound by the bytes of the
+// result (12.6 MB for SAM's global grid), not by the products. On the FMA pipe, a thread per query and table row, the
+// global grid took 44 us and 25 windows of 14 x 14 19 us.
 #pragma once
 
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <stdint.h>
+
+#include <type_traits>
+
+#include "sm100_ptx.cuh"
 
 namespace b200 {
 
@@ -24,100 +30,123 @@ struct RelTermsParams {
   void* rel_h;               // [batch, heads, side * side, side], contiguous
   void* rel_w;
   int batch, heads, side;
+  int parts;                 // CTAs per grid row
+  int tables_wide, out_wide; // both tables / results are 16-byte aligned (else 4-byte)
 };
 
-constexpr int kRelThreads = 256;
-constexpr int kRelMaxSide = 64;  // shared memory: side rows of 64 floats
+constexpr int kRelWarps = 4;
+constexpr int kRelMaxSide = 64;
 
 template <typename T>
-__device__ __forceinline__ float2 rel_unpack2(uint32_t v);
-template <>
-__device__ __forceinline__ float2 rel_unpack2<__half>(uint32_t v) {
-  return __half22float2(*reinterpret_cast<const __half2*>(&v));
-}
-template <>
-__device__ __forceinline__ float2 rel_unpack2<__nv_bfloat16>(uint32_t v) {
-  return make_float2(__uint_as_float(v << 16), __uint_as_float(v & 0xffff0000u));
-}
-template <typename T>
-__device__ __forceinline__ uint32_t rel_pack2(float lo, float hi);
-template <>
-__device__ __forceinline__ uint32_t rel_pack2<__half>(float lo, float hi) {
-  __half2 h = __floats2half2_rn(lo, hi);
-  return *reinterpret_cast<uint32_t*>(&h);
-}
-template <>
-__device__ __forceinline__ uint32_t rel_pack2<__nv_bfloat16>(float lo, float hi) {
-  __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
-  return *reinterpret_cast<uint32_t*>(&h);
+__device__ __forceinline__ void mma_16816(float* c, const uint32_t* a, uint32_t b0, uint32_t b1) {
+  if constexpr (std::is_same<T, __half>::value)
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+  else
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
 template <typename T>
-__global__ void __launch_bounds__(kRelThreads) sam_rel_terms_kernel(const RelTermsParams p) {
-  __shared__ __align__(16) float table[kRelMaxSide][64];  // table[k] = rel_pos[c - k + side - 1]
-  const int side = p.side, n_tokens = side * side;
-  const int which = blockIdx.y;               // 0: rel_h (fixed y), 1: rel_w (fixed x)
-  const int b = blockIdx.x / side, c = blockIdx.x - b * side;
-  const T* rel_pos = static_cast<const T*>(which == 0 ? p.rel_pos_h : p.rel_pos_w);
-  for (int i = threadIdx.x; i < side * 32; i += kRelThreads) {
-    const int k = i >> 5, pair = i & 31;
-    const float2 v = rel_unpack2<T>(reinterpret_cast<const uint32_t*>(rel_pos + static_cast<int64_t>(c - k + side - 1) * 64)[pair]);
-    table[k][2 * pair] = v.x;
-    table[k][2 * pair + 1] = v.y;
+__device__ __forceinline__ uint32_t rel_pack2(float lo, float hi) {
+  if constexpr (std::is_same<T, __half>::value) {
+    __half2 h = __floats2half2_rn(lo, hi);
+    return *reinterpret_cast<uint32_t*>(&h);
+  } else {
+    __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
+    return *reinterpret_cast<uint32_t*>(&h);
+  }
+}
+
+// NT: 8-column tiles of a result row, ceil(side / 8). The order of the 64 products of a sum and of the columns in a tile
+// is free, so both are chosen for wide accesses: a lane's k values are 16-byte chunks of q's and the tables' rows (chunk
+// t and t + 4 of eight), and its columns are the 2 NT consecutive ones from 2 NT t on (t = lane % 4).
+template <typename T, int NT>
+__global__ void __launch_bounds__(kRelWarps * 32) sam_rel_terms_kernel(const RelTermsParams p) {
+  // Table rows as eight 16-byte chunks; odd rows have their halves swapped, so that two neighbouring rows, which a quarter
+  // of a warp reads together, use all banks.
+  extern __shared__ uint4 rel_tables[];
+  const int side = p.side, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int g = lane >> 2, t = lane & 3;
+  const int row_id = blockIdx.x / p.parts, part = blockIdx.x - row_id * p.parts;
+  const int b = row_id / side, y = row_id - b * side;
+  uint4* const table_h = rel_tables;              // row k: rel_pos_h[y - k + side - 1]
+  uint4* const table_w = rel_tables + side * 8;   // rel_pos_w as it is
+  grid_dependency_wait();
+  grid_launch_dependents();
+  const auto load = [&](const void* table, int row, int c) {
+    const uint32_t* src = static_cast<const uint32_t*>(table) + row * 32 + c * 4;
+    return p.tables_wide ? __ldg(reinterpret_cast<const uint4*>(src)) : make_uint4(__ldg(src), __ldg(src + 1), __ldg(src + 2), __ldg(src + 3));
+  };
+  for (int i = threadIdx.x; i < side * 8; i += kRelWarps * 32) {
+    const int k = i >> 3, c = i & 7;
+    table_h[k * 8 + (c ^ ((k & 1) << 2))] = load(p.rel_pos_h, y - k + side - 1, c);
+  }
+  for (int i = threadIdx.x; i < (2 * side - 1) * 8; i += kRelWarps * 32) {
+    const int k = i >> 3, c = i & 7;
+    table_w[k * 8 + (c ^ ((k & 1) << 2))] = load(p.rel_pos_w, k, c);
   }
   __syncthreads();
-  T* out = static_cast<T*>(which == 0 ? p.rel_h : p.rel_w);
-  const int rows = side * p.heads;  // the queries of this CTA: `side` tokens x heads
-  // blockIdx.z splits the rows: every thread has at most one, so that a 64 x 64 grid (768 rows per coordinate) makes
-  // three CTAs per coordinate instead of one CTA that walks three rows per thread on an otherwise idle GPU.
-  for (int r = blockIdx.z * kRelThreads + threadIdx.x; r < rows; r += gridDim.z * kRelThreads) {
-    const int j = r / p.heads, head = r - j * p.heads;
-    const int n = which == 0 ? c * side + j : j * side + c;
-    const uint4* src = reinterpret_cast<const uint4*>(static_cast<const T*>(p.q) + b * p.q_sb + n * p.q_sn + head * p.q_sh);
-    float q[64];
+  const int x_end = side * (part + 1) / p.parts;
+  const int n_tokens = side * side;
+  for (int x = side * part / p.parts + warp; x < x_end; x += kRelWarps) {
+    const int n = y * side + x;
+    const T* q_token = static_cast<const T*>(p.q) + b * p.q_sb + n * p.q_sn;
+    for (int h0 = 0; h0 < p.heads; h0 += 16) {
+      // heads h0 + g and h0 + g + 8, 16-byte chunks t and t + 4 (rows past the last head repeat it; they are not stored)
+      const T* q_lo = q_token + min(h0 + g, p.heads - 1) * p.q_sh;
+      const T* q_hi = q_token + min(h0 + g + 8, p.heads - 1) * p.q_sh;
+      uint4 lo[2], hi[2];
 #pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      const uint4 v = __ldg(src + u);
-      const uint32_t w4[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const float2 f = rel_unpack2<T>(w4[e]);
-        q[u * 8 + e * 2] = f.x;
-        q[u * 8 + e * 2 + 1] = f.y;
+      for (int i = 0; i < 2; ++i) {
+        lo[i] = __ldg(reinterpret_cast<const uint4*>(q_lo) + t + 4 * i);
+        hi[i] = __ldg(reinterpret_cast<const uint4*>(q_hi) + t + 4 * i);
       }
-    }
-    T* dst = out + ((static_cast<int64_t>(b) * p.heads + head) * n_tokens + n) * side;
-    // side is even (checked by the host). Four table rows at a time where they exist: four independent chains of
-    // fused multiply-adds hide the latency of the shared-memory loads behind them; a leftover pair goes alone.
-    int k = 0;
-    for (; k + 4 <= side; k += 4) {
-      float acc[4] = {0.f, 0.f, 0.f, 0.f};
+      uint32_t a[4][4];
 #pragma unroll
-      for (int ch = 0; ch < 64; ch += 4) {
+      for (int i = 0; i < 2; ++i) {
+        a[2 * i][0] = lo[i].x; a[2 * i][1] = hi[i].x; a[2 * i][2] = lo[i].y; a[2 * i][3] = hi[i].y;
+        a[2 * i + 1][0] = lo[i].z; a[2 * i + 1][1] = hi[i].z; a[2 * i + 1][2] = lo[i].w; a[2 * i + 1][3] = hi[i].w;
+      }
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const float4 t = *reinterpret_cast<const float4*>(&table[k + u][ch]);
-          acc[u] = fmaf(q[ch], t.x, acc[u]);
-          acc[u] = fmaf(q[ch + 1], t.y, acc[u]);
-          acc[u] = fmaf(q[ch + 2], t.z, acc[u]);
-          acc[u] = fmaf(q[ch + 3], t.w, acc[u]);
+      for (int which = 0; which < 2; ++which) {
+        float acc[NT][4];
+#pragma unroll
+        for (int j = 0; j < NT; ++j) {
+#pragma unroll
+          for (int e = 0; e < 4; ++e) acc[j][e] = 0.f;
+          // lane group g holds column 2 NT (g / 2) + 2 j + g % 2 of the result: table row for that k
+          const int k = min(2 * NT * (g >> 1) + 2 * j + (g & 1), side - 1);
+          const int row = which == 0 ? k : x - k + side - 1;
+          const uint4* table = (which == 0 ? table_h : table_w) + row * 8;
+#pragma unroll
+          for (int i = 0; i < 2; ++i) {
+            const uint4 v = table[(t + 4 * i) ^ ((row & 1) << 2)];
+            mma_16816<T>(acc[j], a[2 * i], v.x, v.y);
+            mma_16816<T>(acc[j], a[2 * i + 1], v.z, v.w);
+          }
+        }
+        T* out = static_cast<T*>(which == 0 ? p.rel_h : p.rel_w);
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+          const int head = h0 + g + 8 * half;
+          if (head >= p.heads) continue;
+          T* dst = out + ((static_cast<int64_t>(b) * p.heads + head) * n_tokens + n) * side + 2 * NT * t;
+          uint32_t words[NT];
+#pragma unroll
+          for (int j = 0; j < NT; ++j) words[j] = rel_pack2<T>(acc[j][2 * half], acc[j][2 * half + 1]);
+          if (NT % 4 == 0 && side == 8 * NT && p.out_wide) {  // whole 16-byte groups, rows of whole groups
+#pragma unroll
+            for (int j = 0; j + 3 < NT; j += 4) *reinterpret_cast<uint4*>(dst + 2 * j) = make_uint4(words[j], words[j + 1], words[j + 2], words[j + 3]);
+          } else {
+#pragma unroll
+            for (int j = 0; j < NT; ++j)
+              if (2 * NT * t + 2 * j < side) *reinterpret_cast<uint32_t*>(dst + 2 * j) = words[j];  // side is even
+          }
         }
       }
-      *reinterpret_cast<uint32_t*>(dst + k) = rel_pack2<T>(acc[0], acc[1]);
-      *reinterpret_cast<uint32_t*>(dst + k + 2) = rel_pack2<T>(acc[2], acc[3]);
-    }
-    for (; k < side; k += 2) {
-      float acc0 = 0.f, acc1 = 0.f;
-#pragma unroll
-      for (int ch = 0; ch < 64; ch += 4) {
-        const float4 t0 = *reinterpret_cast<const float4*>(&table[k][ch]);
-        const float4 t1 = *reinterpret_cast<const float4*>(&table[k + 1][ch]);
-        acc0 = fmaf(q[ch], t0.x, acc0); acc0 = fmaf(q[ch + 1], t0.y, acc0);
-        acc0 = fmaf(q[ch + 2], t0.z, acc0); acc0 = fmaf(q[ch + 3], t0.w, acc0);
-        acc1 = fmaf(q[ch], t1.x, acc1); acc1 = fmaf(q[ch + 1], t1.y, acc1);
-        acc1 = fmaf(q[ch + 2], t1.z, acc1); acc1 = fmaf(q[ch + 3], t1.w, acc1);
-      }
-      *reinterpret_cast<uint32_t*>(dst + k) = rel_pack2<T>(acc0, acc1);
     }
   }
 }

@@ -97,6 +97,24 @@ def test_producer_kernel_matches_the_oracle(b: int, side: int, dtype: torch.dtyp
     assert_close(rel_w.float().cpu().numpy(), want_w, unit_scale=False, what=f"rel_w side {side} {dtype}")
 
 
+@pytest.mark.parametrize(("b", "side", "heads"), [(1, 2, 1), (2, 6, 3), (1, 10, 17), (1, 16, 16), (1, 22, 24), (3, 32, 12), (1, 40, 5), (1, 48, 33), (2, 50, 12), (1, 62, 7)])
+def test_producer_kernel_at_every_tile_count(b: int, side: int, heads: int) -> None:
+    """Grid sides for each number of eight-column tiles, head counts around the sixteen rows of one product, and a second
+    table whose address is only 4-byte aligned (read word by word)."""
+    from oracle import attention_oracle as ao
+
+    gen = torch.Generator().manual_seed(side * heads)
+    qkv = torch.randn(b, side * side, 3, heads, DIM, generator=gen).half().cuda()
+    values = (torch.randn(2, 2 * side - 1, DIM, generator=gen) * 0.1).half().cuda()
+    room = torch.empty(2 + values[1].numel(), dtype=torch.float16, device="cuda")
+    both = [values[0], room[2:].view_as(values[1]).copy_(values[1])]
+    rel_h, rel_w = ff.sam_rel_terms(qkv[:, :, 0], both[0], both[1], side)
+    want_h, want_w = ao.decomposed_terms(qkv[:, :, 0].float().cpu().numpy().transpose(0, 2, 1, 3), *(t.float().cpu().numpy() for t in both), (side, side))
+    assert_close(rel_h.float().cpu().numpy(), want_h, unit_scale=False, what=f"rel_h side {side}")
+    assert_close(rel_w.float().cpu().numpy(), want_w, unit_scale=False, what=f"rel_w side {side}")
+    assert ff.device_status() == 0
+
+
 def test_producer_kernel_rejects_what_it_cannot_take() -> None:
     q = torch.zeros(1, 25, 2, 64, dtype=torch.float16, device="cuda")
     pos = torch.zeros(9, 64, dtype=torch.float16, device="cuda")
