@@ -10,6 +10,8 @@ from __future__ import annotations
 import ctypes
 import functools
 import hashlib
+import importlib.machinery
+import importlib.util
 import os
 import re
 import shutil
@@ -17,8 +19,12 @@ import subprocess
 import tempfile
 import threading
 from pathlib import Path
+from typing import TYPE_CHECKING
 
 from .errors import KernelUnavailableError
+
+if TYPE_CHECKING:
+    from types import ModuleType
 
 LIBRARY = "b200attn"
 PACKAGE_DIR = Path(__file__).resolve().parent
@@ -36,6 +42,9 @@ HEADERS = (
     PACKAGE_DIR.parent / "include" / "b200_encoder.h",
 )
 SHARED_OBJECT = PACKAGE_DIR / "libb200attn.so"
+# The host side of repeated calls, a CPython extension over torch's C++ interface (no kernels in it).
+HOST_SOURCE = PACKAGE_DIR / "csrc" / "host_ext.cpp"
+HOST_EXTENSION = PACKAGE_DIR / "_b200host.so"
 
 # sm_100a only: the kernels use tcgen05 / TMEM / TMA, which exist in no other target.
 NVCC_FLAGS = (
@@ -236,7 +245,7 @@ def source_hash() -> str:
     """Digest of the sources the shared object is compiled from (16 hex digits). The build passes it to the compiler,
     which puts it into the library's version string, so a binary can be matched with the sources beside it."""
     digest = hashlib.sha256()
-    for path in sorted((*SOURCES, *HEADERS), key=lambda f: f.name):
+    for path in sorted((*SOURCES, *HEADERS, HOST_SOURCE), key=lambda f: f.name):
         digest.update(path.name.encode())
         digest.update(path.read_bytes())
     return digest.hexdigest()[:16]
@@ -245,17 +254,35 @@ def source_hash() -> str:
 _HASH_IN_BINARY = re.compile(rb"b200attn-src:([0-9a-f]{16})")
 
 
-def built_hash() -> str | None:
-    """The source digest compiled into the shared object on disk (read from the file, without loading it), or None."""
-    if not SHARED_OBJECT.exists():
+def built_hash(binary: Path = SHARED_OBJECT) -> str | None:
+    """The source digest compiled into a binary on disk (read from the file, without loading it), or None."""
+    if not binary.exists():
         return None
-    found = _HASH_IN_BINARY.search(SHARED_OBJECT.read_bytes())
+    found = _HASH_IN_BINARY.search(binary.read_bytes())
     return found.group(1).decode() if found else None
 
 
 def needs_build() -> bool:
-    """True when the shared object is missing or was compiled from other sources than the ones beside it."""
-    return built_hash() != source_hash()
+    """True when a binary is missing or was compiled from other sources than the ones beside it."""
+    want = source_hash()
+    return built_hash() != want or built_hash(HOST_EXTENSION) != want
+
+
+def host_build_command(output: Path, digest: str) -> list[str]:
+    """The compiler call for the host extension; it links against the library beside it."""
+    import sysconfig  # noqa: PLC0415
+
+    import torch  # noqa: PLC0415
+
+    root = Path(torch.__file__).parent
+    cuda = Path(shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc").resolve().parent.parent
+    return [
+        shutil.which("g++") or "g++", "-O2", "-std=c++17", "-fPIC", "-shared", f'-DB200_SOURCE_HASH="{digest}"',
+        f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",  # noqa: SLF001
+        f"-I{root / 'include'}", f"-I{root / 'include/torch/csrc/api/include'}", f"-I{cuda / 'include'}", f"-I{sysconfig.get_paths()['include']}",
+        str(HOST_SOURCE), "-o", str(output), f"-L{PACKAGE_DIR}", "-l:libb200attn.so", "-Wl,-rpath,$ORIGIN",
+        f"-L{root / 'lib'}", "-ltorch_python", "-ltorch_cuda", "-ltorch_cpu", "-ltorch", "-lc10_cuda", "-lc10", f"-Wl,-rpath,{root / 'lib'}",
+    ]  # fmt: skip
 
 
 def build(*, force: bool = False, verbose: bool = False) -> Path:
@@ -286,6 +313,12 @@ def build(*, force: bool = False, verbose: bool = False) -> Path:
             tmp.unlink(missing_ok=True)
             raise KernelUnavailableError(LIBRARY, f"linking failed:\n{proc.stdout}\n{proc.stderr}")
     tmp.replace(SHARED_OBJECT)
+    tmp = HOST_EXTENSION.with_suffix(f".{os.getpid()}.tmp.so")
+    proc = subprocess.run(host_build_command(tmp, source_hash()), capture_output=True, text=True, check=False)
+    if proc.returncode != 0:
+        tmp.unlink(missing_ok=True)
+        raise KernelUnavailableError(LIBRARY, f"compiling the host extension failed:\n{proc.stdout}\n{proc.stderr}")
+    tmp.replace(HOST_EXTENSION)
     return SHARED_OBJECT
 
 
@@ -341,6 +374,36 @@ def library() -> ctypes.CDLL:
     lib.b200_attn_version.argtypes = ()
     lib.b200_attn_version.restype = ctypes.c_char_p
     return lib
+
+
+@functools.cache
+def host() -> ModuleType:
+    """The loaded host extension (after `library()`, which checks both binaries against the sources).
+
+    Raises:
+        KernelUnavailableError: It is not built or does not load.
+    """
+    library()
+    loader = importlib.machinery.ExtensionFileLoader("_b200host", str(HOST_EXTENSION))
+    spec = importlib.util.spec_from_file_location("_b200host", str(HOST_EXTENSION), loader=loader)
+    try:
+        module = importlib.util.module_from_spec(spec)
+        loader.exec_module(module)
+    except ImportError as e:
+        raise KernelUnavailableError(LIBRARY, f"cannot load {HOST_EXTENSION.name}: {e}") from e
+    return module
+
+
+# The host extension, once this process has launched an operator the full way (the library is loaded and checked then). Its
+# functions take the plain, valid call of an operator and answer None (False) to anything else.
+fast: ModuleType | None = None
+
+
+def use_fast() -> None:
+    """Let repeated calls go through the host extension."""
+    global fast  # noqa: PLW0603
+    if fast is None:
+        fast = host()
 
 
 def last_error() -> str:

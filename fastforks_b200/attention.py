@@ -199,70 +199,8 @@ def _attach_workspace(a: _lib.B200AttnArgs, index: int) -> None:
         a.workspace, a.workspace_bytes = None, 0
     else:
         a.workspace, a.workspace_bytes = ws.data_ptr(), ws.numel()
-
-
-# Launch descriptions already checked once, per thread: geometry key -> (args struct, output shape). A ViT calls the
-# operator with the same views in every block and every forward; for launch-bound shapes (one image of 197 tokens) the
-# checks and the ctypes set-up of a call cost more than the kernel, so a repeated geometry only has its four
-# pointers and the scale filled in again. The key holds everything `check_operands` looks at.
-_PREPARED = threading.local()
-_PREPARED_LIMIT = 256
-
-
-def _geometry_key(q, k, v, layout, out, schedule, rel=None, bias=None):  # noqa: ANN001, ANN202, PLR0913
-    return (
-        q.dtype, k.dtype, v.dtype, q.device, k.device, v.device, layout, schedule, q.shape, k.shape, v.shape,
-        q.stride(), k.stride(), v.stride(),
-        None if out is None else (out.dtype, out.device, out.shape, out.stride()),
-        None if rel is None else tuple((t.dtype, t.device, t.shape, t.stride()) for t in rel),
-        None if bias is None else (bias.dtype, bias.device, bias.shape, bias.stride(), bias.data_ptr() % 16),
-    )  # fmt: skip
-
-
-def _launch_prepared(q, k, v, scale, layout, out, schedule, rel=None, bias=None):  # noqa: ANN001, ANN202, PLR0913
-    """Launch from a remembered description of this geometry; None when there is none (the full path then runs)."""
-    table = getattr(_PREPARED, "table", None)
-    if table is None:
-        return None
-    try:
-        entry = table.get(_geometry_key(q, k, v, layout, out, schedule, rel, bias))
-    except (AttributeError, TypeError, ValueError):  # not tensors: let the full path raise its ValueError
-        return None
-    if entry is None:
-        return None
-    if (q.requires_grad or k.requires_grad or v.requires_grad) and torch.is_grad_enabled():
-        return None
-    a, o_shape, index = entry
-    if index != torch.cuda.current_device():
-        return None
-    if out is None:
-        o = torch.empty(o_shape, device=q.device, dtype=q.dtype)
-        out = o.transpose(1, 2) if layout == "bhnd" else o
-    a.q, a.k, a.v, a.o = q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr()
-    if rel is not None:  # remembered only where the tables went in as they are (broadcast views of the same memory)
-        a.rel_h, a.rel_w = rel[0].data_ptr(), rel[1].data_ptr()
-    if bias is not None:  # likewise
-        a.bias = bias.data_ptr()
-    a.scale = float(HEAD_DIM**-0.5 if scale is None else scale)
-    _attach_workspace(a, index)
-    code = _lib.library().b200_attn_fwd(ctypes.byref(a), torch._C._cuda_getCurrentRawStream(index))  # noqa: SLF001
-    if code != _lib.OK:
-        _lib.raise_for_code(code, "attention")
-    return out
-
-
-def _remember(a, q, k, v, out, layout, schedule, rel=None, bias=None) -> None:  # noqa: ANN001, PLR0913
-    """Keep the checked description `a` of this geometry for the calling thread (`out` as the caller gave it)."""
-    index = q.device.index
-    if index is None or index != torch.cuda.current_device():
-        return
-    table = getattr(_PREPARED, "table", None)
-    if table is None:
-        table = _PREPARED.table = {}
-    while len(table) >= _PREPARED_LIMIT:  # the oldest description goes (dicts keep insertion order)
-        del table[next(iter(table))]
-    copy = _lib.B200AttnArgs.from_buffer_copy(a)
-    table[_geometry_key(q, k, v, layout, out, schedule, rel, bias)] = (copy, (a.batch, a.q_tokens, a.heads, HEAD_DIM), index)
+        if _lib.fast is not None:
+            _lib.fast.register_workspace(index, torch._C._cuda_getCurrentRawStream(index), ws.data_ptr(), ws.numel())  # noqa: SLF001
 
 
 def attention(  # noqa: PLR0913
@@ -307,8 +245,12 @@ def attention(  # noqa: PLR0913
         KernelUnavailableError: The CUDA library is not built or does not load.
         RuntimeError: A CUDA error at launch.
     """
-    if not _general_merge and not _bias_as_given:
-        done = _launch_prepared(q, k, v, scale, layout, out, schedule, rel, bias)
+    # For launch-bound shapes (one image of 197 tokens) the checks and the ctypes set-up below cost more than the kernel:
+    # the plain call goes through the host extension.
+    host = _lib.fast
+    if host is not None and not _general_merge and not _bias_as_given and layout in LAYOUTS and schedule in _SCHEDULES and (rel is None or len(rel) == 2):  # noqa: PLR2004
+        rel_h, rel_w = rel if rel is not None else (None, None)
+        done = host.attention(q, k, v, scale, layout == "bnhd", _SCHEDULES[schedule], out, bias, rel_h, rel_w, False)  # noqa: FBT003
         if done is not None:
             return done
     check_operands(q, k, v, layout, out)
@@ -321,7 +263,6 @@ def attention(  # noqa: PLR0913
     lib = _lib.library()
     b, n, h = _sizes(q, layout)
     _, nk, _ = _sizes(k, layout)
-    given_out = out
     if out is None:
         o = torch.empty((b, n, h, HEAD_DIM), device=q.device, dtype=q.dtype)
         out = o.transpose(1, 2) if layout == "bhnd" else o
@@ -374,9 +315,7 @@ def attention(  # noqa: PLR0913
         _attach_workspace(a, index)
         code = lib.b200_attn_fwd(ctypes.byref(a), torch._C._cuda_getCurrentRawStream(index))  # noqa: SLF001
     _lib.raise_for_code(code, "attention")
-    if not keep and not _general_merge and not _bias_as_given:
-        # accepted, and made of the caller's own tensors only: the same geometry can be launched from pointers alone
-        _remember(a, q, k, v, given_out, layout, schedule, rel, bias)
+    _lib.use_fast()
     for t in keep:  # the launch is asynchronous: tie temporaries to the stream
         t.record_stream(torch.cuda.current_stream(q.device))
     return out

@@ -17,6 +17,7 @@ from __future__ import annotations
 
 import torch
 
+from . import _lib
 from .attention import HEAD_DIM, attention, check_operands
 
 FLASH_VARIANTS = ("hh", "fh", "ff")
@@ -59,6 +60,10 @@ class Flash64:
     @staticmethod
     def _run(variant: str, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, scale: float) -> torch.Tensor:
         """The one place a launch happens (the reference's tests replace this method to observe launches)."""
+        if _lib.fast is not None and variant in FLASH_VARIANTS:
+            out = _lib.fast.attention(q, k, v, scale, True, 0, None, None, None, None, True)  # noqa: FBT003
+            if out is not None:
+                return out
         _known_variant(variant)
         check_flash64(q, k, v)
         b, n, h, _ = q.shape

@@ -59,6 +59,10 @@ def gemm(  # noqa: PLR0913 - the epilogue terms
         ValueError: Operands outside the contract (checked before the launch).
         KernelUnavailableError: The CUDA library is not built or does not load.
     """
+    if _lib.fast is not None:
+        done = _lib.fast.gemm(x, w, bias, act, scale, res, out)
+        if done is not None:
+            return done
     if x.dtype not in _DTYPES or not x.is_cuda:
         msg = f"gemm: x must be a float16 / bfloat16 CUDA tensor, got {x.dtype} on {x.device}"
         raise ValueError(msg)
@@ -94,4 +98,5 @@ def gemm(  # noqa: PLR0913 - the epilogue terms
     with torch.cuda.device(x.device):
         code = _lib.library().b200_gemm(ctypes.byref(a), torch._C._cuda_getCurrentRawStream(x.device.index))  # noqa: SLF001
     _lib.raise_for_code(code, "gemm")
+    _lib.use_fast()
     return y

@@ -44,6 +44,8 @@ def rope_qk_(qkv: torch.Tensor, cs: torch.Tensor, *, q_scale: float = 1.0) -> to
     Raises:
         ValueError: Operands outside the contract (checked before the launch).
     """
+    if _lib.fast is not None and _lib.fast.rope_qk_(qkv, cs, q_scale):
+        return qkv
     if qkv.dim() != 5 or qkv.shape[2] != 3 or qkv.shape[-1] != HEAD_DIM or not qkv.is_cuda or qkv.dtype not in (torch.float16, torch.bfloat16):  # noqa: PLR2004
         msg = f"rope_qk_: qkv must be a float16 / bfloat16 CUDA [B, N, 3, heads, 64] tensor, got {tuple(qkv.shape)} {qkv.dtype} {qkv.device}"
         raise ValueError(msg)
@@ -70,4 +72,5 @@ def rope_qk_(qkv: torch.Tensor, cs: torch.Tensor, *, q_scale: float = 1.0) -> to
     with torch.cuda.device(qkv.device):
         code = _lib.library().b200_rope_qk(ctypes.byref(a), torch._C._cuda_getCurrentRawStream(qkv.device.index))  # noqa: SLF001
     _lib.raise_for_code(code, "rope_qk_")
+    _lib.use_fast()
     return qkv

@@ -14,6 +14,7 @@ Parameter names are the upstream ones, so a state dict of `ImageEncoderViT` load
 
 from __future__ import annotations
 
+import ctypes
 from dataclasses import dataclass
 
 import torch
@@ -115,10 +116,10 @@ def sam_rel_terms(q: torch.Tensor, rel_pos_h: torch.Tensor, rel_pos_w: torch.Ten
     Raises:
         ValueError: Operands outside the contract (checked before the launch).
     """
-    import ctypes
-
-    from . import _lib
-
+    if _lib.fast is not None:
+        done = _lib.fast.sam_rel_terms(q, rel_pos_h, rel_pos_w, side)
+        if done is not None:
+            return done
     if q.dim() != 4 or q.shape[-1] != 64 or q.stride(-1) != 1 or not q.is_cuda or q.dtype not in (torch.float16, torch.bfloat16):  # noqa: PLR2004
         msg = f"sam_rel_terms: q must be a float16 / bfloat16 CUDA [B, N, heads, 64] view with unit last stride, got {tuple(q.shape)} {q.dtype} {q.device}"
         raise ValueError(msg)
@@ -146,6 +147,7 @@ def sam_rel_terms(q: torch.Tensor, rel_pos_h: torch.Tensor, rel_pos_w: torch.Ten
     with torch.cuda.device(q.device):
         code = _lib.library().b200_sam_rel_terms(ctypes.byref(a), torch._C._cuda_getCurrentRawStream(q.device.index))  # noqa: SLF001
     _lib.raise_for_code(code, "sam_rel_terms")
+    _lib.use_fast()
     return rel_h, rel_w
 
 
