@@ -5,7 +5,7 @@
 // the keys of each in tiles of 128:
 //   * a loader warp stages Q once and K / V tiles through rings of shared-memory stages with TMA
 //     (128-byte swizzle, rows past the end of the sequence read as zero); K runs two tiles ahead of V;
-//   * one thread per query tile issues S = Q K^T (tcgen05.mma, M=128 N=128 K=64) into tensor memory and
+//   * one warp per query tile (one lane of it) issues S = Q K^T (tcgen05.mma, M=128 N=128 K=64) into tensor memory and
 //     O += P V (M=128 N=64 K=128) with P read straight from tensor memory. S_t(j+1) is issued as soon
 //     as the softmax threads have pulled S_t(j) into registers, so the tensor pipe never sits on the
 //     softmax critical path;
@@ -528,7 +528,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   extern __shared__ uint8_t smem_raw[];
   using Smem = std::conditional_t<BIAS == kBiasDenseTiles, AttnSmemDense, AttnSmem>;
   constexpr int kStagesK = Smem::kRing, kStagesV = Smem::kRing;
-  Smem& sm = *reinterpret_cast<Smem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  Smem& sm = *reinterpret_cast<Smem*>(smem_align_1024(smem_raw));
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -579,6 +579,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   // below reads or writes global memory and waits here until the earlier kernel has completed and its writes are
   // visible. Without an earlier kernel, or without the launch attribute, the wait returns at once.
   grid_dependency_wait();
+  grid_launch_dependents();
   const uint32_t tmem = sm.tmem_base;
   volatile uint32_t* abort_flag = &sm.abort;
   const CtaWork& cw = sm.work;
@@ -673,16 +674,19 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       }
       __syncwarp();
     } else if (warp == kMmaWarp || warp == kMmaWarp + 1) {
-      // ======================= MMA issuers: one thread per query tile ==========================
-      const int t = warp - kMmaWarp;
-      if (lane == 0) {
+      // ======================= MMA issuers: one warp per query tile ============================
+      // The warp walks the steps converged and elects a lane around the issue itself (see elect_one): from inside one
+      // lane's branch a product took some 115 clocks to issue, twelve of them per step. One copy of either issue in the
+      // loop: the steps' code streams through the instruction cache, and a second copy of the products cost 10 %.
+      const int t = __shfl_sync(0xffffffffu, warp - kMmaWarp, 0);
+      {
         constexpr uint32_t fmt = std::is_same<T, __half>::value ? UMMA_F16 : UMMA_BF16;
         constexpr uint32_t idesc_qk = umma_idesc_f16(fmt, kTileRows, kTileRows, 0, 0);
         constexpr uint32_t idesc_pv = umma_idesc_f16(fmt, kTileRows, kHeadDim, 0, 1);
         const uint32_t idesc_qk_last = umma_idesc_f16(fmt, kTileRows, kv_last16, 0, 0);
         bool ok = true;
 
-        // Everything the issue loops need is computed once or counted along: one thread feeds the tensor pipe, and
+        // Everything the issue loops need is computed once or counted along: one lane feeds the tensor pipe, and
         // every instruction between two tcgen05.mma shows up as an idle pipe when the MMAs are this small.
         const uint64_t q_desc0 = umma_smem_desc_sw128(smem_u32(sm.q[t][0]), 1024, 16);
         const uint64_t k_desc0 = umma_smem_desc_sw128(smem_u32(sm.k[0]), 1024, 16);
@@ -691,6 +695,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         const uint32_t s_tm = tmem + kTmemS + t * kTileRows;
         const uint32_t o_tm = tmem + kTmemO + t * kHeadDim;
         const uint32_t p_tm = tmem + kTmemP + t * kHeadDim;
+        const auto warp_wait = [&](uint64_t* bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag)) != 0; };
         uint64_t* const s_full = &sm.s_full[t];
         uint64_t* const s_free = &sm.s_free[t];
         uint64_t* const p_full = &sm.p_full[t];
@@ -733,70 +738,70 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           const int slot = x.it & 1;
           // The K tile landed long ago as a rule: its test is issued first and runs behind the wait that does wait.
           const bool k_early = mbar_test_wait(&sm.k_full[x.st], x.ph);
-          if (is_first(x) && !mbar_wait(&sm.q_full[t][slot], (x.it >> 1) & 1, abort_flag)) return false;
-          if (x.gs > 0 && !mbar_wait(s_free, (x.gs - 1) & 1, abort_flag)) return false;  // S_t has been read
-          if (!k_early && !mbar_wait(&sm.k_full[x.st], x.ph, abort_flag)) return false;
+          if (is_first(x) && !warp_wait(&sm.q_full[t][slot], (x.it >> 1) & 1)) return false;
+          if (x.gs > 0 && !warp_wait(s_free, (x.gs - 1) & 1)) return false;  // S_t has been read
+          if (!__all_sync(0xffffffffu, k_early || mbar_wait(&sm.k_full[x.st], x.ph, abort_flag))) return false;
           tc_fence_after_sync();
           const uint64_t a = q_desc0 + static_cast<uint64_t>(slot) * kStageStep;
           const uint64_t bd = k_desc0 + static_cast<uint64_t>(x.st) * kStageStep;
           const uint32_t idesc = (x.j == kv_tiles - 1) ? idesc_qk_last : idesc_qk;
+          if (elect_one()) {
 #pragma unroll
-          for (int kk = 0; kk < kHeadDim / 16; ++kk)  // 32 bytes of K per step inside the swizzle atom
-            umma_ss(s_tm, a + 2 * kk, bd + 2 * kk, idesc, kk > 0 ? 1u : 0u);
-          umma_commit(s_full);
-          umma_commit(&sm.k_empty[x.st]);
-          if (x.it >= my_doubles) umma_commit(&sm.k_empty[x.st]);  // one-tile item: stand in for the absent second tile
-          if (is_last(x)) umma_commit(&sm.q_empty[t][slot]);  // the item's last reader of Q_t
+            for (int kk = 0; kk < kHeadDim / 16; ++kk)  // 32 bytes of K per step inside the swizzle atom
+              umma_ss(s_tm, a + 2 * kk, bd + 2 * kk, idesc, kk > 0 ? 1u : 0u);
+            umma_commit(s_full);
+            umma_commit(&sm.k_empty[x.st]);
+            if (x.it >= my_doubles) umma_commit(&sm.k_empty[x.st]);  // one-tile item: stand in for the absent second tile
+            if (is_last(x)) umma_commit(&sm.q_empty[t][slot]);  // the item's last reader of Q_t
+          }
           return true;
         };
         // O_t (+)= P_t(gs) V, 16 keys (two 8-row groups of the V tile) per MMA.
         auto issue_pv = [&](const Pos& x) -> bool {
           const bool v_early = mbar_test_wait(&sm.v_full[x.st], x.ph);
-          if (!mbar_wait(p_full, x.gs & 1, abort_flag)) return false;
-          if (!v_early && !mbar_wait(&sm.v_full[x.st], x.ph, abort_flag)) return false;
+          if (!warp_wait(p_full, x.gs & 1)) return false;
+          if (!__all_sync(0xffffffffu, v_early || mbar_wait(&sm.v_full[x.st], x.ph, abort_flag))) return false;
           // The first P V of an item overwrites O_t: the previous item's epilogue must have read it.
-          if (is_first(x) && x.it > 0 && !mbar_wait(&sm.o_free[t], (x.it - 1) & 1, abort_flag)) return false;
+          if (is_first(x) && x.it > 0 && !warp_wait(&sm.o_free[t], (x.it - 1) & 1)) return false;
           tc_fence_after_sync();
           const uint64_t bd = v_desc0 + static_cast<uint64_t>(x.st) * kStageStep;
-          if (x.j != kv_tiles - 1) {
-            umma_ts(o_tm, p_tm, bd, idesc_pv, is_first(x) ? 0u : 1u);
-#pragma unroll
-            for (int kk = 1; kk < kTileRows / 16; ++kk)
-              umma_ts(o_tm, p_tm + kk * 8, bd + kk * (2048 >> 4), idesc_pv, 1u);
-          } else {
-            const int steps = kv_last16 / 16;  // at least one
+          if (elect_one()) {
+            const int steps = x.j != kv_tiles - 1 ? kTileRows / 16 : kv_last16 / 16;  // at least one
             umma_ts(o_tm, p_tm, bd, idesc_pv, is_first(x) ? 0u : 1u);
 #pragma unroll
             for (int kk = 1; kk < kTileRows / 16; ++kk)
               if (kk < steps) umma_ts(o_tm, p_tm + kk * 8, bd + kk * (2048 >> 4), idesc_pv, 1u);
+            umma_commit(pv_done);
+            umma_commit(&sm.v_empty[x.st]);
+            if (x.it >= my_doubles) umma_commit(&sm.v_empty[x.st]);
           }
-          umma_commit(pv_done);
-          umma_commit(&sm.v_empty[x.st]);
-          if (x.it >= my_doubles) umma_commit(&sm.v_empty[x.st]);
           return true;
         };
 
-        Pos xq = start;  // the Q K^T stream runs two steps ahead of the P V stream
-        for (int i = 0; i < 2 && xq.gs < total_steps && ok; ++i) {
-          ok = issue_qk(xq);
-          advance(xq);
-        }
-        for (Pos xp = start; xp.gs < total_steps && ok; advance(xp)) {
-          ok = issue_pv(xp);
-          if (ok && xq.gs < total_steps) {
+        Pos xq = start, xp = start;  // the Q K^T stream runs a step ahead of the P V stream
+        bool lead = true;
+#pragma unroll 1
+        while (ok && xp.gs < total_steps) {
+          if (xq.gs < total_steps) {
             ok = issue_qk(xq);
             advance(xq);
           }
+          if (lead) {
+            lead = false;
+            continue;
+          }
+          if (ok) ok = issue_pv(xp);
+          advance(xp);
         }
-        if (!ok) {
+        if (!ok && lane == 0) {
           if (atomicExch(const_cast<uint32_t*>(abort_flag), 1u) == 0) atomicOr(p.status, kStatusMma);
         }
-        if (*abort_flag != 0) {
-          // Some role gave up: products this thread issued may still be running, and their commits must not
+        if (__any_sync(0xffffffffu, *abort_flag != 0)) {
+          // Some role gave up: products this warp issued may still be running, and their commits must not
           // arrive on barriers of a CTA that is gone (nor tensor memory be freed under them). One last commit on
           // a barrier of its own, waited for with the usual limit and without looking at the abort flag.
           uint32_t no_abort = 0;
-          umma_commit(&sm.drain[t]);
+          if (elect_one()) umma_commit(&sm.drain[t]);
           mbar_wait(&sm.drain[t], 0, &no_abort);
         }
       }
@@ -1107,11 +1112,6 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       for (int j = ja; j < jb; ++j) {
         const int rj = j - ja;  // step within this CTA's part of the item
         const int step = g + rj;
-        // One vote per step on whether any lane's wait ran out during the previous one.
-        if (__any_sync(0xffffffffu, bad)) {
-          ok = false;
-          break;
-        }
         bad |= !mbar_wait_warp_after(s_early, &sm.s_full[t], step & 1, abort_flag);
         tc_fence_after_sync();
         // dense-tile bias: the tile's barrier is tested here, its result is needed after the S load
@@ -1135,8 +1135,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         // The token between the warpgroups has two forms. Barrier form: all four warps of the other warpgroup arrive
         // on `turn`. Flag form (kFlagTurn): warp w only waits for warp w of the other warpgroup - the one it shares
         // its SM sub-partition and MUFU unit with - through a counter in shared memory, which is cheaper to poll than
-        // a barrier and does not tie a warp to the slowest of four. Measured per kernel form: the flag form is
-        // 2-6 % faster in the short and the key-split kernels and 4-7 % slower in the plain long one.
+        // a barrier and does not tie a warp to the slowest of four. Measured per kernel form: the flag form is 2-6 % faster
+        // in the short and the key-split kernels and 6 % slower in the plain long one, at every release point.
         constexpr bool kFlagTurn = SHORT || SPLIT;
         const uint32_t turn_need = (t == 0) ? static_cast<uint32_t>(gp + rj) : static_cast<uint32_t>(gp + rj + 1);
         const bool turn_early = (need_turn && !kFlagTurn) ? mbar_test_wait(&sm.turn[t], turn_parity) : true;
@@ -1280,7 +1280,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
             });
           }
         }
-        if (kv_valid < kTileRows) {
+        if (__builtin_expect(kv_valid < kTileRows, 0)) {
           // Short schedule: the ragged tile it is chosen for ends between columns 64 and 96 (197 keys: 69 in the
           // second tile): only those 32 columns need a compare, the last 32 hold no key at all.
           if (SHORT && kv_valid >= 64 && kv_valid <= 96) {
@@ -1343,9 +1343,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         // would leave the unit idle together, and equal loops sharing a unit drift into lockstep). So each
         // may only start a section once the other has released it from inside its previous one: warpgroup 0
         // starts step q+1 after warpgroup 1's release in step q, warpgroup 1 starts step q after warpgroup 0's
-        // release in step q. The release comes after 96 of the 128 columns (measured against 32, 64, 80, 112 and
-        // 128 in the long schedule: 64 was 3 % slower on eleven key tiles, 128 - exclusive sections - 7 %; in the
-        // short one 64 against 96: 1 % slower).
+        // release in step q. The release comes after 64 of the 128 columns in the long schedule ([32,24,1370] us: 16
+        // columns 556, 32 520, 64 510, 96 517, 128 558, no token 562), after 96 in the short one.
         if (need_turn) {
           if constexpr (kFlagTurn) {
             const volatile uint32_t* released = &sm.turn_count[t ^ 1][warp & 3];
@@ -1426,9 +1425,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
             for (int i = 48; i < 64; ++i) pk[i] = 0u;
           }
         } else {
-          exp_columns(integral_constant<int, 2>{}, integral_constant<int, 1>{});
           release_point();
-          exp_columns(integral_constant<int, 3>{}, integral_constant<int, 1>{});
+          exp_columns(integral_constant<int, 2>{}, integral_constant<int, 2>{});
         }
         l_sum += (l2a.x + l2a.y) + (l2b.x + l2b.y);
 
@@ -1436,7 +1434,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         // delivered P_t(j-1), a whole exponential section ago. On the first tile of an item the P V in
         // question is the last one of the previous item, and this is where that item's output is written:
         // its epilogue hides behind this item's first exponentials instead of stalling the pipeline.
-        if (rj == 0) {
+        if (__builtin_expect(rj == 0, 0)) {
           if (pend) {
             ok = finish_item(pv_early, stage_early, std::false_type{});
             if (!ok) break;
@@ -1444,7 +1442,11 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         } else {
           bad |= !mbar_wait_warp_after(pv_early, &sm.pv_done[t], (step - 1) & 1, abort_flag);
           tc_fence_after_sync();
-          if (__any_sync(0xffffffffu, raise)) {
+          if (__builtin_expect(__any_sync(0xffffffffu, raise || bad), 0)) {
+            if (__any_sync(0xffffffffu, bad)) {  // some lane's wait ran out (voted on together with the rescale, which is as rare)
+              ok = false;
+              break;
+            }
             float o[kHeadDim];
             uint32_t* ou = reinterpret_cast<uint32_t*>(o);
             tmem_ld_x64(o_addr, ou);

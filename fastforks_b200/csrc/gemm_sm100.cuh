@@ -169,7 +169,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant
                  const __grid_constant__ CUtensorMap tm_w_tail, const __grid_constant__ CUtensorMap tm_y,
                  const __grid_constant__ CUtensorMap tm_res, const GemmParams p) {
   extern __shared__ uint8_t smem_raw[];
-  PairSmem& sm = *reinterpret_cast<PairSmem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  PairSmem& sm = *reinterpret_cast<PairSmem*>(smem_align_1024(smem_raw));
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rank = static_cast<int>(cluster_cta_rank());  // 0: the leader, rows 0..127 of the tile
   constexpr bool swiglu = ACT == kActSwiGlu;
@@ -488,7 +488,7 @@ __global__ void __launch_bounds__(kSplitThreads)
 gemm_split_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_w, const GemmParams p) {
   using Smem = SplitSmem<S>;
   extern __shared__ uint8_t smem_raw[];
-  Smem& sm = *reinterpret_cast<Smem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  Smem& sm = *reinterpret_cast<Smem*>(smem_align_1024(smem_raw));
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rank = S > 1 ? static_cast<int>(cluster_cta_rank()) : 0;
   const int tile = blockIdx.x / S;
