@@ -46,7 +46,6 @@ static_assert(2 * 128 * kSoftmaxRegs + 128 * kHelperRegs <= kLaunchRegs * kThrea
               "register hand-over does not balance");
 constexpr int kStages = 3;       // K / V ring stages (the dense-tile bias form gives one of each to its bias tiles)
 constexpr int kStagesDense = 2;
-constexpr int kKLead = 2;                             // K tiles are consumed two iterations ahead of V tiles
 constexpr uint32_t kTmemCols = 512;                   // S0 S1 (128 each), O0 O1 (64 each), P0 P1 (64 each)
 constexpr uint32_t kTmemS = 0, kTmemO = 256, kTmemP = 384;
 constexpr float kLog2e = 1.4426950408889634f;
@@ -89,7 +88,14 @@ enum : int { kItemWhole = 0, kItemPartial = 1, kItemOwner = 2 };
 // kBiasDenseTiles is the dense form for 16-bit biases whose rows are 16-byte aligned: the loader warp brings the
 // 128 x 128 bias tile of every (query tile, key tile) into shared memory with TMA, like K and V, instead of every
 // softmax thread walking its own row in global memory.
-enum : int { kBiasNone = 0, kBiasDense = 1, kBiasDecomposed = 2, kBiasDecomposed64 = 3, kBiasDecomposed14 = 4, kBiasDenseTiles = 5 };
+// kBiasDecomposedMma adds the decomposed form on the tensor cores: the row's rel_h and rel_w values (up to 128 of them,
+// 16-bit) are an operand R like Q, the grid coordinates of the keys a one-hot operand E, and S = Q K^T + R E. A 1 in E is
+// 1 / scale, which must be a power of two, so every product is exact and the softmax warps see plain logits. Bounded by the
+// tensor pipe above some 96 values per row and by the softmax step below. us, additions by the softmax warps -> here
+// ([B,H,N]): [4,12,1024] 271 -> 40, [2,12,2304] 853 -> 72, [10,12,400] 170 -> 26, [100,12,36] 113 -> 41; [1,12,4096], whose
+// 64-wide tables had a form of their own (kBiasDecomposed64), 101 -> 99. The 14 x 14 form stays ahead: [400,12,196] 183 against 216.
+enum : int { kBiasNone = 0, kBiasDense = 1, kBiasDecomposed = 2, kBiasDecomposed64 = 3, kBiasDecomposed14 = 4, kBiasDenseTiles = 5, kBiasDecomposedMma = 6 };
+constexpr int kMaxRelChunks = 16;   // kBiasDecomposedMma: groups of eight values per row of R and E
 constexpr int kRelStageWords = 33;  // per-row staging of rel_h | rel_w in shared memory: up to 32 values, odd stride
 
 struct BiasView {
@@ -121,6 +127,10 @@ struct AttnParams {
   uint64_t magic_pairs, magic_singles, magic_heads, magic_rel_kw;  // fast_div constants of pairs_per_head, singles_per_head, heads (the batch size if batch_fastest), rel_kw
   int batch_fastest;   // items are numbered with the batch index running fastest (else the head index): see decode_item
   int rel_staged;      // decomposed form: rel_kh + rel_kw <= 32, rows are staged in shared memory per item
+  // kBiasDecomposedMma: eight-value chunks of rel_h and of rel_w in a row of R, 16-value steps of the product, 1 / scale as
+  // a 16-bit value of the tables' type, and the bytes their rows are aligned to (16, 4 or 2).
+  int rel_chunks_h, rel_chunks_w, rel_steps, rel_align;
+  uint32_t rel_one;
   int bias_vec;        // dense form: rows are 16-byte aligned, full tiles are read with vector loads
   uint32_t* status;    // device word that collects role bits of expired waits
   // Key-split mode (chunked != 0; see kPairCost). pairs_per_head = q_tiles / 2 and singles_per_head = q_tiles % 2 then.
@@ -146,19 +156,23 @@ struct CtaWork {
   int steps_all, steps_pairs;  // key-tile steps of all items and of the two-tile items
 };
 
-template <int STAGES, bool BIAS_TILES>
+enum : int { kRoomRelStage = 0, kRoomBiasTiles = 1, kRoomRelMma = 2 };
+// Q_BUFS: 2 where the next item's Q is loaded while this one computes, 1 in the form that needs the room for R and E.
+template <int STAGES, int Q_BUFS, int ROOM>
 struct alignas(1024) AttnSmemT {
-  static constexpr int kRing = STAGES;
-  uint8_t q[2][2][kTileBytes];  // [query-tile slot][item parity]: the next item's Q is loaded while this one computes
+  static constexpr int kRing = STAGES, kQBufs = Q_BUFS;
+  static constexpr bool BIAS_TILES = ROOM == kRoomBiasTiles, REL_MMA = ROOM == kRoomRelMma;
+  uint8_t q[2][Q_BUFS][kTileBytes];  // [query-tile slot][item number modulo Q_BUFS]
   uint8_t k[STAGES][kTileBytes];
   uint8_t v[STAGES][kTileBytes];
   uint8_t o_stage[2][kTileBytes];  // an item's output tile per query-tile slot, in the TMA tile layout (128-byte swizzle)
-  uint64_t q_full[2][2];   // Q_t of an item has landed                      (TMA)
-  uint64_t q_empty[2][2];  // that item's last Q_t K^T has finished          (MMA commit)
+  uint64_t q_full[2][Q_BUFS];   // Q_t of an item has landed                 (TMA)
+  uint64_t q_empty[2][Q_BUFS];  // that item's last Q_t K^T has finished     (MMA commit)
   uint64_t k_full[STAGES], k_empty[STAGES];
   uint64_t v_full[STAGES], v_empty[STAGES];
   uint64_t bias_full[2];   // dense-tile bias form: the bias tile of query tile t's current step has landed (TMA)
   uint64_t bias_free[2];   // ... and has been read by the softmax warps                                  (4 softmax warps)
+  uint64_t r_full[2];   // R_t of an item is in shared memory             (4 softmax warps)
   uint64_t s_full[2];   // S_t(j) is in tensor memory                     (MMA commit)
   uint64_t s_free[2];   // S_t(j) has been read into registers             (4 softmax warps)
   uint64_t p_full[2];   // P_t(j) is in tensor memory, O_t rescaled        (4 softmax warps)
@@ -178,19 +192,28 @@ struct alignas(1024) AttnSmemT {
   // decomposed forms: each softmax thread's own rel_h | rel_w row, times log2(e); dense-tile form: per query tile the
   // two 64-column halves of the current 128 x 128 bias tile (16-bit, 128-byte swizzle)
   // (a TMA destination with the 128-byte swizzle starts on a 1024-byte boundary)
-  union alignas(BIAS_TILES ? 1024 : 16) {
-    float rel_stage[2][kTileRows][kRelStageWords];
+  // decomposed form on the tensor cores: R per query tile and E, as 128-row tiles of 64 values (128-byte swizzle)
+  union alignas(ROOM != kRoomRelStage ? 1024 : 16) {
+    float rel_stage[2][ROOM == kRoomRelStage ? kTileRows : 1][kRelStageWords];
+    struct {
+      uint8_t r[REL_MMA ? 2 : 1][2][REL_MMA ? kTileBytes : 16];
+      uint8_t e[2][REL_MMA ? kTileBytes : 16];
+    };
     uint8_t bias_tile[BIAS_TILES ? 2 : 1][2][BIAS_TILES ? kTileBytes : 16];
   };
 };
-using AttnSmem = AttnSmemT<kStages, false>;
-using AttnSmemDense = AttnSmemT<kStagesDense, true>;
+using AttnSmem = AttnSmemT<kStages, 2, kRoomRelStage>;
+using AttnSmemDense = AttnSmemT<kStagesDense, 2, kRoomBiasTiles>;
+using AttnSmemRelMma = AttnSmemT<kStagesDense, 1, kRoomRelMma>;
+template <int BIAS>
+using AttnSmemOf = std::conditional_t<BIAS == kBiasDenseTiles, AttnSmemDense, std::conditional_t<BIAS == kBiasDecomposedMma, AttnSmemRelMma, AttnSmem>>;
 // The set-up walks the barriers as one array and picks the arrival count by position.
 static_assert(offsetof(AttnSmem, merge_go) + sizeof(uint64_t[2]) == offsetof(AttnSmem, merge_ready) &&
                   offsetof(AttnSmem, o_free) + 2 * sizeof(uint64_t[2]) == offsetof(AttnSmem, o_staged) &&
                   offsetof(AttnSmem, q_full) < offsetof(AttnSmem, merge_go),
               "barrier order in AttnSmemT: q_full ... o_free, turn, o_staged ... merge_go, nothing else in between");
-static_assert(offsetof(AttnSmemDense, bias_tile) % 1024 == 0, "bias tiles: 1024-byte aligned for the 128-byte swizzle");
+static_assert(offsetof(AttnSmemDense, bias_tile) % 1024 == 0 && offsetof(AttnSmemRelMma, r) % 1024 == 0 && offsetof(AttnSmemRelMma, e) % 1024 == 0,
+              "tiles: 1024-byte aligned for the 128-byte swizzle");
 
 __device__ __forceinline__ float fast_exp2(float x) {
   float y;
@@ -298,6 +321,34 @@ __device__ __forceinline__ void for_bias_dtype(int dtype, F&& f) {
   else f(std::integral_constant<int, 1>{});
 }
 
+// Up to eight 16-bit values at `src`, zeros behind the first `left`; ALIGN: what rows begin on, in bytes (4: whole pairs).
+template <int ALIGN>
+__device__ __forceinline__ uint4 load_rel_chunk(const uint16_t* src, int left) {
+  if constexpr (ALIGN == 16) {  // values behind the row's end belong to the next row or to nobody: loaded only if all eight exist
+    if (left >= 8) return __ldg(reinterpret_cast<const uint4*>(src));
+  }
+  uint32_t w[4];
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    w[e] = 0;
+    if constexpr (ALIGN == 2) {
+      if (2 * e < left) w[e] = __ldg(src + 2 * e);
+      if (2 * e + 1 < left) w[e] |= static_cast<uint32_t>(__ldg(src + 2 * e + 1)) << 16;
+    } else {
+      if (2 * e + 1 < left) w[e] = __ldg(reinterpret_cast<const uint32_t*>(src) + e);
+      else if (2 * e < left) w[e] = __ldg(src + 2 * e);
+    }
+  }
+  return make_uint4(w[0], w[1], w[2], w[3]);
+}
+// Two packed 16-bit values with infinities replaced by the largest finite value of their sign.
+__device__ __forceinline__ uint32_t clamp_finite2(uint32_t v, bool is_half) {
+  const uint32_t inf_lo = is_half ? 0x7c00u : 0x7f80u;
+  if ((v & 0x7fffu) == inf_lo) v -= 1;
+  if (((v >> 16) & 0x7fffu) == inf_lo) v -= 0x10000u;
+  return v;
+}
+
 // n / d for the divisors the host knows at launch: magic = ceil(2^64 / d) (0 stands for d == 1), exact for every
 // n * d < 2^64. An integer division in device code takes its reciprocal from the MUFU unit, which the softmax warps
 // keep saturated; the multiply does not.
@@ -331,7 +382,8 @@ __device__ __forceinline__ void add_rel14(float* s, const float* stage, float c)
   }
 }
 
-static_assert(sizeof(AttnSmem) + 1024 <= 227 * 1024 && sizeof(AttnSmemDense) + 1024 <= 227 * 1024, "shared memory of one CTA");
+static_assert(sizeof(AttnSmem) + 1024 <= 227 * 1024 && sizeof(AttnSmemDense) + 1024 <= 227 * 1024 && sizeof(AttnSmemRelMma) + 1024 <= 227 * 1024,
+              "shared memory of one CTA");
 
 // One unit of work: one or two 128-row query tiles of one (batch, head) over the key tiles [ja, jb).
 struct WorkItem {
@@ -526,8 +578,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
                 const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_o,
                 const __grid_constant__ CUtensorMap tm_bias, const AttnParams p) {
   extern __shared__ uint8_t smem_raw[];
-  using Smem = std::conditional_t<BIAS == kBiasDenseTiles, AttnSmemDense, AttnSmem>;
-  constexpr int kStagesK = Smem::kRing, kStagesV = Smem::kRing;
+  using Smem = AttnSmemOf<BIAS>;
+  constexpr int kStagesK = Smem::kRing, kStagesV = Smem::kRing, kQBufs = Smem::kQBufs;
+  constexpr int kKLead = Smem::kRing - 1;  // K tiles loaded ahead of V tiles: one less than the ring, or V waits for K to come free
+  constexpr bool kPlainLogits = BIAS == kBiasNone || BIAS == kBiasDecomposedMma;  // S is scaled in front of the exponential only
   Smem& sm = *reinterpret_cast<Smem*>(smem_align_1024(smem_raw));
 
   const int warp = threadIdx.x >> 5;
@@ -548,10 +602,12 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     const int n_bars = static_cast<int>(&sm.merge_go[1] - first) + 1;
     for (int i = lane; i < n_bars; i += 32) {
       uint64_t* bar = first + i;
-      const bool four = (bar >= &sm.bias_free[0] && bar <= &sm.bias_free[1]) || (bar >= &sm.s_free[0] && bar <= &sm.s_free[1]) ||
+      const bool four = (bar >= &sm.bias_free[0] && bar <= &sm.bias_free[1]) || (bar >= &sm.r_full[0] && bar <= &sm.r_full[1]) ||
+                        (bar >= &sm.s_free[0] && bar <= &sm.s_free[1]) ||
                         (bar >= &sm.p_full[0] && bar <= &sm.p_full[1]) || (bar >= &sm.o_free[0] && bar <= &sm.o_staged[1]);
-      const bool two = (bar >= &sm.k_empty[0] && bar <= &sm.k_empty[kStagesK - 1]) ||
-                       (bar >= &sm.v_empty[0] && bar <= &sm.v_empty[kStagesV - 1]);
+      // with kBiasDecomposedMma a K tile is there when its TMA transaction and its E are
+      const bool two = (BIAS == kBiasDecomposedMma && bar >= &sm.k_full[0] && bar <= &sm.k_full[kStagesK - 1]) || (bar >= &sm.k_empty[0] && bar <= &sm.k_empty[kStagesK - 1]) ||
+                       (bar >= &sm.v_empty[0] && bar <= &sm.v_empty[kStagesV - 1]) ;
       mbar_init(bar, four ? 4 : two ? 2 : 1);
     }
     if (lane == 0) sm.abort = 0;
@@ -559,6 +615,11 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     mbar_init_fence();
   } else if (threadIdx.x == 32) {
     sm.work = cta_work(p, static_cast<int>(blockIdx.x), static_cast<int>(gridDim.x));
+  }
+  if constexpr (BIAS == kBiasDecomposedMma) {  // E starts without a one
+    uint4* e = reinterpret_cast<uint4*>(sm.e[0]);
+    for (int i = threadIdx.x; i < 2 * kTileBytes / 16; i += kThreads) e[i] = make_uint4(0, 0, 0, 0);
+    fence_proxy_async_smem();
   }
   if (warp == kMmaWarp) {
     tmem_alloc(&sm.tmem_base, kTmemCols);
@@ -589,15 +650,125 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     reg_dealloc<kHelperRegs>();
     if (warp == kLoaderWarp) {
       // ======================= loader =======================================================
-      if (lane == 0) {
+      if constexpr (BIAS == kBiasDecomposedMma) {
+        // The whole warp: one lane issues the copies, and all write E, the grid coordinates of a tile's keys as one-hot
+        // rows (rel_h's values, then rel_w's), which is released and reused with the K tile it belongs to: two buffers where
+        // a row has up to 64 values, one of twice the size above. A lane moves the two ones of four keys. (By the MMA warp
+        // of one query tile, between its products, the same 500 clocks held up the other tile too: +40 %.)
+        bool ok = true;
+        int gk = 0, gv = 0;
+        int q_count[2] = {0, 0};
+        const int e_bufs = p.rel_steps <= 4 ? 2 : 1;
+        const bool e_constant = !SPLIT && kv_tiles <= e_bufs;  // every use of a buffer has the same E: it is written once
+        int e_y[4], e_x[4];  // coordinates of this lane's keys
+        const int e_dy = fast_div(kTileRows, p.magic_rel_kw), e_dx = kTileRows - e_dy * p.rel_kw;
+        // byte offsets of this lane's ones (inside its rows) in the tile before last and in the last one; at first those of
+        // places that hold a zero
+        uint32_t hot_old[4][2] = {}, hot[4][2] = {};
+        const auto warp_wait = [&](uint64_t* bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait_relaxed(bar, parity, abort_flag)) != 0; };
+        for (int it = 0; it < my_items && ok; ++it) {
+          const WorkItem w = decode_item<SPLIT>(p, cw, it);
+          for (int t = 0; t < w.n_tiles && ok; ++t) {
+            ok = warp_wait(&sm.q_empty[t][it % kQBufs], ((it / kQBufs) & 1) ^ 1);
+            if (!ok) break;
+            if (lane == 0) {
+              mbar_arrive_expect_tx(&sm.q_full[t][it % kQBufs], kTileBytes);
+              tma_load_4d(sm.q[t][it % kQBufs], &tm_q, &sm.q_full[t][it % kQBufs], 0, w.q_row0 + t * kTileRows, w.h, w.b);
+            }
+            q_count[t] = it + 1;
+          }
+          const int steps = w.jb - w.ja;
+          for (int i = 0; i < steps + kKLead && ok; ++i) {
+            if (i < steps) {
+              const int st = gk % kStagesK;
+              ok = warp_wait(&sm.k_empty[st], ((gk / kStagesK) & 1) ^ 1);
+              if (!ok) break;
+              if (lane == 0) {
+                mbar_arrive_expect_tx(&sm.k_full[st], kTileBytes);
+                tma_load_4d(sm.k[st], &tm_k, &sm.k_full[st], 0, (w.ja + i) * kTileRows, w.h, w.b);
+              }
+              ++gk;
+            }
+            const int iv = i - kKLead;
+            if (iv >= 0) {
+              const int st = gv % kStagesV;
+              ok = warp_wait(&sm.v_empty[st], ((gv / kStagesV) & 1) ^ 1);
+              if (ok && lane == 0) {
+                mbar_arrive_expect_tx(&sm.v_full[st], kTileBytes);
+                tma_load_4d(sm.v[st], &tm_v, &sm.v_full[st], 0, (w.ja + iv) * kTileRows, w.h, w.b);
+              }
+              gv += ok ? 1 : 0;
+            }
+            if (i < steps) {
+              const int n = gk - 1, st = n % kStagesK;  // the tile whose E is due
+              if (ok && !(e_constant && n >= e_bufs)) {
+                // with one buffer the products of the tile before must have read it
+                if (e_bufs == 1 && n > 0) ok = warp_wait(&sm.k_empty[(n - 1) % kStagesK], ((n - 1) / kStagesK) & 1);
+                const uint32_t e = smem_u32(sm.e[e_bufs == 2 ? st : 0]) + lane * 128, swizzle = (lane & 7) << 4;
+                if (i == 0) {
+#pragma unroll
+                  for (int r = 0; r < 4; ++r) {
+                    const int key = w.ja * kTileRows + lane + 32 * r;
+                    e_y[r] = fast_div(key, p.magic_rel_kw);
+                    e_x[r] = key - e_y[r] * p.rel_kw;
+                  }
+                } else {  // a tile on: 128 keys
+#pragma unroll
+                  for (int r = 0; r < 4; ++r) {
+                    e_y[r] += e_dy;
+                    e_x[r] += e_dx;
+                    const bool carry = e_x[r] >= p.rel_kw;
+                    e_x[r] -= carry ? p.rel_kw : 0;
+                    e_y[r] += carry ? 1 : 0;
+                  }
+                }
+                // Keys behind the last one get ones like the others: their columns of S are masked.
+                uint32_t at[4][2];
+#pragma unroll
+                for (int r = 0; r < 4; ++r)
+#pragma unroll
+                  for (int k = 0; k < 2; ++k) {
+                    const uint32_t f = k == 0 ? min(e_y[r], p.rel_kh - 1) : 8 * p.rel_chunks_h + e_x[r];
+                    at[r][k] = (((f << 1) & 0x7e) ^ swizzle) + ((f << 8) & 0x4000);  // value f of the row: tile f / 64, swizzled chunk f / 8
+                  }
+#pragma unroll
+                for (int r = 0; r < 4; ++r)
+#pragma unroll
+                  for (int k = 0; k < 2; ++k) st_shared_u16(e + r * 32 * 128 + (e_bufs == 2 ? hot_old[r][k] : hot[r][k]), 0);
+#pragma unroll
+                for (int r = 0; r < 4; ++r)
+#pragma unroll
+                  for (int k = 0; k < 2; ++k) {
+                    st_shared_u16(e + r * 32 * 128 + at[r][k], static_cast<uint16_t>(p.rel_one));
+                    hot_old[r][k] = hot[r][k];
+                    hot[r][k] = at[r][k];
+                  }
+                fence_proxy_async_smem();
+              }
+              warp_arrive(&sm.k_full[st], lane);  // on the abort path too: the copy's barrier must complete
+            }
+          }
+        }
+        if (!ok && lane == 0) {
+          if (atomicExch(const_cast<uint32_t*>(abort_flag), 1u) == 0) atomicOr(p.status, kStatusLoader);
+        }
+        if (__any_sync(0xffffffffu, *abort_flag != 0)) {  // let the copies in flight land, as below
+          uint32_t no_abort = 0;
+          for (int t = 0; t < 2; ++t)
+            for (int i = (q_count[t] > kQBufs ? q_count[t] - kQBufs : 0); i < q_count[t]; ++i)
+              mbar_wait_relaxed(&sm.q_full[t][i % kQBufs], (i / kQBufs) & 1, &no_abort);
+          for (int j = (gk > kStagesK ? gk - kStagesK : 0); j < gk; ++j) mbar_wait_relaxed(&sm.k_full[j % kStagesK], (j / kStagesK) & 1, &no_abort);
+          for (int j = (gv > kStagesV ? gv - kStagesV : 0); j < gv; ++j) mbar_wait_relaxed(&sm.v_full[j % kStagesV], (j / kStagesV) & 1, &no_abort);
+        }
+      } else if (lane == 0) {
         bool ok = true;
         int gk = 0, gv = 0;        // K / V tiles issued so far (ring position and phase)
         int q_count[2] = {0, 0};   // Q tiles issued so far per query-tile slot
         for (int it = 0; it < my_items && ok; ++it) {
           const WorkItem w = decode_item<SPLIT>(p, cw, it);
-          const int slot = it & 1;
+          const int slot = it % kQBufs;
           for (int t = 0; t < w.n_tiles && ok; ++t) {
-            ok = mbar_wait_relaxed(&sm.q_empty[t][slot], ((it >> 1) & 1) ^ 1, abort_flag);
+            ok = mbar_wait_relaxed(&sm.q_empty[t][slot], ((it / kQBufs) & 1) ^ 1, abort_flag);
             if (!ok) break;
             mbar_arrive_expect_tx(&sm.q_full[t][slot], kTileBytes);
             tma_load_4d(sm.q[t][slot], &tm_q, &sm.q_full[t][slot], 0, w.q_row0 + t * kTileRows, w.h, w.b);
@@ -632,8 +803,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           // that was issued, so that none writes into shared memory after the CTA has gone.
           uint32_t no_abort = 0;
           for (int t = 0; t < 2; ++t)
-            for (int i = (q_count[t] > 2 ? q_count[t] - 2 : 0); i < q_count[t]; ++i)
-              mbar_wait_relaxed(&sm.q_full[t][i & 1], (i >> 1) & 1, &no_abort);
+            for (int i = (q_count[t] > kQBufs ? q_count[t] - kQBufs : 0); i < q_count[t]; ++i)
+              mbar_wait_relaxed(&sm.q_full[t][i % kQBufs], (i / kQBufs) & 1, &no_abort);
           for (int j = (gk > kStagesK ? gk - kStagesK : 0); j < gk; ++j)
             mbar_wait_relaxed(&sm.k_full[j % kStagesK], (j / kStagesK) & 1, &no_abort);
           for (int j = (gv > kStagesV ? gv - kStagesV : 0); j < gv; ++j)
@@ -733,14 +904,24 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         const Pos start = {0, 0, ja0, my_items == 1 ? jb_last : kv_tiles, 0, 0u};
         static_assert(kStagesK == kStagesV, "one ring position serves both rings");
 
+        [[maybe_unused]] const uint32_t rel_fmt = (p.bias.dtype == 0 ? UMMA_F16 : UMMA_BF16) * ((1u << 7) | (1u << 10));
+        [[maybe_unused]] uint64_t r_desc0 = 0, e_desc0 = 0;
+        if constexpr (BIAS == kBiasDecomposedMma) {
+          r_desc0 = umma_smem_desc_sw128(smem_u32(sm.r[t][0]), 1024, 16);
+          e_desc0 = umma_smem_desc_sw128(smem_u32(sm.e[0]), 1024, 16);
+        }
+
         // S_t(gs) = Q_t K^T. The last key tile of an item only computes the columns that hold keys.
         auto issue_qk = [&](const Pos& x) -> bool {
-          const int slot = x.it & 1;
+          const int slot = x.it % kQBufs;
           // The K tile landed long ago as a rule: its test is issued first and runs behind the wait that does wait.
           const bool k_early = mbar_test_wait(&sm.k_full[x.st], x.ph);
-          if (is_first(x) && !warp_wait(&sm.q_full[t][slot], (x.it >> 1) & 1)) return false;
+          if (is_first(x) && !warp_wait(&sm.q_full[t][slot], (x.it / kQBufs) & 1)) return false;
           if (x.gs > 0 && !warp_wait(s_free, (x.gs - 1) & 1)) return false;  // S_t has been read
           if (!__all_sync(0xffffffffu, k_early || mbar_wait(&sm.k_full[x.st], x.ph, abort_flag))) return false;
+          if constexpr (BIAS == kBiasDecomposedMma) {
+            if (is_first(x) && !warp_wait(&sm.r_full[t], x.it & 1)) return false;
+          }
           tc_fence_after_sync();
           const uint64_t a = q_desc0 + static_cast<uint64_t>(slot) * kStageStep;
           const uint64_t bd = k_desc0 + static_cast<uint64_t>(x.st) * kStageStep;
@@ -749,6 +930,14 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
 #pragma unroll
             for (int kk = 0; kk < kHeadDim / 16; ++kk)  // 32 bytes of K per step inside the swizzle atom
               umma_ss(s_tm, a + 2 * kk, bd + 2 * kk, idesc, kk > 0 ? 1u : 0u);
+            if constexpr (BIAS == kBiasDecomposedMma) {
+              const uint64_t e_desc = e_desc0 + (p.rel_steps <= 4 ? x.st * kStageStep : 0);  // two buffers of E, or one of twice the size
+              const uint32_t idesc_re = (idesc & ~((7u << 7) | (7u << 10))) | rel_fmt;  // the tables' type, else the same
+#pragma unroll
+              for (int kk = 0; kk < kMaxRelChunks / 2; ++kk)
+                if (kk < p.rel_steps)
+                  umma_ss(s_tm, r_desc0 + (kk / 4) * kStageStep + 2 * (kk % 4), e_desc + (kk / 4) * kStageStep + 2 * (kk % 4), idesc_re, 1u);
+            }
             umma_commit(s_full);
             umma_commit(&sm.k_empty[x.st]);
             if (x.it >= my_doubles) umma_commit(&sm.k_empty[x.st]);  // one-tile item: stand in for the absent second tile
@@ -1008,7 +1197,6 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           !__all_sync(0xffffffffu, stage_tested || mbar_wait(&sm.o_stage_free[t], (pend_it - 1) & 1, abort_flag)))
         return false;
       const uint32_t row = smem_u32(sm.o_stage[t]) + row_in_tile * (kHeadDim * 2);
-#pragma unroll
       const float2 inv2 = make_float2(inv, inv), zero2 = make_float2(0.f, 0.f);
 #pragma unroll
       for (int ch = 0; ch < kHeadDim / 8; ++ch) {
@@ -1049,8 +1237,42 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       if constexpr (BIAS != kBiasNone) {
         const int qr = row_valid ? q_row : 0;
         bias_row = b * p.bias.sb + h * p.bias.sh + qr * p.bias.sn;
-        if constexpr (BIAS == kBiasDecomposed || BIAS == kBiasDecomposed64 || BIAS == kBiasDecomposed14)
+        if constexpr (BIAS == kBiasDecomposed || BIAS == kBiasDecomposed64 || BIAS == kBiasDecomposed14 || BIAS == kBiasDecomposedMma)
           bias2_row = b * p.bias2.sb + h * p.bias2.sh + qr * p.bias2.sn;
+        if constexpr (BIAS == kBiasDecomposedMma) {
+          // The row's tables into R. The products that read the last item's R have finished: this thread waited for that
+          // item's last S. (Bringing the rows in from inside the item's last step, or only into L1, was 1-25 % slower.)
+          const uint32_t row = smem_u32(sm.r[t][0]) + row_in_tile * 128;
+          const uint16_t* const src_h = static_cast<const uint16_t*>(p.bias.ptr) + bias_row;
+          const uint16_t* const src_w = static_cast<const uint16_t*>(p.bias2.ptr) + bias2_row;
+          const int chunks = 2 * p.rel_steps;
+          const bool is_half = p.bias.dtype == 0;
+          auto stage_row = [&](auto align_tag) {
+#pragma unroll 1
+            for (int first = 0; first < chunks; first += 8) {
+              uint4 v[8];
+#pragma unroll
+              for (int u = 0; u < 8; ++u) {  // all loads in flight together
+                const int ch = first + u, ch_w = ch - p.rel_chunks_h;
+                const bool in_h = ch_w < 0;
+                v[u] = load_rel_chunk<decltype(align_tag)::value>(in_h ? src_h + 8 * ch : src_w + 8 * ch_w,
+                                                                  in_h ? p.rel_kh - 8 * ch : ch_w < p.rel_chunks_w ? p.rel_kw - 8 * ch_w : 0);
+              }
+#pragma unroll
+              for (int u = 0; u < 8; ++u) {
+                if (first + u >= chunks) break;
+                // an infinity would meet zeros in E: it goes in as the largest finite value
+                st_shared_v4(row + (first >> 3) * kTileBytes + ((u ^ (row_in_tile & 7)) << 4),
+                             make_uint4(clamp_finite2(v[u].x, is_half), clamp_finite2(v[u].y, is_half), clamp_finite2(v[u].z, is_half), clamp_finite2(v[u].w, is_half)));
+              }
+            }
+          };
+          if (p.rel_align == 16) stage_row(std::integral_constant<int, 16>{});
+          else if (p.rel_align == 4) stage_row(std::integral_constant<int, 4>{});
+          else stage_row(std::integral_constant<int, 2>{});
+          fence_proxy_async_smem();
+          warp_arrive(&sm.r_full[t], lane);
+        }
         if constexpr (BIAS == kBiasDecomposed14) {
           // This thread's rows, read back by this thread only: no synchronisation needed.
           float* stage = sm.rel_stage[t][row_in_tile];
@@ -1324,7 +1546,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           mx0 = max3(mx0, s[124], s[125]);  // 12 + 8 * 14 = 124: four columns left
           mx1 = max3(mx1, s[126], s[127]);
           m_tile = fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3));
-          if constexpr (BIAS == kBiasNone) m_tile *= c;
+          if constexpr (kPlainLogits) m_tile *= c;
           if constexpr (BIAS == kBiasDenseTiles) m_tile *= kLog2e;  // natural units -> base-2 units
         }
 
@@ -1360,7 +1582,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           }
         }
         float2 l2a = make_float2(0.f, 0.f), l2b = make_float2(0.f, 0.f);
-        const float2 c2 = (BIAS == kBiasNone)           ? make_float2(c, c)
+        const float2 c2 = kPlainLogits                  ? make_float2(c, c)
                           : (BIAS == kBiasDecomposed64 || BIAS == kBiasDenseTiles) ? make_float2(kLog2e, kLog2e)
                                                         : make_float2(1.f, 1.f);
         float nm = -m_use;

@@ -225,6 +225,29 @@ bool bias_shared_by_the_batch(const B200AttnArgs* a) {
   return dense_bias_in_tiles(a) && a->batch > 1 && a->bias_stride[0] == 0;
 }
 
+// What the rows of both 16-bit tables of a decomposed bias begin on: 16, 4 or 2 bytes.
+int aligned_to(const B200AttnArgs* a) {
+  uint64_t bits = reinterpret_cast<uintptr_t>(a->rel_h) | reinterpret_cast<uintptr_t>(a->rel_w);
+  const int ext[3] = {a->batch, a->heads, a->q_tokens};
+  for (int i = 0; i < 3; ++i)
+    if (ext[i] > 1) bits |= static_cast<uint64_t>(a->rel_h_stride[i]) * 2 | static_cast<uint64_t>(a->rel_w_stride[i]) * 2;
+  return bits % 16 == 0 ? 16 : bits % 4 == 0 ? 4 : 2;
+}
+// Whether 1 / scale is a power of two that the tables' type holds as a normal number; its 16 bits in *one.
+bool inverse_is_exact(float scale, uint32_t dtype, uint32_t* one) {
+  int e = 0;
+  if (std::frexp(scale, &e) != 0.5f) return false;
+  const int exponent = 1 - e;  // scale = 2^(e - 1)
+  if (dtype == B200_ATTN_F16) {
+    if (exponent < -14 || exponent > 15) return false;
+    *one = static_cast<uint32_t>(exponent + 15) << 10;
+  } else {
+    if (exponent < -126 || exponent > 127) return false;
+    *one = static_cast<uint32_t>(exponent + 127) << 7;
+  }
+  return true;
+}
+
 int bias_elem_size(uint32_t dtype) { return dtype == B200_ATTN_F32 ? 4 : 2; }
 
 // The argument checks shared by b200_attn_fwd and b200_attn_query. Sets *bias_mode and *schedule.
@@ -445,7 +468,7 @@ template <typename T, int BIAS, bool SHORT, bool SPLIT>
 int launch(const AttnParams& planned, unsigned grid, DeviceState& dev, const CUtensorMap& mq, const CUtensorMap& mk,
            const CUtensorMap& mv, const CUtensorMap& mo, const CUtensorMap& mb, cudaStream_t stream) {
   auto kernel = attn_fwd_kernel<T, BIAS, SHORT, SPLIT>;
-  constexpr int smem = static_cast<int>(BIAS == kBiasDenseTiles ? sizeof(AttnSmemDense) : sizeof(AttnSmem)) + 1024;
+  constexpr int smem = static_cast<int>(sizeof(AttnSmemOf<BIAS>)) + 1024;
   constexpr int form = (BIAS * 2 + (std::is_same<T, __half>::value ? 0 : 1)) * 3 + (SHORT ? 1 : SPLIT ? 2 : 0);
   static_assert(form < kKernelForms, "kernel form index");
   if (!dev.opted_in[form].load(std::memory_order_acquire)) {
@@ -601,7 +624,18 @@ int b200_attn_fwd(const B200AttnArgs* a, void* stream_ptr) {
     const auto rows16 = [](const void* ptr, const int64_t s[3]) {
       return aligned16(ptr) && s[0] % 8 == 0 && s[1] % 8 == 0 && s[2] % 8 == 0;
     };
-    if (a->rel_kw == 64 && a->rel_kh % 8 == 0 && a->rel_dtype != B200_ATTN_F32 && rows16(a->rel_w, a->rel_w_stride) &&
+    // Added on the tensor cores wherever that is exact and the tables fit (kBiasDecomposedMma), but for 14 x 14, whose own
+    // form is the faster one.
+    const int chunks_h = (a->rel_kh + 7) / 8, chunks_w = (a->rel_kw + 7) / 8;
+    const int aligned = aligned_to(a);
+    if (a->rel_dtype != B200_ATTN_F32 && chunks_h + chunks_w <= kMaxRelChunks && aligned >= 2 && inverse_is_exact(a->scale, a->rel_dtype, &prm.rel_one) &&
+        !(a->rel_kh == 14 && a->rel_kw == 14)) {
+      prm.rel_chunks_h = chunks_h;
+      prm.rel_chunks_w = chunks_w;
+      prm.rel_steps = (chunks_h + chunks_w + 1) / 2;
+      prm.rel_align = aligned;
+      bias_mode = kBiasDecomposedMma;
+    } else if (a->rel_kw == 64 && a->rel_kh % 8 == 0 && a->rel_dtype != B200_ATTN_F32 && rows16(a->rel_w, a->rel_w_stride) &&
         rows16(a->rel_h, a->rel_h_stride))
       bias_mode = kBiasDecomposed64;
     else if (a->rel_kh == 14 && a->rel_kw == 14)
@@ -636,6 +670,9 @@ int b200_attn_fwd(const B200AttnArgs* a, void* stream_ptr) {
     case kBiasDecomposed14:
       return f16 ? launch_sched<__half, kBiasDecomposed14>(short_sched, prm, grid, *dev, mq, mk, mv, mo, mb, stream)
                  : launch_sched<__nv_bfloat16, kBiasDecomposed14>(short_sched, prm, grid, *dev, mq, mk, mv, mo, mb, stream);
+    case kBiasDecomposedMma:
+      return f16 ? launch_sched<__half, kBiasDecomposedMma>(short_sched, prm, grid, *dev, mq, mk, mv, mo, mb, stream)
+                 : launch_sched<__nv_bfloat16, kBiasDecomposedMma>(short_sched, prm, grid, *dev, mq, mk, mv, mo, mb, stream);
     default:
       return f16 ? launch_sched<__half, kBiasDecomposed>(short_sched, prm, grid, *dev, mq, mk, mv, mo, mb, stream)
                  : launch_sched<__nv_bfloat16, kBiasDecomposed>(short_sched, prm, grid, *dev, mq, mk, mv, mo, mb, stream);

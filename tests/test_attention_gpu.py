@@ -312,6 +312,38 @@ def test_full_size_configs_by_properties(b: int, h: int, n: int, dtype: str) -> 
     assert_close(got[:: max(1, b // 2), :, :: max(1, h // 2)].float().cpu().numpy(), ref, unit_scale=True)
 
 
+# One and two buffers of the one-hot operand (up to 64 and up to 128 values per row), rows of 16-, 4- and 2-byte alignment, one
+# key tile, as many as buffers and more, tables wider than high and the reverse, partly filled chunks of eight.
+@pytest.mark.parametrize(("hw", "nq"), [((1, 1), 3), ((6, 6), 36), ((7, 5), 35), ((16, 8), 300), ((33, 31), 130), ((32, 32), 1024), ((25, 40), 140),
+                                        ((34, 34), 257), ((63, 62), 129), ((1, 120), 64), ((120, 1), 64), ((2, 64), 128), ((64, 64), 200)])  # fmt: skip
+@pytest.mark.parametrize("rel_dtype", [torch.float16, torch.bfloat16])
+def test_decomposed_bias_as_a_product(hw: tuple[int, int], nq: int, rel_dtype: torch.dtype) -> None:
+    """The decomposed bias as a second product into the logits, over several items per CTA (batch x heads > SMs / 2)."""
+    kh, kw = hw
+    n = kh * kw
+    b, h = (3, 40) if n <= 256 else (2, 3)
+    gen = torch.Generator().manual_seed(n + nq)
+    q = torch.randn(b, h, nq, 64, generator=gen).half()
+    k, v = (torch.randn(b, h, n, 64, generator=gen).half() for _ in range(2))
+    rel_h, rel_w = (torch.randn(b, h, nq, side, generator=gen).to(rel_dtype) for side in hw)
+    got = ff.scaled_dot_product_attention(q.cuda(), k.cuda(), v.cuda(), rel=(rel_h.cuda(), rel_w.cuda()))
+    ref = c_oracle.attention(*(t.float().numpy() for t in (q, k, v)), 0.125, rel=(rel_h.float().numpy(), rel_w.float().numpy()), threads=8)
+    assert_close(got.float().cpu().numpy(), ref, unit_scale=True, what=f"{hw} {rel_dtype}")
+
+
+def test_decomposed_bias_masks_and_other_scales() -> None:
+    """-inf in a table (the largest finite value takes its place in the product) masks a grid row, and a scale whose inverse
+    is no power of two goes through the softmax warps' own addition."""
+    gen = torch.Generator().manual_seed(8)
+    q, k, v = (torch.randn(1, 2, 400, 64, generator=gen).half() for _ in range(3))
+    rel_h, rel_w = (torch.randn(1, 2, 400, 20, generator=gen).half() for _ in range(2))
+    rel_h[:, 0, :, 7] = float("-inf")
+    for scale in (0.125, 0.1):
+        got = ff.scaled_dot_product_attention(q.cuda(), k.cuda(), v.cuda(), rel=(rel_h.cuda(), rel_w.cuda()), scale=scale)
+        ref = c_oracle.attention(*(t.float().numpy() for t in (q, k, v)), scale, rel=(rel_h.float().numpy(), rel_w.float().numpy()), threads=8)
+        assert_close(got.float().cpu().numpy(), ref, unit_scale=True, what=f"scale {scale}")
+
+
 def oracle_of_heads(qkv: torch.Tensor, picks: list[tuple[int, int]], scale: float, rel: tuple | None = None) -> np.ndarray:
     """Oracle output `[len(picks), N, 64]` for the chosen (batch, head) pairs of a packed `[B, N, 3, H, 64]` tensor,
     one head at a time (a dense 4096 x 4096 bias is 64 MB per head)."""
