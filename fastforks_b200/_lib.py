@@ -254,8 +254,9 @@ def source_hash() -> str:
 _HASH_IN_BINARY = re.compile(rb"b200attn-src:([0-9a-f]{16})")
 
 
-def built_hash(binary: Path = SHARED_OBJECT) -> str | None:
-    """The source digest compiled into a binary on disk (read from the file, without loading it), or None."""
+def built_hash(binary: Path | None = None) -> str | None:
+    """The source digest compiled into a binary on disk (default: the library; read from the file, without loading it), or None."""
+    binary = SHARED_OBJECT if binary is None else binary
     if not binary.exists():
         return None
     found = _HASH_IN_BINARY.search(binary.read_bytes())
