@@ -117,6 +117,10 @@ struct AttnParams {
   // Dealt mode: the last `conv_pairs` two-tile items (those a last, partial round of the grid would hold) are worked on
   // as 2 * conv_pairs one-tile items instead, numbered in front of the other one-tile items; `kept_pairs` stay whole.
   int conv_pairs, kept_pairs;
+  // Dealt mode: the last `twins` two-tile items hold one-tile remainders of two different heads (twin k: remainders k and
+  // k + twins), numbered from `first_twin` on; the one-tile items are the remainders behind them. Each tile of a twin
+  // has K and V tiles of its own. Never together with conv_pairs.
+  int twins, first_twin;
   int kv_tiles;
   float scale_log2;    // scale * log2(e)
   void* o;
@@ -154,6 +158,7 @@ struct CtaWork {
   int first_item, ja0, jb_last, last_parts;
   int first_back, first_fwd;  // CTAs before / after this one that hold other parts of its first item (ja0 > 0)
   int steps_all, steps_pairs;  // key-tile steps of all items and of the two-tile items
+  int twin_item;               // the list's first twin (pairs: none); the two-tile items from it on are twins
 };
 
 enum : int { kRoomRelStage = 0, kRoomBiasTiles = 1, kRoomRelMma = 2 };
@@ -385,9 +390,11 @@ __device__ __forceinline__ void add_rel14(float* s, const float* stage, float c)
 static_assert(sizeof(AttnSmem) + 1024 <= 227 * 1024 && sizeof(AttnSmemDense) + 1024 <= 227 * 1024 && sizeof(AttnSmemRelMma) + 1024 <= 227 * 1024,
               "shared memory of one CTA");
 
-// One unit of work: one or two 128-row query tiles of one (batch, head) over the key tiles [ja, jb).
+// One unit of work: one or two 128-row query tiles over the key tiles [ja, jb), as one of its tiles sees it.
 struct WorkItem {
-  int b, h, q_row0, n_tiles;
+  int b, h, q_row;  // of the tile that was asked for
+  int n_tiles;
+  bool twin;        // the two tiles belong to different heads: each walks K and V tiles of its own
   int ja, jb;  // key tiles of this CTA's part
   int kind;    // kItemWhole, kItemPartial (leaves its result in the workspace) or kItemOwner (merges the later parts)
 };
@@ -442,6 +449,7 @@ __host__ __device__ __forceinline__ CtaWork cta_work(const AttnParams& p, int ct
       while (cta + 1 + cw.first_fwd < grid && chunk_bound(p, cta + 1 + cw.first_fwd, grid) < item_end) ++cw.first_fwd;
     }
     cw.pair_start = cw.pair_stride = cw.single_start = cw.single_stride = 0;
+    cw.twin_item = cw.pairs;
     return cw;
   }
   cw.pair_start = cta;
@@ -465,33 +473,44 @@ __host__ __device__ __forceinline__ CtaWork cta_work(const AttnParams& p, int ct
   cw.last_parts = cw.first_back = cw.first_fwd = 0;
   cw.steps_all = (cw.pairs + cw.singles) * p.kv_tiles;
   cw.steps_pairs = cw.pairs * p.kv_tiles;
+  cw.twin_item = cw.pairs;
+  if (p.twins > 0) {
+    const int before = p.first_twin > cta ? (p.first_twin - cta + grid - 1) / grid : 0;  // items cta, cta + grid, ... below first_twin
+    if (before < cw.pairs) cw.twin_item = before;
+  }
   return cw;
 }
 
-// The it-th item of a CTA's list. SPLIT: the kernel form for key-split mode (the other form never meets a part
-// of an item: every item is whole and its key range a constant, and the code for parts is not even compiled).
-template <bool SPLIT>
-__host__ __device__ __forceinline__ WorkItem decode_item(const AttnParams& p, const CtaWork& cw, int it) {
+// What a kernel form's lists may hold, besides whole items: nothing, twins, or (key-split mode) parts of items. The code for
+// the others is not even compiled: with the twins' rules in it the common form lost 1 % on long and 8 % on short sequences.
+enum ListForm { kListPlain = 0, kListTwins = 1, kListSplit = 2 };
+
+// The it-th item of a CTA's list, seen from its tile t.
+template <int LISTS>
+__host__ __device__ __forceinline__ WorkItem decode_item(const AttnParams& p, const CtaWork& cw, int it, int t) {
+  constexpr bool SPLIT = LISTS == kListSplit;
   WorkItem w;
   int bh;
-  const bool pair = it < cw.pairs;
-  if (pair) {
+  w.twin = LISTS == kListTwins && it >= cw.twin_item && it < cw.pairs;
+  if (it < cw.pairs && !w.twin) {
     const int id = SPLIT ? cw.first_item + it : cw.pair_start + it * cw.pair_stride;
     bh = fast_div(id, p.magic_pairs);
-    w.q_row0 = (id - bh * p.pairs_per_head) * 2 * kTileRows;
+    w.q_row = ((id - bh * p.pairs_per_head) * 2 + t) * kTileRows;
     w.n_tiles = 2;
   } else {
     int id = SPLIT ? cw.first_item + it - p.pair_items : cw.single_start + (it - cw.pairs) * cw.single_stride;
-    if (!SPLIT && id < 2 * p.conv_pairs) {  // one half of a two-tile item that is worked on as two one-tile items
+    if (w.twin) id = cw.pair_start + it * cw.pair_stride - p.first_twin + t * p.twins;
+    w.n_tiles = w.twin ? 2 : 1;
+    if (LISTS == kListPlain && id < 2 * p.conv_pairs) {  // one half of a two-tile item that is worked on as two one-tile items
       const int pair = p.kept_pairs + (id >> 1);
       bh = fast_div(pair, p.magic_pairs);
-      w.q_row0 = (2 * (pair - bh * p.pairs_per_head) + (id & 1)) * kTileRows;
+      w.q_row = (2 * (pair - bh * p.pairs_per_head) + (id & 1)) * kTileRows;
     } else {
-      if (!SPLIT) id -= 2 * p.conv_pairs;
+      if (LISTS == kListPlain) id -= 2 * p.conv_pairs;
+      if (LISTS == kListTwins && !w.twin) id += 2 * p.twins;
       bh = fast_div(id, p.magic_singles);
-      w.q_row0 = (2 * p.pairs_per_head + (id - bh * p.singles_per_head)) * kTileRows;
+      w.q_row = (2 * p.pairs_per_head + (id - bh * p.singles_per_head)) * kTileRows;
     }
-    w.n_tiles = 1;
   }
   // `bh` numbers the (batch, head) pairs head-fastest as a rule: neighbouring CTAs then work on one image's heads.
   // With a dense bias that all images share it is batch-fastest (magic_heads then belongs to the batch size): the
@@ -511,6 +530,40 @@ __host__ __device__ __forceinline__ WorkItem decode_item(const AttnParams& p, co
   }
   return w;
 }
+
+// The second tile of an item whose tiles belong to one head.
+__host__ __device__ __forceinline__ WorkItem second_tile(WorkItem w) {
+  w.q_row += kTileRows;
+  return w;
+}
+
+// Where a role stands in the K or V ring of RING stages: the stage of its next key-tile step and the parity of that use.
+// A barrier's parity tells only neighbouring phases apart, so a role that waits for a use of a stage must have waited for
+// every use before it. Hence, in lists with twins:
+//   * two-tile items, whose tiles share K and V, go round the ring;
+//   * in a twin, tile t keeps to stage t (its next K tile is loaded while the softmax works on this one);
+//   * one-tile items behind twins use the stages that only tile 0 has used since: the first and the third, if there is one.
+// (Going round the ring with the tiles of a twin taking alternate stages let a tile take an old phase of a stage for the one
+// it waited for.)
+template <int RING, bool TWINS>
+struct RingPos {
+  int stage = 0;
+  uint32_t phase = 0;  // parity of the next use: of every stage (a bit each) with twins, else of the stages from `stage` on
+  __device__ __forceinline__ uint32_t parity() const { return TWINS ? (phase >> stage) & 1 : phase; }
+  __device__ __forceinline__ uint32_t last_parity(int s) const {  // of the last use of stage s; 1, which is always complete, before the first
+    return TWINS ? ((phase >> s) & 1) ^ 1 : s < stage ? phase : phase ^ 1;
+  }
+  __device__ __forceinline__ void advance(bool twin, bool behind_twins) {
+    if constexpr (TWINS) {
+      phase ^= 1u << stage;
+      if (behind_twins) stage = RING == 3 ? stage ^ 2 : 0;
+      else if (!twin) stage = stage + 1 == RING ? 0 : stage + 1;
+    } else if (++stage == RING) {
+      stage = 0;
+      phase ^= 1;
+    }
+  }
+};
 
 // Workspace slot of part `part` of a cut item whose first part belongs to CTA `first_cta`: that CTA's last-item
 // slot for part 0, the first-item slot of CTA first_cta + part otherwise.
@@ -572,11 +625,12 @@ __device__ __forceinline__ void merge_parts_to_output(float* ws_partial, T* out_
 // Persistent kernel: every CTA works through its own list of items (cta_work). All barrier phases and ring
 // positions are running counters, so the loader prefetches the next item's Q / K / V while the current one is
 // still being computed and tensor memory and barriers are set up once per CTA.
-template <typename T, int BIAS, bool SHORT, bool SPLIT>
+template <typename T, int BIAS, bool SHORT, int LISTS>
 __global__ void __launch_bounds__(kThreads, 1)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                 const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_o,
                 const __grid_constant__ CUtensorMap tm_bias, const AttnParams p) {
+  constexpr bool SPLIT = LISTS == kListSplit, TWINS = LISTS == kListTwins;
   extern __shared__ uint8_t smem_raw[];
   using Smem = AttnSmemOf<BIAS>;
   constexpr int kStagesK = Smem::kRing, kStagesV = Smem::kRing, kQBufs = Smem::kQBufs;
@@ -656,55 +710,65 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         // a row has up to 64 values, one of twice the size above. A lane moves the two ones of four keys. (By the MMA warp
         // of one query tile, between its products, the same 500 clocks held up the other tile too: +40 %.)
         bool ok = true;
-        int gk = 0, gv = 0;
+        RingPos<kStagesK, TWINS> kr, vr;  // the next K and V tile
+        int last_k = -1;
         int q_count[2] = {0, 0};
+        uint32_t e_written = 0;
+        const bool has_twins = TWINS && cw.twin_item < cw.pairs;
         const int e_bufs = p.rel_steps <= 4 ? 2 : 1;
-        const bool e_constant = !SPLIT && kv_tiles <= e_bufs;  // every use of a buffer has the same E: it is written once
+        const bool e_constant = !SPLIT && (kv_tiles == 1 || (!TWINS && kv_tiles <= e_bufs));  // every use of a buffer has the same E: it is written once
         int e_y[4], e_x[4];  // coordinates of this lane's keys
         const int e_dy = fast_div(kTileRows, p.magic_rel_kw), e_dx = kTileRows - e_dy * p.rel_kw;
-        // byte offsets of this lane's ones (inside its rows) in the tile before last and in the last one; at first those of
-        // places that hold a zero
-        uint32_t hot_old[4][2] = {}, hot[4][2] = {};
+        // byte offsets of this lane's ones (inside its rows) in either buffer; at first those of places that hold a zero
+        uint32_t hot0[4][2] = {}, hot1[4][2] = {};
         const auto warp_wait = [&](uint64_t* bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait_relaxed(bar, parity, abort_flag)) != 0; };
         for (int it = 0; it < my_items && ok; ++it) {
-          const WorkItem w = decode_item<SPLIT>(p, cw, it);
+          const WorkItem w = decode_item<LISTS>(p, cw, it, 0), w1 = TWINS ? decode_item<LISTS>(p, cw, it, 1) : second_tile(w);
           for (int t = 0; t < w.n_tiles && ok; ++t) {
             ok = warp_wait(&sm.q_empty[t][it % kQBufs], ((it / kQBufs) & 1) ^ 1);
             if (!ok) break;
             if (lane == 0) {
               mbar_arrive_expect_tx(&sm.q_full[t][it % kQBufs], kTileBytes);
-              tma_load_4d(sm.q[t][it % kQBufs], &tm_q, &sm.q_full[t][it % kQBufs], 0, w.q_row0 + t * kTileRows, w.h, w.b);
+              tma_load_4d(sm.q[t][it % kQBufs], &tm_q, &sm.q_full[t][it % kQBufs], 0, t == 0 ? w.q_row : w1.q_row, t == 0 ? w.h : w1.h, t == 0 ? w.b : w1.b);
             }
             q_count[t] = it + 1;
           }
           const int steps = w.jb - w.ja;
-          for (int i = 0; i < steps + kKLead && ok; ++i) {
+          const int streams = w.twin ? 2 : 1;  // K and V tiles per step: one for both query tiles, or one each
+          const bool behind = has_twins && it >= cw.pairs;
+          if (has_twins && it == cw.pairs) kr.stage = vr.stage = 0;
+          for (int n = 0; n < (steps + kKLead) * streams && ok; ++n) {
+            const int i = w.twin ? n >> 1 : n;
+            const bool second = w.twin && (n & 1) != 0;
+            const int h = second ? w1.h : w.h, b = second ? w1.b : w.b;
             if (i < steps) {
-              const int st = gk % kStagesK;
-              ok = warp_wait(&sm.k_empty[st], ((gk / kStagesK) & 1) ^ 1);
+              if (w.twin) kr.stage = second ? 1 : 0;
+              ok = warp_wait(&sm.k_empty[kr.stage], kr.parity() ^ 1);
               if (!ok) break;
               if (lane == 0) {
-                mbar_arrive_expect_tx(&sm.k_full[st], kTileBytes);
-                tma_load_4d(sm.k[st], &tm_k, &sm.k_full[st], 0, (w.ja + i) * kTileRows, w.h, w.b);
+                mbar_arrive_expect_tx(&sm.k_full[kr.stage], kTileBytes);
+                tma_load_4d(sm.k[kr.stage], &tm_k, &sm.k_full[kr.stage], 0, (w.ja + i) * kTileRows, h, b);
               }
-              ++gk;
             }
             const int iv = i - kKLead;
             if (iv >= 0) {
-              const int st = gv % kStagesV;
-              ok = warp_wait(&sm.v_empty[st], ((gv / kStagesV) & 1) ^ 1);
-              if (ok && lane == 0) {
-                mbar_arrive_expect_tx(&sm.v_full[st], kTileBytes);
-                tma_load_4d(sm.v[st], &tm_v, &sm.v_full[st], 0, (w.ja + iv) * kTileRows, w.h, w.b);
+              if (w.twin) vr.stage = second ? 1 : 0;
+              ok = warp_wait(&sm.v_empty[vr.stage], vr.parity() ^ 1);
+              if (ok) {
+                if (lane == 0) {
+                  mbar_arrive_expect_tx(&sm.v_full[vr.stage], kTileBytes);
+                  tma_load_4d(sm.v[vr.stage], &tm_v, &sm.v_full[vr.stage], 0, (w.ja + iv) * kTileRows, h, b);
+                }
+                vr.advance(w.twin, behind);
               }
-              gv += ok ? 1 : 0;
             }
             if (i < steps) {
-              const int n = gk - 1, st = n % kStagesK;  // the tile whose E is due
-              if (ok && !(e_constant && n >= e_bufs)) {
+              const int st = kr.stage, buf = e_bufs == 2 ? st : 0;  // the tile whose E is due
+              if (ok && !(e_constant && ((e_written >> buf) & 1) != 0)) {
                 // with one buffer the products of the tile before must have read it
-                if (e_bufs == 1 && n > 0) ok = warp_wait(&sm.k_empty[(n - 1) % kStagesK], ((n - 1) / kStagesK) & 1);
-                const uint32_t e = smem_u32(sm.e[e_bufs == 2 ? st : 0]) + lane * 128, swizzle = (lane & 7) << 4;
+                if (e_bufs == 1 && last_k >= 0 && last_k != st) ok = warp_wait(&sm.k_empty[last_k], kr.last_parity(last_k));
+                e_written |= 1u << buf;
+                const uint32_t e = smem_u32(sm.e[buf]) + lane * 128, swizzle = (lane & 7) << 4;
                 if (i == 0) {
 #pragma unroll
                   for (int r = 0; r < 4; ++r) {
@@ -712,7 +776,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
                     e_y[r] = fast_div(key, p.magic_rel_kw);
                     e_x[r] = key - e_y[r] * p.rel_kw;
                   }
-                } else {  // a tile on: 128 keys
+                } else if (!second) {  // a tile on: 128 keys
 #pragma unroll
                   for (int r = 0; r < 4; ++r) {
                     e_y[r] += e_dy;
@@ -734,18 +798,20 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
 #pragma unroll
                 for (int r = 0; r < 4; ++r)
 #pragma unroll
-                  for (int k = 0; k < 2; ++k) st_shared_u16(e + r * 32 * 128 + (e_bufs == 2 ? hot_old[r][k] : hot[r][k]), 0);
+                  for (int k = 0; k < 2; ++k) st_shared_u16(e + r * 32 * 128 + (buf == 0 ? hot0[r][k] : hot1[r][k]), 0);
 #pragma unroll
                 for (int r = 0; r < 4; ++r)
 #pragma unroll
                   for (int k = 0; k < 2; ++k) {
                     st_shared_u16(e + r * 32 * 128 + at[r][k], static_cast<uint16_t>(p.rel_one));
-                    hot_old[r][k] = hot[r][k];
-                    hot[r][k] = at[r][k];
+                    hot0[r][k] = buf == 0 ? at[r][k] : hot0[r][k];
+                    hot1[r][k] = buf == 0 ? hot1[r][k] : at[r][k];
                   }
                 fence_proxy_async_smem();
               }
               warp_arrive(&sm.k_full[st], lane);  // on the abort path too: the copy's barrier must complete
+              last_k = st;
+              kr.advance(w.twin, behind);
             }
           }
         }
@@ -757,41 +823,51 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           for (int t = 0; t < 2; ++t)
             for (int i = (q_count[t] > kQBufs ? q_count[t] - kQBufs : 0); i < q_count[t]; ++i)
               mbar_wait_relaxed(&sm.q_full[t][i % kQBufs], (i / kQBufs) & 1, &no_abort);
-          for (int j = (gk > kStagesK ? gk - kStagesK : 0); j < gk; ++j) mbar_wait_relaxed(&sm.k_full[j % kStagesK], (j / kStagesK) & 1, &no_abort);
-          for (int j = (gv > kStagesV ? gv - kStagesV : 0); j < gv; ++j) mbar_wait_relaxed(&sm.v_full[j % kStagesV], (j / kStagesV) & 1, &no_abort);
+          for (int i = 0; i < kStagesK; ++i) {
+            mbar_wait_relaxed(&sm.k_full[i], kr.last_parity(i), &no_abort);
+            mbar_wait_relaxed(&sm.v_full[i], vr.last_parity(i), &no_abort);
+          }
         }
       } else if (lane == 0) {
         bool ok = true;
-        int gk = 0, gv = 0;        // K / V tiles issued so far (ring position and phase)
+        RingPos<kStagesK, TWINS> kr, vr;  // the next K and V tile
+        const bool has_twins = TWINS && cw.twin_item < cw.pairs;
         int q_count[2] = {0, 0};   // Q tiles issued so far per query-tile slot
         for (int it = 0; it < my_items && ok; ++it) {
-          const WorkItem w = decode_item<SPLIT>(p, cw, it);
+          const WorkItem w = decode_item<LISTS>(p, cw, it, 0), w1 = TWINS ? decode_item<LISTS>(p, cw, it, 1) : second_tile(w);
           const int slot = it % kQBufs;
           for (int t = 0; t < w.n_tiles && ok; ++t) {
             ok = mbar_wait_relaxed(&sm.q_empty[t][slot], ((it / kQBufs) & 1) ^ 1, abort_flag);
             if (!ok) break;
             mbar_arrive_expect_tx(&sm.q_full[t][slot], kTileBytes);
-            tma_load_4d(sm.q[t][slot], &tm_q, &sm.q_full[t][slot], 0, w.q_row0 + t * kTileRows, w.h, w.b);
+            tma_load_4d(sm.q[t][slot], &tm_q, &sm.q_full[t][slot], 0, t == 0 ? w.q_row : w1.q_row, t == 0 ? w.h : w1.h, t == 0 ? w.b : w1.b);
             q_count[t] = it + 1;
           }
           const int steps = w.jb - w.ja;  // the key tiles of this CTA's part of the item
-          for (int i = 0; i < steps + kKLead && ok; ++i) {
+          // A twin takes two K and two V tiles per step, and K runs one step ahead instead of as far as the ring allows.
+          const int lead = w.twin ? 1 : kKLead, shift = w.twin ? 1 : 0;
+          const bool behind = has_twins && it >= cw.pairs;
+          if (has_twins && it == cw.pairs) kr.stage = vr.stage = 0;
+          for (int n = 0; n < (steps + lead) << shift && ok; ++n) {
+            const int i = n >> shift;
+            const bool second = (n & shift) != 0;
+            const int h = second ? w1.h : w.h, b = second ? w1.b : w.b;
             if (i < steps) {
-              const int st = gk % kStagesK;
-              ok = mbar_wait_relaxed(&sm.k_empty[st], ((gk / kStagesK) & 1) ^ 1, abort_flag);
+              if (w.twin) kr.stage = second ? 1 : 0;
+              ok = mbar_wait_relaxed(&sm.k_empty[kr.stage], kr.parity() ^ 1, abort_flag);
               if (!ok) break;
-              mbar_arrive_expect_tx(&sm.k_full[st], kTileBytes);
-              tma_load_4d(sm.k[st], &tm_k, &sm.k_full[st], 0, (w.ja + i) * kTileRows, w.h, w.b);
-              ++gk;
+              mbar_arrive_expect_tx(&sm.k_full[kr.stage], kTileBytes);
+              tma_load_4d(sm.k[kr.stage], &tm_k, &sm.k_full[kr.stage], 0, (w.ja + i) * kTileRows, h, b);
+              kr.advance(w.twin, behind);
             }
-            const int iv = i - kKLead;
+            const int iv = i - lead;
             if (iv >= 0) {
-              const int st = gv % kStagesV;
-              ok = mbar_wait_relaxed(&sm.v_empty[st], ((gv / kStagesV) & 1) ^ 1, abort_flag);
+              if (w.twin) vr.stage = second ? 1 : 0;
+              ok = mbar_wait_relaxed(&sm.v_empty[vr.stage], vr.parity() ^ 1, abort_flag);
               if (!ok) break;
-              mbar_arrive_expect_tx(&sm.v_full[st], kTileBytes);
-              tma_load_4d(sm.v[st], &tm_v, &sm.v_full[st], 0, (w.ja + iv) * kTileRows, w.h, w.b);
-              ++gv;
+              mbar_arrive_expect_tx(&sm.v_full[vr.stage], kTileBytes);
+              tma_load_4d(sm.v[vr.stage], &tm_v, &sm.v_full[vr.stage], 0, (w.ja + iv) * kTileRows, h, b);
+              vr.advance(w.twin, behind);
             }
           }
         }
@@ -805,10 +881,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           for (int t = 0; t < 2; ++t)
             for (int i = (q_count[t] > kQBufs ? q_count[t] - kQBufs : 0); i < q_count[t]; ++i)
               mbar_wait_relaxed(&sm.q_full[t][i % kQBufs], (i / kQBufs) & 1, &no_abort);
-          for (int j = (gk > kStagesK ? gk - kStagesK : 0); j < gk; ++j)
-            mbar_wait_relaxed(&sm.k_full[j % kStagesK], (j / kStagesK) & 1, &no_abort);
-          for (int j = (gv > kStagesV ? gv - kStagesV : 0); j < gv; ++j)
-            mbar_wait_relaxed(&sm.v_full[j % kStagesV], (j / kStagesV) & 1, &no_abort);
+          for (int i = 0; i < kStagesK; ++i) {
+            mbar_wait_relaxed(&sm.k_full[i], kr.last_parity(i), &no_abort);
+            mbar_wait_relaxed(&sm.v_full[i], vr.last_parity(i), &no_abort);
+          }
         }
       }
       if constexpr (BIAS == kBiasDenseTiles) {
@@ -820,15 +896,16 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           bool ok = true;
           int gb[2] = {0, 0};  // bias tiles issued so far per query-tile slot
           for (int it = 0; it < my_items && ok; ++it) {
-            const WorkItem w = decode_item<SPLIT>(p, cw, it);
-            for (int j = w.ja; j < w.jb && ok; ++j) {
-              for (int t = 0; t < w.n_tiles && ok; ++t) {
+            const WorkItem w0 = decode_item<LISTS>(p, cw, it, 0), w1 = TWINS ? decode_item<LISTS>(p, cw, it, 1) : second_tile(w0);
+            for (int j = w0.ja; j < w0.jb && ok; ++j) {
+              for (int t = 0; t < w0.n_tiles && ok; ++t) {
+                const WorkItem& w = t == 0 ? w0 : w1;
                 ok = mbar_wait_relaxed(&sm.bias_free[t], (gb[t] & 1) ^ 1, abort_flag);
                 if (!ok) break;
                 mbar_arrive_expect_tx(&sm.bias_full[t], 2 * kTileBytes);
                 const int bz = p.bias.sh != 0 ? w.h : 0, bw = p.bias.sb != 0 ? w.b : 0;  // a stride of 0 broadcasts
-                tma_load_4d(sm.bias_tile[t][0], &tm_bias, &sm.bias_full[t], j * kTileRows, w.q_row0 + t * kTileRows, bz, bw);
-                tma_load_4d(sm.bias_tile[t][1], &tm_bias, &sm.bias_full[t], j * kTileRows + 64, w.q_row0 + t * kTileRows, bz, bw);
+                tma_load_4d(sm.bias_tile[t][0], &tm_bias, &sm.bias_full[t], j * kTileRows, w.q_row, bz, bw);
+                tma_load_4d(sm.bias_tile[t][1], &tm_bias, &sm.bias_full[t], j * kTileRows + 64, w.q_row, bz, bw);
                 ++gb[t];
               }
             }
@@ -873,35 +950,40 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         uint64_t* const pv_done = &sm.pv_done[t];
 
         // This slot's items are a prefix of the CTA's list (two-tile items come first), so its key-tile steps form
-        // one stream gs = 0, 1, ...: step gs is key tile j of item it and uses ring tile gs (stage st, in its
-        // ph-th use). S is issued two steps ahead of its use, across item boundaries too, so that a new item starts
-        // at once. The positions are counted along: a division by kv_tiles here would queue its reciprocal behind the
-        // softmax warps' exponentials on the MUFU unit, which cost the long-sequence runs 15 %.
+        // one stream gs = 0, 1, ...: step gs is key tile j of item it. S is issued two steps ahead of its use, across
+        // item boundaries too, so that a new item starts at once. The positions are counted along: a division by kv_tiles here
+        // would queue its reciprocal behind the softmax warps' exponentials on the MUFU unit, which cost the long-sequence runs 15 %.
         const int my_doubles = cw.pairs;
         const int total_steps = t == 0 ? cw.steps_all : cw.steps_pairs;
         // `j` is the key tile and `jend` where this CTA's part of the item ends (the part starts at key tile 0
         // except, in key-split mode, for the CTA's first item).
         struct Pos {
-          int gs, it, j, jend, st;
-          uint32_t ph;
+          int gs, it, j, jend;
+          RingPos<kStagesK, TWINS> ring;
         };
         const int ja0 = SPLIT ? cw.ja0 : 0, jb_last = cw.jb_last;
         // Without key split every part is a whole item: `jend` is never read and costs no register.
         auto is_first = [&](const Pos& x) { return SPLIT ? x.j == (x.it == 0 ? ja0 : 0) : x.j == 0; };
         auto is_last = [&](const Pos& x) { return SPLIT ? x.j == x.jend - 1 : x.j == kv_tiles - 1; };
+        const int twin_item = TWINS ? cw.twin_item : my_doubles;
+        const bool has_twins = TWINS && twin_item < my_doubles;
+        // Whether nobody but this tile reads the K and V tiles of an item: it then frees them for both.
+        auto alone = [&](const Pos& x) { return x.it >= (TWINS ? twin_item : my_doubles); };
         auto advance = [&](Pos& x) {
+          x.ring.advance(TWINS && x.it >= twin_item && x.it < my_doubles, has_twins && x.it >= my_doubles);
           ++x.gs;
           if (SPLIT ? ++x.j == x.jend : ++x.j == kv_tiles) {
             x.j = 0;
             ++x.it;
             x.jend = x.it == my_items - 1 ? jb_last : kv_tiles;
-          }
-          if (++x.st == kStagesK) {
-            x.st = 0;
-            x.ph ^= 1;
+            if (has_twins) {
+              if (x.it == twin_item) x.ring.stage = t;
+              else if (x.it == my_doubles) x.ring.stage = 0;
+            }
           }
         };
-        const Pos start = {0, 0, ja0, my_items == 1 ? jb_last : kv_tiles, 0, 0u};
+        Pos start = {0, 0, ja0, my_items == 1 ? jb_last : kv_tiles, {}};
+        if (has_twins && twin_item == 0) start.ring.stage = t;
         static_assert(kStagesK == kStagesV, "one ring position serves both rings");
 
         [[maybe_unused]] const uint32_t rel_fmt = (p.bias.dtype == 0 ? UMMA_F16 : UMMA_BF16) * ((1u << 7) | (1u << 10));
@@ -915,23 +997,23 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         auto issue_qk = [&](const Pos& x) -> bool {
           const int slot = x.it % kQBufs;
           // The K tile landed long ago as a rule: its test is issued first and runs behind the wait that does wait.
-          const bool k_early = mbar_test_wait(&sm.k_full[x.st], x.ph);
+          const bool k_early = mbar_test_wait(&sm.k_full[x.ring.stage], x.ring.parity());
           if (is_first(x) && !warp_wait(&sm.q_full[t][slot], (x.it / kQBufs) & 1)) return false;
           if (x.gs > 0 && !warp_wait(s_free, (x.gs - 1) & 1)) return false;  // S_t has been read
-          if (!__all_sync(0xffffffffu, k_early || mbar_wait(&sm.k_full[x.st], x.ph, abort_flag))) return false;
+          if (!__all_sync(0xffffffffu, k_early || mbar_wait(&sm.k_full[x.ring.stage], x.ring.parity(), abort_flag))) return false;
           if constexpr (BIAS == kBiasDecomposedMma) {
             if (is_first(x) && !warp_wait(&sm.r_full[t], x.it & 1)) return false;
           }
           tc_fence_after_sync();
           const uint64_t a = q_desc0 + static_cast<uint64_t>(slot) * kStageStep;
-          const uint64_t bd = k_desc0 + static_cast<uint64_t>(x.st) * kStageStep;
+          const uint64_t bd = k_desc0 + static_cast<uint64_t>(x.ring.stage) * kStageStep;
           const uint32_t idesc = (x.j == kv_tiles - 1) ? idesc_qk_last : idesc_qk;
           if (elect_one()) {
 #pragma unroll
             for (int kk = 0; kk < kHeadDim / 16; ++kk)  // 32 bytes of K per step inside the swizzle atom
               umma_ss(s_tm, a + 2 * kk, bd + 2 * kk, idesc, kk > 0 ? 1u : 0u);
             if constexpr (BIAS == kBiasDecomposedMma) {
-              const uint64_t e_desc = e_desc0 + (p.rel_steps <= 4 ? x.st * kStageStep : 0);  // two buffers of E, or one of twice the size
+              const uint64_t e_desc = e_desc0 + (p.rel_steps <= 4 ? x.ring.stage * kStageStep : 0);  // two buffers of E, or one of twice the size
               const uint32_t idesc_re = (idesc & ~((7u << 7) | (7u << 10))) | rel_fmt;  // the tables' type, else the same
 #pragma unroll
               for (int kk = 0; kk < kMaxRelChunks / 2; ++kk)
@@ -939,21 +1021,21 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
                   umma_ss(s_tm, r_desc0 + (kk / 4) * kStageStep + 2 * (kk % 4), e_desc + (kk / 4) * kStageStep + 2 * (kk % 4), idesc_re, 1u);
             }
             umma_commit(s_full);
-            umma_commit(&sm.k_empty[x.st]);
-            if (x.it >= my_doubles) umma_commit(&sm.k_empty[x.st]);  // one-tile item: stand in for the absent second tile
+            umma_commit(&sm.k_empty[x.ring.stage]);
+            if (alone(x)) umma_commit(&sm.k_empty[x.ring.stage]);  // stand in for the other tile
             if (is_last(x)) umma_commit(&sm.q_empty[t][slot]);  // the item's last reader of Q_t
           }
           return true;
         };
         // O_t (+)= P_t(gs) V, 16 keys (two 8-row groups of the V tile) per MMA.
         auto issue_pv = [&](const Pos& x) -> bool {
-          const bool v_early = mbar_test_wait(&sm.v_full[x.st], x.ph);
+          const bool v_early = mbar_test_wait(&sm.v_full[x.ring.stage], x.ring.parity());
           if (!warp_wait(p_full, x.gs & 1)) return false;
-          if (!__all_sync(0xffffffffu, v_early || mbar_wait(&sm.v_full[x.st], x.ph, abort_flag))) return false;
+          if (!__all_sync(0xffffffffu, v_early || mbar_wait(&sm.v_full[x.ring.stage], x.ring.parity(), abort_flag))) return false;
           // The first P V of an item overwrites O_t: the previous item's epilogue must have read it.
           if (is_first(x) && x.it > 0 && !warp_wait(&sm.o_free[t], (x.it - 1) & 1)) return false;
           tc_fence_after_sync();
-          const uint64_t bd = v_desc0 + static_cast<uint64_t>(x.st) * kStageStep;
+          const uint64_t bd = v_desc0 + static_cast<uint64_t>(x.ring.stage) * kStageStep;
           if (elect_one()) {
             const int steps = x.j != kv_tiles - 1 ? kTileRows / 16 : kv_last16 / 16;  // at least one
             umma_ts(o_tm, p_tm, bd, idesc_pv, is_first(x) ? 0u : 1u);
@@ -961,8 +1043,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
             for (int kk = 1; kk < kTileRows / 16; ++kk)
               if (kk < steps) umma_ts(o_tm, p_tm + kk * 8, bd + kk * (2048 >> 4), idesc_pv, 1u);
             umma_commit(pv_done);
-            umma_commit(&sm.v_empty[x.st]);
-            if (x.it >= my_doubles) umma_commit(&sm.v_empty[x.st]);
+            umma_commit(&sm.v_empty[x.ring.stage]);
+            if (alone(x)) umma_commit(&sm.v_empty[x.ring.stage]);
           }
           return true;
         };
@@ -1006,17 +1088,18 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         if (lane == 0) {
           bool ok = true;
           for (int it = 0; it < my_items && ok; ++it) {
-            const WorkItem w = decode_item<SPLIT>(p, cw, it);
-            for (int t = 0; t < w.n_tiles && ok; ++t) {
+            const WorkItem w0 = decode_item<LISTS>(p, cw, it, 0), w1 = TWINS ? decode_item<LISTS>(p, cw, it, 1) : second_tile(w0);
+            for (int t = 0; t < w0.n_tiles && ok; ++t) {
+              const WorkItem& w = t == 0 ? w0 : w1;
               // Slot 1's items are a prefix of the CTA's list, so this is the it-th use of either slot's buffer.
               ok = mbar_wait(&sm.o_staged[t], it & 1, abort_flag);
               if (!ok) break;
-              tma_store_4d(&tm_o, sm.o_stage[t], 0, w.q_row0 + t * kTileRows, w.h, w.b);
+              tma_store_4d(&tm_o, sm.o_stage[t], 0, w.q_row, w.h, w.b);
               tma_store_commit();
             }
             // The buffers are not needed again before the next item's epilogue: one wait for both stores.
             tma_store_wait_read<0>();
-            for (int t = 0; t < w.n_tiles && ok; ++t) mbar_arrive(&sm.o_stage_free[t]);
+            for (int t = 0; t < w0.n_tiles && ok; ++t) mbar_arrive(&sm.o_stage_free[t]);
           }
           // Every store has read its buffer by now (the wait above); the writes themselves complete with the kernel.
           if (!ok) {
@@ -1027,14 +1110,14 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       } else {
         bool ok = true;
         for (int it = 0; it < my_items && ok; ++it) {
-          const WorkItem w = decode_item<SPLIT>(p, cw, it);
+          const WorkItem w = decode_item<LISTS>(p, cw, it, 0);
           for (int t = 0; t < w.n_tiles && ok; ++t) {
             uint32_t what = 1;
             if (lane == 0) {
               ok = mbar_wait(&sm.o_staged[t], it & 1, abort_flag);
               if (ok && w.kind != kItemWhole) what = *reinterpret_cast<volatile uint32_t*>(&sm.o_store[t][it & 1]);
               if (ok && what == 1) {
-                tma_store_4d(&tm_o, sm.o_stage[t], 0, w.q_row0 + t * kTileRows, w.h, w.b);
+                tma_store_4d(&tm_o, sm.o_stage[t], 0, w.q_row + t * kTileRows, w.h, w.b);
                 tma_store_commit();
               }
             }
@@ -1060,7 +1143,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
             }
             last = __shfl_sync(0xffffffffu, last, 0);
             if (last) {
-              const int row0 = w.q_row0 + t * kTileRows;
+              const int row0 = w.q_row + t * kTileRows;
               T* out_tile = static_cast<T*>(p.o) + w.b * p.o_sb + static_cast<int64_t>(row0) * p.o_sn + w.h * p.o_sh;
               merge_parts_to_output<T>(p.ws_partial, out_tile, p.o_sn, p.q_tokens - row0, t, first_cta, n_parts, lane);
             }
@@ -1219,10 +1302,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     };
 
     for (int it = 0; it < my_items && ok; ++it) {
-      const WorkItem w = decode_item<SPLIT>(p, cw, it);
+      const WorkItem w = decode_item<LISTS>(p, cw, it, t);
       if (t >= w.n_tiles) break;  // only one-tile items follow
       const int b = w.b, h = w.h;
-      const int q_row = w.q_row0 + t * kTileRows + row_in_tile;
+      const int q_row = w.q_row + row_in_tile;
       const bool row_valid = q_row < p.q_tokens;
       const bool pingpong = w.n_tiles == 2;
       const int ja = w.ja, jb = w.jb;  // this CTA's key tiles of the item

@@ -333,57 +333,64 @@ unsigned plan_split(AttnParams& prm, long long heads_total, int sms, double* spa
   double best_span = 0;
   int best_pairs = -1;
   struct Plan {
-    int grid, na, ka, kb, a, ea, b, eb, conv;
+    int grid, na, ka, kb, a, ea, b, eb, conv, twins;
   } best{}, cur{};
   const int first = tiles / 2, last = tiles / 2 - 8;
   for (int pairs = first; pairs >= 0 && pairs >= last; --pairs) {
-    const long long P = pairs * heads_total, S = (tiles - 2LL * pairs) * heads_total;
-    const long long grid = P + S < sms ? P + S : sms;
-    cur.grid = static_cast<int>(grid);
-    cur.na = static_cast<int>(P % grid);
-    cur.kb = static_cast<int>(P / grid);
-    cur.ka = cur.kb + 1;
-    if (cur.na == 0) cur.ka = cur.kb;  // no CTA of the first kind
-    // Level the loads with the one-tile items: group A (na CTAs, ka two-tile items), group B (the rest, kb).
-    const long long nb = grid - cur.na;
-    long long a = 0, b = 0, ea = 0, eb = 0, left = S;
-    while (left > 0) {
-      const double level_a = cur.na > 0 ? cur.ka + kDealtSingleCost * a : 1e300;
-      const double level_b = nb > 0 ? cur.kb + kDealtSingleCost * b : 1e300;
-      if (level_b <= level_a) {
-        if (left >= nb) { ++b; left -= nb; } else { eb = left; left = 0; }
-      } else {
-        if (left >= cur.na) { ++a; left -= cur.na; } else { ea = left; left = 0; }
+    const long long P = pairs * heads_total, S_all = (tiles - 2LL * pairs) * heads_total;
+    // The one-tile remainders alone, or two by two as twins: a twin runs at a two-tile item's pace on K and V tiles of its
+    // own, 1.0 for what two one-tile items do in 1.6 ([8,192,49,64] 36 -> 26 us).
+    for (const long long T : {0LL, S_all / 2}) {
+      const long long two = P + T, S = S_all - 2 * T;
+      const long long grid = two + S < sms ? two + S : sms;
+      cur.twins = static_cast<int>(T);
+      cur.grid = static_cast<int>(grid);
+      cur.na = static_cast<int>(two % grid);
+      cur.kb = static_cast<int>(two / grid);
+      cur.ka = cur.kb + 1;
+      if (cur.na == 0) cur.ka = cur.kb;  // no CTA of the first kind
+      // Level the loads with the one-tile items: group A (na CTAs, ka two-tile items), group B (the rest, kb).
+      const long long nb = grid - cur.na;
+      long long a = 0, b = 0, ea = 0, eb = 0, left = S;
+      while (left > 0) {
+        const double level_a = cur.na > 0 ? cur.ka + kDealtSingleCost * a : 1e300;
+        const double level_b = nb > 0 ? cur.kb + kDealtSingleCost * b : 1e300;
+        if (level_b <= level_a) {
+          if (left >= nb) { ++b; left -= nb; } else { eb = left; left = 0; }
+        } else {
+          if (left >= cur.na) { ++a; left -= cur.na; } else { ea = left; left = 0; }
+        }
       }
-    }
-    cur.a = static_cast<int>(a); cur.ea = static_cast<int>(ea); cur.b = static_cast<int>(b); cur.eb = static_cast<int>(eb);
-    double span = 0;
-    if (cur.na > 0) span = std::fmax(span, cur.ka + kDealtSingleCost * (a + (ea > 0 ? 1 : 0)));
-    if (nb > 0) span = std::fmax(span, cur.kb + kDealtSingleCost * (b + (eb > 0 ? 1 : 0)));
-    cur.conv = 0;
-    if (best_pairs < 0 || span < best_span - 1e-9) {
-      best_span = span;
-      best_pairs = pairs;
-      best = cur;
-    }
-    // The same count of two-tile items per head, but the na items of the last, partial round taken apart into 2 na
-    // one-tile items: every CTA then has kb two-tile items and the one-tile items level the rest. It pays when that
-    // round is thin (300 items on 148 CTAs: 4 of them would run a third item while 144 wait) and the lists are short
-    // (measured: -6 % at two items per CTA, -3 % at four, nothing at eight: taken from 3 % of predicted gain on).
-    if (cur.na > 0 && cur.kb > 0) {
-      const long long singles = S + 2LL * cur.na;
-      Plan alt = cur;
-      alt.conv = cur.na;
-      alt.na = 0;
-      alt.ka = cur.kb;
-      alt.a = alt.ea = 0;
-      alt.b = static_cast<int>(singles / grid);
-      alt.eb = static_cast<int>(singles % grid);
-      const double alt_span = cur.kb + kDealtSingleCost * (alt.b + (alt.eb > 0 ? 1 : 0));
-      if (alt_span < 0.97 * span && alt_span < best_span - 1e-9) {
-        best_span = alt_span;
+      cur.a = static_cast<int>(a); cur.ea = static_cast<int>(ea); cur.b = static_cast<int>(b); cur.eb = static_cast<int>(eb);
+      double span = 0;
+      if (cur.na > 0) span = std::fmax(span, cur.ka + kDealtSingleCost * (a + (ea > 0 ? 1 : 0)));
+      if (nb > 0) span = std::fmax(span, cur.kb + kDealtSingleCost * (b + (eb > 0 ? 1 : 0)));
+      cur.conv = 0;
+      if (best_pairs < 0 || span < best_span - 1e-9) {
+        best_span = span;
         best_pairs = pairs;
-        best = alt;
+        best = cur;
+      }
+      // The same, but the na two-tile items of the last, partial round taken apart into 2 na one-tile items (twins first):
+      // every CTA then has kb two-tile items and the one-tile items level the rest. It pays when that
+      // round is thin (300 items on 148 CTAs: 4 of them would run a third item while 144 wait) and the lists are short
+      // (measured: -6 % at two items per CTA, -3 % at four, nothing at eight: taken from 3 % of predicted gain on).
+      if (cur.na > 0 && cur.kb > 0) {
+        const long long singles = S + 2LL * cur.na;
+        Plan alt = cur;
+        alt.conv = cur.na > cur.twins ? cur.na - cur.twins : 0;
+        alt.twins = cur.na > cur.twins ? 0 : cur.twins - cur.na;
+        alt.na = 0;
+        alt.ka = cur.kb;
+        alt.a = alt.ea = 0;
+        alt.b = static_cast<int>(singles / grid);
+        alt.eb = static_cast<int>(singles % grid);
+        const double alt_span = cur.kb + kDealtSingleCost * (alt.b + (alt.eb > 0 ? 1 : 0));
+        if (alt_span < 0.97 * span && alt_span < best_span - 1e-9) {
+          best_span = alt_span;
+          best_pairs = pairs;
+          best = alt;
+        }
       }
     }
   }
@@ -393,6 +400,8 @@ unsigned plan_split(AttnParams& prm, long long heads_total, int sms, double* spa
   prm.split_a = best.a; prm.split_ea = best.ea; prm.split_b = best.b; prm.split_eb = best.eb;
   prm.conv_pairs = best.conv;
   prm.kept_pairs = static_cast<int>(best_pairs * heads_total) - best.conv;
+  prm.twins = best.twins;
+  prm.first_twin = static_cast<int>(best_pairs * heads_total);
   prm.magic_pairs = div_magic(prm.pairs_per_head);
   prm.magic_singles = div_magic(prm.singles_per_head);
   *span_out = best_span;
@@ -427,6 +436,7 @@ unsigned plan_chunks(AttnParams& prm, const B200AttnArgs* a, long long heads_tot
   const double chunked = kSplitStepFactor * run + 0.5 * (run / prm.kv_tiles + 1.0) + kSplitMergeSteps;
   if (chunked > 0.97 * dealt) return 0;
   prm.chunked = 1;
+  prm.twins = 0;
   prm.pairs_per_head = prm.q_tiles / 2;
   prm.singles_per_head = prm.q_tiles % 2;
   prm.magic_pairs = div_magic(prm.pairs_per_head);
@@ -464,12 +474,12 @@ unsigned plan_work(AttnParams& prm, const B200AttnArgs* a, int sms) {
   return grid;
 }
 
-template <typename T, int BIAS, bool SHORT, bool SPLIT>
+template <typename T, int BIAS, bool SHORT, int LISTS>
 int launch(const AttnParams& planned, unsigned grid, DeviceState& dev, const CUtensorMap& mq, const CUtensorMap& mk,
            const CUtensorMap& mv, const CUtensorMap& mo, const CUtensorMap& mb, cudaStream_t stream) {
-  auto kernel = attn_fwd_kernel<T, BIAS, SHORT, SPLIT>;
+  auto kernel = attn_fwd_kernel<T, BIAS, SHORT, LISTS>;
   constexpr int smem = static_cast<int>(sizeof(AttnSmemOf<BIAS>)) + 1024;
-  constexpr int form = (BIAS * 2 + (std::is_same<T, __half>::value ? 0 : 1)) * 3 + (SHORT ? 1 : SPLIT ? 2 : 0);
+  constexpr int form = ((BIAS * 2 + (std::is_same<T, __half>::value ? 0 : 1)) * 2 + (SHORT ? 1 : 0)) * 3 + LISTS;
   static_assert(form < kKernelForms, "kernel form index");
   if (!dev.opted_in[form].load(std::memory_order_acquire)) {
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
@@ -503,11 +513,14 @@ int launch(const AttnParams& planned, unsigned grid, DeviceState& dev, const CUt
 template <typename T, int BIAS>
 int launch_sched(bool short_sched, const AttnParams& planned, unsigned grid, DeviceState& dev, const CUtensorMap& mq,
                  const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mo, const CUtensorMap& mb, cudaStream_t stream) {
-  if (planned.chunked) return launch<T, BIAS, false, true>(planned, grid, dev, mq, mk, mv, mo, mb, stream);
+  if (planned.chunked) return launch<T, BIAS, false, kListSplit>(planned, grid, dev, mq, mk, mv, mo, mb, stream);
+  const bool twins = planned.twins > 0;
   if constexpr (BIAS != kBiasDecomposed64) {
-    if (short_sched) return launch<T, BIAS, true, false>(planned, grid, dev, mq, mk, mv, mo, mb, stream);
+    if (short_sched && twins) return launch<T, BIAS, true, kListTwins>(planned, grid, dev, mq, mk, mv, mo, mb, stream);
+    if (short_sched) return launch<T, BIAS, true, kListPlain>(planned, grid, dev, mq, mk, mv, mo, mb, stream);
   }
-  return launch<T, BIAS, false, false>(planned, grid, dev, mq, mk, mv, mo, mb, stream);
+  if (twins) return launch<T, BIAS, false, kListTwins>(planned, grid, dev, mq, mk, mv, mo, mb, stream);
+  return launch<T, BIAS, false, kListPlain>(planned, grid, dev, mq, mk, mv, mo, mb, stream);
 }
 
 // The dense bias [B | 1, H | 1, Nq, Nk] (a stride of 0 broadcasts that dimension) as a 4-D tensor map whose box is
@@ -709,12 +722,18 @@ int b200_attn_plan(const B200AttnArgs* a, int32_t sms, int32_t cta, int32_t* gri
   if (cta < 0 || cta >= grid) return fail(B200_ATTN_BAD_CONFIG, "b200_attn_plan: cta %d outside the grid of %d", cta, grid);
   const CtaWork cw = cta_work(prm, cta, grid);
   const int n = cw.pairs + cw.singles;
-  *n_items_out = n;
+  *n_items_out = n + (cw.pairs - cw.twin_item);  // a twin is listed as its two one-tile items
   *later_parts_out = cw.last_parts;
-  for (int it = 0; it < n && it < max_items; ++it) {
-    const WorkItem w = prm.chunked ? decode_item<true>(prm, cw, it) : decode_item<false>(prm, cw, it);
-    int32_t* o = items_out + 7 * it;
-    o[0] = w.b; o[1] = w.h; o[2] = w.q_row0; o[3] = w.n_tiles; o[4] = w.ja; o[5] = w.jb; o[6] = w.kind;
+  int at = 0;
+  for (int it = 0; it < n; ++it) {
+    for (int t = 0; t < 2 && at < max_items; ++t) {
+      const WorkItem w = prm.chunked   ? decode_item<kListSplit>(prm, cw, it, t)
+                         : prm.twins > 0 ? decode_item<kListTwins>(prm, cw, it, t)
+                                         : decode_item<kListPlain>(prm, cw, it, t);
+      if (t == 1 && !w.twin) break;
+      int32_t* o = items_out + 7 * at++;
+      o[0] = w.b; o[1] = w.h; o[2] = w.q_row; o[3] = w.twin ? 1 : w.n_tiles; o[4] = w.ja; o[5] = w.jb; o[6] = w.kind;
+    }
   }
   return B200_ATTN_OK;
 }

@@ -30,7 +30,7 @@ int check_view(const char* name, const void* ptr, const int64_t s[3], int batch,
 // status word and which kernels already have their shared-memory opt-in (the opt-in is per device and per kernel).
 // The runtime calls behind these cost more than the rest of the host path of a launch-bound call.
 constexpr int kMaxDevices = 64;
-constexpr int kKernelForms = 42;      // attention: 2 dtypes x 7 bias forms x (short, long, long with key split)
+constexpr int kKernelForms = 84;      // attention: 2 dtypes x 7 bias forms x (short, long) x (plain lists, twins, key split)
 constexpr int kLinearKernels = 20;    // pair GEMM kernels of b200_linear.cu: 5 epilogues x (full, not) x 2 dtypes
 constexpr int kGemmSplits = 6;        // split counts of the split GEMM kernel
 struct DeviceState {

@@ -260,7 +260,7 @@ int b200_rope_qk(const B200RopeArgs* args, void* stream);
  * Describes, without launching and without a GPU, the work the kernel's CTA number `cta` would do for `args` on a
  * device with `sms` SMs (148 on a B200): the grid size in *grid, the CTA's item count in *n_items, up to `max_items`
  * items as 7 integers each in `items` - batch, head, first query row, query tiles (1 or 2), first key tile, end key
- * tile, kind (0 whole item, 1 a part whose result goes to the workspace, 2 the part that merges the later ones) -
+ * tile (two one-tile items of different heads that are worked on side by side are listed one after the other), kind (0 whole item, 1 a part whose result goes to the workspace, 2 the part that merges the later ones) -
  * and in *later_parts how many following CTAs hold later parts of its last item.  The plan is computed by the very
  * functions the kernel runs, so tests can check on a CPU that every (query tile, key tile) of a problem is covered
  * exactly once.  `args->workspace` only matters as NULL / not NULL (with a workspace long sequences may be split).

@@ -615,3 +615,31 @@ def test_both_schedules_give_the_same_result(schedule: str, n: int) -> None:
     assert_close(got.float().cpu().numpy(), oracle_of_packed(qkv, 0.125), unit_scale=True, what=f"{schedule} n={n}")
     other = ff.attention(q, k, v, scale=0.125, layout="bnhd", schedule="long")
     assert torch.equal(got, other)
+
+
+GRIDS = {9: ((3, 3), (9, 1)), 128: ((16, 8), (64, 2)), 190: ((10, 19), (2, 95)), 300: ((12, 25), (100, 3)), 640: ((20, 32), (80, 8))}
+
+
+@pytest.mark.parametrize(("b", "h", "nq"), [(1, 2, 128), (2, 149, 49), (3, 197, 100), (3, 151, 300), (2, 222, 260), (1, 445, 300), (4, 149, 130)])
+@pytest.mark.parametrize("nk", GRIDS)
+@pytest.mark.parametrize(("form", "dtype"), [("plain", "fp16"), ("plain", "bf16"), ("dense", "bf16"), ("rel", "fp16"), ("rel-wide", "bf16")])
+def test_one_tile_remainders_of_two_heads_side_by_side(b: int, h: int, nq: int, nk: int, form: str, dtype: str) -> None:
+    """Lists of one-tile items taken two by two, behind and before other kinds of items, over one to five key tiles (the
+    stages of the K and V rings used once, twice, and round and round), in the forms with two and with three stages and
+    with one and two buffers of one-hot rows. Against float32 on the same 16-bit inputs, every row."""
+    t = DTYPES[dtype]
+    gen = torch.Generator(device="cuda").manual_seed(nq * 1000 + nk)
+    q = torch.randn(b, h, nq, 64, generator=gen, device="cuda").to(t)
+    k, v = (torch.randn(b, h, nk, 64, generator=gen, device="cuda").to(t) for _ in range(2))
+    bias = rel = None
+    logits = torch.einsum("bhqd,bhkd->bhqk", q.float(), k.float()) * 0.125
+    if form == "dense":
+        bias = ff.tile_layout(torch.randn(1, h, nq, nk, generator=gen, device="cuda").to(t))
+        logits += bias.float()
+    elif form != "plain":
+        rel = tuple(torch.randn(b, h, nq, side, generator=gen, device="cuda").to(t) for side in GRIDS[nk][form == "rel-wide"])
+        logits += (rel[0].float()[..., :, None] + rel[1].float()[..., None, :]).reshape(b, h, nq, nk)
+    ref = torch.einsum("bhqk,bhkd->bhqd", logits.softmax(-1), v.float())
+    got = ff.scaled_dot_product_attention(q, k, v, attn_mask=bias, rel=rel)
+    assert ff.device_status() == 0
+    assert_close(got.float().cpu().numpy(), ref.cpu().numpy(), unit_scale=True, what=f"[{b},{h},{nq},{nk}] {form} {dtype}")
