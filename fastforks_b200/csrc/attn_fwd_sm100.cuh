@@ -719,7 +719,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         const bool e_constant = !SPLIT && (kv_tiles == 1 || (!TWINS && kv_tiles <= e_bufs));  // every use of a buffer has the same E: it is written once
         int e_y[4], e_x[4];  // coordinates of this lane's keys
         const int e_dy = fast_div(kTileRows, p.magic_rel_kw), e_dx = kTileRows - e_dy * p.rel_kw;
-        // byte offsets of this lane's ones (inside its rows) in either buffer; at first those of places that hold a zero
+        // byte offsets of this lane's ones (inside its rows), at first those of places that hold a zero: with twins in buffer
+        // 0 and 1, else in the tile before last and in the last one (the buffers alternate)
         uint32_t hot0[4][2] = {}, hot1[4][2] = {};
         const auto warp_wait = [&](uint64_t* bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait_relaxed(bar, parity, abort_flag)) != 0; };
         for (int it = 0; it < my_items && ok; ++it) {
@@ -798,14 +799,14 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
 #pragma unroll
                 for (int r = 0; r < 4; ++r)
 #pragma unroll
-                  for (int k = 0; k < 2; ++k) st_shared_u16(e + r * 32 * 128 + (buf == 0 ? hot0[r][k] : hot1[r][k]), 0);
+                  for (int k = 0; k < 2; ++k) st_shared_u16(e + r * 32 * 128 + ((TWINS ? buf == 0 : e_bufs == 2) ? hot0[r][k] : hot1[r][k]), 0);
 #pragma unroll
                 for (int r = 0; r < 4; ++r)
 #pragma unroll
                   for (int k = 0; k < 2; ++k) {
                     st_shared_u16(e + r * 32 * 128 + at[r][k], static_cast<uint16_t>(p.rel_one));
-                    hot0[r][k] = buf == 0 ? at[r][k] : hot0[r][k];
-                    hot1[r][k] = buf == 0 ? hot1[r][k] : at[r][k];
+                    hot0[r][k] = !TWINS ? hot1[r][k] : buf == 0 ? at[r][k] : hot0[r][k];
+                    hot1[r][k] = TWINS && buf == 0 ? hot1[r][k] : at[r][k];
                   }
                 fence_proxy_async_smem();
               }
@@ -970,7 +971,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         // Whether nobody but this tile reads the K and V tiles of an item: it then frees them for both.
         auto alone = [&](const Pos& x) { return x.it >= (TWINS ? twin_item : my_doubles); };
         auto advance = [&](Pos& x) {
-          x.ring.advance(TWINS && x.it >= twin_item && x.it < my_doubles, has_twins && x.it >= my_doubles);
+          if constexpr (TWINS) x.ring.advance(x.it >= twin_item && x.it < my_doubles, has_twins && x.it >= my_doubles);
           ++x.gs;
           if (SPLIT ? ++x.j == x.jend : ++x.j == kv_tiles) {
             x.j = 0;
@@ -981,6 +982,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
               else if (x.it == my_doubles) x.ring.stage = 0;
             }
           }
+          if constexpr (!TWINS) x.ring.advance(false, false);
         };
         Pos start = {0, 0, ja0, my_items == 1 ? jb_last : kv_tiles, {}};
         if (has_twins && twin_item == 0) start.ring.stage = t;
