@@ -121,6 +121,7 @@ struct Forward {
   cudaStream_t stream;
   char* ws;
   void* x;
+  mutable bool started = false;  // a kernel of this forward is in front: the weights were complete before that one started
 
   void* at(int64_t offset) const { return ws + offset; }
 
@@ -135,6 +136,8 @@ struct Forward {
     NormParams p{};
     p.x = in; p.x_out = x_out; p.delta = delta; p.weight = w; p.bias = b; p.y = out;
     p.rows = rows; p.dim = a->dim; p.eps = eps; p.map = map;
+    p.early_w = started ? 1 : 0;
+    started = true;
     return launch_norm(a->dtype, p, stream);
   }
 
@@ -146,6 +149,7 @@ struct Forward {
     p.grid_h = a->grid_h; p.grid_w = a->grid_w; p.prefix = a->prefix;
     p.k = 3 * a->patch * a->patch; p.k_padded = a->patch_k;
     p.patches = at(l.hid); p.start = a->start; p.x = x; p.dim = a->dim;
+    started = true;
     void* args[] = {&p};
     const void* kernel = a->dtype == B200_ATTN_F16 ? reinterpret_cast<const void*>(encoder_tokens_kernel<__half>) : reinterpret_cast<const void*>(encoder_tokens_kernel<__nv_bfloat16>);
     if (int rc = launch_kernel(kernel, static_cast<unsigned>(a->batch * a->grid_h), 4, kTokensThreads, 0, 1, stream, args, "encoder tokens launch")) return rc;
