@@ -152,7 +152,7 @@ struct Forward {
     started = true;
     void* args[] = {&p};
     const void* kernel = a->dtype == B200_ATTN_F16 ? reinterpret_cast<const void*>(encoder_tokens_kernel<__half>) : reinterpret_cast<const void*>(encoder_tokens_kernel<__nv_bfloat16>);
-    if (int rc = launch_kernel(kernel, static_cast<unsigned>(a->batch * a->grid_h), 4, kTokensThreads, 0, 1, stream, args, "encoder tokens launch")) return rc;
+    if (int rc = launch_kernel(kernel, static_cast<unsigned>(a->batch * a->grid_h), static_cast<unsigned>(tokens_parts(a->patch)), kTokensThreads, 0, 1, stream, args, "encoder tokens launch")) return rc;
     return linear(at(l.hid), static_cast<int>(l.rows), a->patch_k, a->patch_w, nullptr, a->dim, x, kActNone, nullptr, x);
   }
 

