@@ -384,14 +384,9 @@ int b200_rope_qk(const B200RopeArgs* a, void* stream_ptr) {
   prm.tokens = a->tokens;
   prm.prefix = a->prefix;
   prm.q_scale = a->q_scale;
-  // One token per CTA and pass; enough CTAs to fill every SM sixteen times over (128 threads each), no more.
-  const long long rows = static_cast<long long>(a->batch) * a->tokens;
-  const unsigned grid = static_cast<unsigned>(std::min<long long>(rows, static_cast<long long>(dev->sms) * 16));
-  cudaStream_t stream = static_cast<cudaStream_t>(stream_ptr);
-  if (a->dtype == B200_ATTN_F16) rope_qk_kernel<__half><<<grid, kRopeThreads, 0, stream>>>(prm);
-  else rope_qk_kernel<__nv_bfloat16><<<grid, kRopeThreads, 0, stream>>>(prm);
-  const cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return cuda_fail(e, "rope_qk kernel launch");
+  void* args[] = {&prm};
+  const void* kernel = a->dtype == B200_ATTN_F16 ? reinterpret_cast<const void*>(rope_qk_kernel<__half>) : reinterpret_cast<const void*>(rope_qk_kernel<__nv_bfloat16>);
+  if (int rc = launch_kernel(kernel, static_cast<unsigned>(a->tokens), static_cast<unsigned>(std::min(a->batch, 65535)), kRopeThreads, 0, 1, static_cast<cudaStream_t>(stream_ptr), args, "rope_qk kernel launch")) return rc;
   clear_error();
   return B200_ATTN_OK;
 }

@@ -111,3 +111,16 @@ def test_contract_violations_raise_before_launch() -> None:
         ff.rope_qk_(qkv, ff.rope_table(4, 4, 100.0, "cuda"))  # more patch tokens than the sequence has
     with pytest.raises(ValueError, match="q_scale"):
         ff.rope_qk_(qkv, cs, q_scale=0.0)
+
+
+@pytest.mark.parametrize("b", [1, 65535, 65541])
+def test_more_images_than_a_grid_has_rows(b: int) -> None:
+    """The launch's second dimension is the batch, up to its limit of 65535; images behind that are further passes."""
+    gen = torch.Generator().manual_seed(b)
+    qkv = torch.randn(b, 3, 3, 1, 64, generator=gen).half().cuda()
+    before = qkv.clone()
+    cs = ff.rope_table(1, 2, 100.0, "cuda")
+    ff.rope_qk_(qkv, cs, q_scale=0.125)
+    q_ref, k_ref = ro.rope_qk(before[:, :, 0].float().cpu().numpy(), before[:, :, 1].float().cpu().numpy(), cs.cpu().numpy(), 0.125)
+    within_one_ulp(qkv[:, :, 0], q_ref, "fp16", "q")
+    within_one_ulp(qkv[:, :, 1], k_ref, "fp16", "k")
