@@ -34,6 +34,7 @@ HEADERS = (
     PACKAGE_DIR / "csrc" / "linear_host.h",
     PACKAGE_DIR / "csrc" / "sm100_ptx.cuh",
     PACKAGE_DIR / "csrc" / "attn_fwd_sm100.cuh",
+    PACKAGE_DIR / "csrc" / "attn_small_sm100.cuh",
     PACKAGE_DIR / "csrc" / "sam_rel_terms.cuh",
     PACKAGE_DIR / "csrc" / "rope_sm100.cuh",
     PACKAGE_DIR / "csrc" / "gemm_sm100.cuh",

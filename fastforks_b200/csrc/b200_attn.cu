@@ -16,6 +16,7 @@
 #include <type_traits>
 
 #include "attn_fwd_sm100.cuh"
+#include "attn_small_sm100.cuh"
 #include "host_common.h"
 
 namespace {
@@ -109,6 +110,7 @@ int device_state(DeviceState** out) {
       e = cudaGetSymbolAddress(reinterpret_cast<void**>(&d.status), g_status_word);
       if (e != cudaSuccess) return cuda_fail(e, "cudaGetSymbolAddress(status word)");
       for (auto& f : d.opted_in) f.store(false, std::memory_order_relaxed);
+      for (auto& f : d.small_opted_in) f.store(false, std::memory_order_relaxed);
       for (auto& f : d.linear_opted_in) f.store(false, std::memory_order_relaxed);
       d.splits_ready.store(false, std::memory_order_relaxed);
       d.ready.store(true, std::memory_order_release);
@@ -523,6 +525,33 @@ int launch_sched(bool short_sched, const AttnParams& planned, unsigned grid, Dev
   return launch<T, BIAS, false, kListPlain>(planned, grid, dev, mq, mk, mv, mo, mb, stream);
 }
 
+// Whether the call goes to attn_small_kernel: no bias, keys that fit, and few enough blocks of 32 queries that they all run
+// at once. The lines lie where the persistent kernel catches up; us per launch in CUDA graphs, persistent and small:
+// 100 keys 5.3 and 4.0 at 288 blocks (two per SM, as far as it was tried), 197 and 256 keys 6.0 and 5.25 at 192 blocks but
+// 6.2 and 7.1 at 252, 512 keys 8.0 and 5.6 at 96 (a block then takes most of an SM's shared memory: one per SM).
+bool small_call(const B200AttnArgs* a, int sms) {
+  const long long blocks = static_cast<long long>(a->batch) * a->heads * ((a->q_tokens + kSmallRows - 1) / kSmallRows);
+  const int kv = a->kv_tokens;
+  return kv <= 64 * kSmallMaxSteps && 3 * blocks <= (kv <= 128 ? 6 : kv <= 256 ? 4 : 3) * sms;
+}
+
+template <typename T, int STEPS>
+int launch_small(const SmallAttnParams& prm, const B200AttnArgs* a, DeviceState& dev, cudaStream_t stream) {
+  if (STEPS * 64 < a->kv_tokens)
+    if constexpr (STEPS < kSmallMaxSteps) return launch_small<T, STEPS + 1>(prm, a, dev, stream);
+  const void* kernel = reinterpret_cast<const void*>(attn_small_kernel<T, STEPS>);
+  constexpr int smem = small_attn_smem(STEPS);
+  constexpr int form = (std::is_same<T, __half>::value ? 0 : kSmallMaxSteps) + STEPS - 1;
+  static_assert(form < kSmallForms, "kernel form index");
+  if (!dev.small_opted_in[form].load(std::memory_order_acquire)) {
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(shared memory)");
+    dev.small_opted_in[form].store(true, std::memory_order_release);
+  }
+  void* args[] = {const_cast<SmallAttnParams*>(&prm)};
+  return launch_kernel(kernel, (a->q_tokens + kSmallRows - 1) / kSmallRows, a->batch * a->heads, kSmallThreads, smem, 0, stream, args, "attention kernel launch");
+}
+
 // The dense bias [B | 1, H | 1, Nq, Nk] (a stride of 0 broadcasts that dimension) as a 4-D tensor map whose box is
 // 128 rows x 64 columns with the 128-byte swizzle; a broadcast dimension gets extent 1 and the kernel addresses it at 0.
 int make_bias_map(CUtensorMap* map, const B200AttnArgs* a) {
@@ -596,6 +625,17 @@ int b200_attn_fwd(const B200AttnArgs* a, void* stream_ptr) {
   int rc = validate(a, &bias_mode, &sched);
   if (rc != B200_ATTN_OK) return rc;
   cudaStream_t stream = static_cast<cudaStream_t>(stream_ptr);
+  DeviceState* dev = nullptr;
+  if ((rc = device_state(&dev))) return rc;
+
+  if (bias_mode == kBiasNone && small_call(a, dev->sms)) {
+    SmallAttnParams prm{a->q, a->k, a->v, a->o, {}, {}, {}, {}, a->heads, a->q_tokens, a->kv_tokens, a->scale * kLog2e};
+    std::copy_n(a->q_stride, 3, prm.q_stride);
+    std::copy_n(a->k_stride, 3, prm.k_stride);
+    std::copy_n(a->v_stride, 3, prm.v_stride);
+    std::copy_n(a->o_stride, 3, prm.o_stride);
+    return a->dtype == B200_ATTN_F16 ? launch_small<__half, 1>(prm, a, *dev, stream) : launch_small<__nv_bfloat16, 1>(prm, a, *dev, stream);
+  }
 
   CUtensorMap mq, mk, mv, mo;
   if ((rc = cached_tile_map(&mq, a->q, a->dtype, a->batch, a->heads, a->q_tokens, a->q_stride, "q"))) return rc;
@@ -654,8 +694,6 @@ int b200_attn_fwd(const B200AttnArgs* a, void* stream_ptr) {
     else if (a->rel_kh == 14 && a->rel_kw == 14)
       bias_mode = kBiasDecomposed14;
   }
-  DeviceState* dev = nullptr;
-  if ((rc = device_state(&dev))) return rc;
   prm.status = dev->status;
 
   if (bias_shared_by_the_batch(a)) {

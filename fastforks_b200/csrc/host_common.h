@@ -31,6 +31,7 @@ int check_view(const char* name, const void* ptr, const int64_t s[3], int batch,
 // The runtime calls behind these cost more than the rest of the host path of a launch-bound call.
 constexpr int kMaxDevices = 64;
 constexpr int kKernelForms = 84;      // attention: 2 dtypes x 7 bias forms x (short, long) x (plain lists, twins, key split)
+constexpr int kSmallForms = 16;      // attention of small calls: 2 dtypes x 8 key counts
 constexpr int kLinearKernels = 20;    // pair GEMM kernels of b200_linear.cu: 5 epilogues x (full, not) x 2 dtypes
 constexpr int kGemmSplits = 6;        // split counts of the split GEMM kernel
 struct DeviceState {
@@ -38,6 +39,7 @@ struct DeviceState {
   int sms = 0;
   uint32_t* status = nullptr;
   std::atomic<bool> opted_in[kKernelForms];
+  std::atomic<bool> small_opted_in[kSmallForms];
   std::atomic<bool> linear_opted_in[kLinearKernels];
   std::atomic<bool> splits_ready;
   std::atomic<int> split_clusters[kGemmSplits];  // clusters of the split GEMM kernel that run at once

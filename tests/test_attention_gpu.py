@@ -643,3 +643,21 @@ def test_one_tile_remainders_of_two_heads_side_by_side(b: int, h: int, nq: int, 
     got = ff.scaled_dot_product_attention(q, k, v, attn_mask=bias, rel=rel)
     assert ff.device_status() == 0
     assert_close(got.float().cpu().numpy(), ref.cpu().numpy(), unit_scale=True, what=f"[{b},{h},{nq},{nk}] {form} {dtype}")
+
+
+@pytest.mark.parametrize(("b", "h", "nq", "nk"), [(1, 1, 1, 1), (1, 2, 31, 15), (2, 3, 33, 16), (1, 3, 32, 17), (1, 12, 197, 197), (1, 5, 64, 64), (2, 2, 65, 65), (1, 2, 100, 193), (1, 24, 256, 256), (1, 25, 256, 256), (1, 49, 192, 128), (1, 50, 192, 128), (1, 6, 40, 257), (1, 3, 300, 449), (1, 148, 32, 512), (1, 148, 33, 512), (1, 1, 70, 513), (3, 99, 20, 130)])  # fmt: skip
+@pytest.mark.parametrize("dtype", ["fp16", "bf16"])
+def test_small_calls_in_blocks_of_32_queries(b: int, h: int, nq: int, nk: int, dtype: str) -> None:
+    """Key counts around the 16-key steps of a quarter (quarters without keys among them), remainders of 32 queries, and
+    the calls on either side of the rule's lines; views of wider tensors, against float32 on the same operands, and
+    nothing written past the rows."""
+    t = DTYPES[dtype]
+    gen = torch.Generator(device="cuda").manual_seed(nq * 1000 + nk)
+    q = torch.randn(b, nq, 2, h, 64, generator=gen, device="cuda").to(t)[:, :, 0]
+    k, v = torch.randn(b, nk, 3, h, 64, generator=gen, device="cuda").to(t)[:, :, 1:].unbind(2)
+    big = torch.full((b, nq + 2, h, 64), 77.0, dtype=t, device="cuda")
+    ff.attention(q, k, v, scale=0.25, layout="bnhd", out=big[:, 1 : 1 + nq])
+    logits = torch.einsum("bqhd,bkhd->bhqk", q.float(), k.float()) * 0.25
+    ref = torch.einsum("bhqk,bkhd->bqhd", logits.softmax(-1), v.float())
+    assert_close(big[:, 1 : 1 + nq].float().cpu().numpy(), ref.cpu().numpy(), unit_scale=True, what=f"[{b},{h},{nq},{nk}] {dtype}")
+    assert bool((big[:, 0] == 77.0).all()) and bool((big[:, -1] == 77.0).all())
