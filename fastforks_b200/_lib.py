@@ -239,6 +239,12 @@ class B200EncoderArgs(ctypes.Structure):
         ("neck_out", ctypes.c_void_p),
         ("neck_channels", ctypes.c_int32),
         ("neck_eps", ctypes.c_float),
+        ("patch_b", ctypes.c_void_p),
+        ("first", ctypes.c_void_p),
+        ("start_f32", ctypes.c_int32),
+        ("patch_w_raw", ctypes.c_int32),
+        ("neck_w1_conv", ctypes.c_int32),
+        ("reserved", ctypes.c_int32),
     )
 
 

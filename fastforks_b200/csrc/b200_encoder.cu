@@ -20,9 +20,13 @@ int64_t align256(int64_t bytes) { return (bytes + 255) & ~int64_t(255); }
 
 // Buffers of one forward, as offsets into the workspace.
 struct Layout {
-  int64_t x, y, qkv, att, hid, rel_h, rel_w, neck, total;
+  int64_t x, y, qkv, att, hid, rel_h, rel_w, neck, patch_w, neck_w1, total;
   int64_t rows, most_rows;  // tokens of all images; rows of the largest partition into padded windows
 };
+
+// Whether the patch embedding's weights have to be padded, and the neck's 3 x 3 weights reordered, in this call.
+bool pads_patch_w(const B200EncoderArgs* a) { return a->images != nullptr && a->patch_w_raw != 0 && a->patch_k != 3 * a->patch * a->patch; }
+bool reorders_neck_w1(const B200EncoderArgs* a) { return a->neck_w0 != nullptr && a->neck_w1_conv != 0; }
 
 int windows_of(int grid, int side) { return (grid + side - 1) / side; }
 
@@ -59,6 +63,8 @@ Layout layout_of(const B200EncoderArgs* a) {
   l.rel_h = take(rel);
   l.rel_w = take(rel);
   l.neck = take(a->neck_w0 != nullptr ? l.rows * a->neck_channels : 0);
+  l.patch_w = take(pads_patch_w(a) ? static_cast<int64_t>(a->dim) * a->patch_k : 0);
+  l.neck_w1 = take(reorders_neck_w1(a) ? 9LL * a->neck_channels * a->neck_channels : 0);
   l.total = at;
   return l;
 }
@@ -141,7 +147,20 @@ struct Forward {
     return launch_norm(a->dtype, p, stream);
   }
 
+  int repack(const void* src, int rows, int cols, int out_cols, int taps, int64_t to) const {
+    RepackParams p{src, at(to), cols, out_cols, taps};
+    started = true;
+    void* args[] = {&p};
+    return launch_kernel(reinterpret_cast<const void*>(repack_kernel), static_cast<unsigned>(rows), 1, kRepackThreads, 0, 1, stream, args, "weight repacking launch");
+  }
+
   int start_tokens() const {
+    // In front of the kernel that is in front of the product: the product loads its weights ahead of that one.
+    const void* w = a->patch_w;
+    if (pads_patch_w(a)) {
+      w = at(l.patch_w);
+      if (int rc = repack(a->patch_w, a->dim, 3 * a->patch * a->patch, a->patch_k, 0, l.patch_w)) return rc;
+    }
     TokensParams p{};
     p.images = a->images;
     p.image_f32 = a->image_dtype == B200_ATTN_F32;
@@ -149,11 +168,12 @@ struct Forward {
     p.grid_h = a->grid_h; p.grid_w = a->grid_w; p.prefix = a->prefix;
     p.k = 3 * a->patch * a->patch; p.k_padded = a->patch_k;
     p.patches = at(l.hid); p.start = a->start; p.x = x; p.dim = a->dim;
+    p.start_f32 = a->start_f32; p.patch_b = a->patch_b; p.first = a->first;
     started = true;
     void* args[] = {&p};
     const void* kernel = a->dtype == B200_ATTN_F16 ? reinterpret_cast<const void*>(encoder_tokens_kernel<__half>) : reinterpret_cast<const void*>(encoder_tokens_kernel<__nv_bfloat16>);
     if (int rc = launch_kernel(kernel, static_cast<unsigned>(a->batch * a->grid_h), static_cast<unsigned>(tokens_parts(a->patch)), kTokensThreads, 0, 1, stream, args, "encoder tokens launch")) return rc;
-    return linear(at(l.hid), static_cast<int>(l.rows), a->patch_k, a->patch_w, nullptr, a->dim, x, kActNone, nullptr, x);
+    return linear(at(l.hid), static_cast<int>(l.rows), a->patch_k, w, nullptr, a->dim, x, kActNone, nullptr, x);
   }
 
   int attention(const B200EncoderBlock& k, int batch, int tokens, int side) const {
@@ -228,6 +248,11 @@ struct Forward {
   int neck() const {
     const int rows = static_cast<int>(l.rows), ch = a->neck_channels;
     if (int rc = linear(x, rows, a->dim, a->neck_w0, nullptr, ch, at(l.neck), kActNone)) return rc;
+    const void* w1 = a->neck_w1;
+    if (reorders_neck_w1(a)) {  // in front of the next kernel for the same reason as the patch embedding's
+      w1 = at(l.neck_w1);
+      if (int rc = repack(a->neck_w1, ch, 9 * ch, 9 * ch, 9, l.neck_w1)) return rc;
+    }
     NeckParams p{};
     p.x = at(l.neck); p.weight = a->neck_n0_w; p.bias = a->neck_n0_b; p.out = at(l.hid);
     p.batch = a->batch; p.grid_h = a->grid_h; p.grid_w = a->grid_w; p.channels = ch; p.eps = a->neck_eps;
@@ -235,7 +260,7 @@ struct Forward {
     const bool f16 = a->dtype == B200_ATTN_F16;
     const void* im2col = f16 ? reinterpret_cast<const void*>(neck_norm_im2col_kernel<__half>) : reinterpret_cast<const void*>(neck_norm_im2col_kernel<__nv_bfloat16>);
     if (int rc = launch_kernel(im2col, static_cast<unsigned>((rows + kNeckWarps - 1) / kNeckWarps), 1, kNeckWarps * 32, 0, 1, stream, args, "neck norm launch")) return rc;
-    if (int rc = linear(at(l.hid), rows, 9 * ch, a->neck_w1, nullptr, ch, at(l.neck), kActNone)) return rc;
+    if (int rc = linear(at(l.hid), rows, 9 * ch, w1, nullptr, ch, at(l.neck), kActNone)) return rc;
     p.weight = a->neck_n1_w; p.bias = a->neck_n1_b; p.out = a->neck_out;
     const void* chw = f16 ? reinterpret_cast<const void*>(neck_norm_chw_kernel<__half>) : reinterpret_cast<const void*>(neck_norm_chw_kernel<__nv_bfloat16>);
     const int area = a->grid_h * a->grid_w;

@@ -191,7 +191,10 @@ struct TokensParams {
   int grid_h, grid_w, prefix;  // tokens per image: prefix (class token) + grid_h * grid_w
   int k, k_padded;      // 3 * patch * patch, and the row stride of `patches`
   void* patches;        // [batch * tokens, k_padded]: one row of pixels per token (channel, row, column), zeros for prefix tokens
-  const void* start;    // [tokens, dim]: what the patch product is added to (position embedding and bias; class token)
+  const void* start;    // [tokens, dim], fp32 or the encoder's type: what the patch product is added to (position embedding) ...
+  int start_f32;
+  const void* patch_b;  // ... plus, for patch tokens, [dim] (patch bias) ...
+  const void* first;    // ... and, for prefix tokens, [prefix, dim] (class token); either may be null
   void* x;              // [batch * tokens, dim]
   int dim;
 };
@@ -248,8 +251,30 @@ __global__ void __launch_bounds__(kTokensThreads) encoder_tokens_kernel(const To
   const int vec = p.dim / 8;
   const uint4* start = static_cast<const uint4*>(p.start);
   uint4* x = static_cast<uint4*>(p.x) + static_cast<int64_t>(b) * tokens * vec;
+  if (!p.start_f32 && p.patch_b == nullptr && p.first == nullptr) {
 #pragma unroll 4
-  for (int i = n0 * vec + slice * kTokensThreads + threadIdx.x; i < n1 * vec; i += kTokensStarts * kTokensThreads) x[i] = __ldg(start + i);
+    for (int i = n0 * vec + slice * kTokensThreads + threadIdx.x; i < n1 * vec; i += kTokensStarts * kTokensThreads) x[i] = __ldg(start + i);
+  } else {  // the sum in fp32, rounded once
+#pragma unroll 2
+    for (int i = n0 * vec + slice * kTokensThreads + threadIdx.x; i < n1 * vec; i += kTokensStarts * kTokensThreads) {
+      const int n = i / vec;
+      const uint4* add = static_cast<const uint4*>(n < p.prefix ? p.first : p.patch_b);
+      float f[8], a[8];
+      if (p.start_f32) {
+        const float4 lo = __ldg(static_cast<const float4*>(p.start) + 2 * i), hi = __ldg(static_cast<const float4*>(p.start) + 2 * i + 1);
+        f[0] = lo.x; f[1] = lo.y; f[2] = lo.z; f[3] = lo.w;
+        f[4] = hi.x; f[5] = hi.y; f[6] = hi.z; f[7] = hi.w;
+      } else {
+        enc_unpack8<T>(__ldg(start + i), f);
+      }
+      if (add != nullptr) {
+        enc_unpack8<T>(__ldg(add + (n < p.prefix ? i : i - n * vec)), a);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) f[e] += a[e];
+      }
+      x[i] = enc_pack8<T>(f);
+    }
+  }
   if (slice != 0) return;
   T* rows = static_cast<T*>(p.patches) + static_cast<int64_t>(b) * tokens * p.k_padded;
   const T zero = T(0.f);
@@ -259,6 +284,39 @@ __global__ void __launch_bounds__(kTokensThreads) encoder_tokens_kernel(const To
   if (pad > 0)
     for (int i = threadIdx.x; i < p.grid_w * pad; i += kTokensThreads)
       static_cast<T*>(p.patches)[(first_row + i / pad) * p.k_padded + p.k + i % pad] = zero;
+}
+
+// A convolution's weights as the rows of a linear layer, in pairs of 16-bit values, a CTA per row: padded with zeros to a row
+// of whole 16-byte groups (the patch embedding of patches of 14), or with the kernel's positions in front of the channels
+// (the neck's 3 x 3, whose input rows are nine channel vectors). Done in every forward, on 1-2 MB, so that the convolution's
+// own tensor is what a forward reads; a copy kept from the first one would not see that tensor change.
+struct RepackParams {
+  const void* src;  // [rows, cols]; taps > 0: [rows, cols / taps, taps]
+  void* dst;        // [rows, out_cols], zeros from cols on; taps > 0: [rows, taps, cols / taps]
+  int cols, out_cols;
+  int taps;
+};
+constexpr int kRepackThreads = 256;
+constexpr int kRepackMaxCols = 9 * 512;  // with taps: a row lies in shared memory
+
+__global__ void __launch_bounds__(kRepackThreads) repack_kernel(const RepackParams p) {
+  __shared__ uint32_t row[kRepackMaxCols / 2];
+  grid_dependency_wait();
+  grid_launch_dependents();
+  const uint32_t* src = static_cast<const uint32_t*>(p.src) + static_cast<int64_t>(blockIdx.x) * (p.cols >> 1);
+  uint32_t* dst = static_cast<uint32_t*>(p.dst) + static_cast<int64_t>(blockIdx.x) * (p.out_cols >> 1);
+  if (p.taps == 0) {
+    for (int i = threadIdx.x; i < p.out_cols >> 1; i += kRepackThreads) dst[i] = 2 * i < p.cols ? __ldg(src + i) : 0u;
+    return;
+  }
+  for (int i = threadIdx.x; i < p.cols >> 1; i += kRepackThreads) row[i] = __ldg(src + i);
+  __syncthreads();
+  const uint16_t* values = reinterpret_cast<const uint16_t*>(row);
+  const int channels = p.cols / p.taps;  // a multiple of eight: both values of a pair lie at one position
+  for (int i = threadIdx.x; i < p.cols >> 1; i += kRepackThreads) {
+    const int tap = 2 * i / channels, c = 2 * i - tap * channels;
+    dst[i] = values[c * p.taps + tap] | static_cast<uint32_t>(values[(c + 1) * p.taps + tap]) << 16;
+  }
 }
 
 // ---- SAM's neck -------------------------------------------------------------------------------------------------
@@ -275,6 +333,7 @@ struct NeckParams {
 
 constexpr int kNeckWarps = 8;
 constexpr int kNeckChunks = 2;  // up to 512 channels
+static_assert(kRepackMaxCols >= 9 * kNeckChunks * 256, "a row of the neck's 3 x 3 weights");
 
 // The normalised row of one token per warp, in `v` (8 values per lane and chunk).
 template <typename T>

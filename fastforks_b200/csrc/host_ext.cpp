@@ -12,6 +12,7 @@
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <cstring>
+#include <memory>
 #include <mutex>
 #include <vector>
 
@@ -344,6 +345,62 @@ PyObject* py_rel_terms(PyObject*, PyObject* const* args, Py_ssize_t n) {
   return pair;
 }
 
+// What an encoder's table of parameter addresses was made from (encoder.py: Snapshot). The tensors are held, so an address
+// cannot come to mean another one while it is compared with.
+struct Fact {
+  at::Tensor tensor;
+  const void* ptr;
+  c10::SmallVector<int64_t, 4> sizes, strides;
+};
+using Facts = std::vector<Fact>;
+constexpr const char* kFactsName = "_b200host.snapshot";
+
+void free_facts(PyObject* capsule) { delete static_cast<Facts*>(PyCapsule_GetPointer(capsule, kFactsName)); }
+
+// Calls f(tensor) for every value of every dictionary in the tuple `dicts`; false as soon as f says so or one is no tensor.
+template <typename F>
+bool for_each_tensor(PyObject* dicts, F&& f) {
+  if (!PyTuple_Check(dicts)) return false;
+  for (Py_ssize_t i = 0; i < PyTuple_GET_SIZE(dicts); ++i) {
+    PyObject* d = PyTuple_GET_ITEM(dicts, i);
+    if (!PyDict_Check(d)) return false;
+    PyObject *key = nullptr, *value = nullptr;
+    for (Py_ssize_t at = 0; PyDict_Next(d, &at, &key, &value);) {
+      const at::Tensor* t = tensor_of(value);
+      if (t == nullptr || !t->has_storage() || !f(*t)) return false;
+    }
+  }
+  return true;
+}
+
+// snapshot(dicts) -> capsule, or None for anything but dictionaries of plain tensors
+PyObject* py_snapshot(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  if (n != 1) Py_RETURN_NONE;
+  auto facts = std::make_unique<Facts>();
+  const auto take = [&](const at::Tensor& t) {
+    facts->push_back(Fact{t, t.const_data_ptr(), {t.sizes().begin(), t.sizes().end()}, {t.strides().begin(), t.strides().end()}});
+    return true;
+  };
+  if (!for_each_tensor(args[0], take)) Py_RETURN_NONE;
+  PyObject* capsule = PyCapsule_New(facts.get(), kFactsName, free_facts);
+  if (capsule != nullptr) facts.release();
+  return capsule;
+}
+
+// unchanged(capsule, dicts): the same tensors in the same places
+PyObject* py_unchanged(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  if (n != 2 || !PyCapsule_IsValid(args[0], kFactsName)) Py_RETURN_FALSE;
+  const Facts& facts = *static_cast<Facts*>(PyCapsule_GetPointer(args[0], kFactsName));
+  size_t i = 0;
+  const auto same = [&](const at::Tensor& t) {
+    if (i >= facts.size()) return false;
+    const Fact& f = facts[i++];
+    return t.is_same(f.tensor) && t.const_data_ptr() == f.ptr && t.sizes().equals(f.sizes) && t.strides().equals(f.strides);
+  };
+  if (for_each_tensor(args[1], same) && i == facts.size()) Py_RETURN_TRUE;
+  Py_RETURN_FALSE;
+}
+
 // C++ exceptions (an allocation that fails) must not cross into the interpreter: the Python side runs and reports.
 template <PyObject* (*F)(PyObject*, PyObject* const*, Py_ssize_t)>
 PyObject* guarded(PyObject* self, PyObject* const* args, Py_ssize_t n) {
@@ -365,6 +422,8 @@ PyMethodDef methods[] = {
     {"gemm", fast<py_gemm>(), METH_FASTCALL, nullptr},
     {"rope_qk_", fast<py_rope>(), METH_FASTCALL, nullptr},
     {"sam_rel_terms", fast<py_rel_terms>(), METH_FASTCALL, nullptr},
+    {"snapshot", fast<py_snapshot>(), METH_FASTCALL, nullptr},
+    {"unchanged", fast<py_unchanged>(), METH_FASTCALL, nullptr},
     {"register_workspace", fast<py_register_workspace>(), METH_FASTCALL, nullptr},
     {nullptr, nullptr, 0, nullptr},
 };

@@ -30,6 +30,25 @@ def supported(dtype: torch.dtype, dim: int, heads: int, hidden: int) -> bool:
     return dtype in _DTYPES and dim == heads * 64 and dim <= MAX_DIM and hidden % 8 == 0
 
 
+class Snapshot:
+    """The tensors of a model's dictionaries as they were when their addresses were taken: a tensor put in another's place, or
+    given other storage, is seen by `changed`, which every forward asks. (Values written in place need no looking at: the
+    kernels read the tensors themselves.) The tensors are kept alive, so that no address is used again while it is in the table."""
+
+    def __init__(self, *dicts: dict[str, torch.Tensor]) -> None:
+        self._native = None if _lib.fast is None else _lib.fast.snapshot(dicts)
+        self._kept = None if self._native is not None else self._facts(dicts)
+
+    @staticmethod
+    def _facts(dicts: tuple[dict[str, torch.Tensor], ...]) -> list[tuple]:
+        return [(id(t), t.data_ptr(), t.shape, t.stride(), t) for d in dicts for t in d.values()]
+
+    def changed(self, *dicts: dict[str, torch.Tensor]) -> bool:
+        if self._native is not None:
+            return not _lib.fast.unchanged(self._native, dicts)
+        return [f[:-1] for f in self._kept] != [f[:-1] for f in self._facts(dicts)]
+
+
 class NativeEncoder:
     """Blocks of one encoder on one device. `blocks[i]` maps the pointer names of `B200EncoderBlock` to tensors (missing
     names are NULL) and `window` to the window side; the tensors are kept alive here and read in place."""

@@ -178,15 +178,22 @@ class SamEncoder:
             side = cfg.grid if i in cfg.global_blocks else cfg.window
             p = f"blocks.{i}.attn."
             self.tables[i] = (rel_table(side, self.w[p + "rel_pos_h"]), rel_table(side, self.w[p + "rel_pos_w"]), side)
-        # On a CUDA device the whole forward is one native call over the parameters in `self.w`; what the kernels cannot take
-        # (grids of an odd side or above 64, where the producer of the relative terms ends) runs block by block below.
-        self._native: encoder.NativeEncoder | None = None
+        # On a CUDA device the whole forward is one native call that reads the parameters in `self.w`; what the kernels cannot
+        # take (grids of an odd side or above 64, where the producer of the relative terms ends) runs block by block below.
         sides = [cfg.grid if i in cfg.global_blocks else cfg.window for i in range(cfg.depth)]
-        if (self.device.type == "cuda" and encoder.supported(dtype, cfg.dim, cfg.heads, 4 * cfg.dim) and cfg.patch % 2 == 0
-                and all(side % 2 == 0 and side <= MAX_SIDE for side in sides) and cfg.out_chans % 8 == 0 and cfg.out_chans <= MAX_NECK):  # fmt: skip
-            self._make_native()
+        self._has_native = (self.device.type == "cuda" and encoder.supported(dtype, cfg.dim, cfg.heads, 4 * cfg.dim) and cfg.patch % 2 == 0
+                            and all(side % 2 == 0 and side <= MAX_SIDE for side in sides) and cfg.out_chans % 8 == 0 and cfg.out_chans <= MAX_NECK)  # fmt: skip
+        self._native: encoder.NativeEncoder | None = None
+        self._snapshot: encoder.Snapshot | None = None
+        self._native_now()
 
-    def _make_native(self) -> None:
+    def _native_now(self) -> encoder.NativeEncoder | None:
+        """The native encoder over the parameters as they are now; None where there is none for this device or shape."""
+        if self._has_native and (self._snapshot is None or self._snapshot.changed(self.w)):
+            self._native, self._snapshot = self._make_native(), encoder.Snapshot(self.w)
+        return self._native
+
+    def _make_native(self) -> encoder.NativeEncoder:
         w, cfg, blocks = self.w, self.cfg, []
         layers = {"norm1": "norm1", "qkv": "attn.qkv", "proj": "attn.proj", "norm2": "norm2", "fc1": "mlp.lin1", "fc2": "mlp.lin2"}
         for i in range(cfg.depth):
@@ -195,17 +202,12 @@ class SamEncoder:
             tensors |= {"rel_pos_h": w[p + "attn.rel_pos_h"], "rel_pos_w": w[p + "attn.rel_pos_w"],
                         "window": 0 if i in cfg.global_blocks else cfg.window}  # fmt: skip
             blocks.append(tensors)
-        self._native = encoder.NativeEncoder(blocks, dtype=self.dtype, dim=cfg.dim, heads=cfg.heads, hidden=4 * cfg.dim, ffn=encoder.FFN_GELU, eps=1e-5)
-        self._patch_w = F.pad(w["patch_embed.proj.weight"].flatten(1), (0, -3 * cfg.patch**2 % 8)).contiguous()
-        # what the patch products are added to, and the 3 x 3 convolution as rows over (row, column, channel)
-        self._start = (w["pos_embed"].float() + w["patch_embed.proj.bias"].float()).to(self.dtype).reshape(cfg.grid**2, cfg.dim).contiguous()
-        self._neck_w0 = w["neck.0.weight"].flatten(1).contiguous()
-        self._neck_w1 = w["neck.2.weight"].permute(0, 2, 3, 1).reshape(cfg.out_chans, -1).contiguous()
+        return encoder.NativeEncoder(blocks, dtype=self.dtype, dim=cfg.dim, heads=cfg.heads, hidden=4 * cfg.dim, ffn=encoder.FFN_GELU, eps=1e-5)
 
     def _forward_native(self, images: torch.Tensor) -> torch.Tensor | None:
         """The forward as one native call; None when the images are not of a form it takes."""
-        cfg, w = self.cfg, self.w
-        if (self._native is None or images.dim() != 4 or images.shape[1:] != (3, cfg.img, cfg.img) or images.device != self.w["pos_embed"].device  # noqa: PLR2004
+        cfg, w, native = self.cfg, self.w, self._native_now()
+        if (native is None or images.dim() != 4 or images.shape[1:] != (3, cfg.img, cfg.img) or images.device != self.w["pos_embed"].device  # noqa: PLR2004
                 or images.numel() == 0 or cfg.img % 2):  # fmt: skip
             return None
         if images.dtype not in (torch.float32, self.dtype):
@@ -215,16 +217,17 @@ class SamEncoder:
             return None
         extra = {  # "images", "neck_out": any address, the description only needs to know that there are some
             "images": 1, "image_dtype": _lib.F32 if images.dtype == torch.float32 else encoder._DTYPES[self.dtype],  # noqa: SLF001
-            "height": cfg.img, "width": cfg.img, "patch": cfg.patch, "patch_w": self._patch_w.data_ptr(), "patch_k": self._patch_w.shape[1],
-            "start": self._start.data_ptr(), "neck_out": 1, "neck_channels": cfg.out_chans, "neck_eps": cfg.eps,
-            "neck_w0": self._neck_w0.data_ptr(), "neck_w1": self._neck_w1.data_ptr(),
+            "height": cfg.img, "width": cfg.img, "patch": cfg.patch, "patch_k": (3 * cfg.patch**2 + 7) // 8 * 8,
+            "patch_w": w["patch_embed.proj.weight"].data_ptr(), "patch_w_raw": 1, "patch_b": w["patch_embed.proj.bias"].data_ptr(),
+            "start": w["pos_embed"].data_ptr(), "neck_out": 1, "neck_channels": cfg.out_chans, "neck_eps": cfg.eps,
+            "neck_w0": w["neck.0.weight"].data_ptr(), "neck_w1": w["neck.2.weight"].data_ptr(), "neck_w1_conv": 1,
             "neck_n0_w": w["neck.1.weight"].data_ptr(), "neck_n0_b": w["neck.1.bias"].data_ptr(),
             "neck_n1_w": w["neck.3.weight"].data_ptr(), "neck_n1_b": w["neck.3.bias"].data_ptr(),
         }  # fmt: skip
         b, grid = images.shape[0], cfg.grid
-        described = self._native.describe(b, (grid, grid), 0, 0, cfg.depth, extra)
+        described = native.describe(b, (grid, grid), 0, 0, cfg.depth, extra)
         out = torch.empty((b, cfg.out_chans, grid, grid), dtype=self.dtype, device=images.device)
-        self._native.launch(described, images.device, images=images, neck_out=out)
+        native.launch(described, images.device, images=images, neck_out=out)
         return out
 
     def attend(self, i: int, x: torch.Tensor) -> torch.Tensor:

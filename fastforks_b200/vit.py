@@ -141,12 +141,20 @@ class ViTEncoder:
         # this library never uses) a GEMM of its own is bound by the L2 at about 0.8 of the library's rate.
         self.fuse_plain = fuse_plain
         self.scales = {k: v.to(self.device, torch.float32) for k, v in state.items() if k.endswith(".gamma")}
-        # ... and the whole forward is one native call (`encoder`), made from the parameters in `self.w` and `self.scales`.
+        # ... and the whole forward is one native call (`encoder`) that reads the parameters in `self.w` and `self.scales`.
         self._native: encoder.NativeEncoder | None = None
-        if self.fused and self.device.type == "cuda" and encoder.supported(dtype, cfg.dim, cfg.heads, cfg.hidden):
-            self._native = self._make_native()
-            self._start: dict[tuple[int, int], torch.Tensor] = {}
-            self._patch_w = self._patch_matrix()
+        self._snapshot: encoder.Snapshot | None = None
+        self._pos32: dict[tuple[int, int], torch.Tensor] = {}
+        self._native_now()
+
+    def _native_now(self) -> encoder.NativeEncoder | None:
+        """The native encoder over the parameters as they are now; None where there is none for this device or shape."""
+        cfg = self.cfg
+        if not self.fused or self.device.type != "cuda" or not encoder.supported(self.dtype, cfg.dim, cfg.heads, cfg.hidden):
+            return None
+        if self._snapshot is None or self._snapshot.changed(self.w, self.scales):
+            self._native, self._snapshot = self._make_native(), encoder.Snapshot(self.w, self.scales)
+        return self._native
 
     def _make_native(self) -> encoder.NativeEncoder:
         w, cfg, blocks = self.w, self.cfg, []
@@ -161,27 +169,11 @@ class ViTEncoder:
         ffn = encoder.FFN_SWIGLU if cfg.ffn == "swiglu" else encoder.FFN_GELU_TANH
         return encoder.NativeEncoder(blocks, dtype=self.dtype, dim=cfg.dim, heads=cfg.heads, hidden=cfg.hidden, ffn=ffn, eps=cfg.eps)
 
-    def _patch_matrix(self) -> torch.Tensor:
-        """The patch embedding's kernel as rows of a linear layer, padded with zeros to a multiple of eight inputs."""
-        rows = self.w["patch_embed.proj.weight"].flatten(1)
-        return F.pad(rows, (0, -rows.shape[1] % 8)).contiguous()
-
-    def start_tokens(self, gh: int, gw: int) -> torch.Tensor:
-        """What a `gh x gw` image's patch products are added to, per token: position embedding plus the patch bias, and
-        plus the class token in the first row."""
-        key = (gh, gw)
-        if key not in self._start:
-            pos = self.pos_embed_fp32(gh, gw)[0]
-            cls = self.w["cls_token"].reshape(1, -1).float()
-            bias = self.w["patch_embed.proj.bias"].float()
-            self._start[key] = torch.cat([pos[:1] + cls, pos[1:] + bias]).to(self.dtype).contiguous()
-        return self._start[key]
-
     def _forward_native(self, images: torch.Tensor, count: int, taps: tuple[int, ...]) -> list[torch.Tensor] | None:
         """Normalised tokens after the blocks in `taps`, of the first `count` blocks, as one native call; None when the images
         are not of a form it takes."""
-        ps = self.cfg.patch
-        if self._native is None or images.dim() != 4 or images.shape[1] != 3 or images.device.type != "cuda" or images.numel() == 0:  # noqa: PLR2004
+        w, ps, native = self.w, self.cfg.patch, self._native_now()
+        if native is None or images.dim() != 4 or images.shape[1] != 3 or images.device.type != "cuda" or images.numel() == 0:  # noqa: PLR2004
             return None
         if images.dtype not in (torch.float32, self.dtype):
             images = images.to(self.dtype)
@@ -190,15 +182,17 @@ class ViTEncoder:
         gh, gw = height // ps, width // ps
         if width % 2 or gh == 0 or gw == 0 or images.data_ptr() % 16:
             return None
-        start = self.start_tokens(gh, gw)
+        if (gh, gw) not in self._pos32:
+            self._pos32[gh, gw] = self.pos_embed_fp32(gh, gw).contiguous()
         extra = {  # "images": any address, the description only needs to know that there are images
             "images": 1, "image_dtype": _lib.F32 if images.dtype == torch.float32 else encoder._DTYPES[self.dtype],  # noqa: SLF001
-            "height": height, "width": width, "patch": ps, "patch_w": self._patch_w.data_ptr(), "patch_k": self._patch_w.shape[1],
-            "start": start.data_ptr(), "norm_w": self.w["norm.weight"].data_ptr(), "norm_b": self.w["norm.bias"].data_ptr(),
+            "height": height, "width": width, "patch": ps, "patch_w": w["patch_embed.proj.weight"].data_ptr(), "patch_w_raw": 1, "patch_k": (3 * ps * ps + 7) // 8 * 8,
+            "start": self._pos32[gh, gw].data_ptr(), "start_f32": 1, "patch_b": w["patch_embed.proj.bias"].data_ptr(), "first": w["cls_token"].data_ptr(),
+            "norm_w": w["norm.weight"].data_ptr(), "norm_b": w["norm.bias"].data_ptr(),
         }  # fmt: skip
-        described = self._native.describe(b, (gh, gw), 1, 0, count, extra)
+        described = native.describe(b, (gh, gw), 1, 0, count, extra)
         outs = [torch.empty((b, 1 + gh * gw, self.cfg.dim), dtype=self.dtype, device=images.device) for _ in taps]
-        self._native.launch(described, images.device, images=images, taps=list(zip(taps, outs)))
+        native.launch(described, images.device, images=images, taps=list(zip(taps, outs)))
         return outs
 
     def pos_embed(self, gh: int, gw: int) -> torch.Tensor:
@@ -259,9 +253,10 @@ class ViTEncoder:
         src/fastforks/shared/timm_blocks/net/vit.py:60-62). q, k, v are strided views of the packed qkv tensor."""
         w, cfg, p = self.w, self.cfg, f"blocks.{i}."
         b, n, c = x.shape
-        native = self._native is not None and not (x.requires_grad and torch.is_grad_enabled())
-        if native and x.is_cuda and x.dtype == self.dtype and x.is_contiguous() and x.numel() > 0 and x.data_ptr() % 16 == 0:
-            self._native.launch(self._native.describe(b, (n, 1), 0, i, 1, {"x": 1}), x.device, x=x)
+        native = self._native_now()
+        if (native is not None and not (x.requires_grad and torch.is_grad_enabled()) and x.is_cuda and x.dtype == self.dtype and x.is_contiguous()
+                and x.numel() > 0 and x.data_ptr() % 16 == 0):  # fmt: skip
+            native.launch(native.describe(b, (n, 1), 0, i, 1, {"x": 1}), x.device, x=x)
             return x
         heads = cfg.heads
         ls1, ls2 = (p + "ls1.gamma", p + "ls2.gamma") if cfg.layerscale else (None, None)

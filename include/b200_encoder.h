@@ -94,6 +94,14 @@ typedef struct B200EncoderArgs {
   void* neck_out; /* [batch, channels, grid_h, grid_w] */
   int32_t neck_channels;
   float neck_eps;
+  /* Parameters as a model holds them, so that a forward reads the model's own tensors and no prepared copies (all 0 / NULL:
+   * the prepared forms above) */
+  const void* patch_b;  /* [dim], added to the start of every patch token, or NULL */
+  const void* first;    /* [prefix, dim], added to the start of the prefix tokens (class token), or NULL */
+  int32_t start_f32;    /* start is fp32 */
+  int32_t patch_w_raw;  /* patch_w is [dim, 3 * patch * patch], without the columns up to patch_k */
+  int32_t neck_w1_conv; /* neck_w1 is [channels, channels, 3, 3]: (channel, kernel row, kernel column) */
+  int32_t reserved;
 } B200EncoderArgs;
 
 /* Bytes of workspace a call with these sizes needs (pointers are not looked at, except `blocks` for the windows and

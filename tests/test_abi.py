@@ -59,6 +59,20 @@ def test_ctypes_struct_matches_the_c_struct(tmp_path: Path) -> None:
         assert int(out[f]) == getattr(_lib.B200AttnArgs, f).offset, f
 
 
+@pytest.mark.skipif(shutil.which("gcc") is None, reason="needs gcc")
+def test_ctypes_structs_of_the_encoder_match_the_c_structs(tmp_path: Path) -> None:
+    structs = (_lib.B200EncoderBlock, _lib.B200EncoderTap, _lib.B200EncoderArgs)
+    want = {f"{s.__name__}.{f}": getattr(s, f).offset for s in structs for f, *_ in s._fields_}  # noqa: SLF001
+    want |= {s.__name__: ctypes.sizeof(s) for s in structs}
+    src = tmp_path / "layout.c"
+    lines = "\n".join(f'  printf("{name} %zu\n", {"offsetof(" + name.replace(".", ", ") + ")" if "." in name else "sizeof(" + name + ")"});' for name in want)
+    src.write_text(f'#include <stdio.h>\n#include <stddef.h>\n#include "{ROOT / "include" / "b200_encoder.h"}"\nint main(void) {{\n{lines}\n  return 0;\n}}\n')
+    exe = tmp_path / "layout"
+    subprocess.run(["gcc", "-std=c99", "-Wall", "-Werror", "-o", str(exe), str(src)], check=True)
+    out = subprocess.run([str(exe)], check=True, capture_output=True, text=True).stdout.splitlines()
+    assert {name: int(offset) for name, offset in (line.split() for line in out)} == want
+
+
 def _args(**kw: object) -> _lib.B200AttnArgs:
     a = _lib.B200AttnArgs()
     a.struct_size = ctypes.sizeof(_lib.B200AttnArgs)

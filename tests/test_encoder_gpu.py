@@ -15,6 +15,8 @@ import torch.nn.functional as F  # noqa: N812
 import fastforks_b200 as ff
 from conftest import assert_close
 from fastforks_b200 import encoder
+from fastforks_b200.sam import SamConfig, SamEncoder, sam_state_shapes
+from fastforks_b200.vit import ViTConfig, ViTEncoder, state_shapes
 
 pytestmark = pytest.mark.gpu
 
@@ -120,3 +122,58 @@ def test_patches_and_neck(b: int, grid: tuple[int, int], patch: int, extra: tupl
         ref = F.layer_norm(y.permute(0, 2, 3, 1), (channels,), n["n1_w"], n["n1_b"], 1e-6).permute(0, 3, 1, 2)
     assert ff.device_status() == 0
     assert_close(out.float().cpu().numpy(), ref.cpu().numpy(), unit_scale=False, what=f"{b} {grid} {patch} {channels}")
+
+
+def random_state(shapes: dict[str, tuple[int, ...]], seed: int) -> dict[str, torch.Tensor]:
+    """Every parameter different from those of another seed, but `pos_embed`, which an encoder may read once."""
+    gen = torch.Generator().manual_seed(seed)
+    state = {k: torch.randn(*s, generator=gen) * (0.1 if len(s) > 1 else 0.3) + (1.0 if "norm" in k and k.endswith("weight") else 0.0) for k, s in shapes.items()}
+    state["pos_embed"] = torch.randn(*shapes["pos_embed"], generator=torch.Generator().manual_seed(0))
+    return state
+
+
+def give(held: dict[str, torch.Tensor], values: dict[str, torch.Tensor], how: str) -> None:
+    for name, value in values.items():
+        if how == "in place":
+            held[name].copy_(value)
+        elif how == "entry":
+            held[name] = value.clone()
+        else:
+            held[name].data = value.clone()
+
+
+@pytest.mark.parametrize("how", ["in place", "entry", "storage"])
+@pytest.mark.parametrize(("patch", "ffn", "layerscale"), [(14, "mlp", True), (16, "swiglu", False)])
+def test_vit_forward_follows_its_parameters(how: str, patch: int, ffn: str, layerscale: bool) -> None:  # noqa: FBT001
+    """An encoder whose parameters were written in place, replaced in its dictionaries or given other storage computes what a
+    new encoder of those parameters does."""
+    cfg = ViTConfig(128, 2, 2, patch, 4 * patch, ffn=ffn, layerscale=layerscale)
+    enc = ViTEncoder(cfg, random_state(state_shapes(cfg), 1), device="cuda")
+    images = torch.rand(2, 3, 3 * patch, 5 * patch, generator=torch.Generator().manual_seed(3)).cuda()
+    before = enc(images)
+    other = ViTEncoder(cfg, random_state(state_shapes(cfg), 2), device="cuda")
+    give(enc.w, other.w, how)
+    give(enc.scales, other.scales, how)
+    with torch.no_grad():
+        x = torch.randn(1, 9, 128, generator=torch.Generator().manual_seed(4)).half().cuda()
+        assert torch.equal(enc.block(1, x.clone()), other.block(1, x.clone()))
+    after, want = enc(images), other(images)
+    assert torch.equal(after, want) and not torch.equal(after, before)
+    assert all(torch.equal(a, b) for a, b in zip(enc.intermediate(images, (0, 1)), other.intermediate(images, (0, 1)), strict=True))
+    assert ff.device_status() == 0
+
+
+@pytest.mark.parametrize("how", ["in place", "entry", "storage"])
+@pytest.mark.parametrize("patch", [14, 16])
+def test_sam_forward_follows_its_parameters(how: str, patch: int) -> None:
+    cfg = SamConfig(img=6 * patch, patch=patch, dim=128, depth=2, heads=2, out_chans=24, window=4, global_blocks=(1,))
+    enc = SamEncoder(cfg, random_state(sam_state_shapes(cfg), 1), device="cuda")
+    images = torch.rand(2, 3, cfg.img, cfg.img, generator=torch.Generator().manual_seed(3)).cuda()
+    before = enc(images)
+    state = random_state(sam_state_shapes(cfg), 2)
+    state["pos_embed"] = state["pos_embed"] + 1.0
+    other = SamEncoder(cfg, state, device="cuda")
+    give(enc.w, other.w, how)
+    after, want = enc(images), other(images)
+    assert torch.equal(after, want) and not torch.equal(after, before)
+    assert ff.device_status() == 0

@@ -186,3 +186,26 @@ def test_host_attention_contract_is_checked_before_any_copy() -> None:
         check([x, torch.zeros(1, 5, 3, 4, 64, dtype=torch.float16)], [o, torch.zeros(1, 5, 4, 64, dtype=torch.float16)])
     with pytest.raises(ValueError, match="empty"):
         check([x[:0]], [o[:0]])
+
+
+@pytest.mark.parametrize("native", [True, False])
+def test_a_snapshot_sees_tensors_that_were_replaced(native: bool, monkeypatch: pytest.MonkeyPatch) -> None:  # noqa: FBT001
+    """What an encoder's table of parameter addresses rests on: values written in place leave it valid, another tensor, other
+    storage, another shape, one more or one less do not."""
+    from fastforks_b200 import _lib, encoder
+
+    monkeypatch.setattr(_lib, "fast", _lib.host() if native else None)
+    a = {"x": torch.zeros(4, 6), "y": torch.zeros(3, dtype=torch.float16)}
+    b = {"x": torch.zeros(2)}
+    snap = encoder.Snapshot(a, b)
+    a["x"].add_(1.0)
+    assert not snap.changed(a, b)
+    assert snap.changed(a) and snap.changed(b, a) and snap.changed({**a, "z": torch.zeros(1)}, b)
+    assert snap.changed({"x": a["x"].clone(), "y": a["y"]}, b) and snap.changed({"x": a["x"], "y": 3.0}, b) if native else True
+    a["x"].t_()
+    assert snap.changed(a, b)
+    a["x"].t_()
+    assert not snap.changed(a, b)
+    b["x"].data = b["x"].clone()
+    assert snap.changed(a, b)
+    assert not encoder.Snapshot(a, b).changed(a, b)
