@@ -65,7 +65,7 @@ def test_ctypes_structs_of_the_encoder_match_the_c_structs(tmp_path: Path) -> No
     want = {f"{s.__name__}.{f}": getattr(s, f).offset for s in structs for f, *_ in s._fields_}  # noqa: SLF001
     want |= {s.__name__: ctypes.sizeof(s) for s in structs}
     src = tmp_path / "layout.c"
-    lines = "\n".join(f'  printf("{name} %zu\n", {"offsetof(" + name.replace(".", ", ") + ")" if "." in name else "sizeof(" + name + ")"});' for name in want)
+    lines = "\n".join(f'  printf("{name} %zu\\n", {"offsetof(" + name.replace(".", ", ") + ")" if "." in name else "sizeof(" + name + ")"});' for name in want)
     src.write_text(f'#include <stdio.h>\n#include <stddef.h>\n#include "{ROOT / "include" / "b200_encoder.h"}"\nint main(void) {{\n{lines}\n  return 0;\n}}\n')
     exe = tmp_path / "layout"
     subprocess.run(["gcc", "-std=c99", "-Wall", "-Werror", "-o", str(exe), str(src)], check=True)
