@@ -73,9 +73,10 @@ __device__ __forceinline__ uint32_t gemm_pack2(float lo, float hi) {
 // 0.5 v (1 + erf) loses digits. Phi(-x) = exp(-x^2 / 2) t P(t), t = 1 / (1 + 0.3 x), where P is a degree-7 least-maximum
 // fit of 0.5 erfcx(x / sqrt 2) / t on 0 <= x <= 13.5 (relative error 1.3e-7; the whole within 2e-6 of v Phi(v) down to
 // v = -5, where erff gave 1e-3). Two MUFU operations and a dozen multiply-adds: a third of the time of erff, which took
-// longer than the products of a 256 x 256 tile at k = 768.
+// longer than the products of a 256 x 256 tile at k = 768. max(v, 0) is written v / 2 + |v| / 2, which keeps NaN and gives
+// it for -inf as v Phi(v) does; the tail's argument ends where the tail is zero, so that +inf meets no inf * 0.
 __device__ __forceinline__ float gelu_erf(float v) {
-  const float x = fabsf(v);
+  const float a = fabsf(v), x = fminf(a, 64.f);
   float t, e;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(t) : "f"(fmaf(x, 0.3f, 1.f)));
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(x * x * -0.72134752f));
@@ -87,7 +88,7 @@ __device__ __forceinline__ float gelu_erf(float v) {
   p = fmaf(p, t, 0.0996374786f);
   p = fmaf(p, t, 0.120798357f);
   p = fmaf(p, t, 0.119626388f);
-  return fmaxf(v, 0.f) - x * (t * p) * e;
+  return fmaf(0.5f, v, 0.5f * a) - x * (t * p) * e;
 }
 
 template <int ACT>

@@ -64,6 +64,19 @@ def test_activations(act: int, dtype: str) -> None:
     check(ff.gemm(x, w, bias, act=act), x, w, bias, act=act, what=f"act {act} {dtype}")
 
 
+@pytest.mark.parametrize(("m", "n", "k"), [(1, 16, 8), (9500, 2056, 72)])  # the split and the pair kernel
+@pytest.mark.parametrize("act", [ff.ACT_GELU, ff.ACT_GELU_TANH])
+def test_activations_at_the_ends_of_the_range(act: int, m: int, n: int, k: int) -> None:
+    """Infinities, NaN and the largest finite values give what torch's GELU gives (a product of zeros, the values as bias)."""
+    bias = torch.zeros(n)
+    big = torch.finfo(torch.bfloat16).max
+    bias[:8] = torch.tensor([float("inf"), -float("inf"), float("nan"), big, -big, 1e20, -1e20, -200.0])
+    bias = bias.bfloat16().cuda()
+    got = ff.gemm(torch.zeros(m, k, dtype=torch.bfloat16, device="cuda"), torch.zeros(n, k, dtype=torch.bfloat16, device="cuda"), bias, act=act)
+    want = torch.nn.functional.gelu(bias.float(), approximate="tanh" if act == ff.ACT_GELU_TANH else "none").bfloat16()
+    assert torch.equal(got.nan_to_num(nan=7.0, posinf=8.0, neginf=9.0), want.expand(m, n).nan_to_num(nan=7.0, posinf=8.0, neginf=9.0)), (got[0, :8], want[:8])
+
+
 @pytest.mark.parametrize(("m", "n", "k"), [(300, 264, 136), (5480, 1024, 4096), (1370, 1536, 1536)])
 @pytest.mark.parametrize("dtype", ["fp16", "bf16"])
 def test_layerscale_and_in_place_residual(m: int, n: int, k: int, dtype: str) -> None:
