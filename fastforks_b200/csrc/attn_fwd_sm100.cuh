@@ -346,12 +346,27 @@ __device__ __forceinline__ uint4 load_rel_chunk(const uint16_t* src, int left) {
   }
   return make_uint4(w[0], w[1], w[2], w[3]);
 }
-// Two packed 16-bit values with infinities replaced by the largest finite value of their sign.
-__device__ __forceinline__ uint32_t clamp_finite2(uint32_t v, bool is_half) {
-  const uint32_t inf_lo = is_half ? 0x7c00u : 0x7f80u;
-  if ((v & 0x7fffu) == inf_lo) v -= 1;
-  if (((v >> 16) & 0x7fffu) == inf_lo) v -= 0x10000u;
+// Two packed 16-bit values with infinities replaced by the largest finite value of their sign; *any: whether there was one.
+__device__ __forceinline__ uint32_t clamp_finite2(uint32_t v, uint32_t inf, bool* any) {
+  const bool lo = (v & 0x7fffu) == inf, hi = ((v >> 16) & 0x7fffu) == inf;
+  *any |= lo || hi;
+  if (lo) v -= 1;
+  if (hi) v -= 0x10000u;
   return v;
+}
+// What the softmax of a row's logits comes to, as far as the infinities in its tables decide it: NaN if there is a +inf or if a
+// whole table is -inf (no key is left), else 0.
+__device__ __forceinline__ float infinite_row(const uint16_t* h, int nh, const uint16_t* w, int nw, uint32_t inf) {
+  bool positive = false, none_h = true, none_w = true;
+  for (int i = 0; i < nh; ++i) {
+    positive |= h[i] == inf;
+    none_h &= h[i] == (inf | 0x8000u);
+  }
+  for (int i = 0; i < nw; ++i) {
+    positive |= w[i] == inf;
+    none_w &= w[i] == (inf | 0x8000u);
+  }
+  return positive || none_h || none_w ? __int_as_float(0x7fffffff) : 0.f;
 }
 
 // n / d for the divisors the host knows at launch: magic = ceil(2^64 / d) (0 stands for d == 1), exact for every
@@ -1331,7 +1346,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           const uint16_t* const src_h = static_cast<const uint16_t*>(p.bias.ptr) + bias_row;
           const uint16_t* const src_w = static_cast<const uint16_t*>(p.bias2.ptr) + bias2_row;
           const int chunks = 2 * p.rel_steps;
-          const bool is_half = p.bias.dtype == 0;
+          const uint32_t inf = p.bias.dtype == 0 ? 0x7c00u : 0x7f80u;
+          bool any_inf = false;
           auto stage_row = [&](auto align_tag) {
 #pragma unroll 1
             for (int first = 0; first < chunks; first += 8) {
@@ -1346,9 +1362,11 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
 #pragma unroll
               for (int u = 0; u < 8; ++u) {
                 if (first + u >= chunks) break;
-                // an infinity would meet zeros in E: it goes in as the largest finite value
+                // An infinity would meet zeros in E: it goes in as the largest finite value, which masks a key just as well beside
+                // others that are some thousands above it.
                 st_shared_v4(row + (first >> 3) * kTileBytes + ((u ^ (row_in_tile & 7)) << 4),
-                             make_uint4(clamp_finite2(v[u].x, is_half), clamp_finite2(v[u].y, is_half), clamp_finite2(v[u].z, is_half), clamp_finite2(v[u].w, is_half)));
+                             make_uint4(clamp_finite2(v[u].x, inf, &any_inf), clamp_finite2(v[u].y, inf, &any_inf), clamp_finite2(v[u].z, inf, &any_inf),
+                                        clamp_finite2(v[u].w, inf, &any_inf)));
               }
             }
           };
@@ -1357,6 +1375,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           else stage_row(std::integral_constant<int, 2>{});
           fence_proxy_async_smem();
           warp_arrive(&sm.r_full[t], lane);
+          if (__builtin_expect(any_inf, 0)) l_sum = infinite_row(src_h, p.rel_kh, src_w, p.rel_kw, inf);  // a NaN stays in the sum
         }
         if constexpr (BIAS == kBiasDecomposed14) {
           // This thread's rows, read back by this thread only: no synchronisation needed.

@@ -344,6 +344,29 @@ def test_decomposed_bias_masks_and_other_scales() -> None:
         assert_close(got.float().cpu().numpy(), ref, unit_scale=True, what=f"scale {scale}")
 
 
+@pytest.mark.parametrize("hw", [(20, 20), (64, 64), (9, 31), (2, 5)])
+@pytest.mark.parametrize("dtype", ["fp16", "bf16"])
+@pytest.mark.parametrize("scale", [0.125, 0.1])
+def test_decomposed_bias_rows_without_a_key_and_positive_infinities(hw: tuple[int, int], dtype: str, scale: float) -> None:
+    """A query whose keys are all masked (every value of either table -inf) and one with +inf in a table get NaN, as the softmax
+    of such logits is, also where the tables are an operand of the tensor cores; the queries beside them are not touched."""
+    gen = torch.Generator(device="cuda").manual_seed(hw[0])
+    n, nq = hw[0] * hw[1], 300
+    q = torch.randn(1, 2, nq, 64, generator=gen, device="cuda").to(DTYPES[dtype])
+    k, v = (torch.randn(1, 2, n, 64, generator=gen, device="cuda").to(DTYPES[dtype]) for _ in range(2))
+    rel_h, rel_w = (torch.randn(1, 2, nq, side, generator=gen, device="cuda").to(DTYPES[dtype]) for side in hw)
+    inf = float("inf")
+    rel_h[0, 0, 3], rel_w[0, 0, 4], rel_h[0, 1, 200, hw[0] - 1], rel_w[0, 1, 131, 0] = -inf, -inf, inf, inf
+    rel_h[0, 1, 9, 1:], rel_w[0, 0, 290, : hw[1] - 1] = -inf, -inf  # one row or column of keys left
+    rel_h[0, 0, 5, 0], rel_w[0, 0, 5, 1:] = -inf, -inf
+    logits = torch.einsum("bhqd,bhkd->bhqk", q.float(), k.float()) * scale + (rel_h.float()[..., :, None] + rel_w.float()[..., None, :]).reshape(1, 2, nq, n)
+    ref = torch.einsum("bhqk,bhkd->bhqd", logits.softmax(-1), v.float())
+    assert int(ref[..., 0].isnan().sum()) == 4
+    got = ff.scaled_dot_product_attention(q, k, v, rel=(rel_h, rel_w), scale=scale)
+    assert ff.device_status() == 0
+    assert_close(got.float().cpu().numpy(), ref.cpu().numpy(), unit_scale=True, what=f"{hw} {dtype} {scale}")
+
+
 def oracle_of_heads(qkv: torch.Tensor, picks: list[tuple[int, int]], scale: float, rel: tuple | None = None) -> np.ndarray:
     """Oracle output `[len(picks), N, 64]` for the chosen (batch, head) pairs of a packed `[B, N, 3, H, 64]` tensor,
     one head at a time (a dense 4096 x 4096 bias is 64 MB per head)."""
