@@ -248,7 +248,8 @@ def attention(  # noqa: PLR0913
     # For launch-bound shapes (one image of 197 tokens) the checks and the ctypes set-up below cost more than the kernel:
     # the plain call goes through the host extension.
     host = _lib.fast
-    if host is not None and not _general_merge and not _bias_as_given and layout in LAYOUTS and schedule in _SCHEDULES and (rel is None or len(rel) == 2):  # noqa: PLR2004
+    plain_rel = rel is None or (isinstance(rel, (tuple, list)) and len(rel) == 2 and rel[0] is not None)  # noqa: PLR2004
+    if host is not None and not _general_merge and not _bias_as_given and layout in LAYOUTS and schedule in _SCHEDULES and plain_rel:
         rel_h, rel_w = rel if rel is not None else (None, None)
         done = host.attention(q, k, v, scale, layout == "bnhd", _SCHEDULES[schedule], out, bias, rel_h, rel_w, False)  # noqa: FBT003
         if done is not None:

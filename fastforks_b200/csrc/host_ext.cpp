@@ -94,6 +94,14 @@ bool number(PyObject* o, double* v) {
   return true;
 }
 
+// An int and nothing that converts to one, as ctypes has it for the fields these go to.
+bool integer(PyObject* o, int64_t* v) {
+  if (!PyLong_Check(o)) return false;
+  int overflow = 0;
+  *v = PyLong_AsLongLongAndOverflow(o, &overflow);
+  return overflow == 0 && *v >= INT32_MIN && *v <= INT32_MAX;
+}
+
 struct View {  // [batch, tokens, heads, 64] in either layout
   int64_t b, n, h, sb, sn, sh;
 };
@@ -141,8 +149,8 @@ PyObject* py_attention(PyObject*, PyObject* const* args, Py_ssize_t n) {
   double scale = 0.125;
   if (args[3] != Py_None && !number(args[3], &scale)) Py_RETURN_NONE;
   a.scale = static_cast<float>(scale);
-  double schedule = 0;
-  if (!number(args[5], &schedule)) Py_RETURN_NONE;
+  int64_t schedule = 0;
+  if (!integer(args[5], &schedule)) Py_RETURN_NONE;
   a.schedule = static_cast<int32_t>(schedule);
 
   if (args[7] != Py_None) {  // a 16-bit bias the kernel fetches in tiles; a broadcast dimension has stride 0
@@ -235,8 +243,8 @@ PyObject* py_gemm(PyObject*, PyObject* const* args, Py_ssize_t n) {
   a.m = static_cast<int32_t>(m);
   a.n = static_cast<int32_t>(cols);
   a.k = static_cast<int32_t>(k);
-  double act = 0;
-  if (!number(args[3], &act)) Py_RETURN_NONE;
+  int64_t act = 0;
+  if (!integer(args[3], &act)) Py_RETURN_NONE;
   a.act = static_cast<int32_t>(act);
   if (!rows_of(*x, m, k, &a.lda)) Py_RETURN_NONE;
   a.x = x->data_ptr();
@@ -312,10 +320,9 @@ PyObject* py_rope(PyObject*, PyObject* const* args, Py_ssize_t n) {
 PyObject* py_rel_terms(PyObject*, PyObject* const* args, Py_ssize_t n) {
   if (n != 4) Py_RETURN_NONE;
   const at::Tensor *q = tensor_of(args[0]), *ph = tensor_of(args[1]), *pw = tensor_of(args[2]);
-  double side_number = 0;
-  if (q == nullptr || ph == nullptr || pw == nullptr || !number(args[3], &side_number)) Py_RETURN_NONE;
+  int64_t side = 0;
+  if (q == nullptr || ph == nullptr || pw == nullptr || !integer(args[3], &side)) Py_RETURN_NONE;
   const c10::DeviceIndex device = c10::cuda::current_device();
-  const int64_t side = static_cast<int64_t>(side_number);
   View v;
   if (!half_type(*q) || !plain(*q, device) || !view_of(*q, true, &v) || side < 2 || side > 64 || v.n != side * side || v.b > INT32_MAX || v.h > INT32_MAX) Py_RETURN_NONE;
   for (const at::Tensor* t : {ph, pw})

@@ -614,6 +614,29 @@ def test_repeated_geometry_takes_the_remembered_launch_and_still_checks() -> Non
         ff.attention(shifted, shifted, shifted, layout="bnhd")
 
 
+def test_repeated_calls_refuse_what_the_first_one_refuses() -> None:
+    """Arguments that are refused before anything was launched stay refused once the host extension takes repeated calls."""
+    qkv = packed_qkv(1, 16, 2, torch.float16, 1.0, seed=3)
+    q, k, v = qkv.unbind(2)
+    rel = tuple(torch.zeros(1, 2, 16, 4, dtype=torch.float16, device="cuda") for _ in range(2))
+    x = torch.zeros(16, 64, dtype=torch.float16, device="cuda")
+    w = torch.zeros(32, 64, dtype=torch.float16, device="cuda")
+    pos = torch.zeros(7, 64, dtype=torch.float16, device="cuda")
+    for _ in range(2):
+        with pytest.raises(AttributeError):
+            ff.attention(q, k, v, layout="bnhd", rel=(None, None))
+        with pytest.raises(TypeError):
+            ff.gemm(x, w, act=5.0)
+        with pytest.raises(TypeError):
+            ff.sam_rel_terms(q, pos, pos, 4.0)
+        with pytest.raises(ValueError, match="too many values"):
+            ff.attention(q, k, v, layout="bnhd", rel=(*rel, None))
+        given = ff.attention(q, k, v, layout="bnhd", rel=(t for t in rel))  # any two tables that can be unpacked
+        assert torch.equal(given, ff.attention(q, k, v, layout="bnhd", rel=rel))
+        ff.gemm(x, w, act=ff.ACT_GELU)
+        ff.sam_rel_terms(q, pos, pos, 4)
+
+
 @pytest.mark.parametrize(("b", "n", "h"), [(1, 4096, 12), (2, 1370, 16), (1, 1370, 6), (3, 900, 7), (1, 197, 12), (5, 640, 31)])
 def test_mixed_one_and_two_tile_items_cover_every_query_tile_once(b: int, n: int, h: int) -> None:
     """Grids smaller than, about equal to and larger than the SM count, where the host splits each head's query
