@@ -56,7 +56,8 @@ class NativeEncoder:
     def __init__(self, blocks: Sequence[dict], *, dtype: torch.dtype, dim: int, heads: int, hidden: int, ffn: int, eps: float) -> None:  # noqa: PLR0913
         self.dtype, self.dim, self.heads, self.hidden, self.ffn, self.eps = dtype, dim, heads, hidden, ffn, eps
         self._keep = [dict(b) for b in blocks]
-        self.blocks = (_lib.B200EncoderBlock * max(1, len(blocks)))()
+        self.count = len(blocks)
+        self.blocks = (_lib.B200EncoderBlock * max(1, self.count))()
         for entry, tensors in zip(self.blocks, blocks):
             for name in BLOCK_TENSORS:
                 t = tensors.get(name)
@@ -69,7 +70,15 @@ class NativeEncoder:
         self._described: dict[tuple, tuple] = {}  # geometry -> (argument description, workspace bytes)
 
     def describe(self, batch: int, grid: tuple[int, int], prefix: int, first: int, count: int, extra: dict) -> tuple:
-        """The argument description of a geometry and its workspace size; `extra`: further scalar and pointer fields."""
+        """The argument description of `count` blocks from block `first` on at a geometry, and its workspace size; `extra`: further
+        scalar and pointer fields.
+
+        Raises:
+            ValueError: There are no such blocks, or the library cannot take the geometry.
+        """
+        if not 0 <= first <= first + count <= self.count:
+            msg = f"encoder: blocks {first} .. {first + count - 1} of {self.count}"
+            raise ValueError(msg)
         key = (batch, grid, prefix, first, count, tuple(sorted(extra.items())))
         found = self._described.get(key)
         if found is None:
