@@ -67,6 +67,7 @@ class NativeEncoder:
                         raise ValueError(msg)
                     setattr(entry, name, t.data_ptr())
             entry.window = tensors.get("window", 0)
+        self.device = next((t.device for b in blocks for t in b.values() if isinstance(t, torch.Tensor)), None)
         self._described: dict[tuple, tuple] = {}  # geometry -> (argument description, workspace bytes)
 
     def describe(self, batch: int, grid: tuple[int, int], prefix: int, first: int, count: int, extra: dict) -> tuple:
@@ -100,13 +101,21 @@ class NativeEncoder:
 
     def launch(self, described: tuple, device: torch.device, *, x: torch.Tensor | None = None, images: torch.Tensor | None = None,
                taps: Sequence[tuple[int, torch.Tensor]] = (), neck_out: torch.Tensor | None = None) -> None:  # fmt: skip
-        """Launch a described forward on the current stream of `device`."""
+        """Launch a described forward on the current stream of `device`, which is the parameters'.
+
+        Raises:
+            ValueError: A tensor or the parameters are on another device.
+        """
+        tensors = [t for t in (x, images, neck_out, *(out for _, out in taps)) if t is not None]
+        if any(t.device != device for t in tensors) or self.device not in (None, device):
+            msg = f"encoder: parameters on {self.device}, tensors on {[str(t.device) for t in tensors]}, launch on {device}"
+            raise ValueError(msg)
         template, size = described
         a = _lib.B200EncoderArgs.from_buffer_copy(template)
-        index = device.index if device.index is not None else torch.cuda.current_device()
+        index = device.index  # a tensor's device has one
         if index != torch.cuda.current_device():
             with torch.cuda.device(index):
-                self.launch(described, torch.device("cuda", index), x=x, images=images, taps=taps, neck_out=neck_out)
+                self.launch(described, device, x=x, images=images, taps=taps, neck_out=neck_out)
             return
         workspace = torch.empty(max(size, 1), dtype=torch.uint8, device=device)
         a.workspace, a.workspace_bytes = workspace.data_ptr(), size

@@ -173,7 +173,7 @@ class ViTEncoder:
         """Normalised tokens after the blocks in `taps`, of the first `count` blocks, as one native call; None when the images
         are not of a form it takes."""
         w, ps, native = self.w, self.cfg.patch, self._native_now()
-        if native is None or count > self.cfg.depth or images.dim() != 4 or images.shape[1] != 3 or images.device.type != "cuda" or images.numel() == 0:  # noqa: PLR2004
+        if native is None or count > self.cfg.depth or images.dim() != 4 or images.shape[1] != 3 or images.device != native.device or images.numel() == 0:  # noqa: PLR2004
             return None
         if images.dtype not in (torch.float32, self.dtype):
             images = images.to(self.dtype)
@@ -254,8 +254,8 @@ class ViTEncoder:
         w, cfg, p = self.w, self.cfg, f"blocks.{i}."
         b, n, c = x.shape
         native = self._native_now()
-        if (native is not None and type(i) is int and 0 <= i < cfg.depth and not (x.requires_grad and torch.is_grad_enabled()) and x.is_cuda and x.dtype == self.dtype and x.is_contiguous()
-                and x.numel() > 0 and x.data_ptr() % 16 == 0):  # fmt: skip
+        if (native is not None and type(i) is int and 0 <= i < cfg.depth and not (x.requires_grad and torch.is_grad_enabled()) and x.device == native.device
+                and x.dtype == self.dtype and c == cfg.dim and x.is_contiguous() and x.numel() > 0 and x.data_ptr() % 16 == 0):  # fmt: skip
             native.launch(native.describe(b, (n, 1), 0, i, 1, {"x": 1}), x.device, x=x)
             return x
         heads = cfg.heads

@@ -27,11 +27,12 @@ CFG = ViTConfig(128, 2, 2, 14, 56)
 
 @pytest.fixture
 def vit(monkeypatch: pytest.MonkeyPatch) -> ViTEncoder:
-    """A ViT on the CPU that would take its native form where the arguments allow it; a launch fails the test."""
+    """A ViT on the CPU that takes its native form where the arguments allow it; `launched` lists the launches, which do nothing."""
     enc = ViTEncoder(CFG, seeded_state(CFG), device="cpu", dtype=torch.float16)
     enc.scales = {k: v.float() for k, v in enc.scales.items()}
     native = enc._make_native()  # noqa: SLF001
-    monkeypatch.setattr(native, "launch", lambda *a, **k: pytest.fail("launched"))
+    enc.launched = []
+    monkeypatch.setattr(native, "launch", lambda described, *a, **k: enc.launched.append(described[0].n_blocks))
     monkeypatch.setattr(enc, "_native_now", lambda: native)
     monkeypatch.setattr(Flash64, "_run", staticmethod(lambda variant, q, k, v, scale: v.contiguous()))
     return enc
@@ -50,5 +51,30 @@ def test_blocks_that_do_not_exist_are_refused(vit: ViTEncoder, first: int, count
 def test_block_numbers_out_of_range_raise_as_the_layers_do(vit: ViTEncoder, i: int) -> None:
     with pytest.raises(KeyError):
         vit.block(i, torch.zeros(1, 5, 128, dtype=torch.float16))
+    assert vit.launched == []
     with pytest.raises(KeyError):
         vit.intermediate(torch.zeros(1, 3, 28, 28), (0, 2))
+    assert vit.launched == [1, 1]  # the blocks that do exist, one by one
+    vit.block(1, torch.zeros(1, 5, 128, dtype=torch.float16))
+    vit.intermediate(torch.zeros(1, 3, 28, 28), (0, 1))
+    assert vit.launched == [1, 1, 1, 2]
+
+
+@pytest.mark.parametrize("width", [64, 120, 192, 1])
+def test_tokens_of_another_width_are_left_to_the_layers(vit: ViTEncoder, width: int) -> None:
+    with pytest.raises(RuntimeError, match="normalized_shape"):
+        vit.block(0, torch.zeros(1, 5, width, dtype=torch.float16))
+    assert vit.launched == []
+
+
+def test_tensors_on_another_device_are_refused(vit: ViTEncoder) -> None:
+    with pytest.raises(RuntimeError):  # torch's device mismatch
+        vit.block(0, torch.zeros(1, 5, 128, dtype=torch.float16, device="meta"))
+    assert vit._forward_native(torch.zeros(1, 3, 28, 28, device="meta"), 2, (1,)) is None  # noqa: SLF001
+    native = encoder.NativeEncoder([dict(vit.w)], dtype=torch.float16, dim=128, heads=2, hidden=512, ffn=encoder.FFN_GELU, eps=1e-6)
+    described = native.describe(1, (4, 1), 0, 0, 0, {"x": 1})
+    meta = torch.zeros(4, 128, dtype=torch.float16, device="meta")
+    with pytest.raises(ValueError, match="parameters on cpu"):
+        native.launch(described, meta.device, x=meta)
+    with pytest.raises(ValueError, match="launch on cpu"):
+        native.launch(described, torch.device("cpu"), x=meta)
