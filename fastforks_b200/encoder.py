@@ -8,6 +8,7 @@ from torch's caching allocator. Nothing here computes.
 from __future__ import annotations
 
 import ctypes
+import logging
 from typing import TYPE_CHECKING
 
 import torch
@@ -18,16 +19,30 @@ from .attention import reserve_workspace
 if TYPE_CHECKING:
     from collections.abc import Sequence
 
+_LOG = logging.getLogger("fastforks_b200")
 FFN_GELU_TANH, FFN_SWIGLU, FFN_GELU = 0, 1, 2
 MAX_DIM = 2048  # a row of the layer norms lives in one warp's registers
 _DTYPES = {torch.float16: _lib.F16, torch.bfloat16: _lib.BF16}
 BLOCK_TENSORS = tuple(name for name, kind in _lib.B200EncoderBlock._fields_ if kind is ctypes.c_void_p)  # noqa: SLF001
+_REQUIRED = {name for name in BLOCK_TENSORS if name[:5] not in ("gamma", "rel_p")}
 _SPLIT_MIN_KEYS = 257  # shorter sequences never use the attention workspace
 
 
 def supported(dtype: torch.dtype, dim: int, heads: int, hidden: int) -> bool:
     """Whether the native forward takes an encoder of this shape."""
     return dtype in _DTYPES and dim == heads * 64 and dim <= MAX_DIM and hidden % 8 == 0
+
+
+def check_parameter(name: str, t: torch.Tensor, shape: tuple[int, ...], dtype: torch.dtype, device: torch.device) -> None:
+    """Refuse a parameter the kernels cannot read through its address alone.
+
+    Raises:
+        ValueError: It has another shape, type or device, or is not contiguous and 16-byte aligned.
+    """
+    if tuple(t.shape) != shape or t.dtype != dtype or t.device != device or not t.is_contiguous() or t.data_ptr() % 16:
+        msg = (f"encoder: parameter {name} must be contiguous, 16-byte aligned {dtype} {list(shape)} on {device}, "
+               f"got {list(t.shape)} {t.dtype} {t.device} strides {t.stride()}")  # fmt: skip
+        raise ValueError(msg)
 
 
 class Snapshot:
@@ -58,16 +73,23 @@ class NativeEncoder:
         self._keep = [dict(b) for b in blocks]
         self.count = len(blocks)
         self.blocks = (_lib.B200EncoderBlock * max(1, self.count))()
+        self.device = next((t.device for b in blocks for t in b.values() if isinstance(t, torch.Tensor)), None)
+        wide = 2 * hidden if ffn == FFN_SWIGLU else hidden
+        shapes = {"qkv_w": (3 * dim, dim), "qkv_b": (3 * dim,), "proj_w": (dim, dim), "fc1_w": (wide, dim), "fc1_b": (wide,), "fc2_w": (dim, hidden)}
         for entry, tensors in zip(self.blocks, blocks):
+            missing = _REQUIRED - set(tensors)
+            if missing:
+                msg = f"encoder: a block lacks {sorted(missing)}"
+                raise ValueError(msg)
+            entry.window = tensors.get("window", 0)
             for name in BLOCK_TENSORS:
                 t = tensors.get(name)
                 if t is not None:
-                    if not t.is_contiguous() or t.data_ptr() % 16:
-                        msg = f"encoder: parameter {name} must be contiguous and 16-byte aligned"
-                        raise ValueError(msg)
+                    shape = shapes.get(name, (dim,))
+                    if name in ("rel_pos_h", "rel_pos_w"):  # as many rows as the window's side asks for; a grid's side is known at the call
+                        shape = (2 * entry.window - 1, 64) if entry.window else (*t.shape[:1], 64)
+                    check_parameter(name, t, shape, torch.float32 if name.startswith("gamma") else dtype, self.device)
                     setattr(entry, name, t.data_ptr())
-            entry.window = tensors.get("window", 0)
-        self.device = next((t.device for b in blocks for t in b.values() if isinstance(t, torch.Tensor)), None)
         self._described: dict[tuple, tuple] = {}  # geometry -> (argument description, workspace bytes)
 
     def describe(self, batch: int, grid: tuple[int, int], prefix: int, first: int, count: int, extra: dict) -> tuple:
@@ -83,6 +105,12 @@ class NativeEncoder:
         key = (batch, grid, prefix, first, count, tuple(sorted(extra.items())))
         found = self._described.get(key)
         if found is None:
+            for b in self._keep[first : first + count]:
+                for name in ("rel_pos_h", "rel_pos_w"):
+                    t = b.get(name)
+                    if t is not None and not b.get("window", 0) and (grid[0] != grid[1] or t.shape[0] != 2 * grid[0] - 1):
+                        msg = f"encoder: {name} of {t.shape[0]} rows does not fit a grid of {grid[0]} x {grid[1]}"
+                        raise ValueError(msg)
             a = _lib.B200EncoderArgs()
             a.struct_size = ctypes.sizeof(_lib.B200EncoderArgs)
             a.dtype, a.batch, a.prefix, a.eps = _DTYPES[self.dtype], batch, prefix, self.eps
@@ -133,3 +161,13 @@ class NativeEncoder:
                 a.attn_workspace, a.attn_workspace_bytes = scratch.data_ptr(), scratch.numel()
         code = _lib.library().b200_encoder_forward(ctypes.byref(a), torch._C._cuda_getCurrentRawStream(index))  # noqa: SLF001
         _lib.raise_for_code(code, "encoder")
+
+
+def native_or_none(blocks: Sequence[dict], **geometry: object) -> NativeEncoder | None:
+    """The native encoder of a model's blocks, or None where it cannot take the parameters: the model then runs layer by layer, and
+    its layers take them or say what is wrong."""
+    try:
+        return NativeEncoder(blocks, **geometry)
+    except ValueError as e:
+        _LOG.info("layer by layer: %s", e)
+        return None

@@ -193,7 +193,7 @@ class SamEncoder:
             self._native, self._snapshot = self._make_native(), encoder.Snapshot(self.w)
         return self._native
 
-    def _make_native(self) -> encoder.NativeEncoder:
+    def _make_native(self) -> encoder.NativeEncoder | None:
         w, cfg, blocks = self.w, self.cfg, []
         layers = {"norm1": "norm1", "qkv": "attn.qkv", "proj": "attn.proj", "norm2": "norm2", "fc1": "mlp.lin1", "fc2": "mlp.lin2"}
         for i in range(cfg.depth):
@@ -202,7 +202,7 @@ class SamEncoder:
             tensors |= {"rel_pos_h": w[p + "attn.rel_pos_h"], "rel_pos_w": w[p + "attn.rel_pos_w"],
                         "window": 0 if i in cfg.global_blocks else cfg.window}  # fmt: skip
             blocks.append(tensors)
-        return encoder.NativeEncoder(blocks, dtype=self.dtype, dim=cfg.dim, heads=cfg.heads, hidden=4 * cfg.dim, ffn=encoder.FFN_GELU, eps=1e-5)
+        return encoder.native_or_none(blocks, dtype=self.dtype, dim=cfg.dim, heads=cfg.heads, hidden=4 * cfg.dim, ffn=encoder.FFN_GELU, eps=1e-5)
 
     def _forward_native(self, images: torch.Tensor) -> torch.Tensor | None:
         """The forward as one native call; None when the images are not of a form it takes."""

@@ -156,7 +156,7 @@ class ViTEncoder:
             self._native, self._snapshot = self._make_native(), encoder.Snapshot(self.w, self.scales)
         return self._native
 
-    def _make_native(self) -> encoder.NativeEncoder:
+    def _make_native(self) -> encoder.NativeEncoder | None:
         w, cfg, blocks = self.w, self.cfg, []
         fc1, fc2 = ("mlp.w12", "mlp.w3") if cfg.ffn == "swiglu" else ("mlp.fc1", "mlp.fc2")
         for i in range(cfg.depth):
@@ -167,7 +167,7 @@ class ViTEncoder:
                 tensors |= {"gamma1": self.scales[p + "ls1.gamma"], "gamma2": self.scales[p + "ls2.gamma"]}
             blocks.append(tensors)
         ffn = encoder.FFN_SWIGLU if cfg.ffn == "swiglu" else encoder.FFN_GELU_TANH
-        return encoder.NativeEncoder(blocks, dtype=self.dtype, dim=cfg.dim, heads=cfg.heads, hidden=cfg.hidden, ffn=ffn, eps=cfg.eps)
+        return encoder.native_or_none(blocks, dtype=self.dtype, dim=cfg.dim, heads=cfg.heads, hidden=cfg.hidden, ffn=ffn, eps=cfg.eps)
 
     def _forward_native(self, images: torch.Tensor, count: int, taps: tuple[int, ...]) -> list[torch.Tensor] | None:
         """Normalised tokens after the blocks in `taps`, of the first `count` blocks, as one native call; None when the images

@@ -38,6 +38,16 @@ def vit(monkeypatch: pytest.MonkeyPatch) -> ViTEncoder:
     return enc
 
 
+GEOMETRY = {"dtype": torch.float16, "dim": 128, "heads": 2, "hidden": 72, "ffn": encoder.FFN_SWIGLU, "eps": 1e-6}
+SHAPES = {"norm1_w": (128,), "norm1_b": (128,), "qkv_w": (384, 128), "qkv_b": (384,), "proj_w": (128, 128), "proj_b": (128,), "gamma1": (128,),
+          "norm2_w": (128,), "norm2_b": (128,), "fc1_w": (144, 128), "fc1_b": (144,), "fc2_w": (128, 72), "fc2_b": (128,), "gamma2": (128,),
+          "rel_pos_h": (7, 64), "rel_pos_w": (7, 64)}  # fmt: skip
+
+
+def block(window: int = 4) -> dict:
+    return {k: torch.zeros(*s, dtype=torch.float32 if k.startswith("gamma") else torch.float16) for k, s in SHAPES.items()} | {"window": window}
+
+
 @pytest.mark.parametrize(("first", "count"), [(0, 3), (2, 1), (-1, 1), (-1, 2), (1, 2), (3, 0), (0, -1)])
 def test_blocks_that_do_not_exist_are_refused(vit: ViTEncoder, first: int, count: int) -> None:
     native = vit._native_now()  # noqa: SLF001
@@ -71,10 +81,44 @@ def test_tensors_on_another_device_are_refused(vit: ViTEncoder) -> None:
     with pytest.raises(RuntimeError):  # torch's device mismatch
         vit.block(0, torch.zeros(1, 5, 128, dtype=torch.float16, device="meta"))
     assert vit._forward_native(torch.zeros(1, 3, 28, 28, device="meta"), 2, (1,)) is None  # noqa: SLF001
-    native = encoder.NativeEncoder([dict(vit.w)], dtype=torch.float16, dim=128, heads=2, hidden=512, ffn=encoder.FFN_GELU, eps=1e-6)
+    native = encoder.NativeEncoder([block()], **GEOMETRY)
     described = native.describe(1, (4, 1), 0, 0, 0, {"x": 1})
     meta = torch.zeros(4, 128, dtype=torch.float16, device="meta")
     with pytest.raises(ValueError, match="parameters on cpu"):
         native.launch(described, meta.device, x=meta)
     with pytest.raises(ValueError, match="launch on cpu"):
         native.launch(described, torch.device("cpu"), x=meta)
+
+
+@pytest.mark.parametrize("name", SHAPES)
+def test_parameters_the_kernels_would_read_past_are_refused(name: str) -> None:
+    """Shape, type, device, layout and alignment of every parameter whose address goes into the table."""
+    good = block()
+    encoder.NativeEncoder([good], **GEOMETRY)
+    t = good[name]
+    shifted = torch.zeros(t.numel() + 4, dtype=t.dtype)[2:][: t.numel()].view_as(t)  # 4 or 8 bytes off
+    wrong = [t[:-1].clone(), t.expand(2, *t.shape).contiguous(), t.double(), t.to("meta"), shifted]
+    if t.dim() == 2:  # noqa: PLR2004
+        wrong += [t.T.contiguous().T, t[:, :-8].clone()]
+    for bad in wrong:
+        with pytest.raises(ValueError, match=name):
+            encoder.NativeEncoder([good, good | {name: bad}], **GEOMETRY)
+    if not name.startswith(("gamma", "rel_pos")):
+        with pytest.raises(ValueError, match=name):
+            encoder.NativeEncoder([{k: v for k, v in good.items() if k != name}], **GEOMETRY)
+
+
+def test_relative_tables_of_a_grid_are_compared_with_it() -> None:
+    native = encoder.NativeEncoder([block(0)], **GEOMETRY)
+    native.describe(1, (4, 4), 0, 0, 1, {"x": 1})
+    for grid in ((5, 5), (2, 2), (4, 2), (4, 5)):
+        with pytest.raises(ValueError, match="does not fit"):
+            native.describe(1, grid, 0, 0, 1, {"x": 1})
+
+
+@pytest.mark.parametrize("name", ["blocks.0.norm1.weight", "blocks.1.attn.qkv.weight", "blocks.1.mlp.fc2.bias", "blocks.0.ls1.gamma"])
+def test_a_state_of_other_shapes_is_left_to_the_layers(name: str) -> None:
+    state = seeded_state(CFG)
+    state[name] = state[name][:-8].clone()
+    enc = ViTEncoder(CFG, state, device="cpu", dtype=torch.float16)
+    assert enc._make_native() is None  # noqa: SLF001
