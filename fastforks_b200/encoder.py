@@ -163,11 +163,15 @@ class NativeEncoder:
         _lib.raise_for_code(code, "encoder")
 
 
-def native_or_none(blocks: Sequence[dict], **geometry: object) -> NativeEncoder | None:
-    """The native encoder of a model's blocks, or None where it cannot take the parameters: the model then runs layer by layer, and
-    its layers take them or say what is wrong."""
+def native_or_none(blocks: Sequence[dict], others: dict[str, tuple[torch.Tensor, tuple[int, ...]]], **geometry: object) -> NativeEncoder | None:
+    """The native encoder of a model's blocks, or None where the kernels cannot take a parameter, one of the table or one of `others`
+    (those a call names in its description, with their shapes): the model then runs layer by layer, and its layers take the
+    parameter or say what is wrong with it."""
     try:
-        return NativeEncoder(blocks, **geometry)
+        native = NativeEncoder(blocks, **geometry)
+        for name, (t, shape) in others.items():
+            check_parameter(name, t, shape, native.dtype, native.device)
     except ValueError as e:
         _LOG.info("layer by layer: %s", e)
         return None
+    return native

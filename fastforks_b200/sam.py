@@ -202,7 +202,8 @@ class SamEncoder:
             tensors |= {"rel_pos_h": w[p + "attn.rel_pos_h"], "rel_pos_w": w[p + "attn.rel_pos_w"],
                         "window": 0 if i in cfg.global_blocks else cfg.window}  # fmt: skip
             blocks.append(tensors)
-        return encoder.native_or_none(blocks, dtype=self.dtype, dim=cfg.dim, heads=cfg.heads, hidden=4 * cfg.dim, ffn=encoder.FFN_GELU, eps=1e-5)
+        others = {name: (w[name], shape) for name, shape in sam_state_shapes(cfg).items() if not name.startswith("blocks.")}
+        return encoder.native_or_none(blocks, others, dtype=self.dtype, dim=cfg.dim, heads=cfg.heads, hidden=4 * cfg.dim, ffn=encoder.FFN_GELU, eps=1e-5)
 
     def _forward_native(self, images: torch.Tensor) -> torch.Tensor | None:
         """The forward as one native call; None when the images are not of a form it takes."""

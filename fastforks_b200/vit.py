@@ -167,7 +167,9 @@ class ViTEncoder:
                 tensors |= {"gamma1": self.scales[p + "ls1.gamma"], "gamma2": self.scales[p + "ls2.gamma"]}
             blocks.append(tensors)
         ffn = encoder.FFN_SWIGLU if cfg.ffn == "swiglu" else encoder.FFN_GELU_TANH
-        return encoder.native_or_none(blocks, dtype=self.dtype, dim=cfg.dim, heads=cfg.heads, hidden=cfg.hidden, ffn=ffn, eps=cfg.eps)
+        names = ("cls_token", "patch_embed.proj.weight", "patch_embed.proj.bias", "norm.weight", "norm.bias")
+        others = {name: (w[name], state_shapes(cfg)[name]) for name in names}
+        return encoder.native_or_none(blocks, others, dtype=self.dtype, dim=cfg.dim, heads=cfg.heads, hidden=cfg.hidden, ffn=ffn, eps=cfg.eps)
 
     def _forward_native(self, images: torch.Tensor, count: int, taps: tuple[int, ...]) -> list[torch.Tensor] | None:
         """Normalised tokens after the blocks in `taps`, of the first `count` blocks, as one native call; None when the images
@@ -183,11 +185,15 @@ class ViTEncoder:
         if width % 2 or gh == 0 or gw == 0 or images.data_ptr() % 16:
             return None
         if (gh, gw) not in self._pos32:
-            self._pos32[gh, gw] = self.pos_embed_fp32(gh, gw).contiguous()
+            pos = self.pos_embed_fp32(gh, gw).contiguous()
+            self._pos32[gh, gw] = pos.clone() if pos.data_ptr() % 16 else pos
+        pos = self._pos32[gh, gw]
+        if pos.shape != (1, 1 + gh * gw, self.cfg.dim):
+            return None
         extra = {  # "images": any address, the description only needs to know that there are images
             "images": 1, "image_dtype": _lib.F32 if images.dtype == torch.float32 else encoder._DTYPES[self.dtype],  # noqa: SLF001
             "height": height, "width": width, "patch": ps, "patch_w": w["patch_embed.proj.weight"].data_ptr(), "patch_w_raw": 1, "patch_k": (3 * ps * ps + 7) // 8 * 8,
-            "start": self._pos32[gh, gw].data_ptr(), "start_f32": 1, "patch_b": w["patch_embed.proj.bias"].data_ptr(), "first": w["cls_token"].data_ptr(),
+            "start": pos.data_ptr(), "start_f32": 1, "patch_b": w["patch_embed.proj.bias"].data_ptr(), "first": w["cls_token"].data_ptr(),
             "norm_w": w["norm.weight"].data_ptr(), "norm_b": w["norm.bias"].data_ptr(),
         }  # fmt: skip
         described = native.describe(b, (gh, gw), 1, 0, count, extra)

@@ -11,6 +11,7 @@ import torch
 
 from fastforks_b200 import _lib, encoder
 from fastforks_b200.flash64 import Flash64
+from fastforks_b200.sam import SamConfig, SamEncoder, sam_seeded_state
 from fastforks_b200.vit import ViTConfig, ViTEncoder, seeded_state
 
 
@@ -122,3 +123,31 @@ def test_a_state_of_other_shapes_is_left_to_the_layers(name: str) -> None:
     state[name] = state[name][:-8].clone()
     enc = ViTEncoder(CFG, state, device="cpu", dtype=torch.float16)
     assert enc._make_native() is None  # noqa: SLF001
+
+
+VIT_OTHERS = ("cls_token", "patch_embed.proj.weight", "patch_embed.proj.bias", "norm.weight", "norm.bias")
+SAM_OTHERS = ("pos_embed", "patch_embed.proj.weight", "patch_embed.proj.bias", "neck.0.weight", "neck.1.weight", "neck.1.bias", "neck.2.weight", "neck.3.weight", "neck.3.bias")
+
+
+@pytest.mark.parametrize("name", [*(f"vit {n}" for n in VIT_OTHERS), *(f"sam {n}" for n in SAM_OTHERS)])
+def test_parameters_beside_the_blocks_are_looked_at_too(name: str) -> None:
+    """Slices of a flat buffer that begin off a 16-byte boundary, strided views and other shapes run layer by layer."""
+    kind, name = name.split()
+    if kind == "vit":
+        enc = ViTEncoder(CFG, seeded_state(CFG), device="cpu", dtype=torch.float16)
+        enc.scales = {k: v.float() for k, v in enc.scales.items()}
+    else:
+        cfg = SamConfig(img=96, patch=16, dim=128, depth=2, heads=2, out_chans=24, window=4, global_blocks=(1,))
+        enc = SamEncoder(cfg, sam_seeded_state(cfg), device="cpu", dtype=torch.float16)
+    assert enc._make_native() is not None  # noqa: SLF001
+    t = enc.w[name]
+    shifted = torch.zeros(t.numel() + 8, dtype=t.dtype)[2:][: t.numel()].view_as(t)
+    for bad in (shifted, torch.zeros(*t.shape, 2, dtype=t.dtype)[..., 0], t[..., :-1].clone() if t.shape[-1] > 1 else t[:-1].clone()):
+        enc.w[name] = bad
+        assert enc._make_native() is None  # noqa: SLF001
+
+
+def test_a_position_table_of_another_width_is_left_to_the_layers(vit: ViTEncoder) -> None:
+    vit.pos_table = vit.pos_table[..., :64].contiguous()
+    assert vit._forward_native(torch.zeros(1, 3, 28, 28), 2, (1,)) is None  # noqa: SLF001
+    assert vit.launched == []
