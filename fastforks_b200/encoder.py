@@ -127,6 +127,15 @@ class NativeEncoder:
             found = self._described[key] = (a, size.value)
         return found
 
+    def try_describe(self, *geometry: object) -> tuple | None:
+        """`describe`, or None where the library cannot take the geometry (patches of an odd side, more tokens than a launch holds):
+        the model's layers then run one by one."""
+        try:
+            return self.describe(*geometry)
+        except ValueError as e:
+            _LOG.info("layer by layer: %s", e)
+            return None
+
     def launch(self, described: tuple, device: torch.device, *, x: torch.Tensor | None = None, images: torch.Tensor | None = None,
                taps: Sequence[tuple[int, torch.Tensor]] = (), neck_out: torch.Tensor | None = None) -> None:  # fmt: skip
         """Launch a described forward on the current stream of `device`, which is the parameters'.

@@ -226,7 +226,9 @@ class SamEncoder:
             "neck_n1_w": w["neck.3.weight"].data_ptr(), "neck_n1_b": w["neck.3.bias"].data_ptr(),
         }  # fmt: skip
         b, grid = images.shape[0], cfg.grid
-        described = native.describe(b, (grid, grid), 0, 0, cfg.depth, extra)
+        described = native.try_describe(b, (grid, grid), 0, 0, cfg.depth, extra)
+        if described is None:
+            return None
         out = torch.empty((b, cfg.out_chans, grid, grid), dtype=self.dtype, device=images.device)
         native.launch(described, images.device, images=images, neck_out=out)
         return out

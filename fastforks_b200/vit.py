@@ -196,7 +196,9 @@ class ViTEncoder:
             "start": pos.data_ptr(), "start_f32": 1, "patch_b": w["patch_embed.proj.bias"].data_ptr(), "first": w["cls_token"].data_ptr(),
             "norm_w": w["norm.weight"].data_ptr(), "norm_b": w["norm.bias"].data_ptr(),
         }  # fmt: skip
-        described = native.describe(b, (gh, gw), 1, 0, count, extra)
+        described = native.try_describe(b, (gh, gw), 1, 0, count, extra)
+        if described is None:
+            return None
         outs = [torch.empty((b, 1 + gh * gw, self.cfg.dim), dtype=self.dtype, device=images.device) for _ in taps]
         native.launch(described, images.device, images=images, taps=list(zip(taps, outs)))
         return outs
@@ -262,8 +264,10 @@ class ViTEncoder:
         native = self._native_now()
         if (native is not None and type(i) is int and 0 <= i < cfg.depth and not (x.requires_grad and torch.is_grad_enabled()) and x.device == native.device
                 and x.dtype == self.dtype and c == cfg.dim and x.is_contiguous() and x.numel() > 0 and x.data_ptr() % 16 == 0):  # fmt: skip
-            native.launch(native.describe(b, (n, 1), 0, i, 1, {"x": 1}), x.device, x=x)
-            return x
+            described = native.try_describe(b, (n, 1), 0, i, 1, {"x": 1})
+            if described is not None:
+                native.launch(described, x.device, x=x)
+                return x
         heads = cfg.heads
         ls1, ls2 = (p + "ls1.gamma", p + "ls2.gamma") if cfg.layerscale else (None, None)
         qkv = self.linear(F.layer_norm(x, (c,), w[p + "norm1.weight"], w[p + "norm1.bias"], cfg.eps), p + "attn.qkv")

@@ -151,3 +151,18 @@ def test_a_position_table_of_another_width_is_left_to_the_layers(vit: ViTEncoder
     vit.pos_table = vit.pos_table[..., :64].contiguous()
     assert vit._forward_native(torch.zeros(1, 3, 28, 28), 2, (1,)) is None  # noqa: SLF001
     assert vit.launched == []
+
+
+def test_patches_of_an_odd_side_are_left_to_the_layers(monkeypatch: pytest.MonkeyPatch) -> None:
+    cfg = ViTConfig(128, 1, 2, 7, 28)
+    enc = ViTEncoder(cfg, seeded_state(cfg), device="cpu", dtype=torch.float16)
+    enc.scales = {k: v.float() for k, v in enc.scales.items()}
+    native = enc._make_native()  # noqa: SLF001
+    monkeypatch.setattr(enc, "_native_now", lambda: native)
+    assert enc._forward_native(torch.zeros(1, 3, 28, 28), 1, (0,)) is None  # noqa: SLF001
+
+
+def test_more_tokens_than_a_launch_holds_are_left_to_the_layers(vit: ViTEncoder) -> None:
+    native = vit._native_now()  # noqa: SLF001
+    assert native.try_describe(1 << 16, (1 << 12, 1), 0, 0, 1, {"x": 1}) is None
+    assert native.try_describe(1 << 8, (1 << 12, 1), 0, 0, 1, {"x": 1}) is not None
