@@ -262,7 +262,8 @@ class ViTEncoder:
         w, cfg, p = self.w, self.cfg, f"blocks.{i}."
         b, n, c = x.shape
         native = self._native_now()
-        if (native is not None and type(i) is int and 0 <= i < cfg.depth and not (x.requires_grad and torch.is_grad_enabled()) and x.device == native.device
+        wants_grad = torch.is_grad_enabled() and any(t.requires_grad for t in (x, *w.values(), *self.scales.values()))  # refused by the layers
+        if (native is not None and type(i) is int and 0 <= i < cfg.depth and not wants_grad and x.device == native.device
                 and x.dtype == self.dtype and c == cfg.dim and x.is_contiguous() and x.numel() > 0 and x.data_ptr() % 16 == 0):  # fmt: skip
             described = native.try_describe(b, (n, 1), 0, i, 1, {"x": 1})
             if described is not None:

@@ -166,3 +166,18 @@ def test_more_tokens_than_a_launch_holds_are_left_to_the_layers(vit: ViTEncoder)
     native = vit._native_now()  # noqa: SLF001
     assert native.try_describe(1 << 16, (1 << 12, 1), 0, 0, 1, {"x": 1}) is None
     assert native.try_describe(1 << 8, (1 << 12, 1), 0, 0, 1, {"x": 1}) is not None
+
+
+@pytest.mark.parametrize("name", ["tokens", "blocks.1.attn.qkv.weight", "blocks.0.norm1.bias", "scale"])
+def test_a_block_that_is_asked_for_gradients_is_left_to_the_layers(vit: ViTEncoder, name: str, monkeypatch: pytest.MonkeyPatch) -> None:
+    """Attention and gemm refuse operands that require a gradient; so must the block they stand in."""
+    x = torch.zeros(1, 5, 128, dtype=torch.float16)
+    {"tokens": x, "scale": vit.scales["blocks.1.ls1.gamma"]}.get(name, vit.w.get(name)).requires_grad_()
+    reached = []
+    monkeypatch.setattr(vit, "linear", lambda *a, **k: reached.append(a))
+    with pytest.raises(AttributeError, match="view"):  # of what the replaced layer returned
+        vit.block(1, x)
+    assert reached and vit.launched == []
+    with torch.no_grad():
+        vit.block(1, x)
+    assert vit.launched == [1]
