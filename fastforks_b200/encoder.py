@@ -45,6 +45,11 @@ def check_parameter(name: str, t: torch.Tensor, shape: tuple[int, ...], dtype: t
         raise ValueError(msg)
 
 
+def overrides(model: object, base: type, methods: tuple[str, ...]) -> bool:
+    """Whether a subclass of a model or an attribute set on it replaces one of `methods`, which the native call would pass by."""
+    return (type(model) is not base and any(getattr(type(model), m) is not getattr(base, m) for m in methods)) or not vars(model).keys().isdisjoint(methods)
+
+
 class Snapshot:
     """The tensors of a model's dictionaries as they were when their addresses were taken: a tensor put in another's place, or
     given other storage, is seen by `changed`, which every forward asks. (Values written in place need no looking at: the

@@ -69,3 +69,12 @@ class Flash64:
         b, n, h, _ = q.shape
         o = torch.empty((b, n, h, HEAD_DIM), device=q.device, dtype=q.dtype)
         return attention(q, k, v, scale=scale, layout="bnhd", out=o)
+
+
+_OWN_RUN = Flash64._run  # noqa: SLF001
+
+
+def is_stock(attn: object) -> bool:
+    """Whether `attn` launches this library's kernel itself: a caller may put another launcher in a model, or replace
+    `Flash64._run` to observe launches, and must then see every call."""
+    return type(attn) is Flash64 and Flash64._run is _OWN_RUN and "_run" not in vars(attn)  # noqa: SLF001

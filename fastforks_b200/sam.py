@@ -188,7 +188,10 @@ class SamEncoder:
         self._native_now()
 
     def _native_now(self) -> encoder.NativeEncoder | None:
-        """The native encoder over the parameters as they are now; None where there is none for this device or shape."""
+        """The native encoder over the parameters as they are now; None where there is none for this device or shape, or where a step
+        of the forward was replaced."""
+        if encoder.overrides(self, SamEncoder, ("attend", "block", "norm2d")):
+            return None
         if self._has_native and (self._snapshot is None or self._snapshot.changed(self.w)):
             self._native, self._snapshot = self._make_native(), encoder.Snapshot(self.w)
         return self._native

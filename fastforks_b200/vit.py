@@ -21,7 +21,7 @@ import torch
 import torch.nn.functional as F  # noqa: N812
 
 from . import _lib, encoder
-from .flash64 import Flash64
+from .flash64 import Flash64, is_stock
 from .gemm import ACT_GELU_TANH, ACT_NONE, gemm
 
 
@@ -148,8 +148,11 @@ class ViTEncoder:
         self._native_now()
 
     def _native_now(self) -> encoder.NativeEncoder | None:
-        """The native encoder over the parameters as they are now; None where there is none for this device or shape."""
+        """The native encoder over the parameters as they are now; None where there is none for this device or shape, or where the
+        attention launcher or a step of the forward was replaced."""
         cfg = self.cfg
+        if not is_stock(self.attn) or encoder.overrides(self, ViTEncoder, ("tokens", "pos_embed", "linear", "block")):
+            return None
         if not self.fused or self.device.type != "cuda" or not encoder.supported(self.dtype, cfg.dim, cfg.heads, cfg.hidden):
             return None
         if self._snapshot is None or self._snapshot.changed(self.w, self.scales):

@@ -10,7 +10,7 @@ import pytest
 import torch
 
 from fastforks_b200 import _lib, encoder
-from fastforks_b200.flash64 import Flash64
+from fastforks_b200.flash64 import Flash64, is_stock
 from fastforks_b200.sam import SamConfig, SamEncoder, sam_seeded_state
 from fastforks_b200.vit import ViTConfig, ViTEncoder, seeded_state
 
@@ -35,7 +35,6 @@ def vit(monkeypatch: pytest.MonkeyPatch) -> ViTEncoder:
     enc.launched = []
     monkeypatch.setattr(native, "launch", lambda described, *a, **k: enc.launched.append(described[0].n_blocks))
     monkeypatch.setattr(enc, "_native_now", lambda: native)
-    monkeypatch.setattr(Flash64, "_run", staticmethod(lambda variant, q, k, v, scale: v.contiguous()))
     return enc
 
 
@@ -174,10 +173,37 @@ def test_a_block_that_is_asked_for_gradients_is_left_to_the_layers(vit: ViTEncod
     x = torch.zeros(1, 5, 128, dtype=torch.float16)
     {"tokens": x, "scale": vit.scales["blocks.1.ls1.gamma"]}.get(name, vit.w.get(name)).requires_grad_()
     reached = []
-    monkeypatch.setattr(vit, "linear", lambda *a, **k: reached.append(a))
+    monkeypatch.setattr(ViTEncoder, "linear", lambda *a, **k: reached.append(a))
     with pytest.raises(AttributeError, match="view"):  # of what the replaced layer returned
         vit.block(1, x)
     assert reached and vit.launched == []
     with torch.no_grad():
         vit.block(1, x)
     assert vit.launched == [1]
+
+
+def test_replaced_steps_are_seen(monkeypatch: pytest.MonkeyPatch) -> None:
+    """A launcher or a step of the forward that a caller put in a model is what runs."""
+
+    class Sub(ViTEncoder):
+        def block(self, i: int, x: torch.Tensor) -> torch.Tensor:
+            return super().block(i, x)
+
+    class Plain(ViTEncoder):
+        def checked(self, images: torch.Tensor) -> torch.Tensor:
+            return images
+
+    steps = ("tokens", "pos_embed", "linear", "block")
+    enc = ViTEncoder(CFG, seeded_state(CFG), device="cpu")
+    assert is_stock(enc.attn) and not encoder.overrides(enc, ViTEncoder, steps)
+    assert encoder.overrides(Sub(CFG, seeded_state(CFG), device="cpu"), ViTEncoder, steps)
+    assert not encoder.overrides(Plain(CFG, seeded_state(CFG), device="cpu"), ViTEncoder, steps)
+    enc.block = lambda i, x: x
+    assert encoder.overrides(enc, ViTEncoder, steps)
+    assert not is_stock(lambda q, k, v, scale: q)
+    launcher = Flash64("fh")
+    assert is_stock(launcher)
+    launcher._run = Flash64._run  # noqa: SLF001
+    assert not is_stock(launcher)
+    monkeypatch.setattr(Flash64, "_run", staticmethod(lambda *a: None))
+    assert not is_stock(enc.attn)

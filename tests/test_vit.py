@@ -95,6 +95,33 @@ def test_kernels_encoder_with_every_linear_layer_on_the_own_gemm(dtype: torch.dt
 
 
 @pytest.mark.gpu
+def test_a_replaced_launcher_sees_every_call(monkeypatch: pytest.MonkeyPatch) -> None:
+    """The reference's guard tests observe launches by replacing `Flash64._run` (tests/test_flash64_guard.py:29-172), and a caller may
+    give an encoder a launcher of its own."""
+    cfg = CONFIGS["dinov2-vits14"]
+    enc = ViTEncoder(cfg, seeded_state(cfg, 1, qk_gain=4.0), device="cuda", dtype=torch.float16)
+    images = torch.rand(2, 3, 126, 154, generator=torch.Generator().manual_seed(5)).cuda()
+    native = enc(images)
+    run, calls = Flash64._run, []  # noqa: SLF001
+
+    def spy(variant: str, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, scale: float) -> torch.Tensor:
+        calls.append(q.shape)
+        return run(variant, q, k, v, scale)
+
+    with monkeypatch.context() as m:
+        m.setattr(Flash64, "_run", staticmethod(spy))
+        assert cosine(enc(images).float().cpu().numpy(), native.float().cpu().numpy()) > 0.9999
+        assert calls == [(2, 100, 6, 64)] * 12
+        enc.intermediate(images, (3,))
+        assert len(calls) == 16
+    enc.attn = lambda q, k, v, scale: spy("hh", q, k, v, scale)
+    enc(images)
+    assert len(calls) == 28
+    enc.attn = Flash64()
+    assert torch.equal(enc(images), native) and len(calls) == 28
+
+
+@pytest.mark.gpu
 def test_kernels_encoder_batches_are_independent() -> None:
     """Image-wise sharding relies on it: an image's output does not depend on what else is in the batch."""
     cfg = CONFIGS["dinov2-vits14"]
