@@ -120,6 +120,54 @@ int check(const B200EncoderArgs* a) {
   return B200_ATTN_OK;
 }
 
+// What every kernel takes for granted of the addresses: there and on 16-byte boundaries (vector and TMA accesses).
+int check_pointers(const B200EncoderArgs* a) {
+  int rc = B200_ATTN_OK;
+  const auto look = [&](const char* what, int i, const char* name, const void* ptr, bool required) {
+    if (rc != B200_ATTN_OK) return;
+    if (ptr == nullptr && required) rc = fail(B200_ATTN_BAD_CONFIG, "%s %d: %s is NULL", what, i, name);
+    else if (!aligned16(ptr)) rc = fail(B200_ATTN_UNSUPPORTED, "%s %d: %s is not 16-byte aligned", what, i, name);
+  };
+  const bool images = a->images != nullptr, neck = a->neck_w0 != nullptr;
+  look("call", 0, "images", a->images, false);
+  look("call", 0, "x", a->x, false);
+  look("call", 0, "patch_w", a->patch_w, images);
+  look("call", 0, "start", a->start, images);
+  look("call", 0, "patch_b", a->patch_b, false);
+  look("call", 0, "first", a->first, false);
+  if (a->n_taps < 0 || (a->n_taps > 0 && a->taps == nullptr)) return fail(B200_ATTN_BAD_CONFIG, "n_taps %d without taps", a->n_taps);
+  look("call", 0, "norm_w", a->norm_w, a->n_taps > 0);
+  look("call", 0, "norm_b", a->norm_b, a->n_taps > 0);
+  for (int i = 0; i < a->n_taps; ++i) look("tap", i, "out", a->taps[i].out, true);
+  look("neck", 0, "neck_w0", a->neck_w0, false);
+  look("neck", 0, "neck_n0_w", a->neck_n0_w, neck);
+  look("neck", 0, "neck_n0_b", a->neck_n0_b, neck);
+  look("neck", 0, "neck_w1", a->neck_w1, neck);
+  look("neck", 0, "neck_n1_w", a->neck_n1_w, neck);
+  look("neck", 0, "neck_n1_b", a->neck_n1_b, neck);
+  look("neck", 0, "neck_out", a->neck_out, neck);
+  for (int i = 0; i < a->n_blocks; ++i) {
+    const B200EncoderBlock& k = a->blocks[i];
+    look("block", i, "norm1_w", k.norm1_w, true);
+    look("block", i, "norm1_b", k.norm1_b, true);
+    look("block", i, "qkv_w", k.qkv_w, true);
+    look("block", i, "qkv_b", k.qkv_b, false);
+    look("block", i, "proj_w", k.proj_w, true);
+    look("block", i, "proj_b", k.proj_b, false);
+    look("block", i, "gamma1", k.gamma1, false);
+    look("block", i, "norm2_w", k.norm2_w, true);
+    look("block", i, "norm2_b", k.norm2_b, true);
+    look("block", i, "fc1_w", k.fc1_w, true);
+    look("block", i, "fc1_b", k.fc1_b, false);
+    look("block", i, "fc2_w", k.fc2_w, true);
+    look("block", i, "fc2_b", k.fc2_b, false);
+    look("block", i, "gamma2", k.gamma2, false);
+    look("block", i, "rel_pos_h", k.rel_pos_h, k.rel_pos_w != nullptr);
+    look("block", i, "rel_pos_w", k.rel_pos_w, k.rel_pos_h != nullptr);
+  }
+  return rc;
+}
+
 // The launches of one forward.
 struct Forward {
   const B200EncoderArgs* a;
@@ -282,6 +330,7 @@ int b200_encoder_workspace(const B200EncoderArgs* a, int64_t* bytes) {
 
 int b200_encoder_forward(const B200EncoderArgs* a, void* stream_ptr) {
   if (int rc = check(a)) return rc;
+  if (int rc = check_pointers(a)) return rc;
   Forward f{a, layout_of(a), static_cast<cudaStream_t>(stream_ptr), static_cast<char*>(a->workspace), nullptr};
   if (a->workspace == nullptr || (reinterpret_cast<uintptr_t>(a->workspace) & 255) != 0 || a->workspace_bytes < f.l.total)
     return fail(B200_ATTN_BAD_CONFIG, "workspace of %lld bytes: %lld, 256-byte aligned, are needed", static_cast<long long>(a->workspace_bytes), static_cast<long long>(f.l.total));

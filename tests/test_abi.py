@@ -137,3 +137,43 @@ def test_return_codes_map_to_the_reference_exceptions(lib: ctypes.CDLL) -> None:
     with pytest.raises(RuntimeError):
         _lib.raise_for_code(_lib.CUDA_ERROR_BASE + 2, "attention")
     _lib.raise_for_code(_lib.OK, "attention")
+
+
+def _encoder_args(**kw: object) -> _lib.B200EncoderArgs:
+    """An encoder of one SAM block with images, a tap and a neck; addresses are only looked at."""
+    block = (_lib.B200EncoderBlock * 1)()
+    for name, kind in _lib.B200EncoderBlock._fields_:  # noqa: SLF001
+        if kind is ctypes.c_void_p:
+            setattr(block[0], name, kw.pop(f"block.{name}", 0x10000))
+    block[0].window = kw.pop("block.window", 4)
+    tap = (_lib.B200EncoderTap * 1)((0, 0, kw.pop("tap.out", 0x10000)))
+    a = _lib.B200EncoderArgs()
+    a.struct_size = ctypes.sizeof(_lib.B200EncoderArgs)
+    a.batch, a.grid_h, a.grid_w, a.dim, a.heads, a.hidden, a.ffn, a.n_blocks = 1, 6, 6, 128, 2, 512, 2, 1
+    a.blocks, a.taps, a.n_taps = ctypes.addressof(block), ctypes.addressof(tap), 1
+    a.images, a.image_dtype, a.height, a.width, a.patch, a.patch_k = 0x10000, _lib.F32, 96, 96, 16, 768
+    a.neck_channels, a.workspace, a.workspace_bytes = 24, 0x10000, 0
+    for name in ("patch_w", "start", "patch_b", "norm_w", "norm_b", *(f"neck_{n}" for n in ("w0", "n0_w", "n0_b", "w1", "n1_w", "n1_b", "out"))):
+        setattr(a, name, 0x10000)
+    for name, value in kw.items():
+        setattr(a, name, value)
+    a.keep = block, tap
+    return a
+
+
+ENCODER_POINTERS = {"patch_w": True, "start": True, "patch_b": False, "first": False, "norm_w": True, "norm_b": True, "images": None, "x": False, "tap.out": True,
+                    "neck_n0_w": True, "neck_n0_b": True, "neck_w1": True, "neck_n1_w": True, "neck_n1_b": True, "neck_out": True,
+                    **{f"block.{n}": n.startswith(("norm", "rel")) or n.endswith("_w") for n, k in _lib.B200EncoderBlock._fields_ if k is ctypes.c_void_p}}  # fmt: skip
+
+
+@pytest.mark.parametrize("name", ENCODER_POINTERS)
+def test_encoder_forward_looks_at_every_address(lib: ctypes.CDLL, name: str) -> None:
+    """A NULL where something is read and an address off a 16-byte boundary are refused before the first launch."""
+    forward = lambda **kw: lib.b200_encoder_forward(ctypes.byref(_encoder_args(**kw)), None)  # noqa: E731
+    assert forward() == _lib.BAD_CONFIG and "workspace" in lib.b200_attn_last_error().decode()  # everything else is accepted
+    assert forward(**{name: 0x10008}) == _lib.UNSUPPORTED
+    assert name.removeprefix("block.").removeprefix("tap.") in lib.b200_attn_last_error().decode()
+    if ENCODER_POINTERS[name]:
+        assert forward(**{name: None}) in (_lib.BAD_CONFIG, _lib.UNSUPPORTED) and "workspace" not in lib.b200_attn_last_error().decode()
+    elif ENCODER_POINTERS[name] is False:
+        assert forward(**{name: None}) == _lib.BAD_CONFIG and "workspace" in lib.b200_attn_last_error().decode()
