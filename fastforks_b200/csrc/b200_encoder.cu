@@ -179,10 +179,12 @@ struct Forward {
 
   void* at(int64_t offset) const { return ws + offset; }
 
-  // y = act((x w^T + b) * gamma + res). Every product follows a kernel of this forward, so its weights were complete
-  // before that kernel started and are loaded ahead of it.
-  int linear(const void* in, int m, int k, const void* w, const void* b, int n, void* out, int act, const float* gamma = nullptr, const void* res = nullptr) const {
-    const GemmCall c{a->dtype, m, n, k, act, in, k, w, b, gamma, res, n, out, n, true};
+  // y = act((x w^T + b) * gamma + res). A product behind a kernel of this forward may load its weights ahead of that
+  // kernel's end: they were complete before it started. Not so in front (the neck of an encoder without blocks on given
+  // tokens may follow the kernel that writes them), and weights repacked in this forward are left to the wait as well.
+  int linear(const void* in, int m, int k, const void* w, const void* b, int n, void* out, int act, const float* gamma = nullptr, const void* res = nullptr, bool made_here = false) const {
+    const GemmCall c{a->dtype, m, n, k, act, in, k, w, b, gamma, res, n, out, n, started && !made_here};
+    started = true;
     return launch_gemm(c, stream);
   }
 
@@ -203,7 +205,6 @@ struct Forward {
   }
 
   int start_tokens() const {
-    // In front of the kernel that is in front of the product: the product loads its weights ahead of that one.
     const void* w = a->patch_w;
     if (pads_patch_w(a)) {
       w = at(l.patch_w);
@@ -221,7 +222,7 @@ struct Forward {
     void* args[] = {&p};
     const void* kernel = a->dtype == B200_ATTN_F16 ? reinterpret_cast<const void*>(encoder_tokens_kernel<__half>) : reinterpret_cast<const void*>(encoder_tokens_kernel<__nv_bfloat16>);
     if (int rc = launch_kernel(kernel, static_cast<unsigned>(a->batch * a->grid_h), static_cast<unsigned>(tokens_parts(a->patch)), kTokensThreads, 0, 1, stream, args, "encoder tokens launch")) return rc;
-    return linear(at(l.hid), static_cast<int>(l.rows), a->patch_k, w, nullptr, a->dim, x, kActNone, nullptr, x);
+    return linear(at(l.hid), static_cast<int>(l.rows), a->patch_k, w, nullptr, a->dim, x, kActNone, nullptr, x, pads_patch_w(a));
   }
 
   int attention(const B200EncoderBlock& k, int batch, int tokens, int side) const {
@@ -297,7 +298,7 @@ struct Forward {
     const int rows = static_cast<int>(l.rows), ch = a->neck_channels;
     if (int rc = linear(x, rows, a->dim, a->neck_w0, nullptr, ch, at(l.neck), kActNone)) return rc;
     const void* w1 = a->neck_w1;
-    if (reorders_neck_w1(a)) {  // in front of the next kernel for the same reason as the patch embedding's
+    if (reorders_neck_w1(a)) {
       w1 = at(l.neck_w1);
       if (int rc = repack(a->neck_w1, ch, 9 * ch, 9 * ch, 9, l.neck_w1)) return rc;
     }
@@ -308,7 +309,7 @@ struct Forward {
     const bool f16 = a->dtype == B200_ATTN_F16;
     const void* im2col = f16 ? reinterpret_cast<const void*>(neck_norm_im2col_kernel<__half>) : reinterpret_cast<const void*>(neck_norm_im2col_kernel<__nv_bfloat16>);
     if (int rc = launch_kernel(im2col, static_cast<unsigned>((rows + kNeckWarps - 1) / kNeckWarps), 1, kNeckWarps * 32, 0, 1, stream, args, "neck norm launch")) return rc;
-    if (int rc = linear(at(l.hid), rows, 9 * ch, w1, nullptr, ch, at(l.neck), kActNone)) return rc;
+    if (int rc = linear(at(l.hid), rows, 9 * ch, w1, nullptr, ch, at(l.neck), kActNone, nullptr, nullptr, reorders_neck_w1(a))) return rc;
     p.weight = a->neck_n1_w; p.bias = a->neck_n1_b; p.out = a->neck_out;
     const void* chw = f16 ? reinterpret_cast<const void*>(neck_norm_chw_kernel<__half>) : reinterpret_cast<const void*>(neck_norm_chw_kernel<__nv_bfloat16>);
     const int area = a->grid_h * a->grid_w;

@@ -177,3 +177,26 @@ def test_sam_forward_follows_its_parameters(how: str, patch: int) -> None:
     after, want = enc(images), other(images)
     assert torch.equal(after, want) and not torch.equal(after, before)
     assert ff.device_status() == 0
+
+
+def test_the_neck_alone_waits_for_its_weights() -> None:
+    """Given tokens, no blocks: the neck's first product is the first kernel of the call, right behind the one that writes its
+    weights and tokens."""
+    c, channels, grid = 768, 256, (64, 64)
+    weights = params({"w0": (channels, c), "n0_w": (channels,), "n0_b": (channels,), "w1": (channels, 9 * channels), "n1_w": (channels,), "n1_b": (channels,)}, seed=1)
+    tokens = torch.randn(1, 64 * 64, c, generator=torch.Generator().manual_seed(2)).half().cuda()
+    enc = encoder.NativeEncoder([], dtype=torch.float16, dim=c, heads=12, hidden=64, ffn=encoder.FFN_GELU, eps=1e-6)
+    held, x = {k: torch.zeros_like(t) for k, t in weights.items()}, torch.zeros_like(tokens)
+    fields = {f"neck_{name}": t.data_ptr() for name, t in held.items()} | {"x": 1, "neck_out": 1, "neck_channels": channels, "neck_eps": 1e-6}
+    described = enc.describe(1, grid, 0, 0, 0, fields)
+    outs = [torch.empty(1, channels, *grid, dtype=torch.float16, device="cuda") for _ in range(3)]
+    enc.launch(described, x.device, x=x, neck_out=outs[0])
+    for out in outs[1:]:
+        x.copy_(tokens)
+        for name, t in held.items():
+            t.copy_(weights[name]) if name != "w0" else None
+        held["w0"].copy_(weights["w0"])  # last
+        enc.launch(described, x.device, x=x, neck_out=out)
+    torch.cuda.synchronize()
+    assert torch.equal(outs[1], outs[2]) and not torch.equal(outs[0], outs[1])
+    assert ff.device_status() == 0
