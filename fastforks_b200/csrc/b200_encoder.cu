@@ -30,6 +30,11 @@ bool reorders_neck_w1(const B200EncoderArgs* a) { return a->neck_w0 != nullptr &
 
 int windows_of(int grid, int side) { return (grid + side - 1) / side; }
 
+int64_t window_rows(const B200EncoderArgs* a, int side) {
+  return a->batch * static_cast<int64_t>(windows_of(a->grid_h, side)) * windows_of(a->grid_w, side) * side * side;
+}
+constexpr int64_t kMaxRows = 0x3fffffff / 9;  // the neck has nine copies of a row, and row numbers are 32-bit
+
 Layout layout_of(const B200EncoderArgs* a) {
   Layout l{};
   const int64_t tokens = a->prefix + static_cast<int64_t>(a->grid_h) * a->grid_w;
@@ -41,7 +46,7 @@ Layout layout_of(const B200EncoderArgs* a) {
     int64_t rows = l.rows, side = a->grid_h;
     if (k.window > 0) {
       side = k.window;
-      rows = a->batch * static_cast<int64_t>(windows_of(a->grid_h, k.window)) * windows_of(a->grid_w, k.window) * k.window * k.window;
+      rows = window_rows(a, k.window);
       l.most_rows = std::max(l.most_rows, rows);
     }
     if (k.rel_pos_h != nullptr) rel = std::max(rel, rows * a->heads * side);
@@ -101,7 +106,7 @@ int check(const B200EncoderArgs* a) {
   if (a->hidden < 8 || a->hidden % 8 != 0) return fail(B200_ATTN_UNSUPPORTED, "hidden %d must be a positive multiple of 8", a->hidden);
   if (a->ffn < B200_FFN_GELU_TANH || a->ffn > B200_FFN_GELU) return fail(B200_ATTN_BAD_CONFIG, "ffn %d unknown", a->ffn);
   const int64_t rows = a->batch * (a->prefix + static_cast<int64_t>(a->grid_h) * a->grid_w);
-  if (rows > 0x3fffffff / 9) return fail(B200_ATTN_UNSUPPORTED, "too many tokens for one call");
+  if (rows > kMaxRows) return fail(B200_ATTN_UNSUPPORTED, "too many tokens for one call");
   if (a->images != nullptr) {
     if (a->patch < 2 || a->patch % 2 != 0 || a->patch_k < 3 * a->patch * a->patch || a->patch_k % 8 != 0 || a->width % 2 != 0 ||
         a->height < a->grid_h * a->patch || a->width < a->grid_w * a->patch || (a->image_dtype != B200_ATTN_F32 && a->image_dtype != a->dtype))
@@ -114,6 +119,9 @@ int check(const B200EncoderArgs* a) {
     const B200EncoderBlock& k = a->blocks[i];
     if (k.window < 0 || (k.window > 0 && a->prefix != 0)) return fail(B200_ATTN_BAD_CONFIG, "block %d: window %d with %d prefix tokens", i, k.window, a->prefix);
     if (k.rel_pos_h != nullptr && k.window == 0 && a->grid_h != a->grid_w) return fail(B200_ATTN_UNSUPPORTED, "block %d: relative positions need a square grid", i);
+    const int side = k.window > 0 ? k.window : a->grid_h;
+    if (k.rel_pos_h != nullptr && (side < 2 || side > 64 || side % 2 != 0)) return fail(B200_ATTN_UNSUPPORTED, "block %d: relative positions over a side of %d: even, 2 .. 64", i, side);
+    if (k.window > 0 && (k.window > 0x7fff || window_rows(a, k.window) > kMaxRows)) return fail(B200_ATTN_UNSUPPORTED, "block %d: too many tokens in windows of %d for one call", i, k.window);
   }
   if (a->neck_w0 != nullptr && (a->prefix != 0 || a->neck_channels < 8 || a->neck_channels % 8 != 0 || a->neck_channels > kNeckChunks * 256 || a->neck_out == nullptr))
     return fail(B200_ATTN_UNSUPPORTED, "neck of %d channels", a->neck_channels);

@@ -177,3 +177,15 @@ def test_encoder_forward_looks_at_every_address(lib: ctypes.CDLL, name: str) -> 
         assert forward(**{name: None}) in (_lib.BAD_CONFIG, _lib.UNSUPPORTED) and "workspace" not in lib.b200_attn_last_error().decode()
     elif ENCODER_POINTERS[name] is False:
         assert forward(**{name: None}) == _lib.BAD_CONFIG and "workspace" in lib.b200_attn_last_error().decode()
+
+
+@pytest.mark.parametrize("window", [128, 5, 40000, 1 << 20, (1 << 31) - 1])
+def test_encoder_refuses_windows_it_cannot_count(lib: ctypes.CDLL, window: int) -> None:
+    """Padded windows hold more rows than the grid: their number must fit the kernels' 32-bit row numbers too. Sides the
+    relative terms do not take are refused before the first launch, not between two of them."""
+    size = ctypes.c_int64(0)
+    plain = {"block.rel_pos_h": None, "block.rel_pos_w": None}
+    assert lib.b200_encoder_workspace(ctypes.byref(_encoder_args(**{"block.window": 4})), ctypes.byref(size)) == _lib.OK
+    assert lib.b200_encoder_workspace(ctypes.byref(_encoder_args(**{"block.window": window})), ctypes.byref(size)) == _lib.UNSUPPORTED
+    want = _lib.OK if window < 1000 else _lib.UNSUPPORTED  # noqa: PLR2004
+    assert lib.b200_encoder_workspace(ctypes.byref(_encoder_args(**{"block.window": window}, **plain)), ctypes.byref(size)) == want
