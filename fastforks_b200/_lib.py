@@ -16,8 +16,10 @@ import os
 import re
 import shutil
 import subprocess
+import sys
 import tempfile
 import threading
+import warnings
 from pathlib import Path
 from typing import TYPE_CHECKING
 
@@ -270,10 +272,19 @@ def built_hash(binary: Path | None = None) -> str | None:
     return found.group(1).decode() if found else None
 
 
+def host_hash() -> str:
+    """Digest of what the host extension depends on: the sources, and the torch and the interpreter whose C++ and C interfaces are
+    compiled into it (layouts that a binary for another version would silently get wrong)."""
+    import torch  # noqa: PLC0415
+
+    parts = (source_hash(), torch.__version__, str(torch._C._GLIBCXX_USE_CXX11_ABI), str(sys.implementation.cache_tag))  # noqa: SLF001
+    return hashlib.sha256("|".join(parts).encode()).hexdigest()[:16]
+
+
 def needs_build() -> bool:
-    """True when a binary is missing or was compiled from other sources than the ones beside it."""
-    want = source_hash()
-    return built_hash() != want or built_hash(HOST_EXTENSION) != want
+    """True when a binary is missing or was compiled from other sources, or (the host extension) for another torch or Python, than
+    the ones beside it."""
+    return built_hash() != source_hash() or built_hash(HOST_EXTENSION) != host_hash()
 
 
 def host_build_command(output: Path, digest: str) -> list[str]:
@@ -293,15 +304,26 @@ def host_build_command(output: Path, digest: str) -> list[str]:
     ]  # fmt: skip
 
 
+_LOCK = threading.Lock()
+
+
 def build(*, force: bool = False, verbose: bool = False) -> Path:
     """Compile the sources in `csrc/` for sm_100a (one compiler process each, in parallel) and link them into
-    `libb200attn.so` next to this file (needs nvcc, no GPU).
+    `libb200attn.so` next to this file (needs nvcc, no GPU), then the host extension. The extension only saves host time: if it does
+    not compile (no torch headers), a warning says so and the library is complete without it.
 
     Raises:
-        KernelUnavailableError: nvcc is missing or the compilation failed.
+        KernelUnavailableError: nvcc is missing or the compilation of the library failed.
     """
-    if not force and not needs_build():
-        return SHARED_OBJECT
+    with _LOCK:
+        if force or built_hash() != source_hash():
+            _build_library(verbose=verbose)
+        if force or built_hash(HOST_EXTENSION) != host_hash():
+            _build_host()
+    return SHARED_OBJECT
+
+
+def _build_library(*, verbose: bool) -> None:
     nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
     if not Path(nvcc).exists():
         raise KernelUnavailableError(LIBRARY, "nvcc not found: cannot build libb200attn.so")
@@ -321,16 +343,20 @@ def build(*, force: bool = False, verbose: bool = False) -> Path:
             tmp.unlink(missing_ok=True)
             raise KernelUnavailableError(LIBRARY, f"linking failed:\n{proc.stdout}\n{proc.stderr}")
     tmp.replace(SHARED_OBJECT)
+
+
+def _build_host() -> None:
     tmp = HOST_EXTENSION.with_suffix(f".{os.getpid()}.tmp.so")
-    proc = subprocess.run(host_build_command(tmp, source_hash()), capture_output=True, text=True, check=False)
-    if proc.returncode != 0:
-        tmp.unlink(missing_ok=True)
-        raise KernelUnavailableError(LIBRARY, f"compiling the host extension failed:\n{proc.stdout}\n{proc.stderr}")
-    tmp.replace(HOST_EXTENSION)
-    return SHARED_OBJECT
-
-
-_LOCK = threading.Lock()
+    try:
+        proc = subprocess.run(host_build_command(tmp, host_hash()), capture_output=True, text=True, check=False)
+        text = None if proc.returncode == 0 else f"{proc.stdout}\n{proc.stderr}"
+    except OSError as e:  # no compiler
+        text = str(e)
+    if text is None:
+        tmp.replace(HOST_EXTENSION)
+        return
+    tmp.unlink(missing_ok=True)
+    warnings.warn(f"{HOST_EXTENSION.name} did not compile: calls go through ctypes, some microseconds slower each.\n{text}", RuntimeWarning, stacklevel=3)
 
 
 @functools.cache
@@ -340,7 +366,7 @@ def library() -> ctypes.CDLL:
     Raises:
         KernelUnavailableError: The shared object is not built or does not load (the message says which).
     """
-    if needs_build():
+    if built_hash() != source_hash():
         # A binary of other sources must never answer for these, and nothing is built behind the caller's back.
         state = "is not built" if not SHARED_OBJECT.exists() else "was built from other sources than the ones beside it"
         how = "run `python -c 'import fastforks_b200; fastforks_b200.build()'`"
@@ -386,12 +412,15 @@ def library() -> ctypes.CDLL:
 
 @functools.cache
 def host() -> ModuleType:
-    """The loaded host extension (after `library()`, which checks both binaries against the sources).
+    """The loaded host extension.
 
     Raises:
-        KernelUnavailableError: It is not built or does not load.
+        KernelUnavailableError: The library or the extension is not built for these sources, this torch and this Python, or does not
+            load.
     """
     library()
+    if built_hash(HOST_EXTENSION) != host_hash():
+        raise KernelUnavailableError(LIBRARY, f"{HOST_EXTENSION.name} is not built for these sources, this torch and this Python")
     loader = importlib.machinery.ExtensionFileLoader("_b200host", str(HOST_EXTENSION))
     spec = importlib.util.spec_from_file_location("_b200host", str(HOST_EXTENSION), loader=loader)
     try:
@@ -405,13 +434,19 @@ def host() -> ModuleType:
 # The host extension, once this process has launched an operator the full way (the library is loaded and checked then). Its
 # functions take the plain, valid call of an operator and answer None (False) to anything else.
 fast: ModuleType | None = None
+_fast_tried = False
 
 
 def use_fast() -> None:
-    """Let repeated calls go through the host extension."""
-    global fast  # noqa: PLW0603
-    if fast is None:
-        fast = host()
+    """Let repeated calls go through the host extension. Without it every call goes through ctypes, so this never raises (it is
+    called behind a launch): a warning says once that calls are slower than they could be."""
+    global fast, _fast_tried  # noqa: PLW0603
+    if not _fast_tried:
+        _fast_tried = True
+        try:
+            fast = host()
+        except KernelUnavailableError as e:
+            warnings.warn(f"calls go through ctypes, some microseconds slower each: {e}", RuntimeWarning, stacklevel=3)
 
 
 def last_error() -> str:

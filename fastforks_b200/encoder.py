@@ -188,4 +188,5 @@ def native_or_none(blocks: Sequence[dict], others: dict[str, tuple[torch.Tensor,
     except ValueError as e:
         _LOG.info("layer by layer: %s", e)
         return None
+    _lib.use_fast()  # for `Snapshot`
     return native

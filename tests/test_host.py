@@ -5,6 +5,7 @@ signatures, mode resolution. Mirrors the reference's launcher tests that need no
 from __future__ import annotations
 
 import importlib
+import warnings
 
 import pytest
 import torch
@@ -164,6 +165,65 @@ def test_missing_library_fails_loudly(monkeypatch: pytest.MonkeyPatch, tmp_path)
             _lib.library()
     finally:
         _lib.library.cache_clear()
+
+
+def fresh_host(monkeypatch: pytest.MonkeyPatch):  # noqa: ANN201
+    """`_lib` as in a process that has launched nothing yet; its caches are emptied again by the caller."""
+    from fastforks_b200 import _lib
+
+    if _lib.needs_build():
+        _lib.build()
+    monkeypatch.setattr(_lib, "fast", None)
+    monkeypatch.setattr(_lib, "_fast_tried", False)
+    _lib.host.cache_clear()
+    return _lib
+
+
+def test_operators_work_without_the_host_extension(monkeypatch: pytest.MonkeyPatch, tmp_path) -> None:  # noqa: ANN001
+    """The extension only saves host time: missing, for another torch or not loadable it leaves a warning, once, and never an
+    exception, which would come behind a launch."""
+    _lib = fresh_host(monkeypatch)
+    try:
+        with monkeypatch.context() as m:
+            m.setattr(_lib, "HOST_EXTENSION", tmp_path / "absent.so")
+            with pytest.warns(RuntimeWarning, match="ctypes"):
+                _lib.use_fast()
+            assert _lib.fast is None
+            _lib.library.cache_clear()
+            _lib.library()  # which does not ask for the extension
+            with warnings.catch_warnings():
+                warnings.simplefilter("error")
+                _lib.use_fast()
+        with monkeypatch.context() as m:
+            m.setattr(torch, "__version__", "1.0.0+other")
+            m.setattr(_lib, "_fast_tried", False)
+            assert _lib.needs_build()
+            with pytest.warns(RuntimeWarning, match="this torch"):
+                _lib.use_fast()
+        with monkeypatch.context() as m:
+            broken = tmp_path / "broken.so"
+            broken.write_bytes(b"b200attn-src:" + _lib.host_hash().encode())
+            m.setattr(_lib, "HOST_EXTENSION", broken)
+            m.setattr(_lib, "_fast_tried", False)
+            with pytest.warns(RuntimeWarning, match="cannot load"):
+                _lib.use_fast()
+        assert _lib.fast is None
+        monkeypatch.setattr(_lib, "_fast_tried", False)
+        _lib.use_fast()
+        assert _lib.fast is not None
+    finally:
+        _lib.library.cache_clear()
+        _lib.host.cache_clear()
+
+
+def test_a_build_without_torch_headers_still_has_the_library(monkeypatch: pytest.MonkeyPatch, tmp_path) -> None:  # noqa: ANN001
+    _lib = fresh_host(monkeypatch)
+    monkeypatch.setattr(_lib, "HOST_EXTENSION", tmp_path / "_b200host.so")
+    for command in (["false"], [str(tmp_path / "no-such-compiler")]):
+        monkeypatch.setattr(_lib, "host_build_command", lambda *a, command=command: command)
+        with pytest.warns(RuntimeWarning, match="did not compile"):
+            assert _lib.build() == _lib.SHARED_OBJECT
+    assert not _lib.HOST_EXTENSION.exists()
 
 
 def test_host_attention_contract_is_checked_before_any_copy() -> None:
