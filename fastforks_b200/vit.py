@@ -16,6 +16,7 @@ from __future__ import annotations
 
 import math
 from dataclasses import dataclass
+from typing import TYPE_CHECKING
 
 import torch
 import torch.nn.functional as F  # noqa: N812
@@ -23,6 +24,9 @@ import torch.nn.functional as F  # noqa: N812
 from . import _lib, encoder
 from .flash64 import Flash64, is_stock
 from .gemm import ACT_GELU_TANH, ACT_NONE, gemm
+
+if TYPE_CHECKING:
+    from collections.abc import Callable
 
 
 @dataclass(frozen=True)
@@ -187,10 +191,7 @@ class ViTEncoder:
         gh, gw = height // ps, width // ps
         if width % 2 or gh == 0 or gw == 0 or images.data_ptr() % 16:
             return None
-        if (gh, gw) not in self._pos32:
-            pos = self.pos_embed_fp32(gh, gw).contiguous()
-            self._pos32[gh, gw] = pos.clone() if pos.data_ptr() % 16 else pos
-        pos = self._pos32[gh, gw]
+        pos = self._kept(self._pos32, (gh, gw), self._pos_aligned)
         if pos.shape != (1, 1 + gh * gw, self.cfg.dim):
             return None
         extra = {  # "images": any address, the description only needs to know that there are images
@@ -206,12 +207,25 @@ class ViTEncoder:
         native.launch(described, images.device, images=images, taps=list(zip(taps, outs)))
         return outs
 
+    def _kept(self, tables: dict[tuple[int, int], torch.Tensor], grid: tuple[int, int], make: Callable[[int, int], torch.Tensor]) -> torch.Tensor:
+        """`make(*grid)`, kept in `tables` for later calls on any stream: it is waited for once. Under capture it is made in the graph
+        and not kept, since nothing has computed it until the graph is replayed."""
+        if grid not in tables:
+            table = make(*grid)
+            if table.is_cuda and table.data_ptr() != self.pos_table.data_ptr():
+                if torch.cuda.is_current_stream_capturing():
+                    return table
+                torch.cuda.current_stream(table.device).synchronize()
+            tables[grid] = table
+        return tables[grid]
+
     def pos_embed(self, gh: int, gw: int) -> torch.Tensor:
         """Position table for a `gh x gw` patch grid (upstream `interpolate_pos_encoding`, net/dinov2.py:198-237)."""
-        key = (gh, gw)
-        if key not in self._pos:
-            self._pos[key] = self.pos_embed_fp32(gh, gw).to(self.dtype)
-        return self._pos[key]
+        return self._kept(self._pos, (gh, gw), lambda gh, gw: self.pos_embed_fp32(gh, gw).to(self.dtype))
+
+    def _pos_aligned(self, gh: int, gw: int) -> torch.Tensor:
+        pos = self.pos_embed_fp32(gh, gw).contiguous()
+        return pos.clone() if pos.data_ptr() % 16 else pos
 
     def pos_embed_fp32(self, gh: int, gw: int) -> torch.Tensor:
         table = self.pos_table

@@ -110,3 +110,30 @@ def test_one_image_of_vit_b16_eager_against_replayed(capsys: pytest.CaptureFixtu
     with capsys.disabled():
         print(f"\nvit-b16, one image: {eager:.3f} ms per forward eager, {replayed:.3f} ms replayed from a graph")
     assert replayed < eager
+
+
+@pytest.mark.parametrize("native", [True, False])
+def test_a_geometry_first_seen_under_capture_is_not_kept_from_it(native: bool, monkeypatch: pytest.MonkeyPatch) -> None:  # noqa: FBT001
+    """The interpolated position table of a grid that a capture meets first exists when the graph is replayed, not before: an eager
+    call between the two must make its own."""
+    from fastforks_b200.vit import CONFIGS, ViTEncoder, seeded_state
+
+    cfg = CONFIGS["dinov2-vits14"]
+    enc, fresh = (ViTEncoder(cfg, seeded_state(cfg, 1), device="cuda", dtype=torch.float16, fuse_plain=True) for _ in range(2))
+    if not native:
+        for e in (enc, fresh):
+            monkeypatch.setattr(e, "_native_now", lambda: None)
+    other = torch.rand(1, 3, 56, 56, generator=torch.Generator().manual_seed(1)).cuda()
+    images = torch.rand(1, 3, 70, 84, generator=torch.Generator().manual_seed(2)).cuda()
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        enc(other)  # warm-up, at another size
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=side):
+            captured = enc(images)
+    torch.cuda.current_stream().wait_stream(side)
+    want = fresh(images)
+    assert torch.equal(enc(images), want)
+    graph.replay()
+    assert torch.equal(captured, want) and torch.equal(enc(images), want)
