@@ -57,7 +57,7 @@ NVCC_FLAGS = (
 
 # Every symbol include/b200_attn.h declares.
 EXPORTS = (
-    "b200_attn_fwd", "b200_attn_fwd_static", "b200_gemm", "b200_sam_rel_terms", "b200_rope_qk", "b200_attn_query", "b200_attn_plan", "b200_attn_workspace_size", "b200_attn_status",
+    "b200_attn_fwd", "b200_attn_fwd_static", "b200_gemm", "b200_gemm_plan", "b200_sam_rel_terms", "b200_rope_qk", "b200_attn_query", "b200_attn_plan", "b200_attn_workspace_size", "b200_attn_status",
     "b200_attn_selftest_wait_limit", "b200_attn_last_error", "b200_attn_version",
 )  # fmt: skip
 
@@ -397,6 +397,8 @@ def library() -> ctypes.CDLL:
     i32p = ctypes.POINTER(ctypes.c_int32)
     lib.b200_attn_plan.argtypes = (ctypes.POINTER(B200AttnArgs), ctypes.c_int32, ctypes.c_int32, i32p, i32p, ctypes.c_int32, i32p, i32p)
     lib.b200_attn_plan.restype = ctypes.c_int
+    lib.b200_gemm_plan.argtypes = (ctypes.c_int32, ctypes.c_int32, ctypes.c_int32, ctypes.c_int32, i32p, i32p)
+    lib.b200_gemm_plan.restype = ctypes.c_int
     lib.b200_attn_workspace_size.argtypes = (ctypes.POINTER(ctypes.c_int64),)
     lib.b200_attn_workspace_size.restype = ctypes.c_int
     lib.b200_attn_status.argtypes = (ctypes.POINTER(ctypes.c_uint32),)

@@ -301,6 +301,27 @@ int b200_gemm(const B200GemmArgs* a, void* stream_ptr) {
   return B200_ATTN_OK;
 }
 
+int b200_gemm_plan(int32_t m, int32_t n, int32_t k, int32_t sms, const int32_t* clusters, int32_t* plan) {
+  if (m < 1 || n < 1 || k < 1 || sms < 0 || plan == nullptr || (sms > 0 && clusters == nullptr))
+    return fail(B200_ATTN_BAD_CONFIG, "b200_gemm_plan: m %d n %d k %d sms %d, plan and (with sms) split_clusters not NULL", m, n, k, sms);
+  int fit[kGemmSplits];
+  if (sms > 0) {
+    std::copy_n(clusters, kGemmSplits, fit);
+  } else {
+    DeviceState* dev = nullptr;
+    if (int rc = device_state(&dev)) return rc;
+    if (int rc = split_clusters(*dev)) return rc;
+    for (int i = 0; i < kGemmSplits; ++i) fit[i] = dev->split_clusters[i].load(std::memory_order_relaxed);
+    sms = dev->sms;
+  }
+  const GemmPlan p = gemm_plan(m, n, k, false, sms, fit);
+  plan[0] = p.bn;
+  plan[1] = p.split;
+  plan[2] = p.tail_bn;
+  clear_error();
+  return B200_ATTN_OK;
+}
+
 int b200_sam_rel_terms(const B200RelTermsArgs* a, void* stream_ptr) {
   if (a == nullptr) return fail(B200_ATTN_BAD_CONFIG, "args is NULL");
   if (a->struct_size != sizeof(B200RelTermsArgs))

@@ -141,7 +141,7 @@ struct GemmItem {
 };
 // Items are the tiles in groups of `group_m` row tiles, row tiles fastest inside a group: the pairs that run at the same
 // time then share both w tiles and x tiles, and what they read together stays in L2. The tiles behind the last whole
-// round of the grid come in parts (pair_items() in b200_linear.cu says when), parts of a tile one after another.
+// round of the grid come in parts where gemm_plan() in b200_linear.cu says so, parts of a tile one after another.
 __device__ __forceinline__ GemmItem item_at(const GemmParams& p, int item, int out_cols) {
   GemmItem t;
   int tile = item, sub = 0;

@@ -199,6 +199,14 @@ typedef struct B200GemmArgs {
 int b200_gemm(const B200GemmArgs* args, void* stream);
 
 /*
+ * How b200_gemm would cut a product of m x n x k, without launching: plan[0] columns of a tile, plan[1] CTAs that share the k range
+ * of a 128 x 64 tile (0: pairs of CTAs with tiles of 256 rows), plan[2] columns of the narrow parts that the tiles behind the last
+ * whole round are cut into (0: none).  `sms` SMs and `split_clusters[6]` (how many clusters of 1, 2, 3, 4, 6 and 8 CTAs run at once)
+ * describe the device; with sms = 0 they are the current device's and split_clusters is not read.
+ */
+int b200_gemm_plan(int32_t m, int32_t n, int32_t k, int32_t sms, const int32_t* split_clusters, int32_t* plan);
+
+/*
  * The producer of SAM's decomposed bias: for every query (y, x) of a `side` x `side` grid and k = 0 .. side - 1
  *     rel_h[b, head, (y, x), k] = q[b, (y, x), head, :] . rel_pos_h[y - k + side - 1, :]
  *     rel_w[b, head, (y, x), k] = q[b, (y, x), head, :] . rel_pos_w[x - k + side - 1, :]

@@ -189,3 +189,19 @@ def test_encoder_refuses_windows_it_cannot_count(lib: ctypes.CDLL, window: int) 
     assert lib.b200_encoder_workspace(ctypes.byref(_encoder_args(**{"block.window": window})), ctypes.byref(size)) == _lib.UNSUPPORTED
     want = _lib.OK if window < 1000 else _lib.UNSUPPORTED  # noqa: PLR2004
     assert lib.b200_encoder_workspace(ctypes.byref(_encoder_args(**{"block.window": window}, **plain)), ctypes.byref(size)) == want
+
+
+def test_gemm_plan_on_the_host(lib: ctypes.CDLL) -> None:
+    """The plan as a function of sizes and of the device's description, without a GPU."""
+    clusters, plan = (ctypes.c_int32 * 6)(148, 74, 48, 36, 22, 16), (ctypes.c_int32 * 3)()
+    seen = {}
+    for shape in ((197, 768, 3072), (100, 72, 8), (5480, 4096, 1024), (21920, 1536, 4096), (2740, 4096, 200)):
+        assert lib.b200_gemm_plan(*shape, 148, clusters, plan) == _lib.OK
+        seen[shape] = tuple(plan)
+    assert seen[197, 768, 3072][1] > 1  # few tiles: the k range is shared
+    assert seen[100, 72, 8] == (64, 1, 0)
+    assert seen[5480, 4096, 1024][:2] == seen[21920, 1536, 4096][:2] == (256, 0)
+    assert seen[2740, 4096, 200] == (256, 0, 128)  # 176 tiles on 74 pairs: the last round in halves
+    none = (ctypes.c_int32 * 6)(148, 0, 0, 0, 0, 0)  # a device that runs no clusters of the split kernel
+    assert lib.b200_gemm_plan(197, 768, 3072, 148, none, plan) == _lib.OK and plan[1] <= 1
+    assert lib.b200_gemm_plan(0, 8, 8, 148, clusters, plan) == lib.b200_gemm_plan(8, 8, 8, 148, None, plan) == _lib.BAD_CONFIG

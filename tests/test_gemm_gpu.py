@@ -9,11 +9,14 @@ relative form for this library's GEMMs: `|got - ref| <= 2e-2 * max|ref|`, mean w
 
 from __future__ import annotations
 
+import ctypes
+
 import pytest
 import torch
 
 import fastforks_b200 as ff
 from conftest import assert_close
+from fastforks_b200 import _lib
 from oracle import gemm_oracle as go
 
 pytestmark = pytest.mark.gpu
@@ -42,7 +45,7 @@ def check(got: torch.Tensor, x, w, bias=None, scale=None, res=None, act: int = 0
     assert_close(got.float().cpu().numpy(), ref, unit_scale=False, what=what)
 
 
-# tile edges of the three tile shapes (128 x 128, 128 x 256, 256 x 256), k tails, the smallest problem, ViT shapes
+# tile edges (128 x 64 and 256 x 64 .. 256 tiles), k tails, the smallest problem, ViT shapes
 SHAPES = [(1, 8, 8), (128, 128, 64), (129, 136, 72), (255, 256, 64), (257, 264, 200), (300, 1000, 520), (1370, 1152, 384),
           (5480, 1024, 1024), (2740, 3072, 1024), (700, 4096, 1024)]  # fmt: skip
 
@@ -94,7 +97,20 @@ def test_layerscale_and_in_place_residual(m: int, n: int, k: int, dtype: str) ->
 # One shape for every way a product is cut: the split kernel whole and with 2, 3, 4, 6 and 8 CTAs per cluster (uneven k
 # shares, rows that do not divide, a last tile of one row), pair tiles of 64 to 256 columns, and a last round in parts.
 PLANS = [(100, 72, 8), (197, 2304, 776), (257, 1024, 1544), (129, 776, 1000), (60, 64, 3080), (255, 384, 1536), (1, 8, 4096), (1000, 3000, 72),
-         (1500, 768, 768), (1025, 2056, 136), (5480, 1000, 328), (9500, 2056, 72), (2740, 4096, 200)]  # fmt: skip
+         (1500, 768, 768), (1025, 2056, 136), (5480, 1000, 328), (9500, 2056, 72), (2740, 4096, 200), (29, 664, 264), (377, 32, 360), (20682, 8, 248),
+         (5180, 728, 104), (4349, 2912, 512), (10380, 5496, 568)]  # fmt: skip
+
+
+def test_the_shapes_below_are_cut_in_every_way() -> None:
+    """What `b200_gemm_plan` says of them on this device: (columns of a tile, CTAs per split tile, columns of the last round's parts)."""
+    torch.cuda.current_device()
+    plan, found = (ctypes.c_int32 * 3)(), set()
+    for shape in PLANS:
+        assert _lib.library().b200_gemm_plan(*shape, 0, None, plan) == _lib.OK
+        found.add(tuple(plan))
+    splits = {(64, s, 0) for s in (1, 2, 3, 4, 6, 8)}
+    pairs = {(bn, 0, 0) for bn in (64, 128, 192, 256)}
+    assert found == splits | pairs | {(256, 0, 64), (256, 0, 128)}
 
 
 @pytest.mark.parametrize(("m", "n", "k"), PLANS)
