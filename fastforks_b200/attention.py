@@ -234,7 +234,8 @@ def attention(  # noqa: PLR0913
         layout: `"bhnd"` or `"bnhd"`.
         out: Optional output view of q's shape and dtype.
         schedule: `"auto"`, `"long"` or `"short"` tile schedule; `"auto"` takes the short one for at most 256 keys whose last
-            128-key tile holds at most 96 (e.g. 197 tokens). The result does not depend on it.
+            128-key tile holds at most 96 (e.g. 197 tokens). A hint for the persistent kernel: the result does not depend on it, and
+            calls without bias too small to fill the GPU (up to 512 keys) go to a kernel of their own whatever it says.
 
     Returns:
         A tensor of q's shape. Without `out` its memory is `[B, N, heads, 64]`-contiguous in both layouts, so the

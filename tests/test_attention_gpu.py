@@ -104,11 +104,35 @@ def test_flash64_fuzz(variant: str, seed: int) -> None:
 @pytest.mark.parametrize("n", [1, 2, 63, 64, 65, 127, 128, 129, 196, 197, 255, 256, 257, 383, 385, 512, 513, 1370])
 @pytest.mark.parametrize("dtype", ["fp16", "bf16"])
 def test_tile_boundaries(n: int, dtype: str) -> None:
-    """Sequence lengths around every tile edge of the kernel (128-row query tiles, 128-key tiles, two tiles per CTA)."""
+    """Sequence lengths around every tile edge (six heads: up to 512 keys the kernel of small calls answers)."""
     qkv = packed_qkv(2, n, 3, DTYPES[dtype], 1.0, n)
     q, k, v = qkv.unbind(2)
     got = ff.attention(q, k, v, layout="bnhd")
     assert_close(got.float().cpu().numpy(), oracle_of_packed(qkv, 0.125), unit_scale=True, what=f"n{n} {dtype}")
+
+
+@pytest.mark.parametrize("n", [1, 2, 63, 64, 65, 127, 128, 129, 130, 160, 196, 197, 225, 255, 256, 257, 383, 385, 512])
+@pytest.mark.parametrize("dtype", ["fp16", "bf16"])
+def test_tile_boundaries_of_the_persistent_kernel(n: int, dtype: str) -> None:
+    """The same edges (128-row query tiles, 128-key tiles, two tiles per CTA) with more heads than the kernel of small calls takes
+    (300 blocks of queries on 148 SMs), both schedules and the automatic choice with the same bits, and nothing
+    written around the output view."""
+    b, h, dt = 3, 100, DTYPES[dtype]
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    qkv = torch.randn(b, n, 3, h, 64, generator=gen, device="cuda").to(dt)
+    q, k, v = qkv.unbind(2)
+    logits = torch.einsum("bqhd,bkhd->bhqk", q.float(), k.float()) * 0.125
+    ref = torch.einsum("bhqk,bkhd->bqhd", logits.softmax(-1), v.float())
+    outs = []
+    for schedule in ("auto", "long", "short"):
+        big = torch.full((b, n + 7, h + 1, 64), 77.0, dtype=dt, device="cuda")
+        out = big[:, 3 : 3 + n, :h]
+        ff.attention(q, k, v, scale=0.125, layout="bnhd", out=out, schedule=schedule)
+        assert_close(out.float().cpu().numpy(), ref.cpu().numpy(), unit_scale=True, what=f"n{n} {dtype} {schedule}")
+        outs.append(out.clone())
+        out.fill_(77.0)
+        assert bool((big == 77.0).all())
+    assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
 
 
 def test_output_rows_past_the_sequence_are_untouched() -> None:
@@ -654,7 +678,8 @@ def test_mixed_one_and_two_tile_items_cover_every_query_tile_once(b: int, n: int
 def test_both_schedules_give_the_same_result(schedule: str, n: int) -> None:
     """The short schedule skips the exponentials of a last key tile's final 32 columns when they hold no key (197,
     160, 130 keys: taken; 225, 256: tile too full; 1370: only on request). Any hint must give the oracle's result,
-    and the two schedules the same bits."""
+    and the two schedules the same bits. (Six heads: up to 512 keys the kernel of small calls answers whatever the hint; the persistent
+    kernel's schedules are compared at these sizes in test_tile_boundaries_of_the_persistent_kernel.)"""
     qkv = packed_qkv(2, n, 3, torch.float16, 1.0, seed=n)
     q, k, v = qkv.unbind(2)
     got = ff.attention(q, k, v, scale=0.125, layout="bnhd", schedule=schedule)
