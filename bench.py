@@ -273,11 +273,6 @@ def model_throughput(torch, ff, world: int, timed) -> dict | None:  # noqa: ANN0
     ms = timed(forward, steps)
     forward_e2e()
     ms_e2e = timed(forward_e2e, steps)
-    own = ViTEncoder(cfg, seeded_state(cfg, 0), device="cuda", dtype=torch.bfloat16, fuse_plain=True)
-    for _ in range(2):
-        own(images)
-    ms_own = timed(lambda: own(images), steps)
-    del own
     # The launch-bound configuration (one image of ViT-B/16 at 224 px, 197 tokens): the forward as a stream of launches
     # and replayed from a CUDA graph.
     small_cfg = CONFIGS["vit-b16"]
@@ -302,8 +297,7 @@ def model_throughput(torch, ff, world: int, timed) -> dict | None:  # noqa: ANN0
         "images_per_s": batch * steps * world / (ms * 1e-3),
         "ms_per_forward": ms / steps,
         "attention_gflop_per_image": enc.attention_flops(1, side, side) / 1e9,
-        "linear_layers": "proj, fc1, fc2 on this library's GEMM with fused epilogue; qkv (bias only) on torch's library GEMM",
-        "images_per_s_every_linear_layer_own_gemm": batch * steps * world / (ms_own * 1e-3),
+        "linear_layers": "all on this library's GEMM with fused epilogue, launched with the rest of the forward by one native call",
         "e2e": {
             "images_per_s": batch * steps * world / (ms_e2e * 1e-3),
             "h2d_bytes_per_forward": host_images.numel() * 4,

@@ -94,6 +94,7 @@ enum : int { kItemWhole = 0, kItemPartial = 1, kItemOwner = 2 };
 // tensor pipe above some 96 values per row and by the softmax step below. us, additions by the softmax warps -> here
 // ([B,H,N]): [4,12,1024] 271 -> 40, [2,12,2304] 853 -> 72, [10,12,400] 170 -> 26, [100,12,36] 113 -> 41; [1,12,4096], whose
 // 64-wide tables had a form of their own (kBiasDecomposed64), 101 -> 99. The 14 x 14 form stays ahead: [400,12,196] 183 against 216.
+// kBiasDecomposed64 is left for 64-wide tables with more than 64 rows or a scale whose inverse is no power of two.
 enum : int { kBiasNone = 0, kBiasDense = 1, kBiasDecomposed = 2, kBiasDecomposed64 = 3, kBiasDecomposed14 = 4, kBiasDenseTiles = 5, kBiasDecomposedMma = 6 };
 constexpr int kMaxRelChunks = 16;   // kBiasDecomposedMma: groups of eight values per row of R and E
 constexpr int kRelStageWords = 33;  // per-row staging of rel_h | rel_w in shared memory: up to 32 values, odd stride

@@ -289,7 +289,8 @@ __global__ void __launch_bounds__(kTokensThreads) encoder_tokens_kernel(const To
 // A convolution's weights as the rows of a linear layer, in pairs of 16-bit values, a CTA per row: padded with zeros to a row
 // of whole 16-byte groups (the patch embedding of patches of 14), or with the kernel's positions in front of the channels
 // (the neck's 3 x 3, whose input rows are nine channel vectors). Done in every forward, on 1-2 MB, so that the convolution's
-// own tensor is what a forward reads; a copy kept from the first one would not see that tensor change.
+// own tensor is what a forward reads; a copy kept from the first one would not see that tensor change. With the start values
+// summed in fp32 it adds 2.7 us to the 24.7 of patches, product and one norm at four images of 518 x 518 (1024 wide), 1.4 at one.
 struct RepackParams {
   const void* src;  // [rows, cols]; taps > 0: [rows, cols / taps, taps]
   void* dst;        // [rows, out_cols], zeros from cols on; taps > 0: [rows, taps, cols / taps]

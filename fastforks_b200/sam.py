@@ -5,8 +5,9 @@ The caller side of the hot path for SAM: blocks with 14 x 14 windowed attention 
 logits. Written from the math of the upstream module the reference vendors
 (`src/fastforks/promptable_segmentation/models/sam/net/image_encoder.py:17-241, 293-362`): the attention of every
 block is this library's kernel with `rel=(rel_h, rel_w)` - q, k, v stay 64 wide views of the packed qkv tensor -
-where the reference's kernels mode widens q and k instead (`sam/fast.py:92-113`). Everything else is a plain torch
-call. It exists for model-level parity (cosine >= 0.999 against the reference's portable encoder,
+where the reference's kernels mode widens q and k instead (`sam/fast.py:92-113`). On a CUDA device a forward is one
+native call (`encoder`, include/b200_encoder.h) over this library's kernels; block by block (odd grids, replaced steps),
+everything but attention and its relative terms is a plain torch call. It exists for model-level parity (cosine >= 0.999 against the reference's portable encoder,
 `tests/golden/make_golden.py`) and for timing SAM's two attention shapes in place.
 
 Parameter names are the upstream ones, so a state dict of `ImageEncoderViT` loads unchanged.

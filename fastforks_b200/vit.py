@@ -1,10 +1,14 @@
 """Kernels-mode ViT encoder around the attention operator: the caller side of the hot path.
 
 A harness of the DINOv2 / timm ViT block family: layer norms, packed qkv, attention on strided `[B, N, heads, 64]`
-views of it through `Flash64`, projection with LayerScale and residual, MLP or fused SwiGLU. On a CUDA device every
-linear layer is one launch of this library's GEMM with the fused epilogue (bias, GELU, LayerScale, in-place residual:
-what the reference's kernels mode does with its `dpt_fused` library, `src/fastforks/shared/depth_anything_v2/
-fast_vit.py:192-208`) and the attention is the B200 kernel; LayerNorm, the patch embedding and SiLU stay torch calls.
+views of it, projection with LayerScale and residual, MLP or SwiGLU. On a CUDA device a forward is one native call
+(`encoder`, include/b200_encoder.h) that launches this library's kernels for all of it, patch embedding and norms
+included; the reference's kernels mode does as much with its `dpt_fused` library and torch calls in between
+(`src/fastforks/shared/depth_anything_v2/fast_vit.py:192-208`). What the native call does not take runs layer by layer:
+images of an odd width or off a 16-byte boundary, patches of an odd side, parameters that are strided views or of other
+shapes, tokens that require a gradient, a model whose attention launcher or steps were replaced. Attention is then
+`Flash64`, the linear layers are this library's GEMM with the fused epilogue (bias, GELU, LayerScale, in-place residual),
+and LayerNorm, patch embedding and SiLU are torch calls.
 It exists to measure whole-model throughput and to check model-level parity (cosine >= 0.999 against the reference's
 portable network, `tests/golden/make_golden.py`), not to replace the reference's model zoo.
 
@@ -140,9 +144,8 @@ class ViTEncoder:
         # On a CUDA device the linear layers run on this library's GEMM with the fused epilogue, which takes the
         # LayerScale factors as fp32 vectors; elsewhere (CPU harness tests) they are torch calls.
         self.fused = self.device.type == "cuda" if fused is None else fused
-        # Layers with nothing but a bias behind the product (qkv, SwiGLU's w12) go to torch's library GEMM unless
-        # `fuse_plain`: without an epilogue to fuse there is no traffic to save, and without cluster multicast (which
-        # this library never uses) a GEMM of its own is bound by the L2 at about 0.8 of the library's rate.
+        # Layer by layer, those with nothing but a bias behind the product (qkv, SwiGLU's w12) go to torch's library GEMM unless
+        # `fuse_plain`. The native call has every product on this library's GEMM and does not ask.
         self.fuse_plain = fuse_plain
         self.scales = {k: v.to(self.device, torch.float32) for k, v in state.items() if k.endswith(".gamma")}
         # ... and the whole forward is one native call (`encoder`) that reads the parameters in `self.w` and `self.scales`.

@@ -81,17 +81,21 @@ def test_kernels_encoder_matches_reference_network(name: str, dtype: torch.dtype
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("fuse_plain", [False, True])
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
-def test_kernels_encoder_with_every_linear_layer_on_the_own_gemm(dtype: torch.dtype) -> None:
-    """By default the layers with nothing to fuse behind the product (qkv) go to torch's library GEMM; with
-    `fuse_plain` all four linear layers of every block run on this library's GEMM."""
+def test_layer_by_layer_form_matches_the_reference_network(dtype: torch.dtype, fuse_plain: bool, monkeypatch: pytest.MonkeyPatch) -> None:  # noqa: FBT001
+    """What runs where the native call does not take a model or its images: every layer a call of its own, those with nothing to fuse
+    behind the product (qkv) on torch's library GEMM or, with `fuse_plain`, on this library's like the others."""
     import fastforks_b200 as ff
 
     g, state, images = golden_inputs("model_dinov2_vits14_sharp")
-    enc = ViTEncoder(CONFIGS["dinov2-vits14"], state, device="cuda", dtype=dtype, fuse_plain=True)
+    enc = ViTEncoder(CONFIGS["dinov2-vits14"], state, device="cuda", dtype=dtype, fuse_plain=fuse_plain)
+    native = enc(images).float().cpu().numpy()
+    monkeypatch.setattr(enc, "_native_now", lambda: None)
     out = enc(images).float().cpu().numpy()
     assert ff.device_status() == 0 and np.isfinite(out).all()
     assert cosine(out, g["out"]) >= 0.999, cosine(out, g["out"])
+    assert cosine(out, native) >= 0.999 and not np.array_equal(out, native)
 
 
 @pytest.mark.gpu
