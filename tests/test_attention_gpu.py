@@ -618,8 +618,8 @@ def test_host_operands_pipeline_matches_the_device_call(depth: int) -> None:
 
 
 def test_repeated_geometry_takes_the_remembered_launch_and_still_checks() -> None:
-    """The second call with the same views goes through the remembered description: same result, new pointers are
-    used, and a call that breaks the contract is still rejected before the launch."""
+    """The second call goes through the host extension: same result, new pointers are used, and a call that breaks the contract
+    is still rejected before the launch."""
     qkv = packed_qkv(2, 197, 4, torch.float16, 1.0, seed=3)
     q, k, v = qkv.unbind(2)
     first = ff.attention(q, k, v, layout="bnhd")
