@@ -56,7 +56,9 @@ class Snapshot:
     kernels read the tensors themselves.) The tensors are kept alive, so that no address is used again while it is in the table."""
 
     def __init__(self, *dicts: dict[str, torch.Tensor]) -> None:
-        self._native = None if _lib.fast is None else _lib.fast.snapshot(dicts)
+        _lib.use_fast()
+        self._host = _lib.fast
+        self._native = None if self._host is None else self._host.snapshot(dicts)
         self._kept = None if self._native is not None else self._facts(dicts)
 
     @staticmethod
@@ -65,7 +67,7 @@ class Snapshot:
 
     def changed(self, *dicts: dict[str, torch.Tensor]) -> bool:
         if self._native is not None:
-            return not _lib.fast.unchanged(self._native, dicts)
+            return not self._host.unchanged(self._native, dicts)
         return [f[:-1] for f in self._kept] != [f[:-1] for f in self._facts(dicts)]
 
 
@@ -188,5 +190,4 @@ def native_or_none(blocks: Sequence[dict], others: dict[str, tuple[torch.Tensor,
     except ValueError as e:
         _LOG.info("layer by layer: %s", e)
         return None
-    _lib.use_fast()  # for `Snapshot`
     return native

@@ -194,7 +194,8 @@ class SamEncoder:
         if encoder.overrides(self, SamEncoder, ("attend", "block", "norm2d")):
             return None
         if self._has_native and (self._snapshot is None or self._snapshot.changed(self.w)):
-            self._native, self._snapshot = self._make_native(), encoder.Snapshot(self.w)
+            snapshot = encoder.Snapshot(self.w)  # first: what changes while the table is made is seen by the next call
+            self._native, self._snapshot = self._make_native(), snapshot
         return self._native
 
     def _make_native(self) -> encoder.NativeEncoder | None:

@@ -163,7 +163,8 @@ class ViTEncoder:
         if not self.fused or self.device.type != "cuda" or not encoder.supported(self.dtype, cfg.dim, cfg.heads, cfg.hidden):
             return None
         if self._snapshot is None or self._snapshot.changed(self.w, self.scales):
-            self._native, self._snapshot = self._make_native(), encoder.Snapshot(self.w, self.scales)
+            snapshot = encoder.Snapshot(self.w, self.scales)  # first: what changes while the table is made is seen by the next call
+            self._native, self._snapshot = self._make_native(), snapshot
         return self._native
 
     def _make_native(self) -> encoder.NativeEncoder | None:

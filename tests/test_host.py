@@ -255,6 +255,7 @@ def test_a_snapshot_sees_tensors_that_were_replaced(native: bool, monkeypatch: p
     from fastforks_b200 import _lib, encoder
 
     monkeypatch.setattr(_lib, "fast", _lib.host() if native else None)
+    monkeypatch.setattr(_lib, "_fast_tried", True)
     a = {"x": torch.zeros(4, 6), "y": torch.zeros(3, dtype=torch.float16)}
     b = {"x": torch.zeros(2)}
     snap = encoder.Snapshot(a, b)
