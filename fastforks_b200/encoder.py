@@ -33,6 +33,14 @@ def supported(dtype: torch.dtype, dim: int, heads: int, hidden: int) -> bool:
     return dtype in _DTYPES and dim == heads * 64 and dim <= MAX_DIM and hidden % 8 == 0
 
 
+class HoldsNative:
+    """What a model that holds a native encoder is copied and pickled as: without it, since it is made of addresses. It is made
+    again from the copy's own tensors."""
+
+    def __getstate__(self) -> dict:
+        return {**self.__dict__, "_native": None, "_snapshot": None}
+
+
 def check_parameter(name: str, t: torch.Tensor, shape: tuple[int, ...], dtype: torch.dtype, device: torch.device) -> None:
     """Refuse a parameter the kernels cannot read through its address alone.
 

@@ -163,7 +163,7 @@ def rel_terms(q: torch.Tensor, table_h: torch.Tensor, table_w: torch.Tensor, sid
     return rel_h, rel_w
 
 
-class SamEncoder:
+class SamEncoder(encoder.HoldsNative):
     """`images [B, 3, 1024, 1024]` -> `[B, 256, 64, 64]`, every block's attention on the B200 kernels."""
 
     def __init__(self, cfg: SamConfig, state: dict[str, torch.Tensor], device: torch.device | str = "cuda",

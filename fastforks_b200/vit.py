@@ -123,7 +123,7 @@ def seeded_state(cfg: ViTConfig, seed: int = 0, *, std: float = 0.02, qk_gain: f
     return state
 
 
-class ViTEncoder:
+class ViTEncoder(encoder.HoldsNative):
     """`images [B, 3, H, W]` -> normalised tokens `[B, N, dim]`, every block's attention on the B200 kernels."""
 
     def __init__(self, cfg: ViTConfig, state: dict[str, torch.Tensor], device: torch.device | str = "cuda",

@@ -6,6 +6,9 @@ replaced where a test reaches it.
 
 from __future__ import annotations
 
+import copy
+import pickle
+
 import pytest
 import torch
 
@@ -207,3 +210,20 @@ def test_replaced_steps_are_seen(monkeypatch: pytest.MonkeyPatch) -> None:
     assert not is_stock(launcher)
     monkeypatch.setattr(Flash64, "_run", staticmethod(lambda *a: None))
     assert not is_stock(enc.attn)
+
+
+@pytest.mark.parametrize("kind", ["vit", "sam"])
+@pytest.mark.parametrize("duplicate", [copy.deepcopy, lambda enc: pickle.loads(pickle.dumps(enc))])  # noqa: S301
+def test_encoders_can_be_copied_and_pickled(kind: str, duplicate) -> None:  # noqa: ANN001
+    """The native table holds addresses of the original's tensors: a copy makes its own."""
+    if kind == "vit":
+        enc = ViTEncoder(CFG, seeded_state(CFG), device="cpu", dtype=torch.float16)
+        enc.scales = {k: v.float() for k, v in enc.scales.items()}
+    else:
+        cfg = SamConfig(img=96, patch=16, dim=128, depth=2, heads=2, out_chans=24, window=4, global_blocks=(1,))
+        enc = SamEncoder(cfg, sam_seeded_state(cfg), device="cpu", dtype=torch.float16)
+    enc._native, enc._snapshot = enc._make_native(), encoder.Snapshot(enc.w)  # noqa: SLF001
+    other = duplicate(enc)
+    assert other._native is None and other._snapshot is None and enc._native is not None  # noqa: SLF001
+    assert all(torch.equal(other.w[k], v) and other.w[k] is not v for k, v in enc.w.items())
+    assert other._make_native() is not None  # noqa: SLF001
