@@ -176,16 +176,24 @@ int split_clusters(DeviceState& dev) {
   return B200_ATTN_OK;
 }
 
-// [dtype][act][scale or residual]; SwiGLU layers have neither.
+// [dtype][act][form]; SwiGLU layers have neither scale nor residual.
 int pair_act_index(int act) { return act == kActNone ? 0 : act == kActRelu ? 1 : act == kActGelu ? 2 : act == kActGeluTanh ? 3 : 4; }
+template <typename T, int ACT>
+const void* pair_kernel_of(int form) {
+  switch (form) {
+    case kPairResidual: return reinterpret_cast<const void*>(gemm_pair_kernel<T, ACT, kPairResidual>);
+    case kPairScaled: return reinterpret_cast<const void*>(gemm_pair_kernel<T, ACT, kPairScaled>);
+    default: return reinterpret_cast<const void*>(gemm_pair_kernel<T, ACT, kPairPlain>);
+  }
+}
 template <typename T>
-const void* pair_kernel(int act, bool full) {
+const void* pair_kernel(int act, int form) {
   switch (act) {
-    case kActRelu: return full ? reinterpret_cast<const void*>(gemm_pair_kernel<T, kActRelu, true>) : reinterpret_cast<const void*>(gemm_pair_kernel<T, kActRelu, false>);
-    case kActGelu: return full ? reinterpret_cast<const void*>(gemm_pair_kernel<T, kActGelu, true>) : reinterpret_cast<const void*>(gemm_pair_kernel<T, kActGelu, false>);
-    case kActGeluTanh: return full ? reinterpret_cast<const void*>(gemm_pair_kernel<T, kActGeluTanh, true>) : reinterpret_cast<const void*>(gemm_pair_kernel<T, kActGeluTanh, false>);
-    case kActSwiGlu: return reinterpret_cast<const void*>(gemm_pair_kernel<T, kActSwiGlu, false>);
-    default: return full ? reinterpret_cast<const void*>(gemm_pair_kernel<T, kActNone, true>) : reinterpret_cast<const void*>(gemm_pair_kernel<T, kActNone, false>);
+    case kActRelu: return pair_kernel_of<T, kActRelu>(form);
+    case kActGelu: return pair_kernel_of<T, kActGelu>(form);
+    case kActGeluTanh: return pair_kernel_of<T, kActGeluTanh>(form);
+    case kActSwiGlu: return reinterpret_cast<const void*>(gemm_pair_kernel<T, kActSwiGlu, kPairPlain>);
+    default: return pair_kernel_of<T, kActNone>(form);
   }
 }
 
@@ -228,10 +236,10 @@ int launch_gemm(const GemmCall& c, cudaStream_t stream) {
     mr = my;
     if (c.res != nullptr && (c.res != c.y || c.lres != c.ldy))
       if (int rc = matrix_map(&mr, c.res, c.dtype, c.m, c.n, c.lres, 32, "res")) return rc;
-    const bool full = c.scale != nullptr || c.res != nullptr;
-    const void* kernel = f16 ? pair_kernel<__half>(c.act, full) : pair_kernel<__nv_bfloat16>(c.act, full);
+    const int form = c.scale != nullptr ? kPairScaled : c.res != nullptr ? kPairResidual : kPairPlain;
+    const void* kernel = f16 ? pair_kernel<__half>(c.act, form) : pair_kernel<__nv_bfloat16>(c.act, form);
     const int smem = static_cast<int>(sizeof(PairSmem)) + 1024;
-    if (int rc = opt_in(*dev, (pair_act_index(c.act) * 2 + (full ? 1 : 0)) * 2 + (f16 ? 0 : 1), kernel, smem)) return rc;
+    if (int rc = opt_in(*dev, (pair_act_index(c.act) * 3 + form) * 2 + (f16 ? 0 : 1), kernel, smem)) return rc;
     void* args[] = {&mx, &mw, &mwt, &my, &mr, &prm};
     return launch_kernel(kernel, static_cast<unsigned>(2 * std::min<long long>(items, dev->sms / 2)), 1, kPairThreads, smem, 2, stream, args, "gemm kernel launch");
   }

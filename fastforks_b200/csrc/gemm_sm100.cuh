@@ -69,37 +69,76 @@ __device__ __forceinline__ uint32_t gemm_pack2(float lo, float hi) {
   }
 }
 
+// Two values at a time: the packed forms move as many values per clock as the plain ones in half the instructions, and two
+// epilogue warps per SM sub-partition are bound by instructions. us, plain -> packed: [4096,3072,768] with erf GELU 24.8 -> 23.5,
+// with its tanh form 20.8 -> 19.9, [5480,4096,1024] with that 39.4 -> 38.0.
+__device__ __forceinline__ float2 gemm_fma2(float2 a, float2 b, float2 c) {
+  uint64_t ra, rb, rc, rd;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(ra) : "f"(a.x), "f"(a.y));
+  asm("mov.b64 %0, {%1, %2};" : "=l"(rb) : "f"(b.x), "f"(b.y));
+  asm("mov.b64 %0, {%1, %2};" : "=l"(rc) : "f"(c.x), "f"(c.y));
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(rd) : "l"(ra), "l"(rb), "l"(rc));
+  float2 d;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(d.x), "=f"(d.y) : "l"(rd));
+  return d;
+}
+__device__ __forceinline__ float2 gemm_mul2(float2 a, float2 b) {
+  uint64_t ra, rb, rd;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(ra) : "f"(a.x), "f"(a.y));
+  asm("mov.b64 %0, {%1, %2};" : "=l"(rb) : "f"(b.x), "f"(b.y));
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(rd) : "l"(ra), "l"(rb));
+  float2 d;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(d.x), "=f"(d.y) : "l"(rd));
+  return d;
+}
+__device__ __forceinline__ float2 gemm_add2(float2 a, float2 b) {
+  uint64_t ra, rb, rd;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(ra) : "f"(a.x), "f"(a.y));
+  asm("mov.b64 %0, {%1, %2};" : "=l"(rb) : "f"(b.x), "f"(b.y));
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(rd) : "l"(ra), "l"(rb));
+  float2 d;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(d.x), "=f"(d.y) : "l"(rd));
+  return d;
+}
+
 // v Phi(v) with Phi the normal distribution, as max(v, 0) - |v| Phi(-|v|): no cancellation on the negative side, where
 // 0.5 v (1 + erf) loses digits. Phi(-x) = exp(-x^2 / 2) t P(t), t = 1 / (1 + 0.3 x), where P is a degree-7 least-maximum
 // fit of 0.5 erfcx(x / sqrt 2) / t on 0 <= x <= 13.5 (relative error 1.3e-7; the whole within 2e-6 of v Phi(v) down to
 // v = -5, where erff gave 1e-3). Two MUFU operations and a dozen multiply-adds: a third of the time of erff, which took
 // longer than the products of a 256 x 256 tile at k = 768. max(v, 0) is written v / 2 + |v| / 2, which keeps NaN and gives
 // it for -inf as v Phi(v) does; the tail's argument ends where the tail is zero, so that +inf meets no inf * 0.
-__device__ __forceinline__ float gelu_erf(float v) {
-  const float a = fabsf(v), x = fminf(a, 64.f);
-  float t, e;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(t) : "f"(fmaf(x, 0.3f, 1.f)));
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(x * x * -0.72134752f));
-  float p = 0.0359317549f;
-  p = fmaf(p, t, -0.158276081f);
-  p = fmaf(p, t, 0.208206728f);
-  p = fmaf(p, t, -0.0553939454f);
-  p = fmaf(p, t, 0.129469246f);
-  p = fmaf(p, t, 0.0996374786f);
-  p = fmaf(p, t, 0.120798357f);
-  p = fmaf(p, t, 0.119626388f);
-  return fmaf(0.5f, v, 0.5f * a) - x * (t * p) * e;
+__device__ __forceinline__ float2 gelu_erf2(float2 v) {
+  const auto both = [](float c) { return make_float2(c, c); };
+  const float2 a = make_float2(fabsf(v.x), fabsf(v.y)), x = make_float2(fminf(a.x, 64.f), fminf(a.y, 64.f));
+  const float2 s = gemm_fma2(x, both(0.3f), both(1.f)), g = gemm_mul2(gemm_mul2(x, x), both(-0.72134752f));
+  float2 t, e;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(t.x) : "f"(s.x));
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(t.y) : "f"(s.y));
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e.x) : "f"(g.x));
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e.y) : "f"(g.y));
+  float2 p = both(0.0359317549f);
+  p = gemm_fma2(p, t, both(-0.158276081f));
+  p = gemm_fma2(p, t, both(0.208206728f));
+  p = gemm_fma2(p, t, both(-0.0553939454f));
+  p = gemm_fma2(p, t, both(0.129469246f));
+  p = gemm_fma2(p, t, both(0.0996374786f));
+  p = gemm_fma2(p, t, both(0.120798357f));
+  p = gemm_fma2(p, t, both(0.119626388f));
+  const float2 tail = gemm_mul2(make_float2(-x.x, -x.y), gemm_mul2(t, p));
+  return gemm_fma2(tail, e, gemm_fma2(both(0.5f), v, gemm_mul2(both(0.5f), a)));
 }
 
 template <int ACT>
-__device__ __forceinline__ float gemm_act(float v) {
-  if constexpr (ACT == kActRelu) return fmaxf(v, 0.f);
-  if constexpr (ACT == kActGelu) return gelu_erf(v);
+__device__ __forceinline__ float2 gemm_act2(float2 v) {
+  if constexpr (ACT == kActRelu) return make_float2(fmaxf(v.x, 0.f), fmaxf(v.y, 0.f));
+  if constexpr (ACT == kActGelu) return gelu_erf2(v);
   if constexpr (ACT == kActGeluTanh) {
-    float t;
-    const float u = 0.7978845608028654f * v * (1.f + 0.044715f * v * v);
-    asm("tanh.approx.f32 %0, %1;" : "=f"(t) : "f"(u));
-    return 0.5f * v * (1.f + t);
+    const auto both = [](float c) { return make_float2(c, c); };
+    const float2 u = gemm_mul2(gemm_mul2(both(0.7978845608028654f), v), gemm_fma2(gemm_mul2(both(0.044715f), v), v, both(1.f)));
+    float2 t;
+    asm("tanh.approx.f32 %0, %1;" : "=f"(t.x) : "f"(u.x));
+    asm("tanh.approx.f32 %0, %1;" : "=f"(t.y) : "f"(u.y));
+    return gemm_mul2(gemm_mul2(both(0.5f), v), gemm_add2(both(1.f), t));
   }
   return v;
 }
@@ -162,9 +201,12 @@ __device__ __forceinline__ GemmItem item_at(const GemmParams& p, int item, int o
   return t;
 }
 
-// Bounded by the L2 -> SM operand traffic and, above about 1.4 PFLOP/s sustained, the power cap. ACT and FULL (there is a
-// scale or a residual) are template parameters: decided at run time, the branches alone cost 400 clocks per piece.
-template <typename T, int ACT, bool FULL>
+// Bounded by the L2 -> SM operand traffic and, above about 1.4 PFLOP/s sustained, the power cap. ACT and FORM are template
+// parameters: decided at run time, the branches alone cost 400 clocks per piece.
+// A residual without a scale (ViT-B, SAM) has a form of its own: two shuffles less per pair of columns, [4096,768,768] 9.3 -> 9.0 us,
+// [4096,768,3072] 20.8 -> 20.3.
+enum : int { kPairPlain = 0, kPairResidual = 1, kPairScaled = 2 };  // ... ; a residual; a scale, and a residual or none
+template <typename T, int ACT, int FORM>
 __global__ void __launch_bounds__(kPairThreads, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_w,
                  const __grid_constant__ CUtensorMap tm_w_tail, const __grid_constant__ CUtensorMap tm_y,
@@ -173,7 +215,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant
   PairSmem& sm = *reinterpret_cast<PairSmem*>(smem_align_1024(smem_raw));
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rank = static_cast<int>(cluster_cta_rank());  // 0: the leader, rows 0..127 of the tile
-  constexpr bool swiglu = ACT == kActSwiGlu;
+  constexpr bool swiglu = ACT == kActSwiGlu, FULL = FORM != kPairPlain;
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < kPairMaxStages; ++i) {
@@ -418,14 +460,13 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant
                   x[2 * i] = gemm_swiglu(v[at_v] + b.x, u[at_v] + bu.x);
                   x[2 * i + 1] = gemm_swiglu(v[at_v + 1] + b.y, u[at_v + 1] + bu.y);
                 } else {
-                  const float2 r = gemm_unpack2<T>(rw[i]);
-                  float2 y = make_float2(v[at_v] + b.x, v[at_v + 1] + b.y);
-                  if constexpr (FULL) {
-                    y.x = fmaf(y.x, __shfl_sync(0xffffffffu, piece_scale.x, pair), r.x);
-                    y.y = fmaf(y.y, __shfl_sync(0xffffffffu, piece_scale.y, pair), r.y);
-                  }
-                  x[2 * i] = gemm_act<ACT>(y.x);
-                  x[2 * i + 1] = gemm_act<ACT>(y.y);
+                  float2 y = gemm_add2(make_float2(v[at_v], v[at_v + 1]), b);
+                  if constexpr (FORM == kPairResidual) y = gemm_add2(y, gemm_unpack2<T>(rw[i]));
+                  if constexpr (FORM == kPairScaled)
+                    y = gemm_fma2(y, make_float2(__shfl_sync(0xffffffffu, piece_scale.x, pair), __shfl_sync(0xffffffffu, piece_scale.y, pair)), gemm_unpack2<T>(rw[i]));
+                  y = gemm_act2<ACT>(y);
+                  x[2 * i] = y.x;
+                  x[2 * i + 1] = y.y;
                 }
               }
               st_shared_v4(spot, make_uint4(gemm_pack2<T>(x[0], x[1]), gemm_pack2<T>(x[2], x[3]), gemm_pack2<T>(x[4], x[5]), gemm_pack2<T>(x[6], x[7])));
@@ -648,13 +689,11 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
           x.x += o.x; x.y += o.y; x.z += o.z; x.w += o.w;
         }
         const float2 r0 = gemm_unpack2<T>(res[i].x), r1 = gemm_unpack2<T>(res[i].y);
-        x.x = fmaf(x.x + b0.x, scale.x, r0.x);
-        x.y = fmaf(x.y + b0.y, scale.y, r0.y);
-        x.z = fmaf(x.z + b1.x, scale.z, r1.x);
-        x.w = fmaf(x.w + b1.y, scale.w, r1.y);
+        const float2 y0 = gemm_act2<kAct>(gemm_fma2(gemm_add2(make_float2(x.x, x.y), b0), make_float2(scale.x, scale.y), r0));
+        const float2 y1 = gemm_act2<kAct>(gemm_fma2(gemm_add2(make_float2(x.z, x.w), b1), make_float2(scale.z, scale.w), r1));
         if (col_in && row0 + 8 * i < row_end)
           *reinterpret_cast<uint2*>(static_cast<T*>(p.y) + static_cast<int64_t>(row0 + 8 * i) * p.ldy + col) =
-              make_uint2(gemm_pack2<T>(gemm_act<kAct>(x.x), gemm_act<kAct>(x.y)), gemm_pack2<T>(gemm_act<kAct>(x.z), gemm_act<kAct>(x.w)));
+              make_uint2(gemm_pack2<T>(y0.x, y0.y), gemm_pack2<T>(y1.x, y1.y));
       }
     });
   }

@@ -94,6 +94,17 @@ def test_layerscale_and_in_place_residual(m: int, n: int, k: int, dtype: str) ->
     check(other, x, w, None, None, before, act=ff.ACT_RELU, what="no bias + residual + relu")
 
 
+@pytest.mark.parametrize(("m", "n", "k"), [(129, 72, 72), (2740, 776, 264), (9500, 2056, 72)])  # the split kernel and two pair tiles, ragged
+@pytest.mark.parametrize("act", [0, ff.ACT_RELU, ff.ACT_GELU, ff.ACT_GELU_TANH])
+@pytest.mark.parametrize("scaled", [False, True])
+def test_residual_and_scale_each_alone(scaled: bool, act: int, m: int, n: int, k: int) -> None:
+    """A residual without a scale and a scale without a residual, with every activation (each a form of the pair kernel's epilogue)."""
+    x, w, bias, scale, res = (t.cuda() for t in operands(m, n, k, torch.float16, seed=m + act))
+    extra = {"scale": scale} if scaled else {"res": res}
+    out = torch.full((m, n), float("nan"), dtype=torch.float16, device="cuda")
+    check(ff.gemm(x, w, bias, act=act, out=out, **extra), x, w, bias, act=act, what=f"[{m},{n},{k}] act {act}", **extra)
+
+
 # One shape for every way a product is cut: the split kernel whole and with 2, 3, 4, 6 and 8 CTAs per cluster (uneven k
 # shares, rows that do not divide, a last tile of one row), pair tiles of 64 to 256 columns, and a last round in parts.
 PLANS = [(100, 72, 8), (197, 2304, 776), (257, 1024, 1544), (129, 776, 1000), (60, 64, 3080), (255, 384, 1536), (1, 8, 4096), (1000, 3000, 72),
