@@ -12,7 +12,9 @@
 //   * two softmax warpgroups, one per query tile, own one row of S per thread: they read the row
 //     from tensor memory, keep the running maximum and sum, and write P back as 16-bit values.
 //     The exponential section is passed between the two warpgroups like a token ("ping-pong"), so
-//     one warpgroup saturates the MUFU unit while the other loads, reduces and stores.
+//     one warpgroup saturates the MUFU unit while the other loads, reduces and stores;
+//   * in the forms that have registers left for it (RolesOf) a third warpgroup divides by the row sums and stages the
+//     output tiles, in the others the softmax warps do, inside the next item's first step.
 // The running maximum is only raised when it grows by more than 2^8, so rescaling O (a tensor-memory
 // round trip) is rare; the final division by the row sum happens once in the epilogue.
 //
@@ -34,16 +36,28 @@ namespace b200 {
 constexpr int kTileRows = 128;                        // query rows per tile == keys per tile
 constexpr int kHeadDim = 64;                          // the only head dim of this path
 constexpr int kTileBytes = kTileRows * kHeadDim * 2;  // one Q / K / V tile in shared memory
-constexpr int kLoaderWarp = 8;
-constexpr int kMmaWarp = 9;                           // warps 9 and 10 issue the MMAs of query tile 0 and 1
-constexpr int kStoreWarp = 11;                        // issues the TMA stores of the output tiles
-constexpr int kThreads = 384;                         // 2 softmax warpgroups + 1 warpgroup of helpers
-constexpr int kSoftmaxRegs = 224, kHelperRegs = 56;   // per-thread register budgets after the hand-over
-constexpr int kLaunchRegs = 168;                      // what a 384-thread CTA gets per thread at launch
-// setmaxnreg.inc blocks until the CTA's pool holds the registers: the budgets must fit what the launch
-// allocated, or the second warpgroup waits for ever.
-static_assert(2 * 128 * kSoftmaxRegs + 128 * kHelperRegs <= kLaunchRegs * kThreads,
-              "register hand-over does not balance");
+constexpr int kEpilogueWarp = 8;
+// The warps of a CTA: two softmax warpgroups (one per query tile), in some forms a warpgroup that writes the output tiles, and one
+// of helpers: loader, the issuers of query tile 0's and 1's products, store warp.
+// EPILOGUE: an item's output is worked on beside the next item's first step instead of inside it, where it cost the softmax
+// warps some 800 of the about 1400 clocks that a change of item takes. us, inside -> beside: [100,12,196] with 14 x 14 tables 56.4 ->
+// 50.1, [25,12,196] with them 17.6 -> 16.6, without 14.2 -> 13.8, [256,12,197] 85.7 -> 83.9, [8,16,577] 27.5 -> 27.1, [8,6,1370]
+// 39.3 -> 39.1. The forms whose softmax or loader warps need the registers do without: key split [1,12,4096] 76.0 against 79.2,
+// decomposed bias as a product [4,12,1024] 37.1 against 48.6; and dense tiles lose more than they gain ([8,192,49] 25.3 against
+// 26.9, [8,16,577] 35.8 against 35.6).
+template <bool EPILOGUE>
+struct RolesOf {
+  static constexpr int kLoaderWarp = EPILOGUE ? 12 : 8;
+  static constexpr int kMmaWarp = kLoaderWarp + 1;    // and the next one
+  static constexpr int kStoreWarp = kLoaderWarp + 3;  // issues the TMA stores of the output tiles
+  static constexpr int kThreads = 32 * (kLoaderWarp + 4);
+  // per-thread register budgets after the hand-over, and what the launch gives every thread
+  static constexpr int kSoftmaxRegs = EPILOGUE ? 192 : 224, kEpilogueRegs = EPILOGUE ? 80 : 0, kHelperRegs = EPILOGUE ? 48 : 56;
+  static constexpr int kLaunchRegs = EPILOGUE ? 128 : 168;
+  // setmaxnreg.inc blocks until the CTA's pool holds the registers: the budgets must fit what the launch
+  // allocated, or the second warpgroup waits for ever.
+  static_assert(2 * 128 * kSoftmaxRegs + 128 * (kEpilogueRegs + kHelperRegs) <= kLaunchRegs * kThreads, "register hand-over does not balance");
+};
 constexpr int kStages = 3;       // K / V ring stages (the dense-tile bias form gives one of each to its bias tiles)
 constexpr int kStagesDense = 2;
 constexpr uint32_t kTmemCols = 512;                   // S0 S1 (128 each), O0 O1 (64 each), P0 P1 (64 each)
@@ -183,9 +197,10 @@ struct alignas(1024) AttnSmemT {
   uint64_t s_free[2];   // S_t(j) has been read into registers             (4 softmax warps)
   uint64_t p_full[2];   // P_t(j) is in tensor memory, O_t rescaled        (4 softmax warps)
   uint64_t pv_done[2];  // O_t += P_t(j) V(j) has finished                 (MMA commit)
-  uint64_t o_free[2];   // the item's O_t has been read by its epilogue     (4 softmax warps)
+  uint64_t l_full[2];   // EPILOGUE: the row sums of the item are in o_stage[t]  (4 softmax warps)
+  uint64_t o_free[2];   // the item's O_t has been read by its epilogue     (4 softmax or epilogue warps)
   uint64_t turn[2];     // the other warpgroup has released t from inside its exponentials: t may start (4 warps; barrier form of the token)
-  uint64_t o_staged[2];      // the item's output tile t is in o_stage[t]           (4 softmax warps)
+  uint64_t o_staged[2];      // the item's output tile t is in o_stage[t]           (4 softmax or epilogue warps)
   uint64_t o_stage_free[2];  // the TMA store of that tile has read o_stage[t]       (store thread)
   uint64_t drain[2];         // abort path only: the MMAs query tile t's thread had in flight have finished (MMA commit)
   uint64_t merge_go[2];      // the owner's first thread has looked at the item's counter and set `merge_ready` (1)
@@ -263,10 +278,18 @@ __device__ __forceinline__ float2 fadd2(float2 a, float2 b) {
   return d;
 }
 
-// One arrival for the whole warp, after all its lanes have reached this point.
+// One arrival for the whole warp, after all its lanes have reached this point. Predicated: a branch costs some 70 clocks.
 __device__ __forceinline__ void warp_arrive(uint64_t* bar, int lane) {
   __syncwarp();
-  if (lane == 0) mbar_arrive(bar);
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p;\n\t"
+      "setp.eq.s32 p, %1, 0;\n\t"
+      "@p mbarrier.arrive.shared::cta.b64 _, [%0];\n\t"
+      "}\n"
+      :
+      : "r"(smem_u32(bar)), "r"(lane)
+      : "memory");
 }
 
 // The same, pinned in the instruction stream: `dep` is routed through the instruction, so every later
@@ -641,12 +664,17 @@ __device__ __forceinline__ void merge_parts_to_output(float* ws_partial, T* out_
 // Persistent kernel: every CTA works through its own list of items (cta_work). All barrier phases and ring
 // positions are running counters, so the loader prefetches the next item's Q / K / V while the current one is
 // still being computed and tensor memory and barriers are set up once per CTA.
+template <int BIAS, int LISTS>
+using Roles = RolesOf<(BIAS == kBiasNone || BIAS == kBiasDecomposed14) && LISTS != kListSplit>;
 template <typename T, int BIAS, bool SHORT, int LISTS>
-__global__ void __launch_bounds__(kThreads, 1)
+__global__ void __launch_bounds__(Roles<BIAS, LISTS>::kThreads, 1)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                 const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_o,
                 const __grid_constant__ CUtensorMap tm_bias, const AttnParams p) {
   constexpr bool SPLIT = LISTS == kListSplit, TWINS = LISTS == kListTwins;
+  using R = Roles<BIAS, LISTS>;
+  constexpr bool EPILOGUE = R::kEpilogueRegs > 0;
+  constexpr int kLoaderWarp = R::kLoaderWarp, kMmaWarp = R::kMmaWarp, kStoreWarp = R::kStoreWarp, kThreads = R::kThreads;
   extern __shared__ uint8_t smem_raw[];
   using Smem = AttnSmemOf<BIAS>;
   constexpr int kStagesK = Smem::kRing, kStagesV = Smem::kRing, kQBufs = Smem::kQBufs;
@@ -674,7 +702,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       uint64_t* bar = first + i;
       const bool four = (bar >= &sm.bias_free[0] && bar <= &sm.bias_free[1]) || (bar >= &sm.r_full[0] && bar <= &sm.r_full[1]) ||
                         (bar >= &sm.s_free[0] && bar <= &sm.s_free[1]) ||
-                        (bar >= &sm.p_full[0] && bar <= &sm.p_full[1]) || (bar >= &sm.o_free[0] && bar <= &sm.o_staged[1]);
+                        (bar >= &sm.p_full[0] && bar <= &sm.p_full[1]) || (bar >= &sm.l_full[0] && bar <= &sm.l_full[1]) || (bar >= &sm.o_free[0] && bar <= &sm.o_staged[1]);
       // with kBiasDecomposedMma a K tile is there when its TMA transaction and its E are
       const bool two = (BIAS == kBiasDecomposedMma && bar >= &sm.k_full[0] && bar <= &sm.k_full[kStagesK - 1]) || (bar >= &sm.k_empty[0] && bar <= &sm.k_empty[kStagesK - 1]) ||
                        (bar >= &sm.v_empty[0] && bar <= &sm.v_empty[kStagesV - 1]) ;
@@ -717,7 +745,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   const int my_items = cw.pairs + cw.singles;
 
   if (warp >= kLoaderWarp) {
-    reg_dealloc<kHelperRegs>();
+    reg_dealloc<R::kHelperRegs>();
     if (warp == kLoaderWarp) {
       // ======================= loader =======================================================
       if constexpr (BIAS == kBiasDecomposedMma) {
@@ -1178,9 +1206,56 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         __syncwarp();
       }
     }
+  } else if (EPILOGUE && warp >= kEpilogueWarp) {
+    // ======================= epilogue warps ====================================================
+    // O_t / l -> staging buffer -> (store thread) global, tile after tile, each warp 32 rows; frees O_t for the next item's first P V.
+    reg_dealloc<EPILOGUE ? R::kEpilogueRegs : R::kHelperRegs>();
+    const int quarter = warp & 3;
+    const uint32_t lane_addr = static_cast<uint32_t>(quarter * 32) << 16;
+    int steps[2] = {0, 0};  // key-tile steps of either slot up to and with the item
+    bool ok = true;
+    for (int it = 0; it < my_items && ok; ++it) {
+      const int n_tiles = it < cw.pairs ? 2 : 1;
+      for (int t = 0; t < n_tiles && ok; ++t) {
+        steps[t] += kv_tiles;
+        // The row sums come after the item's last P, so that only the last phase of pv_done can be pending then.
+        ok = __all_sync(0xffffffffu, mbar_wait(&sm.l_full[t], it & 1, abort_flag) && mbar_wait(&sm.pv_done[t], (steps[t] - 1) & 1, abort_flag)) != 0;
+        if (!ok) break;
+        tc_fence_after_sync();
+        const uint32_t stage = smem_u32(sm.o_stage[t]) + quarter * (32 * kHeadDim * 2);
+        const float inv = 1.f / ld_shared_f32(stage + lane * 4);
+        __syncwarp();  // all sums are read before a row of the tile is written over them
+        const float2 inv2 = make_float2(inv, inv), zero2 = make_float2(0.f, 0.f);
+#pragma unroll 1
+        for (int half = 0; half < 2; ++half) {
+          float o[kHeadDim / 2];
+          tmem_ld_x32(tmem + lane_addr + kTmemO + t * kHeadDim + half * (kHeadDim / 2), reinterpret_cast<uint32_t*>(o));
+          if (half == 1) {
+            tc_fence_before_sync();
+            warp_arrive(&sm.o_free[t], lane);
+          }
+#pragma unroll
+          for (int ch = 0; ch < kHeadDim / 16; ++ch) {
+            uint32_t val[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              const float2 x = ffma2(make_float2(o[ch * 8 + 2 * e], o[ch * 8 + 2 * e + 1]), inv2, zero2);  // rounds like x * inv
+              val[e] = pack2<T>(x.x, x.y);
+            }
+            st_shared_v4(stage + lane * (kHeadDim * 2) + (((half * 4 + ch) ^ (lane & 7)) << 4), make_uint4(val[0], val[1], val[2], val[3]));
+          }
+        }
+        fence_proxy_async_smem();  // the TMA store reads what these generic-proxy stores wrote
+        warp_arrive(&sm.o_staged[t], lane);
+      }
+    }
+    if (!ok && lane == 0) {
+      if (atomicExch(const_cast<uint32_t*>(abort_flag), 1u) == 0) atomicOr(p.status, kStatusSoftmax);
+    }
+    __syncwarp();
   } else {
     // ======================= softmax warpgroups ================================================
-    reg_alloc<kSoftmaxRegs>();
+    reg_alloc<R::kSoftmaxRegs>();
     const int t = warp >> 2;  // query-tile slot of this warpgroup
     const int row_in_tile = (warp & 3) * 32 + lane;
     const uint32_t lane_addr = static_cast<uint32_t>((warp & 3) * 32) << 16;
@@ -1199,7 +1274,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     float pend_l = 0.f;
     float pend_m_of_split = 0.f;  // key-split form only: the pending item's reference maximum
     int pend_it = 0;
-    // O_t / l -> staging buffer -> (store thread) global for the pending item; frees O_t for the next item's first P V.
+    // (Without epilogue warps.) O_t / l -> staging buffer -> (store thread) global for the pending item; frees O_t for the next item's first P V.
     // Each thread writes its 128-byte row as eight 16-byte chunks at the positions of the 128-byte swizzle.
     // `pv_tested`, `stage_tested`: results of early tests of the two barriers (false = not tested or still pending).
     // A part of an item that is cut along the keys (key-split mode) either folds the other parts into its O_t and
@@ -1448,8 +1523,16 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         float s[kTileRows];
         {
           uint32_t* su = reinterpret_cast<uint32_t*>(s);
-          // One 128-column load (a quarter of the tcgen05 instructions of four 32-column ones: -2 %).
-          tmem_ld_x128(s_addr, su);
+          // One 128-column load (a quarter of the instructions of four 32-column ones: -2 %), or, where the launch allows too few
+          // registers for it, a short, a long and a short one, each waited for: us [8,6,1370] 39.1, two of 64 columns
+          // with one wait 39.5, with two 39.4.
+          if constexpr (EPILOGUE) {
+            tmem_ld_x32(s_addr, su);
+            tmem_ld_1x64(s_addr + 32, su + 32);
+            tmem_ld_x32(s_addr + 96, su + 96);
+          } else {
+            tmem_ld_x128(s_addr, su);
+          }
         }
         // S_t is in registers: the tensor pipe may overwrite it with the tile after next.
         tc_fence_before_sync();
@@ -1670,8 +1753,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         // would leave the unit idle together, and equal loops sharing a unit drift into lockstep). So each
         // may only start a section once the other has released it from inside its previous one: warpgroup 0
         // starts step q+1 after warpgroup 1's release in step q, warpgroup 1 starts step q after warpgroup 0's
-        // release in step q. The release comes after 64 of the 128 columns in the long schedule ([32,24,1370] us: 16
-        // columns 556, 32 520, 64 510, 96 517, 128 558, no token 562), after 96 in the short one.
+        // release in step q. The release comes after 96 of the 128 columns ([8,16,577] us: 32 columns 28.0, 64 27.9, 96 27.1,
+        // 128 28.4, no token 28.7).
         if (need_turn) {
           if constexpr (kFlagTurn) {
             const volatile uint32_t* released = &sm.turn_count[t ^ 1][warp & 3];
@@ -1711,11 +1794,15 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
               warp_arrive_pinned(&sm.turn[t ^ 1], lane, nm);
             }
           }
-          // On an item's first tile the P V in question is the last one of the pending item (same barrier, and
-          // (step - 1) & 1 is that item's last phase), waited for by its epilogue together with the staging buffer.
-          pv_early = (rj > 0 || pend) ? mbar_test_wait(&sm.pv_done[t], (step - 1) & 1) : true;
-          stage_early = (rj == 0 && pend && pend_it > 0) ? mbar_test_wait(&sm.o_stage_free[t], (pend_it - 1) & 1) : false;
-          s_early = mbar_test_wait(&sm.s_full[t], (step + 1) & 1);  // the next step's S (unused after the last step)
+          // On an item's first tile the P V in question is the last one of the item before (same barrier, and
+          // (step - 1) & 1 is that item's last phase); without epilogue warps its epilogue waits for it, together with the
+          // staging buffer.
+          pv_early = step > 0 ? mbar_test_wait(&sm.pv_done[t], (step - 1) & 1) : true;
+          if constexpr (EPILOGUE) {
+            if (j == jb - 1) stage_early = it == 0 || mbar_test_wait(&sm.o_stage_free[t], (it - 1) & 1);
+          } else {
+            stage_early = (rj == 0 && pend && pend_it > 0) ? mbar_test_wait(&sm.o_stage_free[t], (pend_it - 1) & 1) : false;
+          }
         };
         // Exponentials of 32 * CHUNKS columns from column 32 * FIRST on.
         auto exp_columns = [&](auto first, auto chunks) {
@@ -1736,14 +1823,14 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           }
         };
         using std::integral_constant;
-        exp_columns(integral_constant<int, 0>{}, integral_constant<int, 2>{});
+        constexpr int kRelease = BIAS == kBiasDecomposed64 ? 2 : 3;  // columns before the release, in 32s (that form's sections are halves)
+        exp_columns(integral_constant<int, 0>{}, integral_constant<int, kRelease>{});
         if constexpr (SHORT) {
           // Short-sequence schedule. The last 32 columns of a ragged last key tile that hold no key at all (197 keys:
           // 69 in the second tile) need no exponentials: their logits are -inf and their P is never read (P V stops
           // at the last key's k-step). One CTA-uniform branch: -6 % on [256,12,197,64]. With eleven key tiles
           // the branch is taken once in eleven steps and its effect on the step's schedule costs more than it
           // saves (+4 % on [32,24,1370,64] bf16), hence a schedule of its own.
-          exp_columns(integral_constant<int, 2>{}, integral_constant<int, 1>{});
           release_point();
           if (kv_valid > 96) {
             exp_columns(integral_constant<int, 3>{}, integral_constant<int, 1>{});
@@ -1753,37 +1840,41 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           }
         } else {
           release_point();
-          exp_columns(integral_constant<int, 2>{}, integral_constant<int, 2>{});
+          exp_columns(integral_constant<int, kRelease>{}, integral_constant<int, 4 - kRelease>{});
         }
         l_sum += (l2a.x + l2a.y) + (l2b.x + l2b.y);
 
         // P_t and O_t may only change once P_t(j-1) V has finished: it was issued when this warpgroup
         // delivered P_t(j-1), a whole exponential section ago. On the first tile of an item the P V in
-        // question is the last one of the previous item, and this is where that item's output is written:
+        // question is the last one of the previous item; without epilogue warps this is where that item's output is written:
         // its epilogue hides behind this item's first exponentials instead of stalling the pipeline.
-        if (__builtin_expect(rj == 0, 0)) {
+        if (!EPILOGUE && __builtin_expect(rj == 0, 0)) {
           if (pend) {
             ok = finish_item(pv_early, stage_early, std::false_type{});
             if (!ok) break;
           }
-        } else {
+        } else if (__builtin_expect(__any_sync(0xffffffffu, (raise && rj > 0) || bad || !pv_early), 0)) {
+          // One vote for all that is rare: a wait on the path every step takes costs some 100 clocks even on a completed phase.
           bad |= !mbar_wait_warp_after(pv_early, &sm.pv_done[t], (step - 1) & 1, abort_flag);
-          tc_fence_after_sync();
-          if (__builtin_expect(__any_sync(0xffffffffu, raise || bad), 0)) {
-            if (__any_sync(0xffffffffu, bad)) {  // some lane's wait ran out (voted on together with the rescale, which is as rare)
-              ok = false;
-              break;
-            }
-            float o[kHeadDim];
-            uint32_t* ou = reinterpret_cast<uint32_t*>(o);
-            tmem_ld_x64(o_addr, ou);
+          if (__any_sync(0xffffffffu, bad)) {
+            ok = false;
+            break;
+          }
+          if (rj > 0 && __any_sync(0xffffffffu, raise)) {
+            tc_fence_after_sync();
+#pragma unroll 1
+            for (int c0 = 0; c0 < kHeadDim; c0 += 16) {  // in pieces: the P values stay in registers meanwhile
+              float o[16];
+              tmem_ld_x16(o_addr + c0, reinterpret_cast<uint32_t*>(o));
 #pragma unroll
-            for (int i = 0; i < kHeadDim; ++i) o[i] *= alpha;
-            tmem_st_x32(o_addr, ou);
-            tmem_st_x32(o_addr + 32, ou + 32);
+              for (int i = 0; i < 16; ++i) o[i] *= alpha;
+              tmem_st_x16(o_addr + c0, reinterpret_cast<uint32_t*>(o));
+            }
           }
         }
+        tc_fence_after_sync();
         tmem_st_x64(p_addr, pk);
+        s_early = mbar_test_wait(&sm.s_full[t], (step + 1) & 1);  // the next step's S (unused after the last step)
         tmem_st_wait();
         tc_fence_before_sync();
         warp_arrive(&sm.p_full[t], lane);
@@ -1794,16 +1885,27 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         break;
       }
 
-      // The item's output is written later (see above); remember what its epilogue needs.
-      pend = true;
-      pend_phase = (g + (jb - ja) - 1) & 1;
-      pend_l = l_sum;
-      if constexpr (SPLIT) pend_m_of_split = m_ref;
-      pend_it = it;
+      if constexpr (EPILOGUE) {
+        // The row sums go to the epilogue in the staging area, each warp's in front of the rows it belongs to: the last item's
+        // output has to be out of it.
+        if (!__all_sync(0xffffffffu, stage_early || mbar_wait(&sm.o_stage_free[t], (it - 1) & 1, abort_flag))) {
+          ok = false;
+          break;
+        }
+        st_shared_f32(smem_u32(sm.o_stage[t]) + (warp & 3) * (32 * kHeadDim * 2) + lane * 4, l_sum);
+        warp_arrive(&sm.l_full[t], lane);
+      } else {
+        // The item's output is written later (see above); remember what its epilogue needs.
+        pend = true;
+        pend_phase = (g + (jb - ja) - 1) & 1;
+        pend_l = l_sum;
+        if constexpr (SPLIT) pend_m_of_split = m_ref;
+        pend_it = it;
+      }
       g += jb - ja;
       if (w.n_tiles == 2) gp += jb - ja;
     }
-    if (ok && pend) ok = finish_item(false, false, std::true_type{});
+    if (!EPILOGUE && ok && pend) ok = finish_item(false, false, std::true_type{});
     if (!ok && lane == 0) {
       if (atomicExch(const_cast<uint32_t*>(abort_flag), 1u) == 0) atomicOr(p.status, kStatusSoftmax);
     }

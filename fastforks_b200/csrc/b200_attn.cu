@@ -495,7 +495,7 @@ int launch(const AttnParams& planned, unsigned grid, DeviceState& dev, const CUt
   // predecessor's tail.
   cudaLaunchConfig_t config = {};
   config.gridDim = dim3(grid);
-  config.blockDim = dim3(kThreads);
+  config.blockDim = dim3(Roles<BIAS, LISTS>::kThreads);
   config.dynamicSmemBytes = smem;
   config.stream = stream;
   cudaLaunchAttribute attribute[1];

@@ -368,6 +368,24 @@ def test_decomposed_bias_masks_and_other_scales() -> None:
         assert_close(got.float().cpu().numpy(), ref, unit_scale=True, what=f"scale {scale}")
 
 
+# Lists of three items and more per CTA, so that row sums, staging buffers and output tiles are handed over again and again: twins of
+# one and of four key tiles, two-tile items of one, two and three, and one-tile items behind them.
+@pytest.mark.parametrize(("b", "h", "n", "side"), [(40, 24, 60, 0), (50, 16, 97, 0), (40, 12, 250, 0), (30, 12, 384, 0), (9, 48, 390, 0), (50, 12, 196, 14)])
+@pytest.mark.parametrize("dtype", ["fp16", "bf16"])
+def test_many_items_per_cta(b: int, h: int, n: int, side: int, dtype: str) -> None:
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    q, k, v = torch.randn(b, n, 3, h, 64, generator=gen, device="cuda").to(DTYPES[dtype]).unbind(2)
+    q, k, v = (t.transpose(1, 2) for t in (q, k, v))
+    rel, bias = None, 0.0
+    if side:
+        rel = tuple(torch.randn(b, h, n, side, generator=gen, device="cuda").to(DTYPES[dtype]) for _ in range(2))
+        bias = (rel[0].float()[..., :, None] + rel[1].float()[..., None, :]).reshape(b, h, n, n)
+    ref = ((q.float() @ k.float().mT) * 0.125 + bias).softmax(-1) @ v.float()
+    got = ff.scaled_dot_product_attention(q, k, v, rel=rel, scale=0.125) if side else ff.scaled_dot_product_attention(q, k, v, scale=0.125)
+    assert ff.device_status() == 0
+    assert_close(got.float().cpu().numpy(), ref.cpu().numpy(), unit_scale=True, what=f"[{b},{h},{n}] {dtype}")
+
+
 @pytest.mark.parametrize("hw", [(20, 20), (64, 64), (9, 31), (2, 5)])
 @pytest.mark.parametrize("dtype", ["fp16", "bf16"])
 @pytest.mark.parametrize("scale", [0.125, 0.1])
