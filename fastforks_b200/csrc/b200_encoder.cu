@@ -264,7 +264,7 @@ struct Forward {
       r.rel_pos_h = k.rel_pos_h; r.rel_pos_w = k.rel_pos_w;
       r.rel_h = at(l.rel_h); r.rel_w = at(l.rel_w);
       r.batch = batch; r.heads = a->heads; r.side = side; r.head_dim = 64;
-      if (int rc = b200_sam_rel_terms(&r, stream)) return rc;
+      if (int rc = launch_rel_terms(&r, started, stream)) return rc;  // always behind a product of this forward
       t.rel_h = r.rel_h; t.rel_w = r.rel_w;
       t.rel_dtype = a->dtype;
       t.rel_kh = t.rel_kw = side;

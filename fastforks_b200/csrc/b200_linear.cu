@@ -275,9 +275,75 @@ const void* rel_kernel_of(int tiles) {
     default: return reinterpret_cast<const void*>(sam_rel_terms_kernel<T, 8>);
   }
 }
+// Sides from which the terms are computed by lines; us by lines and by tokens: side 32 [1,12] 5.1 and 3.8, [8,16] 16.4 and 14.3; side 40
+// [1,12] 5.9 and 6.6; side 48 [4,12] 16.0 and 21.5. Rows and addresses in whole 16-byte groups, heads to divide by.
+constexpr int kRelLinesSide = 40;
 const void* rel_kernel(bool f16, int tiles) { return f16 ? rel_kernel_of<__half>(tiles) : rel_kernel_of<__nv_bfloat16>(tiles); }
 
 }  // namespace
+
+int launch_rel_terms(const B200RelTermsArgs* a, bool early_tables, cudaStream_t stream) {
+  if (a == nullptr) return fail(B200_ATTN_BAD_CONFIG, "args is NULL");
+  if (a->struct_size != sizeof(B200RelTermsArgs))
+    return fail(B200_ATTN_BAD_CONFIG, "struct_size %u does not match this library's B200RelTermsArgs (%zu bytes)",
+                a->struct_size, sizeof(B200RelTermsArgs));
+  if (a->dtype != B200_ATTN_F16 && a->dtype != B200_ATTN_BF16)
+    return fail(B200_ATTN_BAD_CONFIG, "dtype %u: q, the tables and the results must be fp16 (0) or bf16 (1)", a->dtype);
+  if (a->head_dim != kHeadDim) return fail(B200_ATTN_UNSUPPORTED, "head_dim %d: only head dim 64 is built", a->head_dim);
+  if (a->batch < 1 || a->heads < 1 || a->side < 2 || a->side > kRelMaxSide || a->side % 2 != 0)
+    return fail(B200_ATTN_UNSUPPORTED, "batch %d heads %d side %d: side must be even, 2 .. %d", a->batch, a->heads, a->side, kRelMaxSide);
+  if (static_cast<int64_t>(a->batch) * a->side > 0x7fffffffLL) return fail(B200_ATTN_UNSUPPORTED, "batch too large for one launch");
+  const int tokens = a->side * a->side;
+  if (int rc = check_view("q", a->q, a->q_stride, a->batch, a->heads, tokens)) return rc;
+  const struct { const char* name; const void* ptr; int align; } ptrs[] = {
+      {"rel_pos_h", a->rel_pos_h, 4}, {"rel_pos_w", a->rel_pos_w, 4}, {"rel_h", a->rel_h, 4}, {"rel_w", a->rel_w, 4}};
+  for (const auto& x : ptrs) {
+    if (x.ptr == nullptr) return fail(B200_ATTN_BAD_CONFIG, "%s is NULL", x.name);
+    if (reinterpret_cast<uintptr_t>(x.ptr) % x.align != 0) return fail(B200_ATTN_UNSUPPORTED, "%s is not 4-byte aligned", x.name);
+  }
+  RelTermsParams prm{};
+  prm.q = a->q;
+  prm.q_sb = a->q_stride[0];
+  prm.q_sn = a->q_stride[1];
+  prm.q_sh = a->q_stride[2];
+  prm.rel_pos_h = a->rel_pos_h;
+  prm.rel_pos_w = a->rel_pos_w;
+  prm.rel_h = a->rel_h;
+  prm.rel_w = a->rel_w;
+  prm.batch = a->batch;
+  prm.heads = a->heads;
+  prm.side = a->side;
+  prm.tables_wide = aligned16(a->rel_pos_h) && aligned16(a->rel_pos_w);
+  prm.out_wide = aligned16(a->rel_h) && aligned16(a->rel_w);
+  prm.early_tables = early_tables ? 1 : 0;
+  const long long lines = 2LL * a->batch * a->side;
+  if (a->side % 8 == 0 && a->side >= kRelLinesSide && prm.tables_wide && prm.out_wide && a->heads > 1 && a->heads <= 1024 && lines <= 0x7fffffffLL) {
+    DeviceState* dev = nullptr;
+    if (int rc = device_state(&dev)) return rc;
+    prm.status = dev->status;
+    prm.magic_heads = static_cast<uint32_t>((uint64_t(1) << 32) / static_cast<uint32_t>(a->heads) + 1);  // exact for 64 * heads rows
+    const bool f16 = a->dtype == B200_ATTN_F16;
+    const void* kernel = f16 ? reinterpret_cast<const void*>(sam_rel_lines_kernel<__half>) : reinterpret_cast<const void*>(sam_rel_lines_kernel<__nv_bfloat16>);
+    if (int rc = opt_in(*dev, kLinearKernels - (f16 ? 2 : 1), kernel, rel_lines_smem(kRelLineTiles))) return rc;
+    const int smem = rel_lines_smem(std::min((a->side * a->heads + 127) / 128, kRelLineTiles));
+    void* args[] = {&prm};
+    if (int rc = launch_kernel(kernel, static_cast<unsigned>(lines), 1, kRelLineThreads, smem, 1, stream, args, "sam_rel_terms kernel launch")) return rc;
+    clear_error();
+    return B200_ATTN_OK;
+  }
+  // A token per warp.
+  const long long grid_rows = static_cast<long long>(a->batch) * a->side;
+  prm.parts = (a->side + kRelWarps - 1) / kRelWarps;
+  if (grid_rows * prm.parts > 0x7fffffffLL) return fail(B200_ATTN_UNSUPPORTED, "batch too large for one launch");
+  const void* kernel = rel_kernel(a->dtype == B200_ATTN_F16, (a->side + 7) / 8);
+  void* args[] = {&prm};
+  const size_t smem = static_cast<size_t>(2 * a->side - 1 + (a->side + prm.parts - 1) / prm.parts) * 128;
+  if (int rc = launch_kernel(kernel, static_cast<unsigned>(grid_rows * prm.parts), 1, kRelWarps * 32, smem, 1, stream, args,
+                             "sam_rel_terms kernel launch"))
+    return rc;
+  clear_error();
+  return B200_ATTN_OK;
+}
 
 }  // namespace b200
 
@@ -334,54 +400,7 @@ int b200_gemm_plan(int32_t m, int32_t n, int32_t k, int32_t sms, const int32_t* 
   return B200_ATTN_OK;
 }
 
-int b200_sam_rel_terms(const B200RelTermsArgs* a, void* stream_ptr) {
-  if (a == nullptr) return fail(B200_ATTN_BAD_CONFIG, "args is NULL");
-  if (a->struct_size != sizeof(B200RelTermsArgs))
-    return fail(B200_ATTN_BAD_CONFIG, "struct_size %u does not match this library's B200RelTermsArgs (%zu bytes)",
-                a->struct_size, sizeof(B200RelTermsArgs));
-  if (a->dtype != B200_ATTN_F16 && a->dtype != B200_ATTN_BF16)
-    return fail(B200_ATTN_BAD_CONFIG, "dtype %u: q, the tables and the results must be fp16 (0) or bf16 (1)", a->dtype);
-  if (a->head_dim != kHeadDim) return fail(B200_ATTN_UNSUPPORTED, "head_dim %d: only head dim 64 is built", a->head_dim);
-  if (a->batch < 1 || a->heads < 1 || a->side < 2 || a->side > kRelMaxSide || a->side % 2 != 0)
-    return fail(B200_ATTN_UNSUPPORTED, "batch %d heads %d side %d: side must be even, 2 .. %d", a->batch, a->heads, a->side, kRelMaxSide);
-  if (static_cast<int64_t>(a->batch) * a->side > 0x7fffffffLL) return fail(B200_ATTN_UNSUPPORTED, "batch too large for one launch");
-  const int tokens = a->side * a->side;
-  if (int rc = check_view("q", a->q, a->q_stride, a->batch, a->heads, tokens)) return rc;
-  const struct { const char* name; const void* ptr; int align; } ptrs[] = {
-      {"rel_pos_h", a->rel_pos_h, 4}, {"rel_pos_w", a->rel_pos_w, 4}, {"rel_h", a->rel_h, 4}, {"rel_w", a->rel_w, 4}};
-  for (const auto& x : ptrs) {
-    if (x.ptr == nullptr) return fail(B200_ATTN_BAD_CONFIG, "%s is NULL", x.name);
-    if (reinterpret_cast<uintptr_t>(x.ptr) % x.align != 0) return fail(B200_ATTN_UNSUPPORTED, "%s is not 4-byte aligned", x.name);
-  }
-  RelTermsParams prm{};
-  prm.q = a->q;
-  prm.q_sb = a->q_stride[0];
-  prm.q_sn = a->q_stride[1];
-  prm.q_sh = a->q_stride[2];
-  prm.rel_pos_h = a->rel_pos_h;
-  prm.rel_pos_w = a->rel_pos_w;
-  prm.rel_h = a->rel_h;
-  prm.rel_w = a->rel_w;
-  prm.batch = a->batch;
-  prm.heads = a->heads;
-  prm.side = a->side;
-  DeviceState* dev = nullptr;
-  if (int rc = device_state(&dev)) return rc;
-  prm.tables_wide = aligned16(a->rel_pos_h) && aligned16(a->rel_pos_w);
-  prm.out_wide = aligned16(a->rel_h) && aligned16(a->rel_w);
-  // One CTA per grid row, and several where there are few rows: about four CTAs per SM, a token per warp at least.
-  const long long grid_rows = static_cast<long long>(a->batch) * a->side;
-  prm.parts = static_cast<int>(std::max(1LL, std::min<long long>((4LL * dev->sms + grid_rows - 1) / grid_rows, (a->side + kRelWarps - 1) / kRelWarps)));
-  if (grid_rows * prm.parts > 0x7fffffffLL) return fail(B200_ATTN_UNSUPPORTED, "batch too large for one launch");
-  const void* kernel = rel_kernel(a->dtype == B200_ATTN_F16, (a->side + 7) / 8);
-  void* args[] = {&prm};
-  const size_t smem = static_cast<size_t>(3 * a->side - 1) * 128;
-  if (int rc = launch_kernel(kernel, static_cast<unsigned>(grid_rows * prm.parts), 1, kRelWarps * 32, smem, 1, static_cast<cudaStream_t>(stream_ptr), args,
-                             "sam_rel_terms kernel launch"))
-    return rc;
-  clear_error();
-  return B200_ATTN_OK;
-}
+int b200_sam_rel_terms(const B200RelTermsArgs* a, void* stream_ptr) { return launch_rel_terms(a, false, static_cast<cudaStream_t>(stream_ptr)); }
 
 int b200_rope_qk(const B200RopeArgs* a, void* stream_ptr) {
   if (a == nullptr) return fail(B200_ATTN_BAD_CONFIG, "args is NULL");

@@ -32,7 +32,7 @@ int check_view(const char* name, const void* ptr, const int64_t s[3], int batch,
 constexpr int kMaxDevices = 64;
 constexpr int kKernelForms = 84;      // attention: 2 dtypes x 7 bias forms x (short, long) x (plain lists, twins, key split)
 constexpr int kSmallForms = 16;      // attention of small calls: 2 dtypes x 8 key counts
-constexpr int kLinearKernels = 30;    // pair GEMM kernels of b200_linear.cu: 5 activations x 3 epilogue forms x 2 dtypes
+constexpr int kLinearKernels = 32;    // of b200_linear.cu, with an opt-in: pair GEMM (5 activations x 3 epilogue forms x 2 dtypes), SAM's terms by lines (2 dtypes)
 constexpr int kGemmSplits = 6;        // split counts of the split GEMM kernel
 struct DeviceState {
   std::atomic<bool> ready{false};

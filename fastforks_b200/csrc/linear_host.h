@@ -5,6 +5,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "../../include/b200_attn.h"
+
 namespace b200 {
 
 // One product with its epilogue (gemm_sm100.cuh). `n` counts the columns of y; a SwiGLU layer (act = kActSwiGlu) has
@@ -24,6 +26,9 @@ struct GemmCall {
   bool early_w;
 };
 int launch_gemm(const GemmCall& c, cudaStream_t stream);
+
+// b200_sam_rel_terms; early_tables: see RelTermsParams.
+int launch_rel_terms(const B200RelTermsArgs* a, bool early_tables, cudaStream_t stream);
 
 // How a product is cut: the pair kernel with tiles of 256 x bn, those behind the last whole round of the grid cut into
 // parts of 256 x tail_bn if tail_bn > 0, or, split > 0, the split kernel with 128 x 64 tiles and the k range cut in `split`.

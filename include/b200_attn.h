@@ -216,7 +216,7 @@ int b200_gemm_plan(int32_t m, int32_t n, int32_t k, int32_t sms, const int32_t* 
  * packed qkv tensor (element (b, n, head, d) at q + b*q_stride[0] + n*q_stride[1] + head*q_stride[2] + d, strides in
  * elements, multiples of 8, base 16-byte aligned), `rel_pos_h` / `rel_pos_w` are the module's parameters themselves,
  * `[2 * side - 1, 64]` contiguous, and the results are `[batch, heads, side * side, side]` contiguous, all of `dtype`.
- * `side` must be even and at most 64 (SAM: 14 for the windows, 64 for the global blocks).
+ * `side` must be even and at most 64 (SAM: 14 for the windows, 64 for the global blocks). Status bit 512: a wait of this kernel.
  */
 typedef struct B200RelTermsArgs {
   uint32_t struct_size; /* sizeof(B200RelTermsArgs) */

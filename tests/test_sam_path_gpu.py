@@ -115,6 +115,23 @@ def test_producer_kernel_at_every_tile_count(b: int, side: int, heads: int) -> N
     assert ff.device_status() == 0
 
 
+@pytest.mark.parametrize(("b", "side", "heads"), [(2, 40, 2), (1, 40, 5), (2, 48, 3), (1, 56, 12), (1, 64, 16), (1, 64, 33)])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_producer_kernel_by_lines(b: int, side: int, heads: int, dtype: torch.dtype) -> None:
+    """Aligned tables at the sides a line at a time is computed for: one tile of rows and less, ragged last tiles, more tiles than
+    tensor memory holds at once, and numbers of columns that are no multiple of the product's sixteen."""
+    from oracle import attention_oracle as ao
+
+    gen = torch.Generator().manual_seed(side + heads)
+    qkv = torch.randn(b, side * side, 3, heads, DIM, generator=gen).to(dtype).cuda()
+    pos_h, pos_w = ((torch.randn(2 * side - 1, DIM, generator=gen) * 0.1).to(dtype).cuda() for _ in range(2))
+    rel_h, rel_w = ff.sam_rel_terms(qkv[:, :, 1], pos_h, pos_w, side)
+    want_h, want_w = ao.decomposed_terms(qkv[:, :, 1].float().cpu().numpy().transpose(0, 2, 1, 3), pos_h.float().cpu().numpy(), pos_w.float().cpu().numpy(), (side, side))
+    assert ff.device_status() == 0
+    assert_close(rel_h.float().cpu().numpy(), want_h, unit_scale=False, what=f"rel_h side {side}")
+    assert_close(rel_w.float().cpu().numpy(), want_w, unit_scale=False, what=f"rel_w side {side}")
+
+
 def test_producer_kernel_rejects_what_it_cannot_take() -> None:
     q = torch.zeros(1, 25, 2, 64, dtype=torch.float16, device="cuda")
     pos = torch.zeros(9, 64, dtype=torch.float16, device="cuda")
