@@ -201,7 +201,6 @@ __global__ void __launch_bounds__(kRelLineThreads, 2) sam_rel_lines_kernel(const
   };
   if (p.early_tables) load_table();
   grid_dependency_wait();
-  grid_launch_dependents();
   if (!p.early_tables) load_table();
   bool ok = true;
   uint32_t phase = 0;
@@ -219,6 +218,9 @@ __global__ void __launch_bounds__(kRelLineThreads, 2) sam_rel_lines_kernel(const
     if (t0 == 0 && warp == 1) {  // behind the loads: another CTA of this SM may still hold the columns
       tmem_alloc(&tmem_base, tmem_cols);
       tmem_relinquish();
+      // Only now: a kernel behind this one allocates in its set-up and then waits for this grid. Started any earlier, a CTA of it could
+      // take columns this one has yet to get, and both would wait for ever.
+      grid_launch_dependents();
     }
     cp_async_wait<0>();
     fence_proxy_async_smem();  // the products read what these copies wrote

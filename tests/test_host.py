@@ -270,3 +270,19 @@ def test_a_snapshot_sees_tensors_that_were_replaced(native: bool, monkeypatch: p
     b["x"].data = b["x"].clone()
     assert snap.changed(a, b)
     assert not encoder.Snapshot(a, b).changed(a, b)
+
+
+def test_kernels_hold_their_tensor_memory_before_they_let_the_next_kernel_start() -> None:
+    """A kernel that starts early allocates tensor memory in its set-up and then waits for the grid in front of it. If that grid let it
+    start before all of its own CTAs had theirs, the two could wait for each other for ever (an allocation has no time limit)."""
+    from fastforks_b200 import _lib
+
+    checked = 0
+    for path in (*_lib.SOURCES, *_lib.HEADERS):
+        for body in path.read_text().split("__global__")[1:]:
+            if "tmem_alloc" not in body or "grid_launch_dependents();" not in body:
+                continue
+            name = body[: body.index("(", body.index("_kernel"))].split()[-1]
+            assert body.index("tmem_alloc") < body.index("grid_launch_dependents();"), f"{path.name}: {name}"
+            checked += 1
+    assert checked == 4  # attention, pair and split GEMM, SAM's terms by lines

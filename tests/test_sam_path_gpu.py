@@ -132,6 +132,27 @@ def test_producer_kernel_by_lines(b: int, side: int, heads: int, dtype: torch.dt
     assert_close(rel_w.float().cpu().numpy(), want_w, unit_scale=False, what=f"rel_w side {side}")
 
 
+@pytest.mark.parametrize(("b", "side", "heads"), [(1, 40, 2), (3, 40, 6), (2, 64, 4), (2, 64, 12), (1, 64, 33)])
+def test_producer_by_lines_with_kernels_close_behind(b: int, side: int, heads: int) -> None:
+    """Kernels that allocate tensor memory in their set-up, each started while the one in front drains: lines of one to eight tiles and
+    more, then a product cut along k, one in pairs, and attention. Every round gives what the first one gave."""
+    gen = torch.Generator(device="cuda").manual_seed(side * heads)
+    q, k, v = torch.randn(b, side * side, 3, heads, DIM, generator=gen, device="cuda").half().unbind(2)
+    pos_h, pos_w = ((torch.randn(2 * side - 1, DIM, generator=gen, device="cuda") * 0.1).half() for _ in range(2))
+    small, wide, w = (torch.randn(m, 512, generator=gen, device="cuda").half() for m in (100, 4000, 1024))
+    first = None
+    for _ in range(12):
+        rel = ff.sam_rel_terms(q, pos_h, pos_w, side)
+        out = [*rel, ff.gemm(small, w)]
+        out += [*ff.sam_rel_terms(k, pos_h, pos_w, side), ff.gemm(wide, w)]
+        out += [*ff.sam_rel_terms(v, pos_h, pos_w, side), ff.attention(q, k, v, scale=DIM**-0.5, layout="bnhd", rel=rel)]
+        first = first or out
+        assert all(torch.equal(x, y) for x, y in zip(out, first, strict=True))
+    assert ff.device_status() == 0
+    for got, x in ((first[2], small), (first[5], wide)):
+        assert_close(got.float().cpu().numpy(), (x.float() @ w.float().T).cpu().numpy(), unit_scale=False, what=f"product behind [{b},{side},{heads}]")
+
+
 def test_producer_kernel_rejects_what_it_cannot_take() -> None:
     q = torch.zeros(1, 25, 2, 64, dtype=torch.float16, device="cuda")
     pos = torch.zeros(9, 64, dtype=torch.float16, device="cuda")
