@@ -132,6 +132,20 @@ def test_producer_kernel_by_lines(b: int, side: int, heads: int, dtype: torch.dt
     assert_close(rel_w.float().cpu().numpy(), want_w, unit_scale=False, what=f"rel_w side {side}")
 
 
+@pytest.mark.parametrize(("b", "side", "heads"), [(1, 40, 12), (1, 48, 5), (2, 56, 3), (1, 64, 12), (1, 64, 17)])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_producer_kernels_give_the_same_bits(b: int, side: int, heads: int, dtype: torch.dtype) -> None:
+    """The same tables on 16 bytes (by lines) and on 4 (by tokens): both add a term's 64 products in the same order."""
+    gen = torch.Generator(device="cuda").manual_seed(side + heads)
+    q = torch.randn(b, side * side, heads, DIM, generator=gen, device="cuda").to(dtype)
+    pos = (torch.randn(2, 2 * side - 1, DIM, generator=gen, device="cuda") * 0.1).to(dtype)
+    apart = torch.empty(2, 2 + pos[0].numel(), dtype=dtype, device="cuda")[:, 2:].unflatten(1, pos.shape[1:]).copy_(pos)
+    assert [t.data_ptr() % 16 for t in pos] == [0, 0]
+    assert [t.data_ptr() % 16 != 0 for t in apart] == [True, True]
+    for by_lines, by_tokens in zip(ff.sam_rel_terms(q, *pos, side), ff.sam_rel_terms(q, *apart, side), strict=True):
+        assert torch.equal(by_lines, by_tokens)
+
+
 @pytest.mark.parametrize(("b", "side", "heads"), [(1, 40, 2), (3, 40, 6), (2, 64, 4), (2, 64, 12), (1, 64, 33)])
 def test_producer_by_lines_with_kernels_close_behind(b: int, side: int, heads: int) -> None:
     """Kernels that allocate tensor memory in their set-up, each started while the one in front drains: lines of one to eight tiles and
