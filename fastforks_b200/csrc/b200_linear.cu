@@ -262,23 +262,42 @@ int launch_gemm(const GemmCall& c, cudaStream_t stream) {
 
 namespace {
 
+template <typename T, int NT>
+const void* rel_kernel_at(bool rows) {
+  if constexpr (NT <= 4 || NT == 8)  // sides rel_by_tokens() may choose
+    if (!rows) return reinterpret_cast<const void*>(sam_rel_terms_kernel<T, NT>);
+  return reinterpret_cast<const void*>(sam_rel_rows_kernel<T, NT>);
+}
 template <typename T>
-const void* rel_kernel_of(int tiles) {
+const void* rel_kernel_of(int tiles, bool rows) {
   switch (tiles) {
-    case 1: return reinterpret_cast<const void*>(sam_rel_terms_kernel<T, 1>);
-    case 2: return reinterpret_cast<const void*>(sam_rel_terms_kernel<T, 2>);
-    case 3: return reinterpret_cast<const void*>(sam_rel_terms_kernel<T, 3>);
-    case 4: return reinterpret_cast<const void*>(sam_rel_terms_kernel<T, 4>);
-    case 5: return reinterpret_cast<const void*>(sam_rel_terms_kernel<T, 5>);
-    case 6: return reinterpret_cast<const void*>(sam_rel_terms_kernel<T, 6>);
-    case 7: return reinterpret_cast<const void*>(sam_rel_terms_kernel<T, 7>);
-    default: return reinterpret_cast<const void*>(sam_rel_terms_kernel<T, 8>);
+    case 1: return rel_kernel_at<T, 1>(rows);
+    case 2: return rel_kernel_at<T, 2>(rows);
+    case 3: return rel_kernel_at<T, 3>(rows);
+    case 4: return rel_kernel_at<T, 4>(rows);
+    case 5: return rel_kernel_at<T, 5>(rows);
+    case 6: return rel_kernel_at<T, 6>(rows);
+    case 7: return rel_kernel_at<T, 7>(rows);
+    default: return rel_kernel_at<T, 8>(rows);
   }
 }
-// Sides from which the terms are computed by lines; us by lines and by tokens: side 32 [1,12] 5.1 and 3.8, [8,16] 16.4 and 14.3; side 40
-// [1,12] 5.9 and 6.6; side 48 [4,12] 16.0 and 21.5. Rows and addresses in whole 16-byte groups, heads to divide by.
-constexpr int kRelLinesSide = 40;
-const void* rel_kernel(bool f16, int tiles) { return f16 ? rel_kernel_of<__half>(tiles) : rel_kernel_of<__nv_bfloat16>(tiles); }
+// Which of the three kernels; us ([images, heads, side]) by rows, by tokens and by lines.
+// By lines (rows and addresses in whole 16-byte groups, heads to divide by) from side 48 on: [1,12,48] 7.6, 7.8, 7.2; [2,12,48] 10.8, 13.9,
+// 11.7; [4,12,48] 19.7, 24.8, 16.3; [1,12,64] 12.0, 10.0, 7.9; [4,12,64] 27.5, 30.4, 22.8; [16,16,56] 178, 195, 87; [16,16,64] 99.7, 127, 105. At side 40
+// where an SM has one line or at least four: [1,12,40] 6.5, 6.0, 6.0; [2,12,40] 7.9, 9.6, 9.3; [4,12,40] 12.3, 13.8, 12.9; [16,12,40] 39.5, 46, 35.1.
+bool rel_by_lines(int side, long long lines, int sms) { return side >= 48 || (side >= 40 && (lines <= sms || lines >= 4LL * sms)); }
+// Two CTAs fit an SM's shared memory with six tiles at a time: one loads while the other holds the tensor memory. us, eight at a
+// time and the fewest even shares of at most six: [2,16,56] 17.4 and 15.1, [4,16,64] 37.3 and 31.0, [8,16,64] 66.7 and 54.7; at a line per SM there is
+// nothing to overlap, [1,16,64] 9.5 and 10.6.
+int rel_line_tiles(int tiles, long long lines, int sms) {
+  const int most = lines <= sms ? kRelLineTiles : 6, passes = (tiles + most - 1) / most;
+  return (tiles + passes - 1) / passes;
+}
+// By tokens up to side 32 and at 64 (whole 16-byte groups per row; in between its stores are pieces of four bytes, a sector each), and
+// up to 13 CTAs per SM, by rows beyond: [25,12,14] 6.1 and 4.9, [50,16,14] 11.1 and 8.4, [64,12,14] 9.9 and 10.1, [100,12,14] 12.6 and
+// 14.4, [400,12,14] 44 and 58; [32,12,20] 17.1 and 13.5, [64,12,20] 23.7 and 25.0; [8,12,32] 11.5 and 8.8, [16,12,32] 15.1 and 16.1; [4,12,44] 15.5 and
+// 22.1; [4,12,62] 55 and 63; [1,1,64] 11.1 and 8.1, [4,1,64] 23.7 and 24.5.
+bool rel_by_tokens(int side, long long ctas, int sms) { return (side <= 32 || side == 64) && ctas <= 13LL * sms; }
 
 }  // namespace
 
@@ -316,30 +335,32 @@ int launch_rel_terms(const B200RelTermsArgs* a, bool early_tables, cudaStream_t 
   prm.tables_wide = aligned16(a->rel_pos_h) && aligned16(a->rel_pos_w);
   prm.out_wide = aligned16(a->rel_h) && aligned16(a->rel_w);
   prm.early_tables = early_tables ? 1 : 0;
+  DeviceState* dev = nullptr;
+  if (int rc = device_state(&dev)) return rc;
+  const bool f16 = a->dtype == B200_ATTN_F16;
   const long long lines = 2LL * a->batch * a->side;
-  if (a->side % 8 == 0 && a->side >= kRelLinesSide && prm.tables_wide && prm.out_wide && a->heads > 1 && a->heads <= 1024 && lines <= 0x7fffffffLL) {
-    DeviceState* dev = nullptr;
-    if (int rc = device_state(&dev)) return rc;
+  if (a->side % 8 == 0 && rel_by_lines(a->side, lines, dev->sms) && prm.tables_wide && prm.out_wide && a->heads > 1 && a->heads <= 1024 && lines <= 0x7fffffffLL) {
     prm.status = dev->status;
     prm.magic_heads = static_cast<uint32_t>((uint64_t(1) << 32) / static_cast<uint32_t>(a->heads) + 1);  // exact for 64 * heads rows
-    const bool f16 = a->dtype == B200_ATTN_F16;
+    prm.tiles = rel_line_tiles((a->side * a->heads + 127) / 128, lines, dev->sms);
     const void* kernel = f16 ? reinterpret_cast<const void*>(sam_rel_lines_kernel<__half>) : reinterpret_cast<const void*>(sam_rel_lines_kernel<__nv_bfloat16>);
     if (int rc = opt_in(*dev, kLinearKernels - (f16 ? 2 : 1), kernel, rel_lines_smem(kRelLineTiles))) return rc;
-    const int smem = rel_lines_smem(std::min((a->side * a->heads + 127) / 128, kRelLineTiles));
     void* args[] = {&prm};
-    if (int rc = launch_kernel(kernel, static_cast<unsigned>(lines), 1, kRelLineThreads, smem, 1, stream, args, "sam_rel_terms kernel launch")) return rc;
+    if (int rc = launch_kernel(kernel, static_cast<unsigned>(lines), 1, kRelLineThreads, rel_lines_smem(prm.tiles), 1, stream, args, "sam_rel_terms kernel launch")) return rc;
     clear_error();
     return B200_ATTN_OK;
   }
-  // A token per warp.
   const long long grid_rows = static_cast<long long>(a->batch) * a->side;
   prm.parts = (a->side + kRelWarps - 1) / kRelWarps;
+  const bool rows = !rel_by_tokens(a->side, grid_rows * prm.parts, dev->sms);
+  if (rows)  // one CTA per grid row, and several where there are few rows: about four CTAs per SM, a token per warp at least
+    prm.parts = static_cast<int>(std::max(1LL, std::min<long long>((4LL * dev->sms + grid_rows - 1) / grid_rows, (a->side + kRelRowWarps - 1) / kRelRowWarps)));
   if (grid_rows * prm.parts > 0x7fffffffLL) return fail(B200_ATTN_UNSUPPORTED, "batch too large for one launch");
-  const void* kernel = rel_kernel(a->dtype == B200_ATTN_F16, (a->side + 7) / 8);
+  const int tiles = (a->side + 7) / 8;
+  const void* kernel = f16 ? rel_kernel_of<__half>(tiles, rows) : rel_kernel_of<__nv_bfloat16>(tiles, rows);
   void* args[] = {&prm};
-  const size_t smem = static_cast<size_t>(2 * a->side - 1 + (a->side + prm.parts - 1) / prm.parts) * 128;
-  if (int rc = launch_kernel(kernel, static_cast<unsigned>(grid_rows * prm.parts), 1, kRelWarps * 32, smem, 1, stream, args,
-                             "sam_rel_terms kernel launch"))
+  const int table_rows = rows ? 3 * a->side - 1 : 2 * a->side - 1 + (a->side + prm.parts - 1) / prm.parts;
+  if (int rc = launch_kernel(kernel, static_cast<unsigned>(grid_rows * prm.parts), 1, (rows ? kRelRowWarps : kRelWarps) * 32, table_rows * 128, 1, stream, args, "sam_rel_terms kernel launch"))
     return rc;
   clear_error();
   return B200_ATTN_OK;

@@ -5,11 +5,12 @@
 // parameters themselves ([2 * side - 1, 64]): the [side, side, 64] gather the upstream code builds first
 // (get_rel_pos) never exists.
 //
-// Two kernels, launch_rel_terms() in b200_linear.cu chooses. sam_rel_terms_kernel, for small grids and odd alignments: one query
-// token is a 16 x 64 operand (its heads) against `side` rows of either table, two small products on the same left operand;
-// mma.sync fits operands of 16 rows that change their table rows from token to token. sam_rel_lines_kernel, for sides of 40 and
-// more: the tokens of a grid row or column share their table rows and go through tensor memory together. Both are bound by
-// latency at one image and by the bytes of the result (12.6 MB for SAM's global grid) at several.
+// Three kernels, launch_rel_terms() in b200_linear.cu chooses; all add the 64 products of a term in the same order, so the choice
+// shows in no bit. In two of them one query token is a 16 x 64 operand (its heads) against `side` rows of either table, two small
+// products on the same left operand; mma.sync fits operands of 16 rows that change their table rows from token to token:
+// sam_rel_terms_kernel has a warp per token, for small grids, sam_rel_rows_kernel takes a grid row's tokens in turn behind whole
+// tables, for many. sam_rel_lines_kernel, for large sides: the tokens of a grid row or column share their table rows and go through
+// tensor memory together. All are bound by latency at one image and by the bytes of the result (12.6 MB for SAM's global grid) at several.
 #pragma once
 
 #include <cuda_bf16.h>
@@ -30,14 +31,15 @@ struct RelTermsParams {
   void* rel_h;               // [batch, heads, side * side, side], contiguous
   void* rel_w;
   int batch, heads, side;
-  int parts;                 // CTAs per grid row: a token per warp
+  int parts;                 // CTAs per grid row
   int tables_wide, out_wide; // both tables / results are 16-byte aligned (else 4-byte)
   uint32_t magic_heads;      // ceil(2^32 / heads)
+  int tiles;                 // by lines: tiles of 128 rows at a time
   uint32_t* status;
   int early_tables;          // the tables were complete before the kernel in front of this one started: load them without waiting for that one
 };
 
-constexpr int kRelWarps = 8;
+constexpr int kRelWarps = 8, kRelRowWarps = 4;
 constexpr int kRelMaxSide = 64;
 
 template <typename T>
@@ -54,16 +56,84 @@ __device__ __forceinline__ uint32_t rel_pack2(float lo, float hi) {
 // NT: 8-column tiles of a result row, ceil(side / 8). The order of the 64 products of a sum and of the columns in a tile
 // is free, so both are chosen for wide accesses: a lane's k values are 16-byte chunks of q's and the tables' rows (chunk
 // t and t + 4 of eight), and its columns are the 2 NT consecutive ones from 2 NT t on (t = lane % 4).
-// A token per warp and the rows of the tables that the CTA's tokens need, all in flight together with q. us, four warps that took
-// tokens in turn behind whole tables -> this ([images, heads, side]): [25,12,14] 6.4 -> 5.0, [2,16,32] 5.1 -> 3.7, [1,12,20] 3.1 -> 2.4,
-// [100,12,14] 15.9 and 16.1.
+// Table rows are eight 16-byte chunks in shared memory; odd rows have their halves swapped, so that two neighbouring rows, which a
+// quarter of a warp reads together, use all banks.
+
+// Sixteen heads of a token from h0 on, chunks t and t + 4 of heads h0 + g (lo) and h0 + g + 8 (hi); rows past the last head repeat
+// it and are not stored.
+template <typename T>
+__device__ __forceinline__ void rel_load_q(const RelTermsParams& p, const T* q_token, int g, int t, int h0, uint4* lo, uint4* hi) {
+  const T* q_lo = q_token + min(h0 + g, p.heads - 1) * p.q_sh;
+  const T* q_hi = q_token + min(h0 + g + 8, p.heads - 1) * p.q_sh;
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    lo[i] = __ldg(reinterpret_cast<const uint4*>(q_lo) + t + 4 * i);
+    hi[i] = __ldg(reinterpret_cast<const uint4*>(q_hi) + t + 4 * i);
+  }
+}
+
+// Both products of those heads of token n, in grid column x, and their stores, MOST tiles at a time. Row k of table_h belongs to column
+// k of rel_h, row k of table_w is rel_pos_w[w_first + k].
+template <typename T, int NT, int MOST>
+__device__ __forceinline__ void rel_token(const RelTermsParams& p, const uint4* lo, const uint4* hi, const uint4* table_h, const uint4* table_w, int w_first, int x, int b, int n, int n_tokens, int side, int g, int t, int h0) {
+  uint32_t a[4][4];
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    a[2 * i][0] = lo[i].x; a[2 * i][1] = hi[i].x; a[2 * i][2] = lo[i].y; a[2 * i][3] = hi[i].y;
+    a[2 * i + 1][0] = lo[i].z; a[2 * i + 1][1] = hi[i].z; a[2 * i + 1][2] = lo[i].w; a[2 * i + 1][3] = hi[i].w;
+  }
+#pragma unroll
+  for (int which = 0; which < 2; ++which) {
+    T* const out = static_cast<T*>(which == 0 ? p.rel_h : p.rel_w);
+#pragma unroll
+    for (int j0 = 0; j0 < NT; j0 += MOST) {
+      float acc[MOST][4];
+#pragma unroll
+      for (int j = 0; j < MOST; ++j) {
+        if (j0 + j >= NT) continue;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[j][e] = 0.f;
+        // lane group g holds column 2 NT (g / 2) + 2 (j0 + j) + g % 2 of the result: table row for that k
+        const int k = min(2 * NT * (g >> 1) + 2 * (j0 + j) + (g & 1), side - 1);
+        const int row = which == 0 ? k : x - w_first - k + side - 1;
+        const uint4* table = (which == 0 ? table_h : table_w) + row * 8;
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const uint4 v = table[(t + 4 * i) ^ ((row & 1) << 2)];
+          mma_16816<T>(acc[j], a[2 * i], v.x, v.y);
+          mma_16816<T>(acc[j], a[2 * i + 1], v.z, v.w);
+        }
+      }
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        const int head = h0 + g + 8 * half;
+        if (head >= p.heads) continue;
+        T* dst = out + ((static_cast<int64_t>(b) * p.heads + head) * n_tokens + n) * side + 2 * NT * t + 2 * j0;
+        uint32_t words[MOST];
+#pragma unroll
+        for (int j = 0; j < MOST; ++j)
+          if (j0 + j < NT) words[j] = rel_pack2<T>(acc[j][2 * half], acc[j][2 * half + 1]);
+        if constexpr (NT % 4 == 0) {
+          if (side == 8 * NT && p.out_wide) {  // whole 16-byte groups, rows of whole groups
+#pragma unroll
+            for (int j = 0; j < MOST; j += 4) *reinterpret_cast<uint4*>(dst + 2 * j) = make_uint4(words[j], words[j + 1], words[j + 2], words[j + 3]);
+            continue;
+          }
+        }
+#pragma unroll
+        for (int j = 0; j < MOST; ++j)
+          if (j0 + j < NT && 2 * NT * t + 2 * (j0 + j) < side) *reinterpret_cast<uint32_t*>(dst + 2 * j) = words[j];  // side is even
+      }
+    }
+  }
+}
+
+// A token per warp and the rows of the tables that the CTA's tokens need, all in flight together with q.
+// Four tiles at a time: registers for four CTAs per SM (and up to 80 bytes of spills).
 template <typename T, int NT>
 __global__ void __launch_bounds__(kRelWarps * 32, 4) sam_rel_terms_kernel(const RelTermsParams p) {
-  // Table rows as eight 16-byte chunks; odd rows have their halves swapped, so that two neighbouring rows, which a quarter
-  // of a warp reads together, use all banks.
   extern __shared__ uint4 rel_tables[];
-  const int side = p.side, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int g = lane >> 2, t = lane & 3;
+  const int side = p.side, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3, n_tokens = side * side;
   const int row_id = blockIdx.x / p.parts, part = blockIdx.x - row_id * p.parts;
   const int b = row_id / side, y = row_id - b * side;
   const int x_begin = side * part / p.parts, x_end = side * (part + 1) / p.parts;  // at most kRelWarps tokens
@@ -85,76 +155,52 @@ __global__ void __launch_bounds__(kRelWarps * 32, 4) sam_rel_terms_kernel(const 
   grid_dependency_wait();
   grid_launch_dependents();
   if (!p.early_tables) load_tables();
-  const int n_tokens = side * side;
   const int x = x_begin + warp, n = y * side + x;
   const bool here = x < x_end;
   const T* const q_token = static_cast<const T*>(p.q) + b * p.q_sb + (here ? n : 0) * p.q_sn;
-  // heads h0 + g and h0 + g + 8, 16-byte chunks t and t + 4 (rows past the last head repeat it; they are not stored)
   uint4 lo[2], hi[2];
-  const auto load_q = [&](int h0) {
-    const T* q_lo = q_token + min(h0 + g, p.heads - 1) * p.q_sh;
-    const T* q_hi = q_token + min(h0 + g + 8, p.heads - 1) * p.q_sh;
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      lo[i] = __ldg(reinterpret_cast<const uint4*>(q_lo) + t + 4 * i);
-      hi[i] = __ldg(reinterpret_cast<const uint4*>(q_hi) + t + 4 * i);
-    }
-  };
-  load_q(0);
+  rel_load_q(p, q_token, g, t, 0, lo, hi);
   cp_async_wait<0>();
   __syncthreads();
   if (!here) return;
   for (int h0 = 0; h0 < p.heads; h0 += 16) {
-    if (h0 > 0) load_q(h0);
-    uint32_t a[4][4];
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      a[2 * i][0] = lo[i].x; a[2 * i][1] = hi[i].x; a[2 * i][2] = lo[i].y; a[2 * i][3] = hi[i].y;
-      a[2 * i + 1][0] = lo[i].z; a[2 * i + 1][1] = hi[i].z; a[2 * i + 1][2] = lo[i].w; a[2 * i + 1][3] = hi[i].w;
-    }
-#pragma unroll
-    for (int which = 0; which < 2; ++which) {
-      T* const out = static_cast<T*>(which == 0 ? p.rel_h : p.rel_w);
-#pragma unroll
-      for (int j0 = 0; j0 < NT; j0 += 4) {  // four tiles at a time: registers for four CTAs per SM
-        constexpr int kMost = NT < 4 ? NT : 4;
-        float acc[kMost][4];
-#pragma unroll
-        for (int j = 0; j < kMost; ++j) {
-          if (j0 + j >= NT) continue;
-#pragma unroll
-          for (int e = 0; e < 4; ++e) acc[j][e] = 0.f;
-          // lane group g holds column 2 NT (g / 2) + 2 (j0 + j) + g % 2 of the result: table row for that k
-          const int k = min(2 * NT * (g >> 1) + 2 * (j0 + j) + (g & 1), side - 1);
-          const int row = which == 0 ? k : x - x_begin - k + side - 1;
-          const uint4* table = (which == 0 ? table_h : table_w) + row * 8;
-#pragma unroll
-          for (int i = 0; i < 2; ++i) {
-            const uint4 v = table[(t + 4 * i) ^ ((row & 1) << 2)];
-            mma_16816<T>(acc[j], a[2 * i], v.x, v.y);
-            mma_16816<T>(acc[j], a[2 * i + 1], v.z, v.w);
-          }
-        }
-#pragma unroll
-        for (int half = 0; half < 2; ++half) {
-          const int head = h0 + g + 8 * half;
-          if (head >= p.heads) continue;
-          T* dst = out + ((static_cast<int64_t>(b) * p.heads + head) * n_tokens + n) * side + 2 * NT * t + 2 * j0;
-          uint32_t words[kMost];
-#pragma unroll
-          for (int j = 0; j < kMost; ++j)
-            if (j0 + j < NT) words[j] = rel_pack2<T>(acc[j][2 * half], acc[j][2 * half + 1]);
-          if constexpr (NT % 4 == 0) {
-            if (side == 8 * NT && p.out_wide) {  // whole 16-byte groups, rows of whole groups
-              *reinterpret_cast<uint4*>(dst) = make_uint4(words[0], words[1], words[2], words[3]);
-              continue;
-            }
-          }
-#pragma unroll
-          for (int j = 0; j < kMost; ++j)
-            if (j0 + j < NT && 2 * NT * t + 2 * (j0 + j) < side) *reinterpret_cast<uint32_t*>(dst + 2 * j) = words[j];  // side is even
-        }
-      }
+    if (h0 > 0) rel_load_q(p, q_token, g, t, h0, lo, hi);
+    rel_token<T, NT, NT < 4 ? NT : 4>(p, lo, hi, table_h, table_w, x_begin, x, b, n, n_tokens, side, g, t, h0);
+  }
+}
+
+// The tokens of a grid row, or of a part of it, in turn on four warps: each row of the tables is read once for all of them.
+template <typename T, int NT>
+__global__ void __launch_bounds__(kRelRowWarps * 32) sam_rel_rows_kernel(const RelTermsParams p) {
+  extern __shared__ uint4 rel_tables[];
+  const int side = p.side, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3, n_tokens = side * side;
+  const int row_id = blockIdx.x / p.parts, part = blockIdx.x - row_id * p.parts;
+  const int b = row_id / side, y = row_id - b * side;
+  uint4* const table_h = rel_tables;              // row k: rel_pos_h[y - k + side - 1]
+  uint4* const table_w = rel_tables + side * 8;   // rel_pos_w as it is
+  grid_dependency_wait();
+  grid_launch_dependents();
+  const auto load = [&](const void* table, int row, int c) {
+    const uint32_t* src = static_cast<const uint32_t*>(table) + row * 32 + c * 4;
+    return p.tables_wide ? __ldg(reinterpret_cast<const uint4*>(src)) : make_uint4(__ldg(src), __ldg(src + 1), __ldg(src + 2), __ldg(src + 3));
+  };
+  for (int i = threadIdx.x; i < side * 8; i += kRelRowWarps * 32) {
+    const int k = i >> 3, c = i & 7;
+    table_h[k * 8 + (c ^ ((k & 1) << 2))] = load(p.rel_pos_h, y - k + side - 1, c);
+  }
+  for (int i = threadIdx.x; i < (2 * side - 1) * 8; i += kRelRowWarps * 32) {
+    const int k = i >> 3, c = i & 7;
+    table_w[k * 8 + (c ^ ((k & 1) << 2))] = load(p.rel_pos_w, k, c);
+  }
+  __syncthreads();
+  const int x_end = side * (part + 1) / p.parts;
+  for (int x = side * part / p.parts + warp; x < x_end; x += kRelRowWarps) {
+    const int n = y * side + x;
+    const T* const q_token = static_cast<const T*>(p.q) + b * p.q_sb + n * p.q_sn;
+    for (int h0 = 0; h0 < p.heads; h0 += 16) {
+      uint4 lo[2], hi[2];
+      rel_load_q(p, q_token, g, t, h0, lo, hi);
+      rel_token<T, NT, NT>(p, lo, hi, table_h, table_w, 0, x, b, n, n_tokens, side, g, t, h0);
     }
   }
 }
@@ -163,9 +209,8 @@ __global__ void __launch_bounds__(kRelWarps * 32, 4) sam_rel_terms_kernel(const 
 // The queries of one grid row (rel_h) or column (rel_w), all heads, use the same `side` table rows: a product of side * heads
 // rows, `side` columns and 64 values for the tensor memory. A CTA takes such a line: its q rows and table rows come into shared
 // memory together (128-byte swizzle), the products are a handful of tcgen05.mma, and a warp writes whole rows of the result (a
-// thread per row, 16 bytes of 32 rows per instruction, cost the 64 x 64 grid another 1.8 us). us, by tokens with the first form of
-// the kernel above -> by lines: [1,12,64] 12.8 -> 8.0, [4,12,64] 31.2 -> 22.7, [1,12,48] 7.9 -> 7.0, [1,12,40] 6.6 -> 5.9.
-constexpr int kRelLineThreads = 256, kRelLineTiles = 8;  // tiles of 128 rows at a time: all of tensor memory at 64 columns
+// thread per row, 16 bytes of 32 rows per instruction, cost the 64 x 64 grid another 1.8 us).
+constexpr int kRelLineThreads = 256, kRelLineTiles = 8;  // at most so many tiles of 128 rows at a time: all of tensor memory at 64 columns
 constexpr int rel_lines_smem(int tiles) { return 1024 + 64 * 128 + tiles * 128 * 128; }  // tables, q tiles
 enum : uint32_t { kStatusRelTerms = 512 };
 
@@ -180,7 +225,7 @@ __global__ void __launch_bounds__(kRelLineThreads, 2) sam_rel_lines_kernel(const
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int line = blockIdx.x % side, which = (blockIdx.x / side) & 1, b = blockIdx.x / (2 * side);
   const int n_rows = side * p.heads, n_tiles = (n_rows + 127) >> 7;
-  const uint32_t tmem_cols = n_tiles >= 5 ? 8 * stride_cols : n_tiles >= 3 ? 4 * stride_cols : 2 * stride_cols;
+  const uint32_t tmem_cols = p.tiles >= 5 ? 8 * stride_cols : p.tiles >= 3 ? 4 * stride_cols : 2 * stride_cols;
   if (threadIdx.x == 0) {
     mbar_init(&done, 1);
     abort = 0;
@@ -213,8 +258,8 @@ __global__ void __launch_bounds__(kRelLineThreads, 2) sam_rel_lines_kernel(const
   if (!p.early_tables) load_table();
   bool ok = true;
   uint32_t phase = 0;
-  for (int t0 = 0; t0 < n_tiles; t0 += kRelLineTiles) {
-    const int now = min(n_tiles - t0, kRelLineTiles);
+  for (int t0 = 0; t0 < n_tiles; t0 += p.tiles) {
+    const int now = min(n_tiles - t0, p.tiles);
     for (int i = threadIdx.x; i < now * 128 * 8; i += kRelLineThreads) {
       const int row = i >> 3, c = i & 7, r = t0 * 128 + row;
       int head = 0;

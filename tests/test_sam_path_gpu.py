@@ -97,7 +97,8 @@ def test_producer_kernel_matches_the_oracle(b: int, side: int, dtype: torch.dtyp
     assert_close(rel_w.float().cpu().numpy(), want_w, unit_scale=False, what=f"rel_w side {side} {dtype}")
 
 
-@pytest.mark.parametrize(("b", "side", "heads"), [(1, 2, 1), (2, 6, 3), (1, 10, 17), (1, 16, 16), (1, 22, 24), (3, 32, 12), (1, 40, 5), (1, 48, 33), (2, 50, 12), (1, 62, 7)])
+@pytest.mark.parametrize(("b", "side", "heads"), [(1, 2, 1), (2, 6, 3), (1, 10, 17), (1, 16, 16), (1, 22, 24), (3, 32, 12), (1, 40, 5), (1, 48, 33), (2, 50, 12), (1, 62, 7),
+                                                  (1, 64, 1), (1, 64, 17), (3, 56, 2), (70, 14, 2)])  # fmt: skip
 def test_producer_kernel_at_every_tile_count(b: int, side: int, heads: int) -> None:
     """Grid sides for each number of eight-column tiles, head counts around the sixteen rows of one product, and a second
     table whose address is only 4-byte aligned (read word by word)."""
@@ -144,6 +145,19 @@ def test_producer_kernels_give_the_same_bits(b: int, side: int, heads: int, dtyp
     assert [t.data_ptr() % 16 != 0 for t in apart] == [True, True]
     for by_lines, by_tokens in zip(ff.sam_rel_terms(q, *pos, side), ff.sam_rel_terms(q, *apart, side), strict=True):
         assert torch.equal(by_lines, by_tokens)
+
+
+@pytest.mark.parametrize(("b", "side", "heads"), [(80, 8, 3), (70, 14, 17), (54, 20, 2), (31, 26, 1), (16, 32, 3), (8, 40, 2), (4, 40, 3), (3, 64, 1), (3, 64, 12), (2, 64, 16), (2, 64, 17)])
+def test_producer_gives_an_image_the_same_bits_alone_and_in_a_batch(b: int, side: int, heads: int) -> None:
+    """One image goes by tokens or by lines, as many tiles of rows at a time as there are; the batch by rows, by lines, or by lines with
+    fewer tiles at a time."""
+    gen = torch.Generator(device="cuda").manual_seed(side + heads)
+    q = torch.randn(b, side * side, heads, DIM, generator=gen, device="cuda").half()
+    pos = (torch.randn(2, 2 * side - 1, DIM, generator=gen, device="cuda") * 0.1).half()
+    together = ff.sam_rel_terms(q, *pos, side)
+    for i in {0, b // 2, b - 1}:
+        for whole, alone in zip(together, ff.sam_rel_terms(q[i : i + 1], *pos, side), strict=True):
+            assert torch.equal(whole[i], alone[0])
 
 
 @pytest.mark.parametrize(("b", "side", "heads"), [(1, 40, 2), (3, 40, 6), (2, 64, 4), (2, 64, 12), (1, 64, 33)])
