@@ -82,8 +82,11 @@ double pair_k_block_us(int bn) { return bn == 256 ? 0.298 : bn == 192 ? 0.25 : b
 constexpr double kPairRoundUs = 0.15;
 // Row tiles per raster group: 74 pairs then work on four rows of x tiles and a dozen or two of w tiles at a time. us with groups of
 // 16 and of 4 (1 to 6 are within 0.5 %): [5480,3072,1024] 33.7 and 32.9, [5480,1024,4096] 49.2 and 48.3, [4096,3072,768] 25.5 and 24.1,
-// [32928,3072,1024] 172.8 and 169.9, [21920,4608,1536] 236.1 and 233.9, all in loops of some milliseconds.
-constexpr int kPairGroup = 4;
+// [32928,3072,1024] 172.8 and 169.9, [21920,4608,1536] 236.1 and 233.9, all in loops of some milliseconds; of few products
+// [21920,1536,4096] 181 and 175, [4096,8192,1024] 54.1 and 50.0, [16384,9216,1024] 218 and 215, but [4096,4096,4096] 91.7 and 92.5. With more than
+// 10240 rows of w every group reads a w that the outputs have pushed out of L2: [16384,16384,1024] 387 and 401,
+// [4096,12288,4096] 264 and 279, [4096,16384,2048] 182 and 190.
+constexpr int pair_group(int64_t w_rows) { return w_rows > 10240 ? 16 : 4; }
 // A CTA of the split kernel: 2.5 for set-up, first loads and epilogue, 0.2 per k-block, 0.3 for the merge of a cluster.
 constexpr double kSplitRoundUs = 2.5, kSplitKBlockUs = 0.2, kSplitMergeUs = 0.3, kSplitLaunchUs = 0.6;
 static_assert(kGemmSplits == 6, "split counts");
@@ -223,7 +226,7 @@ int launch_gemm(const GemmCall& c, cudaStream_t stream) {
     const int out_cols = swiglu ? 128 : plan.bn;
     prm.tiles_m = (c.m + 255) / 256;
     prm.tiles_n = (c.n + out_cols - 1) / out_cols;
-    prm.group_m = std::min(prm.tiles_m, kPairGroup);
+    prm.group_m = std::min(prm.tiles_m, pair_group(w_rows));
     const long long tiles = static_cast<long long>(prm.tiles_m) * prm.tiles_n;
     if (tiles > 0x3fffffffLL) return fail(B200_ATTN_UNSUPPORTED, "problem too large for one launch");
     prm.stages = std::min(kPairMaxStages, kPairRingBytes / (kGemmTileBytes + plan.bn * kGemmBK));

@@ -105,6 +105,14 @@ def test_residual_and_scale_each_alone(scaled: bool, act: int, m: int, n: int, k
     check(ff.gemm(x, w, bias, act=act, out=out, **extra), x, w, bias, act=act, what=f"[{m},{n},{k}] act {act}", **extra)
 
 
+@pytest.mark.parametrize(("m", "n", "k"), [(1500, 10240, 72), (1500, 10248, 72), (4400, 10504, 40)])
+def test_raster_groups_of_narrow_and_wide_products(m: int, n: int, k: int) -> None:
+    """Both sides of the width from which sixteen row tiles share a column of tiles; fewer and more row tiles than that."""
+    x, w, bias, _, _ = (t.cuda() for t in operands(m, n, k, torch.float16, seed=n))
+    out = torch.full((m, n), float("nan"), dtype=torch.float16, device="cuda")
+    check(ff.gemm(x, w, bias, out=out), x, w, bias, what=f"[{m},{n},{k}]")
+
+
 # One shape for every way a product is cut: the split kernel whole and with 2, 3, 4, 6 and 8 CTAs per cluster (uneven k
 # shares, rows that do not divide, a last tile of one row), pair tiles of 64 to 256 columns, and a last round in parts.
 PLANS = [(100, 72, 8), (197, 2304, 776), (257, 1024, 1544), (129, 776, 1000), (60, 64, 3080), (255, 384, 1536), (1, 8, 4096), (1000, 3000, 72),
