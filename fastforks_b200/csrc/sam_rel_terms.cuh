@@ -217,7 +217,7 @@ enum : uint32_t { kStatusRelTerms = 512 };
 template <typename T>
 __global__ void __launch_bounds__(kRelLineThreads, 2) sam_rel_lines_kernel(const RelTermsParams p) {
   extern __shared__ uint8_t rel_smem_raw[];
-  __shared__ uint64_t done;
+  __shared__ uint64_t done, drain;  // a round's products have finished; abort path: all of this CTA's have
   __shared__ uint32_t tmem_base, abort;
   uint8_t* const table = smem_align_1024(rel_smem_raw);
   const int side = p.side, n_cols = (side + 15) & ~15, stride_cols = n_cols <= 32 ? 32 : 64;
@@ -228,6 +228,7 @@ __global__ void __launch_bounds__(kRelLineThreads, 2) sam_rel_lines_kernel(const
   const uint32_t tmem_cols = p.tiles >= 5 ? 8 * stride_cols : p.tiles >= 3 ? 4 * stride_cols : 2 * stride_cols;
   if (threadIdx.x == 0) {
     mbar_init(&done, 1);
+    mbar_init(&drain, 1);
     abort = 0;
     mbar_init_fence();
   }
@@ -256,7 +257,6 @@ __global__ void __launch_bounds__(kRelLineThreads, 2) sam_rel_lines_kernel(const
   if (p.early_tables) load_table();
   grid_dependency_wait();
   if (!p.early_tables) load_table();
-  bool ok = true;
   uint32_t phase = 0;
   for (int t0 = 0; t0 < n_tiles; t0 += p.tiles) {
     const int now = min(n_tiles - t0, p.tiles);
@@ -293,7 +293,7 @@ __global__ void __launch_bounds__(kRelLineThreads, 2) sam_rel_lines_kernel(const
       }
       __syncwarp();
     }
-    ok = __all_sync(0xffffffffu, mbar_wait(&done, phase, &abort)) != 0;
+    const bool ok = __all_sync(0xffffffffu, mbar_wait(&done, phase, &abort)) != 0;
     if (!ok && lane == 0 && atomicExch(&abort, 1u) == 0) atomicOr(p.status, kStatusRelTerms);
     phase ^= 1;
     tc_fence_after_sync();
@@ -324,6 +324,15 @@ __global__ void __launch_bounds__(kRelLineThreads, 2) sam_rel_lines_kernel(const
     tc_fence_before_sync();
     __syncthreads();  // tiles and tensor memory have been read
     tc_fence_after_sync();
+    if (abort != 0) {  // written in front of that barrier only, so all leave together: the products may still read the tiles
+      if (warp == 1) {  // no product may be running when tensor memory is freed
+        uint32_t no_abort = 0;
+        if (elect_one()) umma_commit(&drain);
+        mbar_wait(&drain, 0, &no_abort);
+        __syncwarp();
+      }
+      break;
+    }
   }
   if (warp == 1) tmem_dealloc(tmem_base, tmem_cols);
 }

@@ -5,6 +5,7 @@ signatures, mode resolution. Mirrors the reference's launcher tests that need no
 from __future__ import annotations
 
 import importlib
+import re
 import warnings
 
 import pytest
@@ -286,3 +287,26 @@ def test_kernels_hold_their_tensor_memory_before_they_let_the_next_kernel_start(
             assert body.index("tmem_alloc") < body.index("grid_launch_dependents();"), f"{path.name}: {name}"
             checked += 1
     assert checked == 4  # attention, pair and split GEMM, SAM's terms by lines
+
+
+def test_kernels_that_give_up_wait_for_their_products_before_they_free_tensor_memory() -> None:
+    """A wait that runs out ends a kernel early. Products in flight still read its shared memory and write its tensor memory, so none may
+    free that without a wait behind a last commit that looks at no abort flag; and a loop that would overwrite operands ends first.
+    (Read, not run: nothing makes a wait on products run out on a healthy GPU.)"""
+    from fastforks_b200 import _lib
+
+    checked = {}
+    for path in (*_lib.SOURCES, *_lib.HEADERS):
+        for body in path.read_text().split("__global__")[1:]:
+            if "tmem_dealloc" not in body:
+                continue
+            name = body[: body.index("(", body.index("_kernel"))].split()[-1]
+            drained = re.search(r"umma_commit(_pair)?\(&(sm\.)?(drain(\[t\])?|acc_full)\);", body)
+            assert drained, name
+            assert drained.start() < body.index("tmem_dealloc"), name
+            checked[name] = body
+    assert len(checked) == 4  # attention, pair and split GEMM, SAM's terms by lines
+    lines = checked["sam_rel_lines_kernel"]
+    gives_up = lines.index("if (abort != 0)")
+    assert lines.rindex("__syncthreads();", 0, gives_up) > lines.index("mbar_wait(&done")  # the flag is looked at where all warps see the same
+    assert "break;" in lines[gives_up : lines.index("tmem_dealloc")]
