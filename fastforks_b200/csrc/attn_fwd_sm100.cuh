@@ -1753,8 +1753,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         // would leave the unit idle together, and equal loops sharing a unit drift into lockstep). So each
         // may only start a section once the other has released it from inside its previous one: warpgroup 0
         // starts step q+1 after warpgroup 1's release in step q, warpgroup 1 starts step q after warpgroup 0's
-        // release in step q. The release comes after 96 of the 128 columns ([8,16,577] us: 32 columns 28.0, 64 27.9, 96 27.1,
-        // 128 28.4, no token 28.7).
+        // release in step q. The release comes after 96 of the 128 columns. us, 64 and 96:
+        // [32,24,1370] 564 and 497, [32,16,1029] 261 and 229, [16,16,577] 47.9 and 43.4, [4,16,1370] 57.7 and 53.5, [8,6,1370] 44.2 and 40.9; the same
+        // within 1 % on one-wave calls ([1,12,4096] in key splits, [2,12,2304]), dense tiles and the product form. [8,16,577] after 32, 64, 96, 128
+        // columns and without a token: 28.0, 27.9, 27.1, 28.4, 28.7.
         if (need_turn) {
           if constexpr (kFlagTurn) {
             const volatile uint32_t* released = &sm.turn_count[t ^ 1][warp & 3];
@@ -1824,6 +1826,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         };
         using std::integral_constant;
         constexpr int kRelease = BIAS == kBiasDecomposed64 ? 2 : 3;  // columns before the release, in 32s (that form's sections are halves)
+        static_assert(!SHORT || kRelease == 3, "the short schedule goes on at column 96");
         exp_columns(integral_constant<int, 0>{}, integral_constant<int, kRelease>{});
         if constexpr (SHORT) {
           // Short-sequence schedule. The last 32 columns of a ragged last key tile that hold no key at all (197 keys:

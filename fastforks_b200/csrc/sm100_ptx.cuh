@@ -492,15 +492,6 @@ __device__ __forceinline__ void tmem_st_x16(uint32_t taddr, const uint32_t* v) {
       : "memory");
 }
 
-__device__ __forceinline__ void tmem_st_x32(uint32_t taddr, const uint32_t* v) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
-      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
-      "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};\n"
-      :
-      : "r"(taddr), B200_W16(v, 0), B200_W16(v, 16)
-      : "memory");
-}
 
 // 128 columns with one instruction. It needs 128 result registers at once: a kernel whose launch bound allows fewer
 // than about 146 registers per thread does not assemble with it, whatever setmaxnreg raises the budget to later.
