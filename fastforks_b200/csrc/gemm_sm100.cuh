@@ -69,37 +69,9 @@ __device__ __forceinline__ uint32_t gemm_pack2(float lo, float hi) {
   }
 }
 
-// Two values at a time: the packed forms move as many values per clock as the plain ones in half the instructions, and two
-// epilogue warps per SM sub-partition are bound by instructions. us, plain -> packed: [4096,3072,768] with erf GELU 24.8 -> 23.5,
-// with its tanh form 20.8 -> 19.9, [5480,4096,1024] with that 39.4 -> 38.0.
-__device__ __forceinline__ float2 gemm_fma2(float2 a, float2 b, float2 c) {
-  uint64_t ra, rb, rc, rd;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(ra) : "f"(a.x), "f"(a.y));
-  asm("mov.b64 %0, {%1, %2};" : "=l"(rb) : "f"(b.x), "f"(b.y));
-  asm("mov.b64 %0, {%1, %2};" : "=l"(rc) : "f"(c.x), "f"(c.y));
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(rd) : "l"(ra), "l"(rb), "l"(rc));
-  float2 d;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(d.x), "=f"(d.y) : "l"(rd));
-  return d;
-}
-__device__ __forceinline__ float2 gemm_mul2(float2 a, float2 b) {
-  uint64_t ra, rb, rd;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(ra) : "f"(a.x), "f"(a.y));
-  asm("mov.b64 %0, {%1, %2};" : "=l"(rb) : "f"(b.x), "f"(b.y));
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(rd) : "l"(ra), "l"(rb));
-  float2 d;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(d.x), "=f"(d.y) : "l"(rd));
-  return d;
-}
-__device__ __forceinline__ float2 gemm_add2(float2 a, float2 b) {
-  uint64_t ra, rb, rd;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(ra) : "f"(a.x), "f"(a.y));
-  asm("mov.b64 %0, {%1, %2};" : "=l"(rb) : "f"(b.x), "f"(b.y));
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(rd) : "l"(ra), "l"(rb));
-  float2 d;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(d.x), "=f"(d.y) : "l"(rd));
-  return d;
-}
+// The epilogues work on two values at a time: ffma2 and its like move as many values per clock as the plain forms in half the
+// instructions, and two epilogue warps per SM sub-partition are bound by instructions. us, plain -> packed: [4096,3072,768] with erf
+// GELU 24.8 -> 23.5, with its tanh form 20.8 -> 19.9, [5480,4096,1024] with that 39.4 -> 38.0.
 
 // v Phi(v) with Phi the normal distribution, as max(v, 0) - |v| Phi(-|v|): no cancellation on the negative side, where
 // 0.5 v (1 + erf) loses digits. Phi(-x) = exp(-x^2 / 2) t P(t), t = 1 / (1 + 0.3 x), where P is a degree-7 least-maximum
@@ -110,22 +82,22 @@ __device__ __forceinline__ float2 gemm_add2(float2 a, float2 b) {
 __device__ __forceinline__ float2 gelu_erf2(float2 v) {
   const auto both = [](float c) { return make_float2(c, c); };
   const float2 a = make_float2(fabsf(v.x), fabsf(v.y)), x = make_float2(fminf(a.x, 64.f), fminf(a.y, 64.f));
-  const float2 s = gemm_fma2(x, both(0.3f), both(1.f)), g = gemm_mul2(gemm_mul2(x, x), both(-0.72134752f));
+  const float2 s = ffma2(x, both(0.3f), both(1.f)), g = fmul2(fmul2(x, x), both(-0.72134752f));
   float2 t, e;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(t.x) : "f"(s.x));
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(t.y) : "f"(s.y));
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e.x) : "f"(g.x));
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e.y) : "f"(g.y));
   float2 p = both(0.0359317549f);
-  p = gemm_fma2(p, t, both(-0.158276081f));
-  p = gemm_fma2(p, t, both(0.208206728f));
-  p = gemm_fma2(p, t, both(-0.0553939454f));
-  p = gemm_fma2(p, t, both(0.129469246f));
-  p = gemm_fma2(p, t, both(0.0996374786f));
-  p = gemm_fma2(p, t, both(0.120798357f));
-  p = gemm_fma2(p, t, both(0.119626388f));
-  const float2 tail = gemm_mul2(make_float2(-x.x, -x.y), gemm_mul2(t, p));
-  return gemm_fma2(tail, e, gemm_fma2(both(0.5f), v, gemm_mul2(both(0.5f), a)));
+  p = ffma2(p, t, both(-0.158276081f));
+  p = ffma2(p, t, both(0.208206728f));
+  p = ffma2(p, t, both(-0.0553939454f));
+  p = ffma2(p, t, both(0.129469246f));
+  p = ffma2(p, t, both(0.0996374786f));
+  p = ffma2(p, t, both(0.120798357f));
+  p = ffma2(p, t, both(0.119626388f));
+  const float2 tail = fmul2(make_float2(-x.x, -x.y), fmul2(t, p));
+  return ffma2(tail, e, ffma2(both(0.5f), v, fmul2(both(0.5f), a)));
 }
 
 template <int ACT>
@@ -134,11 +106,11 @@ __device__ __forceinline__ float2 gemm_act2(float2 v) {
   if constexpr (ACT == kActGelu) return gelu_erf2(v);
   if constexpr (ACT == kActGeluTanh) {
     const auto both = [](float c) { return make_float2(c, c); };
-    const float2 u = gemm_mul2(gemm_mul2(both(0.7978845608028654f), v), gemm_fma2(gemm_mul2(both(0.044715f), v), v, both(1.f)));
+    const float2 u = fmul2(fmul2(both(0.7978845608028654f), v), ffma2(fmul2(both(0.044715f), v), v, both(1.f)));
     float2 t;
     asm("tanh.approx.f32 %0, %1;" : "=f"(t.x) : "f"(u.x));
     asm("tanh.approx.f32 %0, %1;" : "=f"(t.y) : "f"(u.y));
-    return gemm_mul2(gemm_mul2(both(0.5f), v), gemm_add2(both(1.f), t));
+    return fmul2(fmul2(both(0.5f), v), fadd2(both(1.f), t));
   }
   return v;
 }
@@ -460,10 +432,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant
                   x[2 * i] = gemm_swiglu(v[at_v] + b.x, u[at_v] + bu.x);
                   x[2 * i + 1] = gemm_swiglu(v[at_v + 1] + b.y, u[at_v + 1] + bu.y);
                 } else {
-                  float2 y = gemm_add2(make_float2(v[at_v], v[at_v + 1]), b);
-                  if constexpr (FORM == kPairResidual) y = gemm_add2(y, gemm_unpack2<T>(rw[i]));
+                  float2 y = fadd2(make_float2(v[at_v], v[at_v + 1]), b);
+                  if constexpr (FORM == kPairResidual) y = fadd2(y, gemm_unpack2<T>(rw[i]));
                   if constexpr (FORM == kPairScaled)
-                    y = gemm_fma2(y, make_float2(__shfl_sync(0xffffffffu, piece_scale.x, pair), __shfl_sync(0xffffffffu, piece_scale.y, pair)), gemm_unpack2<T>(rw[i]));
+                    y = ffma2(y, make_float2(__shfl_sync(0xffffffffu, piece_scale.x, pair), __shfl_sync(0xffffffffu, piece_scale.y, pair)), gemm_unpack2<T>(rw[i]));
                   y = gemm_act2<ACT>(y);
                   x[2 * i] = y.x;
                   x[2 * i + 1] = y.y;
@@ -689,8 +661,8 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
           x.x += o.x; x.y += o.y; x.z += o.z; x.w += o.w;
         }
         const float2 r0 = gemm_unpack2<T>(res[i].x), r1 = gemm_unpack2<T>(res[i].y);
-        const float2 y0 = gemm_act2<kAct>(gemm_fma2(gemm_add2(make_float2(x.x, x.y), b0), make_float2(scale.x, scale.y), r0));
-        const float2 y1 = gemm_act2<kAct>(gemm_fma2(gemm_add2(make_float2(x.z, x.w), b1), make_float2(scale.z, scale.w), r1));
+        const float2 y0 = gemm_act2<kAct>(ffma2(fadd2(make_float2(x.x, x.y), b0), make_float2(scale.x, scale.y), r0));
+        const float2 y1 = gemm_act2<kAct>(ffma2(fadd2(make_float2(x.z, x.w), b1), make_float2(scale.z, scale.w), r1));
         if (col_in && row0 + 8 * i < row_end)
           *reinterpret_cast<uint2*>(static_cast<T*>(p.y) + static_cast<int64_t>(row0 + 8 * i) * p.ldy + col) =
               make_uint2(gemm_pack2<T>(y0.x, y0.y), gemm_pack2<T>(y1.x, y1.y));

@@ -33,7 +33,7 @@ struct RelTermsParams {
   int batch, heads, side;
   int parts;                 // CTAs per grid row
   int tables_wide, out_wide; // both tables / results are 16-byte aligned (else 4-byte)
-  uint32_t magic_heads;      // ceil(2^32 / heads)
+  uint32_t magic_heads;      // floor(2^32 / heads) + 1
   int tiles;                 // by lines: tiles of 128 rows at a time
   uint32_t* status;
   int early_tables;          // the tables were complete before the kernel in front of this one started: load them without waiting for that one
@@ -220,7 +220,8 @@ __global__ void __launch_bounds__(kRelLineThreads, 2) sam_rel_lines_kernel(const
   __shared__ uint64_t done, drain;  // a round's products have finished; abort path: all of this CTA's have
   __shared__ uint32_t tmem_base, abort;
   uint8_t* const table = smem_align_1024(rel_smem_raw);
-  const int side = p.side, n_cols = (side + 15) & ~15, stride_cols = n_cols <= 32 ? 32 : 64;
+  const int side = p.side, n_cols = (side + 15) & ~15;
+  constexpr int stride_cols = 64;
   uint8_t* const tiles = table + 64 * 128;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int line = blockIdx.x % side, which = (blockIdx.x / side) & 1, b = blockIdx.x / (2 * side);
