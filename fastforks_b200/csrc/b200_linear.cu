@@ -285,12 +285,12 @@ const void* rel_kernel_of(int tiles, bool rows) {
   }
 }
 // Which of the three kernels; us ([images, heads, side]) by rows, by tokens and by lines.
-// By lines (rows and addresses in whole 16-byte groups, heads to divide by) from side 48 on: [1,12,48] 7.6, 7.8, 7.2; [2,12,48] 10.8, 13.9,
-// 11.7; [4,12,48] 19.7, 24.8, 16.3; [1,12,64] 12.0, 10.0, 7.9; [4,12,64] 27.5, 30.4, 22.8; [16,16,56] 178, 195, 87; [16,16,64] 99.7, 127, 105. At side 40
-// where an SM has one line or at least four: [1,12,40] 6.5, 6.0, 6.0; [2,12,40] 7.9, 9.6, 9.3; [4,12,40] 12.3, 13.8, 12.9; [16,12,40] 39.5, 46, 35.1.
+// By lines (rows and addresses in whole 16-byte groups, heads to divide by) from side 48 on: [1,12,48] 7.6, 7.8, 7.1; [2,12,48] 10.8, 13.9,
+// 11.5; [4,12,48] 19.7, 24.8, 16.0; [1,12,64] 12.0, 10.0, 7.6; [4,12,64] 27.5, 30.4, 22.5; [16,16,56] 178, 195, 87; [16,16,64] 99.7, 127, 105. At side 40
+// where an SM has one line or at least four: [1,12,40] 6.5, 6.0, 5.9; [2,12,40] 7.9, 9.6, 9.3; [4,12,40] 12.3, 13.8, 12.9; [16,12,40] 39.5, 46, 35.1.
 bool rel_by_lines(int side, long long lines, int sms) { return side >= 48 || (side >= 40 && (lines <= sms || lines >= 4LL * sms)); }
 // Two CTAs fit an SM's shared memory with six tiles at a time: one loads while the other holds the tensor memory. us, eight at a
-// time and the fewest even shares of at most six: [2,16,56] 17.4 and 15.1, [4,16,64] 37.3 and 31.0, [8,16,64] 66.7 and 54.7; at a line per SM there is
+// time and the fewest even shares of at most six: [2,16,56] 17.4 and 14.6, [4,16,64] 37.3 and 30.1, [8,16,64] 66.7 and 53.6; at a line per SM there is
 // nothing to overlap, [1,16,64] 9.5 and 10.6.
 int rel_line_tiles(int tiles, long long lines, int sms) {
   const int most = lines <= sms ? kRelLineTiles : 6, passes = (tiles + most - 1) / most;

@@ -235,8 +235,8 @@ __global__ void __launch_bounds__(kRelLineThreads, 2) sam_rel_lines_kernel(const
   }
   // Chunk c of a 128-byte row, from the halves of two chunks of `src`: a product's 16 values are those the kernel above takes together,
   // the first four of chunks 0 to 3, then their last four, then those of chunks 4 to 7, and the two kernels give the same bits. (By
-  // whole chunks, some 4 in 10000 values were the other neighbour.) us, whole chunks -> halves: [1,12,64] 7.65 -> 7.74,
-  // [4,12,64] 21.8 -> 22.7, [4,16,56] 33.3 -> 34.0.
+  // whole chunks, some 4 in 10000 values were the other neighbour.) us, whole chunks -> halves: [1,12,64] 7.65 -> 7.6,
+  // [4,12,64] 21.8 -> 22.5, [8,12,64] 40.8 -> 40.9.
   const auto stage = [](uint8_t* to, int row, int c, const void* src, bool valid) {
 #pragma unroll
     for (int e = 0; e < 2; ++e)
