@@ -30,13 +30,15 @@ if TYPE_CHECKING:
 
 LIBRARY = "b200attn"
 PACKAGE_DIR = Path(__file__).resolve().parent
-SOURCES = (PACKAGE_DIR / "csrc" / "b200_attn.cu", PACKAGE_DIR / "csrc" / "b200_linear.cu", PACKAGE_DIR / "csrc" / "b200_encoder.cu")
+SOURCES = tuple(PACKAGE_DIR / "csrc" / name for name in ("b200_attn.cu", "b200_window.cu", "b200_linear.cu", "b200_encoder.cu"))
 HEADERS = (
     PACKAGE_DIR / "csrc" / "host_common.h",
     PACKAGE_DIR / "csrc" / "linear_host.h",
     PACKAGE_DIR / "csrc" / "sm100_ptx.cuh",
     PACKAGE_DIR / "csrc" / "attn_fwd_sm100.cuh",
     PACKAGE_DIR / "csrc" / "attn_small_sm100.cuh",
+    PACKAGE_DIR / "csrc" / "attn_window_sm100.cuh",
+    PACKAGE_DIR / "csrc" / "window_host.h",
     PACKAGE_DIR / "csrc" / "sam_rel_terms.cuh",
     PACKAGE_DIR / "csrc" / "rope_sm100.cuh",
     PACKAGE_DIR / "csrc" / "gemm_sm100.cuh",

@@ -18,6 +18,7 @@
 #include "attn_fwd_sm100.cuh"
 #include "attn_small_sm100.cuh"
 #include "host_common.h"
+#include "window_host.h"
 
 namespace {
 
@@ -635,6 +636,17 @@ int b200_attn_fwd(const B200AttnArgs* a, void* stream_ptr) {
     std::copy_n(a->v_stride, 3, prm.v_stride);
     std::copy_n(a->o_stride, 3, prm.o_stride);
     return a->dtype == B200_ATTN_F16 ? launch_small<__half, 1>(prm, a, *dev, stream) : launch_small<__nv_bfloat16, 1>(prm, a, *dev, stream);
+  }
+
+  // Few keys (attn_window_sm100.cuh): without a bias, with one in rows on 16 bytes, or with tables that the product with a one-hot
+  // operand adds exactly.
+  const bool in_tiles = bias_mode == kBiasDense && dense_bias_in_tiles(a);
+  if (bias_mode == kBiasNone || in_tiles || bias_mode == kBiasDecomposed) {
+    WindowCall call{bias_mode == kBiasNone ? kWindowCallPlain : in_tiles ? kWindowCallDense : kWindowCallRel, in_tiles && bias_shared_by_the_batch(a), 0, 0};
+    const bool exact = bias_mode != kBiasDecomposed ||
+                       (a->rel_dtype == a->dtype && inverse_is_exact(a->scale, a->rel_dtype, &call.rel_one));
+    if (bias_mode == kBiasDecomposed) call.rel_align = aligned_to(a);
+    if (exact && window_pays(a, call, dev->sms)) return launch_window(a, call, stream);
   }
 
   CUtensorMap mq, mk, mv, mo;

@@ -750,3 +750,45 @@ def test_small_calls_in_blocks_of_32_queries(b: int, h: int, nq: int, nk: int, d
     ref = torch.einsum("bhqk,bkhd->bqhd", logits.softmax(-1), v.float())
     assert_close(big[:, 1 : 1 + nq].float().cpu().numpy(), ref.cpu().numpy(), unit_scale=True, what=f"[{b},{h},{nq},{nk}] {dtype}")
     assert bool((big[:, 0] == 77.0).all()) and bool((big[:, -1] == 77.0).all())
+
+
+@pytest.mark.parametrize(("b", "h", "nq", "hw"), [(3, 70, 1, (1, 1)), (2, 90, 15, (3, 5)), (3, 70, 16, (4, 4)), (2, 99, 33, (1, 17)), (5, 67, 49, (7, 7)), (2, 120, 64, (8, 8)), (1, 200, 130, (9, 7)), (2, 70, 65, (13, 5)), (4, 60, 81, (9, 9)), (2, 100, 98, (7, 14)), (3, 50, 128, (8, 16)), (1, 481, 128, (16, 8)), (1, 482, 128, (16, 8)), (1, 300, 20, (3, 31))])  # fmt: skip
+@pytest.mark.parametrize("form", ["plain", "dense", "dense-per-image", "dense-other-type", "rel", "rel-odd-rows"])
+@pytest.mark.parametrize("dtype", ["fp16", "bf16"])
+def test_few_keys_in_blocks_of_64_queries(b: int, h: int, nq: int, hw: tuple[int, int], form: str, dtype: str) -> None:
+    """Key counts around the 16-key groups, query counts around the 16 rows of a warp and the 64 of a block, calls on either side of
+    the rule's line; views of wider tensors, a bias with broken last groups of eight, masked columns and rows without a key, tables
+    whose rows begin on four and on two bytes; against float32 on the same operands, and nothing written past the rows."""
+    t, nk = DTYPES[dtype], hw[0] * hw[1]
+    gen = torch.Generator(device="cuda").manual_seed(nq * 1000 + nk)
+    q = torch.randn(b, nq, 2, h, 64, generator=gen, device="cuda").to(t)[:, :, 0]
+    k, v = torch.randn(b, nk, 3, h, 64, generator=gen, device="cuda").to(t)[:, :, 1:].unbind(2)
+    logits, kw, dead = torch.einsum("bqhd,bkhd->bhqk", q.float(), k.float()) * 0.25, {}, None
+    if form.startswith("dense"):
+        bias_type = {torch.float16: torch.bfloat16, torch.bfloat16: torch.float16}[t] if form == "dense-other-type" else t
+        bias = torch.randn(b if form == "dense-per-image" else 1, h, nq, nk, generator=gen, device="cuda").to(bias_type)
+        bias[..., nk - nk // 5 :] = float("-inf")
+        if nq > 3:
+            bias[:, 1, 3] = float("-inf")
+            dead = (slice(None), 3, 1)
+        wide = torch.full((*bias.shape[:3], nk + 15), float("nan"), dtype=bias_type, device="cuda")[..., : nk + (-nk) % 8]
+        kw["bias"] = ff.tile_layout(wide[..., :nk].copy_(bias))
+        logits = logits + bias.float()
+    elif form.startswith("rel"):
+        pad = 1 if form == "rel-odd-rows" else 0
+        rel = [torch.randn(b, h, nq, side + pad, generator=gen, device="cuda").to(t)[..., :side] for side in hw]
+        if hw[0] > 1 and nq > 3:
+            rel[0][:, 0, :, 1] = float("-inf")
+            rel[1][:, 1, 3] = float("-inf")
+            dead = (slice(None), 3, 1)
+        kw["rel"] = tuple(rel)
+        logits = logits + (rel[0].float()[..., :, None] + rel[1].float()[..., None, :]).reshape(b, h, nq, nk)
+    big = torch.full((b, nq + 2, h, 64), 77.0, dtype=t, device="cuda")
+    ff.attention(q, k, v, scale=0.25, layout="bnhd", out=big[:, 1 : 1 + nq], **kw)
+    ref = torch.einsum("bhqk,bkhd->bqhd", logits.softmax(-1), v.float())
+    got = big[:, 1 : 1 + nq].float()
+    if dead is not None:  # a row without a key is NaN, as its softmax is
+        assert bool(got[dead].isnan().all()) and bool(ref[dead].isnan().all())
+        got[dead] = ref[dead] = 0.0
+    assert_close(got.cpu().numpy(), ref.cpu().numpy(), unit_scale=True, what=f"[{b},{h},{nq},{nk}] {form} {dtype}")
+    assert bool((big[:, 0] == 77.0).all()) and bool((big[:, -1] == 77.0).all())
