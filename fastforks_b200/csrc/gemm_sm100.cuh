@@ -23,6 +23,7 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
+#include <cstddef>
 #include <type_traits>
 
 #include "sm100_ptx.cuh"
@@ -143,6 +144,8 @@ struct PairSmem {
   uint32_t tmem_base;
   uint32_t abort;
 };
+constexpr int kPairBarriers = 2 * kPairMaxStages + 2 + 2 + 16 + 1;
+static_assert(offsetof(PairSmem, drain) == offsetof(PairSmem, full) + (kPairBarriers - 1) * sizeof(uint64_t), "the set-up walks the barriers as one array");
 static_assert(sizeof(PairSmem) + 1024 <= 227 * 1024, "shared memory of one CTA");
 
 struct GemmItem {
@@ -176,7 +179,7 @@ __device__ __forceinline__ GemmItem item_at(const GemmParams& p, int item, int o
 // Bounded by the L2 -> SM operand traffic and, above about 1.4 PFLOP/s sustained, the power cap. ACT and FORM are template
 // parameters: decided at run time, the branches alone cost 400 clocks per piece.
 // A residual without a scale (ViT-B, SAM) has a form of its own: two shuffles less per pair of columns, [4096,768,768] 9.3 -> 9.0 us,
-// [4096,768,3072] 20.8 -> 20.3.
+// [4096,768,3072] 20.8 -> 20.3. Sixteen epilogue warps with a piece each instead of eight with two: [4096,3072,768] 16.6 -> 17.5.
 enum : int { kPairPlain = 0, kPairResidual = 1, kPairScaled = 2 };  // ... ; a residual; a scale, and a residual or none
 template <typename T, int ACT, int FORM>
 __global__ void __launch_bounds__(kPairThreads, 1)
@@ -189,36 +192,39 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant
   const int rank = static_cast<int>(cluster_cta_rank());  // 0: the leader, rows 0..127 of the tile
   constexpr bool swiglu = ACT == kActSwiGlu, FULL = FORM != kPairPlain;
 
-  if (threadIdx.x == 0) {
-    for (int i = 0; i < kPairMaxStages; ++i) {
-      mbar_init(&sm.full[i], 1);
-      mbar_init(&sm.empty[i], 1);
-    }
-    for (int i = 0; i < 2; ++i) {
-      mbar_init(&sm.acc_full[i], 1);
-      mbar_init(&sm.acc_empty[i], 16);
-    }
-    for (int i = 0; i < 16; ++i) mbar_init(&sm.res_full[0][0] + i, 1);
-    mbar_init(&sm.drain, 1);
-    sm.abort = 0;
+  // Set-up. The loader goes on as soon as both CTAs' barriers exist, the other warps once tensor memory has been allocated too.
+  // Neither this hand-over, nor that of an accumulator, nor the one at the end passes data through memory: relaxed, without the
+  // wait for a thread's own traffic that a release brings, they take some 100 clocks instead of 1000. us of a launch, before and
+  // with both: [4096,768,768] 9.2 and 8.0, [4096,2304,768] 13.9 and 12.6, [4096,3072,768] with erf GELU 22.4 and 19.6,
+  // [1370,1536,384] 7.3 and 5.9.
+  if (warp == 0) {
+    uint64_t* const first = &sm.full[0];  // the barriers lie one after another
+    for (int i = lane; i < kPairBarriers; i += 32) mbar_init(first + i, first + i == &sm.acc_empty[0] || first + i == &sm.acc_empty[1] ? 16 : 1);
+    if (lane == 0) sm.abort = 0;
     mbar_init_fence();
+    __syncwarp();
   }
-  if (warp == 1) {
-    tmem_alloc_pair(&sm.tmem_base, 512);
-    tmem_relinquish_pair();
+  cluster_arrive_relaxed();
+  if (warp == 0) {
+    named_barrier_arrive(1, kPairThreads);
+    if (lane == 0) {
+      tma_prefetch_desc(&tm_x);
+      tma_prefetch_desc(&tm_w);
+      tma_prefetch_desc(&tm_y);
+      if (FULL && p.res != nullptr) tma_prefetch_desc(&tm_res);
+    }
+    __syncwarp();
+  } else {
+    if (warp == 1) {
+      tmem_alloc_pair(&sm.tmem_base, 512);
+      tmem_relinquish_pair();
+    }
+    tc_fence_before_sync();
+    named_barrier_sync(1, kPairThreads);
+    tc_fence_after_sync();
   }
-  if (warp == 0 && lane == 0) {
-    tma_prefetch_desc(&tm_x);
-    tma_prefetch_desc(&tm_w);
-    tma_prefetch_desc(&tm_y);
-    if (FULL && p.res != nullptr) tma_prefetch_desc(&tm_res);
-  }
-  tc_fence_before_sync();
-  __syncthreads();
-  cluster_arrive();  // the other CTA's barriers exist before anything of this one reaches for them
-  cluster_wait();
-  tc_fence_after_sync();
-  const uint32_t tmem = sm.tmem_base;
+  cluster_wait();  // the other CTA's barriers exist before anything of this one reaches for them
+  const uint32_t tmem = sm.tmem_base;  // (not the loader's)
   volatile uint32_t* abort_flag = &sm.abort;
   const int items = p.whole_tiles + (p.tiles_m * p.tiles_n - p.whole_tiles) * p.tail_parts;
   const int first_tile = blockIdx.x >> 1, tile_step = gridDim.x >> 1;
@@ -348,6 +354,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant
       const int pieces = swiglu ? 2 : t.bn / 64;
       // What the epilogue needs besides the accumulator is asked for before the wait for it: the residual of this warp's
       // two pieces, one per buffer, and bias and scale.
+      // The first tile's residual stands back (for a while) until the ring's first loads are in, which it held up. With this and the
+      // waits below where they are: [4096,768,768] 8.0 -> 7.7, [4096,768,3072] 16.5 -> 16.0.
+      if (it == 0 && has_res)
+        for (int polls = 0; polls < 32 && !mbar_test_wait(&sm.empty[0], 0); ++polls) {}
       if (has_res && lane == 0) {
         tma_store_wait_read<0>();  // the stores of the tile before have read both buffers
         for (int i = 0; i < 2; ++i) {
@@ -371,6 +381,16 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant
           if (p.scale != nullptr) scale2[i] = __ldg(reinterpret_cast<const float2*>(p.scale + c));
         }
       }
+      // The residual has landed long before the accumulator is finished: its waits cost nothing here, some 350 clocks each behind that.
+      if (has_res) {
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+          if (part + 2 * i < pieces && inside(row0, col0 + (part + 2 * i) * 64)) {
+            ok = ok && __all_sync(0xffffffffu, mbar_wait(&sm.res_full[e][i], loads[i] & 1, abort_flag)) != 0;
+            loads[i] += ok ? 1 : 0;
+          }
+        if (!ok) break;
+      }
       if (!__all_sync(0xffffffffu, mbar_wait(&sm.acc_full[it & 1], (it >> 1) & 1, abort_flag))) {
         ok = false;
         break;
@@ -386,19 +406,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant
         const int buf = c >> 1;
         const int col = col0 + c * 64;
         const bool here = inside(row0, col);
-        if (has_res) {
-          if (here) {
-            if (!__all_sync(0xffffffffu, mbar_wait(&sm.res_full[e][buf], loads[buf] & 1, abort_flag))) {
-              ok = false;
-              break;
-            }
-            ++loads[buf];
-          }
-        } else {
-          if (lane == 0) {  // the store that used this buffer last has read it
-            if (part + 2 < pieces) tma_store_wait_read<1>();
-            else tma_store_wait_read<0>();
-          }
+        if (!has_res && lane == 0) {  // the store that used this buffer last has read it
+          if (part + 2 < pieces) tma_store_wait_read<1>();
+          else tma_store_wait_read<0>();
         }
         __syncwarp();
         if (here) {
@@ -468,7 +478,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant
 
   tc_fence_before_sync();
   __syncthreads();
-  cluster_arrive();  // neither CTA goes while the other may still signal its barriers or multiply into its tensor memory
+  cluster_arrive_relaxed();  // neither CTA goes while the other may still signal its barriers or multiply into its tensor memory
   cluster_wait();
   if (warp == 1) {
     tc_fence_after_sync();
