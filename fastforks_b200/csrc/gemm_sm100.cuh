@@ -487,8 +487,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant
 }
 
 // ---- split kernel ---------------------------------------------------------------------------------------------
-constexpr int kSplitThreads = 192;  // warp 0 loader, warp 1 MMA, warps 2..5 epilogue
-constexpr int kSplitStages = 6;     // a round trip to L2 covers some four stages
+constexpr int kSplitEpilogueThreads = 256;
+constexpr int kSplitThreads = 64 + kSplitEpilogueThreads;  // warp 0 loader, warp 1 MMA, warps 2..9 epilogue
+// A round trip to L2 covers some four stages; with six a CTA left no room on its SM for one of the kernels in front or behind.
+constexpr int kSplitStages = 4;
 constexpr int kSplitBN = 64;
 
 template <int S>
@@ -540,7 +542,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
-  if constexpr (S > 1) cluster_arrive();  // this CTA runs; waited for before anybody writes into its receive area
+  if constexpr (S > 1) cluster_arrive_relaxed();  // this CTA runs; waited for before anybody writes into its receive area
   const uint32_t tmem = sm.tmem_base;
   volatile uint32_t* abort_flag = &sm.abort;
 
@@ -615,9 +617,9 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
     __syncwarp();
   }
 
-  // Epilogue thread: four columns (the same for all its items) of every eighth row. What the epilogue needs besides the
+  // Epilogue thread: four columns (the same for all its items) of every sixteenth row. What the epilogue needs besides the
   // sums is in flight while the products run.
-  constexpr int kItems = (Smem::kRows * (kSplitBN / 4) + 127) / 128;
+  constexpr int kItems = (Smem::kRows * (kSplitBN / 4) + kSplitEpilogueThreads - 1) / kSplitEpilogueThreads, kRowStep = kSplitEpilogueThreads / 16;
   const int et = threadIdx.x - 64, c4 = et & 15;
   const int first_row = rank * Smem::kRows, end_row = min(min(first_row + Smem::kRows, 128), p.m - tm * 128);  // in the tile
   const int row0 = tm * 128 + first_row + (et >> 4), row_end = tm * 128 + end_row, col = tn * kSplitBN + c4 * 4;
@@ -631,8 +633,8 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
 #pragma unroll
     for (int i = 0; i < kItems; ++i) {
       res[i] = make_uint2(0, 0);
-      if (p.res != nullptr && col_in && row0 + 8 * i < row_end)
-        res[i] = *reinterpret_cast<const uint2*>(static_cast<const T*>(p.res) + static_cast<int64_t>(row0 + 8 * i) * p.lres + col);
+      if (p.res != nullptr && col_in && row0 + kRowStep * i < row_end)
+        res[i] = *reinterpret_cast<const uint2*>(static_cast<const T*>(p.res) + static_cast<int64_t>(row0 + kRowStep * i) * p.lres + col);
     }
     if (!__all_sync(0xffffffffu, mbar_wait(&sm.acc_full, 0, abort_flag)) && lane == 0 &&
         atomicExch(const_cast<uint32_t*>(abort_flag), 1u) == 0)
@@ -641,13 +643,13 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
   }
   if constexpr (S > 1) cluster_wait();
   if (warp >= 2) {
-    const int row = (warp & 3) * 32 + lane;  // this thread's row of the tile
-    float v[kSplitBN];
-    tmem_ld_x64(tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16), reinterpret_cast<uint32_t*>(v));
-    uint32_t dst = smem_u32(&sm.recv[rank][0][row % Smem::kRows]);
+    const int row = (warp & 3) * 32 + lane, half = (warp - 2) >> 2;  // this thread's row of the tile, its 32 columns
+    float v[kSplitBN / 2];
+    tmem_ld_x32(tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16) + half * (kSplitBN / 2), reinterpret_cast<uint32_t*>(v));
+    uint32_t dst = smem_u32(&sm.recv[rank][half * (kSplitBN / 8)][row % Smem::kRows]);
     if constexpr (S > 1) dst = cluster_map(dst, row / Smem::kRows);
 #pragma unroll
-    for (int c4 = 0; c4 < kSplitBN / 4; ++c4)
+    for (int c4 = 0; c4 < kSplitBN / 8; ++c4)
       st_cluster_v4(dst + c4 * (Smem::kStride * 16), make_float4(v[4 * c4], v[4 * c4 + 1], v[4 * c4 + 2], v[4 * c4 + 3]));
   }
   tc_fence_before_sync();
@@ -663,7 +665,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
       constexpr int kAct = decltype(act_tag)::value;
 #pragma unroll
       for (int i = 0; i < kItems; ++i) {
-        const int r = min((et >> 4) + 8 * i, Smem::kRows - 1);  // past the last row: read what is there, write nothing
+        const int r = min((et >> 4) + kRowStep * i, Smem::kRows - 1);  // past the last row: read what is there, write nothing
         float4 x = sm.recv[0][c4][r];
 #pragma unroll
         for (int s = 1; s < S; ++s) {
@@ -673,8 +675,8 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
         const float2 r0 = gemm_unpack2<T>(res[i].x), r1 = gemm_unpack2<T>(res[i].y);
         const float2 y0 = gemm_act2<kAct>(ffma2(fadd2(make_float2(x.x, x.y), b0), make_float2(scale.x, scale.y), r0));
         const float2 y1 = gemm_act2<kAct>(ffma2(fadd2(make_float2(x.z, x.w), b1), make_float2(scale.z, scale.w), r1));
-        if (col_in && row0 + 8 * i < row_end)
-          *reinterpret_cast<uint2*>(static_cast<T*>(p.y) + static_cast<int64_t>(row0 + 8 * i) * p.ldy + col) =
+        if (col_in && row0 + kRowStep * i < row_end)
+          *reinterpret_cast<uint2*>(static_cast<T*>(p.y) + static_cast<int64_t>(row0 + kRowStep * i) * p.ldy + col) =
               make_uint2(gemm_pack2<T>(y0.x, y0.y), gemm_pack2<T>(y1.x, y1.y));
       }
     });
