@@ -5,8 +5,11 @@
 // all its keys, a warp 16 of the queries: mma.sync on operands of 16 rows, the whole row of logits in registers, no running maximum.
 // Bound by latency: load, two short products, store. Nothing is overlapped inside a CTA; the CTAs of an SM (window_ctas) cover each
 // other. (Persistent CTAs with K and V in a TMA ring and 32 queries per warp held too few warps for that: [8,192,49] 20 us.)
-// us per launch in CUDA graphs, persistent kernel and this one: [8,192,49] with a dense bias 25.0 and 11.3, without 18.1 and 8.8,
-// [64,16,64] with a dense bias 17.0 and 8.3, [64,12,64] 10.4 and 5.5, [100,12,36] with 6 x 6 tables 24.4 and 8.1.
+// us per launch in CUDA graphs, persistent kernel and this one: [8,192,49] with a dense bias 25.0 and 10.5, without 18.1 and 8.8,
+// [64,16,64] with a dense bias 17.0 and 8.3, [64,12,64] 10.4 and 5.7, [100,12,36] with 6 x 6 tables 24.4 and 8.0.
+// Issue slots count next: 870 instructions a warp took 4.6 of [8,192,49]'s 11.5 us. The bias comes in pairs of columns as the logits lie
+// (11.5 -> 10.9; in rows of 16 bytes turned by shuffles before), the block number is taken apart by multiplies (-> 10.5). Outputs in pairs
+// instead of 16 bytes turned by shuffles: 12.1. Prefetching the next round's rows into L2: 11.0.
 #pragma once
 
 #include <cuda_bf16.h>
@@ -25,9 +28,9 @@ constexpr int kWindowMaxKeys = 128;
 constexpr int kWindowMaxRel = 32;  // values of a decomposed bias per row (rel_kh + rel_kw)
 constexpr int kWindowRows = 64;    // queries per CTA
 constexpr int kWindowThreads = 128;
-// CTAs per SM, by registers: 80 a thread hold 64 logits of two rows, 128 hold 128. us [8,192,49] / [64,192,49] with a bias at 5, 6 and 8:
-// 11.4 / 84.8, 11.2 / 81.6, 12.0 / 79.6.
-constexpr int window_ctas(int groups) { return groups <= 4 ? 6 : 4; }
+// CTAs per SM, by registers: 72 a thread hold 64 logits of two rows, 128 hold 128. us at 6 and 7: [8,192,49] / [64,192,49] with a bias
+// 10.5 / 76.6 and 10.5 / 74.8, [8,64,64] 7.1 and 5.8, [100,12,36] with tables 8.4 and 8.0, but [64,12,64] without either 5.7 and 6.3.
+constexpr int window_ctas(int groups, int bias) { return groups > 4 ? 4 : bias == kWindowPlain ? 6 : 7; }
 
 struct WindowParams {
   const void* q;
@@ -37,6 +40,7 @@ struct WindowParams {
   int64_t q_stride[3], k_stride[3], v_stride[3], o_stride[3];  // batch, token, head; elements
   int batch, heads, q_tokens, kv_tokens;
   int q_blocks;        // ceil(q_tokens / 64)
+  uint64_t magic_blocks, magic_inner;  // fast_div constants of q_blocks and of the index that runs fastest
   float scale_log2, scale;
   int batch_fastest;   // heads are numbered with the batch index running fastest (a bias every image shares is then read side by side)
   const void* bias;    // dense form
@@ -73,19 +77,6 @@ __device__ __forceinline__ uint32_t onehot_chunk(uint32_t base, int row, int chu
 
 // Loads through L2 only (the kernel in front may have written the data while this one was already on the SM), nothing where !valid.
 // Written as predicated instructions, so that a row's loads are all in flight before the first is used.
-__device__ __forceinline__ uint4 load_v4_if(const uint16_t* src, bool valid) {
-  uint4 v;
-  asm volatile(
-      "{\n\t"
-      ".reg .pred p;\n\t"
-      "setp.ne.s32 p, %5, 0;\n\t"
-      "mov.b32 %0, 0;\n\tmov.b32 %1, 0;\n\tmov.b32 %2, 0;\n\tmov.b32 %3, 0;\n\t"
-      "@p ld.global.cg.v4.u32 {%0, %1, %2, %3}, [%4];\n\t"
-      "}\n"
-      : "=&r"(v.x), "=&r"(v.y), "=&r"(v.z), "=&r"(v.w)
-      : "l"(src), "r"(valid ? 1 : 0));
-  return v;
-}
 __device__ __forceinline__ uint32_t load_u32_if(const uint16_t* src, bool valid) {
   uint32_t v;
   asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.s32 p, %2, 0;\n\tmov.b32 %0, 0;\n\t@p ld.global.cg.u32 %0, [%1];\n\t}\n" : "=&r"(v) : "l"(src), "r"(valid ? 1 : 0));
@@ -109,7 +100,7 @@ __device__ __forceinline__ void window_load(uint32_t smem, const T* rows, int64_
 
 // GROUPS = ceil(kv_tokens / 16). Grid: q_blocks * batch * heads.
 template <typename T, int BIAS, int GROUPS>
-__global__ void __launch_bounds__(kWindowThreads, window_ctas(GROUPS)) attn_window_kernel(const WindowParams p) {
+__global__ void __launch_bounds__(kWindowThreads, window_ctas(GROUPS, BIAS)) attn_window_kernel(const WindowParams p) {
   __shared__ __align__(128) uint8_t smem_q[kWindowRows * 128];
   __shared__ __align__(128) uint8_t smem_k[GROUPS * 16 * 128];
   __shared__ __align__(128) uint8_t smem_v[GROUPS * 16 * 128];
@@ -118,8 +109,8 @@ __global__ void __launch_bounds__(kWindowThreads, window_ctas(GROUPS)) attn_wind
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
   constexpr float kNone = -__builtin_huge_valf();
 
-  const int item = static_cast<int>(blockIdx.x) / p.q_blocks, row0 = (static_cast<int>(blockIdx.x) - item * p.q_blocks) * kWindowRows;
-  const int inner = p.batch_fastest ? p.batch : p.heads, outer = item / inner, rest = item - outer * inner;
+  const int item = fast_div(static_cast<int>(blockIdx.x), p.magic_blocks), row0 = (static_cast<int>(blockIdx.x) - item * p.q_blocks) * kWindowRows;
+  const int inner = p.batch_fastest ? p.batch : p.heads, outer = fast_div(item, p.magic_inner), rest = item - outer * inner;
   const int b = p.batch_fastest ? rest : outer, h = p.batch_fastest ? outer : rest;
   const int my_row0 = row0 + warp * 16;
   auto row_of = [&](int r) { return my_row0 + 8 * r + g; };
@@ -146,31 +137,19 @@ __global__ void __launch_bounds__(kWindowThreads, window_ctas(GROUPS)) attn_wind
   window_load<T, GROUPS * 16>(sv, static_cast<const T*>(p.v) + b * p.v_stride[0] + h * p.v_stride[2], p.v_stride[1], p.kv_tokens);
   cp_async_commit();
 
-  // The rows' bias: in flight with the operands.
-  constexpr int kHalves = (GROUPS + 1) / 2;  // 32 keys each: a lane loads eight of them per row
-  [[maybe_unused]] uint32_t bw[2][kHalves][4];
+  // The rows' bias, in flight with the operands: a lane loads the pairs of columns whose logits it will hold. A pair never reaches behind
+  // the row's end.
+  [[maybe_unused]] uint32_t bw[2][2 * GROUPS];
   if constexpr (BIAS == kWindowDense) {
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
       const bool valid = row_of(r) < p.q_tokens;
-      const uint16_t* src = static_cast<const uint16_t*>(p.bias) + b * p.bias_stride[0] + h * p.bias_stride[1] + (valid ? row_of(r) : 0) * p.bias_stride[2];
+      const uint16_t* src = static_cast<const uint16_t*>(p.bias) + b * p.bias_stride[0] + h * p.bias_stride[1] + (valid ? row_of(r) : 0) * p.bias_stride[2] + 2 * t;
 #pragma unroll
-      for (int i = 0; i < kHalves; ++i) {
-        const uint4 v = load_v4_if(src + 32 * i + 8 * t, valid && 32 * i + 8 * t + 8 <= p.kv_tokens);
-        bw[r][i][0] = v.x; bw[r][i][1] = v.y; bw[r][i][2] = v.z; bw[r][i][3] = v.w;
-      }
-      // The row's last, broken group of eight: pair by pair, so that nothing is read behind the row's end.
-      if ((p.kv_tokens & 7) != 0) {
-        const int at = p.kv_tokens & ~7, left = p.kv_tokens & 7;
+      for (int j = 0; j < 2 * GROUPS; ++j) bw[r][j] = load_u32_if(src + 8 * j, valid && 8 * j + 2 * t + 1 < p.kv_tokens);
+      if ((p.kv_tokens & 1) != 0) {  // the last key's half of its pair
 #pragma unroll
-        for (int i = 0; i < kHalves; ++i) {
-          const bool mine = valid && 32 * i + 8 * t == at;
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            bw[r][i][e] |= load_u32_if(src + at + 2 * e, mine && 2 * e + 1 < left);
-            bw[r][i][e] |= load_u16_if(src + at + 2 * e, mine && 2 * e + 1 == left);
-          }
-        }
+        for (int j = 2 * GROUPS - 2; j < 2 * GROUPS; ++j) bw[r][j] |= load_u16_if(src + 8 * j, valid && 8 * j + 2 * t + 1 == p.kv_tokens);
       }
     }
   }
@@ -243,10 +222,8 @@ __global__ void __launch_bounds__(kWindowThreads, window_ctas(GROUPS)) attn_wind
     for (int r = 0; r < 2; ++r) {
       if constexpr (BIAS == kWindowDense) {  // natural units, s * scale + bias; log2(e) rides on the FMA in front of the exponential
 #pragma unroll
-        for (int i = 0; i < kHalves; ++i) quad_transpose(bw[r][i], lane);
-#pragma unroll
         for (int j = 0; j < 2 * GROUPS; ++j) {
-          const float2 x = ffma2(make_float2(s[j][2 * r], s[j][2 * r + 1]), make_float2(p.scale, p.scale), unpack2(bw[r][j / 4][j % 4], p.bias_half != 0));
+          const float2 x = ffma2(make_float2(s[j][2 * r], s[j][2 * r + 1]), make_float2(p.scale, p.scale), unpack2(bw[r][j], p.bias_half != 0));
           s[j][2 * r] = x.x;
           s[j][2 * r + 1] = x.y;
         }

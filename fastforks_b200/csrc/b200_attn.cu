@@ -42,9 +42,6 @@ __global__ void wait_limit_selftest_kernel(uint64_t limit_ns, uint32_t* status) 
   if (!done && threadIdx.x == 0) atomicOr(status, 8u);
 }
 
-// ceil(2^64 / d) for the kernel's fast_div; 0 stands for d <= 1.
-uint64_t div_magic(int d) { return d <= 1 ? 0 : ~uint64_t(0) / static_cast<uint64_t>(d) + 1; }
-
 thread_local char tl_error[512] = "";
 DeviceState g_devices[kMaxDevices];
 std::mutex g_devices_mutex;

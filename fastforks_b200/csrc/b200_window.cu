@@ -57,6 +57,8 @@ int launch_window(const B200AttnArgs* a, const WindowCall& call, cudaStream_t st
   prm.q_tokens = a->q_tokens;
   prm.kv_tokens = a->kv_tokens;
   prm.q_blocks = (a->q_tokens + kWindowRows - 1) / kWindowRows;
+  prm.magic_blocks = div_magic(prm.q_blocks);
+  prm.magic_inner = div_magic(call.batch_fastest ? a->batch : a->heads);
   prm.scale = a->scale;
   prm.scale_log2 = a->scale * kLog2e;
   prm.batch_fastest = call.batch_fastest ? 1 : 0;

@@ -21,6 +21,9 @@ using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t
                                    CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 EncodeTiledFn encode_tiled_fn();
 
+// ceil(2^64 / d) for the attention kernels' fast_div; 0 stands for d <= 1.
+inline uint64_t div_magic(int d) { return d <= 1 ? 0 : ~uint64_t(0) / static_cast<uint64_t>(d) + 1; }
+
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
 // Checks a [batch, tokens, heads, 64] view's pointer and strides against what the kernels take.
