@@ -261,7 +261,6 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant
       }
     }
     grid_dependency_wait();
-    grid_launch_dependents();
     for (int tile = first_tile; tile < items && ok; tile += tile_step) {
       const GemmItem t = item_at(p, tile, out_cols);
       for (int kb = 0; kb < k_blocks; ++kb, ++g) {
@@ -290,6 +289,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant
     __syncwarp();
   } else if (warp == 1) {
     // ======================= MMA issuer (leader only) =================================================
+    // The next kernel may start from here on: this warp's CTA holds its tensor memory, which the loader does not wait for.
+    grid_dependency_wait();
+    grid_launch_dependents();
     if (rank == 0) {
       constexpr uint32_t fmt = std::is_same<T, __half>::value ? UMMA_F16 : UMMA_BF16;
       const uint32_t idesc_whole = umma_idesc_f16(fmt, 256, p.bn, 0, 0), idesc_tail = umma_idesc_f16(fmt, 256, p.tail_bn, 0, 0);
