@@ -108,8 +108,13 @@ enum : int { kItemWhole = 0, kItemPartial = 1, kItemOwner = 2 };
 // tensor pipe above some 96 values per row and by the softmax step below. us, additions by the softmax warps -> here
 // ([B,H,N]): [4,12,1024] 271 -> 40, [2,12,2304] 853 -> 72, [10,12,400] 170 -> 26, [100,12,36] 113 -> 41; [1,12,4096], whose
 // 64-wide tables had a form of their own (kBiasDecomposed64), 101 -> 99. The 14 x 14 form stays ahead: [400,12,196] 183 against 216.
+// kBiasDecomposedWide is that form for 57 and more grid rows: of E's columns for rel_h a key tile has ones in a few neighbours only, and the
+// 16-value steps without one are left out (three of SAM's eight at 64 x 64, a quarter of the step's products). us: [4,12,4096] 361 -> 345,
+// [1,12,4096] 96.5 -> 95.5 (in a long loop, at the power cap, with the producer 108.4 -> 104.0). Narrower grids had nothing from it, and lost
+// up to 8 % by the test in front of each product ([4,16,1600] 84 -> 91, [2,12,3136] 114 -> 114): a form of its own.
 // kBiasDecomposed64 is left for 64-wide tables with more than 64 rows or a scale whose inverse is no power of two.
-enum : int { kBiasNone = 0, kBiasDense = 1, kBiasDecomposed = 2, kBiasDecomposed64 = 3, kBiasDecomposed14 = 4, kBiasDenseTiles = 5, kBiasDecomposedMma = 6 };
+enum : int { kBiasNone = 0, kBiasDense = 1, kBiasDecomposed = 2, kBiasDecomposed64 = 3, kBiasDecomposed14 = 4, kBiasDenseTiles = 5, kBiasDecomposedMma = 6, kBiasDecomposedWide = 7 };
+constexpr bool is_rel_mma(int bias) { return bias == kBiasDecomposedMma || bias == kBiasDecomposedWide; }
 constexpr int kMaxRelChunks = 16;   // kBiasDecomposedMma: groups of eight values per row of R and E
 constexpr int kRelStageWords = 33;  // per-row staging of rel_h | rel_w in shared memory: up to 32 values, odd stride
 
@@ -206,6 +211,7 @@ struct alignas(1024) AttnSmemT {
   uint64_t merge_go[2];      // the owner's first thread has looked at the item's counter and set `merge_ready` (1)
   uint32_t merge_ready[2];   // every later part of the owner's item is counted: the owner folds them in itself
   uint32_t o_store[2][2];    // [t][item parity] what the hand-over o_staged[t] of a cut item means: 1 a staged tile, 2 a part in the workspace
+  uint32_t rel_needed;        // kBiasDecomposedWide: the 16-value steps of E (a bit each) with a one in them; written with E
   uint32_t turn_count[2][4];  // flag form of the token: releases so far by warp w of warpgroup t (see kFlagTurn)
   uint32_t tmem_base;
   uint32_t abort;
@@ -227,7 +233,7 @@ using AttnSmem = AttnSmemT<kStages, 2, kRoomRelStage>;
 using AttnSmemDense = AttnSmemT<kStagesDense, 2, kRoomBiasTiles>;
 using AttnSmemRelMma = AttnSmemT<kStagesDense, 1, kRoomRelMma>;
 template <int BIAS>
-using AttnSmemOf = std::conditional_t<BIAS == kBiasDenseTiles, AttnSmemDense, std::conditional_t<BIAS == kBiasDecomposedMma, AttnSmemRelMma, AttnSmem>>;
+using AttnSmemOf = std::conditional_t<BIAS == kBiasDenseTiles, AttnSmemDense, std::conditional_t<is_rel_mma(BIAS), AttnSmemRelMma, AttnSmem>>;
 // The set-up walks the barriers as one array and picks the arrival count by position.
 static_assert(offsetof(AttnSmem, merge_go) + sizeof(uint64_t[2]) == offsetof(AttnSmem, merge_ready) &&
                   offsetof(AttnSmem, o_free) + 2 * sizeof(uint64_t[2]) == offsetof(AttnSmem, o_staged) &&
@@ -649,7 +655,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   using Smem = AttnSmemOf<BIAS>;
   constexpr int kStagesK = Smem::kRing, kStagesV = Smem::kRing, kQBufs = Smem::kQBufs;
   constexpr int kKLead = Smem::kRing - 1;  // K tiles loaded ahead of V tiles: one less than the ring, or V waits for K to come free
-  constexpr bool kPlainLogits = BIAS == kBiasNone || BIAS == kBiasDecomposedMma;  // S is scaled in front of the exponential only
+  constexpr bool kPlainLogits = BIAS == kBiasNone || is_rel_mma(BIAS);  // S is scaled in front of the exponential only
   Smem& sm = *reinterpret_cast<Smem*>(smem_align_1024(smem_raw));
 
   const int warp = threadIdx.x >> 5;
@@ -674,7 +680,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
                         (bar >= &sm.s_free[0] && bar <= &sm.s_free[1]) ||
                         (bar >= &sm.p_full[0] && bar <= &sm.p_full[1]) || (bar >= &sm.l_full[0] && bar <= &sm.l_full[1]) || (bar >= &sm.o_free[0] && bar <= &sm.o_staged[1]);
       // with kBiasDecomposedMma a K tile is there when its TMA transaction and its E are
-      const bool two = (BIAS == kBiasDecomposedMma && bar >= &sm.k_full[0] && bar <= &sm.k_full[kStagesK - 1]) || (bar >= &sm.k_empty[0] && bar <= &sm.k_empty[kStagesK - 1]) ||
+      const bool two = (is_rel_mma(BIAS) && bar >= &sm.k_full[0] && bar <= &sm.k_full[kStagesK - 1]) || (bar >= &sm.k_empty[0] && bar <= &sm.k_empty[kStagesK - 1]) ||
                        (bar >= &sm.v_empty[0] && bar <= &sm.v_empty[kStagesV - 1]) ;
       mbar_init(bar, four ? 4 : two ? 2 : 1);
     }
@@ -684,7 +690,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   } else if (threadIdx.x == 32) {
     sm.work = cta_work(p, static_cast<int>(blockIdx.x), static_cast<int>(gridDim.x));
   }
-  if constexpr (BIAS == kBiasDecomposedMma) {  // E starts without a one
+  if constexpr (is_rel_mma(BIAS)) {  // E starts without a one
     uint4* e = reinterpret_cast<uint4*>(sm.e[0]);
     for (int i = threadIdx.x; i < 2 * kTileBytes / 16; i += kThreads) e[i] = make_uint4(0, 0, 0, 0);
     fence_proxy_async_smem();
@@ -718,7 +724,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     reg_dealloc<R::kHelperRegs>();
     if (warp == kLoaderWarp) {
       // ======================= loader =======================================================
-      if constexpr (BIAS == kBiasDecomposedMma) {
+      if constexpr (is_rel_mma(BIAS)) {
         // The whole warp: one lane issues the copies, and all write E, the grid coordinates of a tile's keys as one-hot
         // rows (rel_h's values, then rel_w's), which is released and reused with the K tile it belongs to: two buffers where
         // a row has up to 64 values, one of twice the size above. A lane moves the two ones of four keys. (By the MMA warp
@@ -800,6 +806,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
                     e_x[r] -= carry ? p.rel_kw : 0;
                     e_y[r] += carry ? 1 : 0;
                   }
+                }
+                if constexpr (BIAS == kBiasDecomposedWide) {
+                  const int first_y = min(__shfl_sync(0xffffffffu, e_y[0], 0), p.rel_kh - 1), last_y = min(__shfl_sync(0xffffffffu, e_y[3], 31), p.rel_kh - 1);
+                  if (lane == 0) *reinterpret_cast<volatile uint32_t*>(&sm.rel_needed) = ((2u << (last_y >> 4)) - (1u << (first_y >> 4))) | (~0u << (p.rel_chunks_h >> 1));
                 }
                 // Keys behind the last one get ones like the others: their columns of S are masked.
                 uint32_t at[4][2];
@@ -1004,7 +1014,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
 
         [[maybe_unused]] const uint32_t rel_fmt = (p.bias.dtype == 0 ? UMMA_F16 : UMMA_BF16) * ((1u << 7) | (1u << 10));
         [[maybe_unused]] uint64_t r_desc0 = 0, e_desc0 = 0;
-        if constexpr (BIAS == kBiasDecomposedMma) {
+        if constexpr (is_rel_mma(BIAS)) {
           r_desc0 = umma_smem_desc_sw128(smem_u32(sm.r[t][0]), 1024, 16);
           e_desc0 = umma_smem_desc_sw128(smem_u32(sm.e[0]), 1024, 16);
         }
@@ -1017,7 +1027,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           if (is_first(x) && !warp_wait(&sm.q_full[t][slot], (x.it / kQBufs) & 1)) return false;
           if (x.gs > 0 && !warp_wait(s_free, (x.gs - 1) & 1)) return false;  // S_t has been read
           if (!__all_sync(0xffffffffu, k_early || mbar_wait(&sm.k_full[x.ring.stage], x.ring.parity(), abort_flag))) return false;
-          if constexpr (BIAS == kBiasDecomposedMma) {
+          if constexpr (is_rel_mma(BIAS)) {
             if (is_first(x) && !warp_wait(&sm.r_full[t], x.it & 1)) return false;
           }
           tc_fence_after_sync();
@@ -1028,12 +1038,14 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
 #pragma unroll
             for (int kk = 0; kk < kHeadDim / 16; ++kk)  // 32 bytes of K per step inside the swizzle atom
               umma_ss(s_tm, a + 2 * kk, bd + 2 * kk, idesc, kk > 0 ? 1u : 0u);
-            if constexpr (BIAS == kBiasDecomposedMma) {
+            if constexpr (is_rel_mma(BIAS)) {
               const uint64_t e_desc = e_desc0 + (p.rel_steps <= 4 ? x.ring.stage * kStageStep : 0);  // two buffers of E, or one of twice the size
               const uint32_t idesc_re = (idesc & ~((7u << 7) | (7u << 10))) | rel_fmt;  // the tables' type, else the same
+              [[maybe_unused]] uint32_t needed = 0;
+              if constexpr (BIAS == kBiasDecomposedWide) needed = *reinterpret_cast<volatile uint32_t*>(&sm.rel_needed);
 #pragma unroll
               for (int kk = 0; kk < kMaxRelChunks / 2; ++kk)
-                if (kk < p.rel_steps)
+                if (kk < p.rel_steps && (BIAS != kBiasDecomposedWide || ((needed >> kk) & 1) != 0))
                   umma_ss(s_tm, r_desc0 + (kk / 4) * kStageStep + 2 * (kk % 4), e_desc + (kk / 4) * kStageStep + 2 * (kk % 4), idesc_re, 1u);
             }
             umma_commit(s_full);
@@ -1383,9 +1395,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       if constexpr (BIAS != kBiasNone) {
         const int qr = row_valid ? q_row : 0;
         bias_row = b * p.bias.sb + h * p.bias.sh + qr * p.bias.sn;
-        if constexpr (BIAS == kBiasDecomposed || BIAS == kBiasDecomposed64 || BIAS == kBiasDecomposed14 || BIAS == kBiasDecomposedMma)
+        if constexpr (BIAS == kBiasDecomposed || BIAS == kBiasDecomposed64 || BIAS == kBiasDecomposed14 || is_rel_mma(BIAS))
           bias2_row = b * p.bias2.sb + h * p.bias2.sh + qr * p.bias2.sn;
-        if constexpr (BIAS == kBiasDecomposedMma) {
+        if constexpr (is_rel_mma(BIAS)) {
           // The row's tables into R. The products that read the last item's R have finished: this thread waited for that
           // item's last S. (Bringing the rows in from inside the item's last step, or only into L1, was 1-25 % slower.)
           const uint32_t row = smem_u32(sm.r[t][0]) + row_in_tile * 128;

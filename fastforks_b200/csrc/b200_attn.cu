@@ -508,14 +508,14 @@ int launch(const AttnParams& planned, unsigned grid, DeviceState& dev, const CUt
 }
 
 // The short schedule exists for every bias form but the 64-wide one (its key counts are multiples of 64, where the
-// long schedule loses nothing worth a second set of kernels); the key-split form only for the long schedule (a
+// long schedule loses nothing worth a second set of kernels) and the one for many grid rows; the key-split form only for the long schedule (a
 // sequence of at most two key tiles is never split).
 template <typename T, int BIAS>
 int launch_sched(bool short_sched, const AttnParams& planned, unsigned grid, DeviceState& dev, const CUtensorMap& mq,
                  const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mo, const CUtensorMap& mb, cudaStream_t stream) {
   if (planned.chunked) return launch<T, BIAS, false, kListSplit>(planned, grid, dev, mq, mk, mv, mo, mb, stream);
   const bool twins = planned.twins > 0;
-  if constexpr (BIAS != kBiasDecomposed64) {
+  if constexpr (BIAS != kBiasDecomposed64 && BIAS != kBiasDecomposedWide) {
     if (short_sched && twins) return launch<T, BIAS, true, kListTwins>(planned, grid, dev, mq, mk, mv, mo, mb, stream);
     if (short_sched) return launch<T, BIAS, true, kListPlain>(planned, grid, dev, mq, mk, mv, mo, mb, stream);
   }
@@ -696,7 +696,7 @@ int b200_attn_fwd(const B200AttnArgs* a, void* stream_ptr) {
       prm.rel_chunks_w = chunks_w;
       prm.rel_steps = (chunks_h + chunks_w + 1) / 2;
       prm.rel_align = aligned;
-      bias_mode = kBiasDecomposedMma;
+      bias_mode = chunks_h >= 8 ? kBiasDecomposedWide : kBiasDecomposedMma;
     } else if (a->rel_kw == 64 && a->rel_kh % 8 == 0 && a->rel_dtype != B200_ATTN_F32 && rows16(a->rel_w, a->rel_w_stride) &&
         rows16(a->rel_h, a->rel_h_stride))
       bias_mode = kBiasDecomposed64;
@@ -730,6 +730,9 @@ int b200_attn_fwd(const B200AttnArgs* a, void* stream_ptr) {
     case kBiasDecomposed14:
       return f16 ? launch_sched<__half, kBiasDecomposed14>(short_sched, prm, grid, *dev, mq, mk, mv, mo, mb, stream)
                  : launch_sched<__nv_bfloat16, kBiasDecomposed14>(short_sched, prm, grid, *dev, mq, mk, mv, mo, mb, stream);
+    case kBiasDecomposedWide:
+      return f16 ? launch_sched<__half, kBiasDecomposedWide>(false, prm, grid, *dev, mq, mk, mv, mo, mb, stream)
+                 : launch_sched<__nv_bfloat16, kBiasDecomposedWide>(false, prm, grid, *dev, mq, mk, mv, mo, mb, stream);
     case kBiasDecomposedMma:
       return f16 ? launch_sched<__half, kBiasDecomposedMma>(short_sched, prm, grid, *dev, mq, mk, mv, mo, mb, stream)
                  : launch_sched<__nv_bfloat16, kBiasDecomposedMma>(short_sched, prm, grid, *dev, mq, mk, mv, mo, mb, stream);

@@ -33,7 +33,7 @@ int check_view(const char* name, const void* ptr, const int64_t s[3], int batch,
 // status word and which kernels already have their shared-memory opt-in (the opt-in is per device and per kernel).
 // The runtime calls behind these cost more than the rest of the host path of a launch-bound call.
 constexpr int kMaxDevices = 64;
-constexpr int kKernelForms = 84;      // attention: 2 dtypes x 7 bias forms x (short, long) x (plain lists, twins, key split)
+constexpr int kKernelForms = 96;      // attention: 2 dtypes x 8 bias forms x (short, long) x (plain lists, twins, key split)
 constexpr int kSmallForms = 16;      // attention of small calls: 2 dtypes x 8 key counts
 constexpr int kLinearKernels = 32;    // of b200_linear.cu, with an opt-in: pair GEMM (5 activations x 3 epilogue forms x 2 dtypes), SAM's terms by lines (2 dtypes)
 constexpr int kGemmSplits = 6;        // split counts of the split GEMM kernel

@@ -792,3 +792,21 @@ def test_few_keys_in_blocks_of_64_queries(b: int, h: int, nq: int, hw: tuple[int
         got[dead] = ref[dead] = 0.0
     assert_close(got.cpu().numpy(), ref.cpu().numpy(), unit_scale=True, what=f"[{b},{h},{nq},{nk}] {form} {dtype}")
     assert bool((big[:, 0] == 77.0).all()) and bool((big[:, -1] == 77.0).all())
+
+
+@pytest.mark.parametrize(("b", "h", "nq", "hw"), [(3, 5, 70, (57, 1)), (2, 7, 130, (64, 2)), (5, 31, 200, (60, 5)), (2, 9, 257, (63, 17)), (1, 6, 300, (120, 8)), (7, 29, 128, (100, 20)), (2, 3, 512, (72, 56)), (1, 5, 385, (64, 64)), (1, 3, 129, (96, 32))])  # fmt: skip
+@pytest.mark.parametrize("dtype", ["fp16", "bf16"])
+def test_many_grid_rows_leave_out_the_steps_without_a_one(b: int, h: int, nq: int, hw: tuple[int, int], dtype: str) -> None:
+    """Key tiles that lie in one to all of the 16-row groups of rel_h, ragged last tiles, tables whose groups of eight do not pair up,
+    heads for items of one and two tiles and for twins; a masked row of the grid and one that is all that is left; against float32."""
+    t, nk = DTYPES[dtype], hw[0] * hw[1]
+    gen = torch.Generator(device="cuda").manual_seed(nq * 1000 + nk)
+    q, k, v = (torch.randn(b, n, h, 64, generator=gen, device="cuda").to(t) for n in (nq, nk, nk))
+    rel = [torch.randn(b, h, nq, side, generator=gen, device="cuda").to(t) for side in hw]
+    rel[0][:, 0, :, hw[0] // 2] = float("-inf")
+    rel[0][:, 1, :, : hw[0] - 1] -= 40.0  # the last row of the grid decides
+    logits = torch.einsum("bqhd,bkhd->bhqk", q.float(), k.float()) * 0.125 + (rel[0].float()[..., :, None] + rel[1].float()[..., None, :]).reshape(b, h, nq, nk)
+    ref = torch.einsum("bhqk,bkhd->bqhd", logits.softmax(-1), v.float())
+    got = ff.attention(q, k, v, scale=0.125, layout="bnhd", rel=tuple(rel))
+    assert_close(got.float().cpu().numpy(), ref.cpu().numpy(), unit_scale=True, what=f"[{b},{h},{nq}] {hw} {dtype}")
+    assert ff.device_status() == 0
