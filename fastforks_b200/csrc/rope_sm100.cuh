@@ -60,8 +60,11 @@ __global__ void __launch_bounds__(kRopeThreads) rope_qk_kernel(const RopeParams 
   grid_dependency_wait();
   grid_launch_dependents();
   const int units = 8 * p.heads;  // per token: (q | k) x heads x four groups of eight dims
-  const int n = blockIdx.x, np = n - p.prefix;
-  for (int b = blockIdx.y; b < p.batch; b += gridDim.y) {
+  // From the last token of the last image on: where the packed tensor does not fit L2, its end is what the layer in front left there,
+  // and its beginning is then what attention finds. us, forwards and backwards, [32,1029,3,16,64] in CUDA graphs: qkv layer and this 194 and
+  // 189, with the attention behind them 469 and 448.
+  const int n = static_cast<int>(gridDim.x - 1 - blockIdx.x), np = n - p.prefix;
+  for (int b = p.batch - 1 - static_cast<int>(blockIdx.y); b >= 0; b -= gridDim.y) {
     for (int u = threadIdx.x; u < units; u += kRopeThreads) {
       const int is_k = u >= 4 * p.heads ? 1 : 0;
       const int v = u - is_k * 4 * p.heads;
