@@ -190,8 +190,8 @@ struct Forward {
   // y = act((x w^T + b) * gamma + res). A product behind a kernel of this forward may load its weights ahead of that
   // kernel's end: they were complete before it started. Not so in front (the neck of an encoder without blocks on given
   // tokens may follow the kernel that writes them), and weights repacked in this forward are left to the wait as well.
-  int linear(const void* in, int m, int k, const void* w, const void* b, int n, void* out, int act, const float* gamma = nullptr, const void* res = nullptr, bool made_here = false) const {
-    const GemmCall c{a->dtype, m, n, k, act, in, k, w, b, gamma, res, n, out, n, started && !made_here};
+  int linear(const void* in, int m, int k, const void* w, const void* b, int n, void* out, int act, const float* gamma = nullptr, const void* res = nullptr, bool made_here = false, bool backwards = false) const {
+    const GemmCall c{a->dtype, m, n, k, act, in, k, w, b, gamma, res, n, out, n, started && !made_here, backwards};
     started = true;
     return launch_gemm(c, stream);
   }
@@ -277,8 +277,14 @@ struct Forward {
     return b200_attn_fwd(&t, stream);
   }
 
+  // Activations of a large batch do not fit L2. What a kernel wrote last is still there, and one that begins with that finds it: with norms
+  // and attention going forwards through the rows, qkv, projection and fc1 go backwards, and fc2 forwards. us per forward, all forwards and
+  // so: ViT-g/14 at 16 images of 518 px 52737 and 52389, ViT-L/14 at 16 17257 and 17023, ViT-B/14 at 16 5686 and 5612, ViT-B/16 at 110 of 224 px
+  // 4567 and 4486; ViT-L/14 at 4, whose widest tensors of 34 and 45 MB fit, 4848 and 4865.
+  static constexpr int64_t kLargeQkvBytes = 64 << 20;
   int block(const B200EncoderBlock& k) const {
     const int rows = static_cast<int>(l.rows), dim = a->dim;
+    const bool back = l.rows * 6 * dim > kLargeQkvBytes;
     const int tokens = a->prefix + a->grid_h * a->grid_w;
     if (k.window > 0) {
       // Windowed attention (SAM): the first norm writes the padded windows, the projection stays in window order, and the
@@ -286,19 +292,19 @@ struct Forward {
       const WindowMap map{k.window, a->grid_h, a->grid_w, windows_of(a->grid_w, k.window), windows_of(a->grid_h, k.window)};
       const int windows = a->batch * map.per_row * map.per_col, area = k.window * k.window, wrows = windows * area;
       if (int rc = norm(x, k.norm1_w, k.norm1_b, at(l.y), wrows, a->eps, map)) return rc;
-      if (int rc = linear(at(l.y), wrows, dim, k.qkv_w, k.qkv_b, 3 * dim, at(l.qkv), kActNone)) return rc;
+      if (int rc = linear(at(l.y), wrows, dim, k.qkv_w, k.qkv_b, 3 * dim, at(l.qkv), kActNone, nullptr, nullptr, false, back)) return rc;
       if (int rc = attention(k, windows, area, k.window)) return rc;
-      if (int rc = linear(at(l.att), wrows, dim, k.proj_w, k.proj_b, dim, at(l.y), kActNone, k.gamma1)) return rc;
+      if (int rc = linear(at(l.att), wrows, dim, k.proj_w, k.proj_b, dim, at(l.y), kActNone, k.gamma1, nullptr, false, back)) return rc;
       if (int rc = norm(x, k.norm2_w, k.norm2_b, at(l.att), rows, a->eps, map, x, at(l.y))) return rc;
     } else {
       if (int rc = norm(x, k.norm1_w, k.norm1_b, at(l.y), rows, a->eps)) return rc;
-      if (int rc = linear(at(l.y), rows, dim, k.qkv_w, k.qkv_b, 3 * dim, at(l.qkv), kActNone)) return rc;
+      if (int rc = linear(at(l.y), rows, dim, k.qkv_w, k.qkv_b, 3 * dim, at(l.qkv), kActNone, nullptr, nullptr, false, back)) return rc;
       if (int rc = attention(k, a->batch, tokens, a->grid_h)) return rc;
-      if (int rc = linear(at(l.att), rows, dim, k.proj_w, k.proj_b, dim, x, kActNone, k.gamma1, x)) return rc;
+      if (int rc = linear(at(l.att), rows, dim, k.proj_w, k.proj_b, dim, x, kActNone, k.gamma1, x, false, back)) return rc;
       if (int rc = norm(x, k.norm2_w, k.norm2_b, at(l.att), rows, a->eps)) return rc;
     }
     const int act = a->ffn == B200_FFN_SWIGLU ? kActSwiGlu : a->ffn == B200_FFN_GELU ? kActGelu : kActGeluTanh;
-    if (int rc = linear(at(l.att), rows, dim, k.fc1_w, k.fc1_b, a->hidden, at(l.hid), act)) return rc;
+    if (int rc = linear(at(l.att), rows, dim, k.fc1_w, k.fc1_b, a->hidden, at(l.hid), act, nullptr, nullptr, false, back)) return rc;
     return linear(at(l.hid), rows, a->hidden, k.fc2_w, k.fc2_b, dim, x, kActNone, k.gamma2, x);
   }
 

@@ -217,6 +217,7 @@ int launch_gemm(const GemmCall& c, cudaStream_t stream) {
   prm.bias = c.bias; prm.scale = c.scale; prm.res = c.res; prm.lres = c.lres;
   prm.y = c.y; prm.ldy = c.ldy; prm.act = c.act;
   prm.early_w = c.early_w ? 1 : 0;
+  prm.backwards = c.backwards ? 1 : 0;
   prm.status = dev->status;
   const int64_t w_rows = swiglu ? 2LL * c.n : c.n;
   CUtensorMap mx, mw;
@@ -397,7 +398,7 @@ int b200_gemm(const B200GemmArgs* a, void* stream_ptr) {
     if (x.ptr == nullptr && x.required) return fail(B200_ATTN_BAD_CONFIG, "%s is NULL", x.name);
     if (!aligned16(x.ptr)) return fail(B200_ATTN_UNSUPPORTED, "%s is not 16-byte aligned", x.name);
   }
-  const GemmCall call{a->dtype, a->m, a->n, a->k, a->act, a->x, a->lda, a->w, a->bias, a->scale, a->res, a->lres, a->y, a->ldy, false};
+  const GemmCall call{a->dtype, a->m, a->n, a->k, a->act, a->x, a->lda, a->w, a->bias, a->scale, a->res, a->lres, a->y, a->ldy, false, false};
   if (int rc = launch_gemm(call, static_cast<cudaStream_t>(stream_ptr))) return rc;
   clear_error();
   return B200_ATTN_OK;

@@ -51,6 +51,7 @@ struct GemmParams {
   int64_t ldy;
   int act;
   int early_w;         // w was complete before the kernel in front of this one started: load it without waiting for that one
+  int backwards;       // pair kernel: row tiles from the last to the first
   uint32_t* status;
 };
 
@@ -172,6 +173,7 @@ __device__ __forceinline__ GemmItem item_at(const GemmParams& p, int item, int o
   const int rows = min(p.group_m, p.tiles_m - g * p.group_m);
   const int tn = in / rows;
   t.tm = g * p.group_m + (in - tn * rows);
+  if (p.backwards) t.tm = p.tiles_m - 1 - t.tm;
   t.col0 = tn * out_cols + sub;
   return t;
 }

@@ -24,6 +24,7 @@ struct GemmCall {
   void* y;
   int64_t ldy;
   bool early_w;
+  bool backwards;  // a hint: rows from the last to the first, so that what the kernel in front wrote last is read first
 };
 int launch_gemm(const GemmCall& c, cudaStream_t stream);
 
