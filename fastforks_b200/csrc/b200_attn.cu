@@ -638,7 +638,7 @@ int b200_attn_fwd(const B200AttnArgs* a, void* stream_ptr) {
   // Few keys (attn_window_sm100.cuh): without a bias, with one in rows on 16 bytes, or with tables that the product with a one-hot
   // operand adds exactly.
   const bool in_tiles = bias_mode == kBiasDense && dense_bias_in_tiles(a);
-  if (bias_mode == kBiasNone || in_tiles || bias_mode == kBiasDecomposed) {
+  if (a->kv_tokens <= kWindowCallMaxKeys && (bias_mode == kBiasNone || in_tiles || bias_mode == kBiasDecomposed)) {
     WindowCall call{bias_mode == kBiasNone ? kWindowCallPlain : in_tiles ? kWindowCallDense : kWindowCallRel, in_tiles && bias_shared_by_the_batch(a), 0, 0};
     const bool exact = bias_mode != kBiasDecomposed ||
                        (a->rel_dtype == a->dtype && inverse_is_exact(a->scale, a->rel_dtype, &call.rel_one));

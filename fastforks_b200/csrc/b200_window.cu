@@ -13,6 +13,7 @@ namespace b200 {
 constexpr int kWindowGroupsPerSm = 52;
 
 bool window_pays(const B200AttnArgs* a, const WindowCall& call, int sms) {
+  static_assert(kWindowCallMaxKeys == kWindowMaxKeys, "one limit");
   if (a->kv_tokens > kWindowMaxKeys) return false;
   if (call.bias == kWindowCallRel && a->rel_kh + a->rel_kw > kWindowMaxRel) return false;
   const int64_t blocks = (static_cast<int64_t>(a->q_tokens) + kWindowRows - 1) / kWindowRows * a->batch * a->heads;

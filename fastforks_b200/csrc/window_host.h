@@ -13,6 +13,7 @@ struct WindowCall {
   int rel_align;        // decomposed: bytes the rows of both tables begin on (16, 4 or 2)
   uint32_t rel_one;     // decomposed: 1 / scale, 16 bits
 };
+constexpr int kWindowCallMaxKeys = 128;  // no call with more keys goes there: nothing else needs to be looked at
 // Whether a call that passed validation goes to the kernel, and the launch.
 bool window_pays(const B200AttnArgs* a, const WindowCall& call, int sms);
 int launch_window(const B200AttnArgs* a, const WindowCall& call, cudaStream_t stream);
