@@ -30,7 +30,10 @@ constexpr int kWindowRows = 64;    // queries per CTA
 constexpr int kWindowThreads = 128;
 // CTAs per SM, by registers: 72 a thread hold 64 logits of two rows, 128 hold 128. us at 6 and 7: [8,192,49] / [64,192,49] with a bias
 // 10.5 / 76.6 and 10.5 / 74.8, [8,64,64] 7.1 and 5.8, [100,12,36] with tables 8.4 and 8.0, but [64,12,64] without either 5.7 and 6.3.
-constexpr int window_ctas(int groups, int bias) { return groups > 4 ? 4 : bias == kWindowPlain ? 6 : 7; }
+constexpr int window_ctas(int eights, int bias) { return eights > 8 ? 4 : bias == kWindowPlain ? 6 : 7; }
+// 7 x 7 windows and the 50 tokens of a 224 px image in patches of 32 need no eighth group of eight. us with it and without: [64,192,49] with a
+// bias 74.5 and 72.5, [8,192,49] 10.6 and 10.5, [64,12,50] 5.85 and 5.55. (At 64 registers and eight CTAs an SM: 77.1, 10.6, 6.5.)
+constexpr int window_eights(int keys) { return keys > 48 && keys <= 56 ? 7 : (keys + 15) / 16 * 2; }
 
 struct WindowParams {
   const void* q;
@@ -98,9 +101,11 @@ __device__ __forceinline__ void window_load(uint32_t smem, const T* rows, int64_
   }
 }
 
-// GROUPS = ceil(kv_tokens / 16). Grid: q_blocks * batch * heads.
-template <typename T, int BIAS, int GROUPS>
-__global__ void __launch_bounds__(kWindowThreads, window_ctas(GROUPS, BIAS)) attn_window_kernel(const WindowParams p) {
+// EIGHTS = ceil(kv_tokens / 8), of which an odd number is only told from the next even one where window_eights() says so. Grid: q_blocks *
+// batch * heads.
+template <typename T, int BIAS, int EIGHTS>
+__global__ void __launch_bounds__(kWindowThreads, window_ctas(EIGHTS, BIAS)) attn_window_kernel(const WindowParams p) {
+  constexpr int GROUPS = (EIGHTS + 1) / 2;  // of 16 keys: what a step of the second product takes
   __shared__ __align__(128) uint8_t smem_q[kWindowRows * 128];
   __shared__ __align__(128) uint8_t smem_k[GROUPS * 16 * 128];
   __shared__ __align__(128) uint8_t smem_v[GROUPS * 16 * 128];
@@ -139,17 +144,17 @@ __global__ void __launch_bounds__(kWindowThreads, window_ctas(GROUPS, BIAS)) att
 
   // The rows' bias, in flight with the operands: a lane loads the pairs of columns whose logits it will hold. A pair never reaches behind
   // the row's end.
-  [[maybe_unused]] uint32_t bw[2][2 * GROUPS];
+  [[maybe_unused]] uint32_t bw[2][EIGHTS];
   if constexpr (BIAS == kWindowDense) {
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
       const bool valid = row_of(r) < p.q_tokens;
       const uint16_t* src = static_cast<const uint16_t*>(p.bias) + b * p.bias_stride[0] + h * p.bias_stride[1] + (valid ? row_of(r) : 0) * p.bias_stride[2] + 2 * t;
 #pragma unroll
-      for (int j = 0; j < 2 * GROUPS; ++j) bw[r][j] = load_u32_if(src + 8 * j, valid && 8 * j + 2 * t + 1 < p.kv_tokens);
+      for (int j = 0; j < EIGHTS; ++j) bw[r][j] = load_u32_if(src + 8 * j, valid && 8 * j + 2 * t + 1 < p.kv_tokens);
       if ((p.kv_tokens & 1) != 0) {  // the last key's half of its pair
 #pragma unroll
-        for (int j = 2 * GROUPS - 2; j < 2 * GROUPS; ++j) bw[r][j] |= load_u16_if(src + 8 * j, valid && 8 * j + 2 * t + 1 == p.kv_tokens);
+        for (int j = EIGHTS - 2 < 0 ? 0 : EIGHTS - 2; j < EIGHTS; ++j) bw[r][j] |= load_u16_if(src + 8 * j, valid && 8 * j + 2 * t + 1 == p.kv_tokens);
       }
     }
   }
@@ -186,9 +191,9 @@ __global__ void __launch_bounds__(kWindowThreads, window_ctas(GROUPS, BIAS)) att
   __syncthreads();
   if (my_row0 < p.q_tokens) {
     const int k_row = (lane & 7) + ((lane >> 4) << 3), k_chunk = (lane >> 3) & 1;  // ldmatrix addresses: 16 keys x 16 of the head dim
-    float s[2 * GROUPS][4];  // rows g and g + 8, keys 8 j + 2 t and + 1
+    float s[EIGHTS][4];  // rows g and g + 8, keys 8 j + 2 t and + 1
 #pragma unroll
-    for (int j = 0; j < 2 * GROUPS; ++j)
+    for (int j = 0; j < EIGHTS; ++j)
 #pragma unroll
       for (int e = 0; e < 4; ++e) s[j][e] = 0.f;
 #pragma unroll
@@ -200,7 +205,7 @@ __global__ void __launch_bounds__(kWindowThreads, window_ctas(GROUPS, BIAS)) att
         uint32_t kk[4];
         ldmatrix_x4(kk, window_chunk(sk, i * 16 + k_row, 2 * d + k_chunk));
         mma_16816<T>(s[2 * i], a, kk[0], kk[1]);
-        mma_16816<T>(s[2 * i + 1], a, kk[2], kk[3]);
+        if (2 * i + 1 < EIGHTS) mma_16816<T>(s[2 * i + 1], a, kk[2], kk[3]);
       }
     }
     if constexpr (BIAS == kWindowRel) {
@@ -212,36 +217,37 @@ __global__ void __launch_bounds__(kWindowThreads, window_ctas(GROUPS, BIAS)) att
           uint32_t kk[4];
           ldmatrix_x4(kk, onehot_chunk(smem_u32(smem_e), i * 16 + k_row, 2 * c + k_chunk));
           mma_16816<T>(s[2 * i], ra[c], kk[0], kk[1]);
-          mma_16816<T>(s[2 * i + 1], ra[c], kk[2], kk[3]);
+          if (2 * i + 1 < EIGHTS) mma_16816<T>(s[2 * i + 1], ra[c], kk[2], kk[3]);
         }
       }
     }
     const float unit = BIAS == kWindowDense ? kLog2e : p.scale_log2;
     uint32_t probs[2 * GROUPS][2];
+    if constexpr (EIGHTS % 2 != 0) probs[EIGHTS][0] = probs[EIGHTS][1] = 0;
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
       if constexpr (BIAS == kWindowDense) {  // natural units, s * scale + bias; log2(e) rides on the FMA in front of the exponential
 #pragma unroll
-        for (int j = 0; j < 2 * GROUPS; ++j) {
+        for (int j = 0; j < EIGHTS; ++j) {
           const float2 x = ffma2(make_float2(s[j][2 * r], s[j][2 * r + 1]), make_float2(p.scale, p.scale), unpack2(bw[r][j], p.bias_half != 0));
           s[j][2 * r] = x.x;
           s[j][2 * r + 1] = x.y;
         }
       }
 #pragma unroll
-      for (int j = 2 * GROUPS - 2; j < 2 * GROUPS; ++j)  // the keys that pad the last group
+      for (int j = EIGHTS - 2 < 0 ? 0 : EIGHTS - 2; j < EIGHTS; ++j)  // the keys that pad the last group
 #pragma unroll
         for (int e = 0; e < 2; ++e)
           if (8 * j + 2 * t + e >= p.kv_tokens) s[j][2 * r + e] = kNone;
       float top = fmaxf(s[0][2 * r], s[0][2 * r + 1]);
 #pragma unroll
-      for (int j = 1; j < 2 * GROUPS; ++j) top = max3(top, s[j][2 * r], s[j][2 * r + 1]);
+      for (int j = 1; j < EIGHTS; ++j) top = max3(top, s[j][2 * r], s[j][2 * r + 1]);
       top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 1));
       top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 2)) * unit;
       const float shift = top == kNone ? 0.f : -top;
       float2 part = make_float2(0.f, 0.f);
 #pragma unroll
-      for (int j = 0; j < 2 * GROUPS; ++j) {
+      for (int j = 0; j < EIGHTS; ++j) {
         const float2 x = ffma2(make_float2(s[j][2 * r], s[j][2 * r + 1]), make_float2(unit, unit), make_float2(shift, shift));
         const float2 e = make_float2(fast_exp2(x.x), fast_exp2(x.y));
         part = fadd2(part, e);

@@ -24,21 +24,22 @@ bool window_pays(const B200AttnArgs* a, const WindowCall& call, int sms) {
 namespace {
 
 template <typename T, int BIAS>
-const void* window_kernel(int groups) {
-  switch (groups) {
-    case 1: return reinterpret_cast<const void*>(attn_window_kernel<T, BIAS, 1>);
+const void* window_kernel(int keys) {
+  switch (window_eights(keys)) {
     case 2: return reinterpret_cast<const void*>(attn_window_kernel<T, BIAS, 2>);
-    case 3: return reinterpret_cast<const void*>(attn_window_kernel<T, BIAS, 3>);
     case 4: return reinterpret_cast<const void*>(attn_window_kernel<T, BIAS, 4>);
-    case 5: return reinterpret_cast<const void*>(attn_window_kernel<T, BIAS, 5>);
     case 6: return reinterpret_cast<const void*>(attn_window_kernel<T, BIAS, 6>);
     case 7: return reinterpret_cast<const void*>(attn_window_kernel<T, BIAS, 7>);
-    default: return reinterpret_cast<const void*>(attn_window_kernel<T, BIAS, 8>);
+    case 8: return reinterpret_cast<const void*>(attn_window_kernel<T, BIAS, 8>);
+    case 10: return reinterpret_cast<const void*>(attn_window_kernel<T, BIAS, 10>);
+    case 12: return reinterpret_cast<const void*>(attn_window_kernel<T, BIAS, 12>);
+    case 14: return reinterpret_cast<const void*>(attn_window_kernel<T, BIAS, 14>);
+    default: return reinterpret_cast<const void*>(attn_window_kernel<T, BIAS, 16>);
   }
 }
 template <typename T>
-const void* window_kernel(int bias, int groups) {
-  return bias == kWindowDense ? window_kernel<T, kWindowDense>(groups) : bias == kWindowRel ? window_kernel<T, kWindowRel>(groups) : window_kernel<T, kWindowPlain>(groups);
+const void* window_kernel(int bias, int keys) {
+  return bias == kWindowDense ? window_kernel<T, kWindowDense>(keys) : bias == kWindowRel ? window_kernel<T, kWindowRel>(keys) : window_kernel<T, kWindowPlain>(keys);
 }
 
 }  // namespace
@@ -77,8 +78,7 @@ int launch_window(const B200AttnArgs* a, const WindowCall& call, cudaStream_t st
     prm.rel_pairs = call.rel_align >= 4 && a->rel_kh % 2 == 0 && a->rel_kw % 2 == 0;
     prm.rel_one = call.rel_one;
   }
-  const int groups = (a->kv_tokens + 15) / 16;
-  const void* kernel = a->dtype == B200_ATTN_F16 ? window_kernel<__half>(call.bias, groups) : window_kernel<__nv_bfloat16>(call.bias, groups);
+  const void* kernel = a->dtype == B200_ATTN_F16 ? window_kernel<__half>(call.bias, a->kv_tokens) : window_kernel<__nv_bfloat16>(call.bias, a->kv_tokens);
   void* args[] = {&prm};
   return launch_kernel(kernel, static_cast<unsigned>(prm.q_blocks * a->batch * a->heads), 1, kWindowThreads, 0, 1, stream, args, "attention kernel launch");
 }

@@ -794,6 +794,14 @@ def test_few_keys_in_blocks_of_64_queries(b: int, h: int, nq: int, hw: tuple[int
     assert bool((big[:, 0] == 77.0).all()) and bool((big[:, -1] == 77.0).all())
 
 
+@pytest.mark.parametrize(("b", "h", "nq", "hw"), [(4, 60, 50, (5, 10)), (3, 70, 55, (5, 11)), (2, 90, 70, (7, 8)), (2, 90, 57, (3, 19))])
+@pytest.mark.parametrize("form", ["plain", "dense", "rel"])
+@pytest.mark.parametrize("dtype", ["fp16", "bf16"])
+def test_few_keys_in_seven_groups_of_eight(b: int, h: int, nq: int, hw: tuple[int, int], form: str, dtype: str) -> None:
+    """Key counts at either end of the form that has no eighth group, and the one behind it."""
+    test_few_keys_in_blocks_of_64_queries(b, h, nq, hw, form, dtype)
+
+
 @pytest.mark.parametrize(("b", "h", "nq", "hw"), [(3, 5, 70, (57, 1)), (2, 7, 130, (64, 2)), (5, 31, 200, (60, 5)), (2, 9, 257, (63, 17)), (1, 6, 300, (120, 8)), (7, 29, 128, (100, 20)), (2, 3, 512, (72, 56)), (1, 5, 385, (64, 64)), (1, 3, 129, (96, 32))])  # fmt: skip
 @pytest.mark.parametrize("dtype", ["fp16", "bf16"])
 def test_many_grid_rows_leave_out_the_steps_without_a_one(b: int, h: int, nq: int, hw: tuple[int, int], dtype: str) -> None:
