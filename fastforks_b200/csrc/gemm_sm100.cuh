@@ -328,6 +328,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant
           ph = next_ph;
         }
       }
+      // The other CTA's epilogue warps signal `acc_empty` here, a lane per barrier: those of the last two items are waited for by nobody else,
+      // and they have landed before this CTA goes. (In a warp that has nothing else to do any more: no launch took longer.)
+      if (ok) ok = __all_sync(0xffffffffu, lane >= min(it, 2) || mbar_wait(&sm.acc_empty[lane], ((it - 1 - lane) / 2) & 1, abort_flag));
       if (!ok && lane == 0 && atomicExch(const_cast<uint32_t*>(abort_flag), 1u) == 0) atomicOr(p.status, kStatusGemmMma);
       if (__any_sync(0xffffffffu, *abort_flag != 0)) {  // no product may be running when tensor memory is freed
         uint32_t no_abort = 0;
@@ -482,7 +485,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant
 
   tc_fence_before_sync();
   __syncthreads();
-  cluster_arrive_relaxed();  // neither CTA goes while the other may still signal its barriers or multiply into its tensor memory
+  // Neither CTA goes while the other may still multiply into its tensor memory or signal its barriers. The barrier itself, relaxed, orders no such
+  // signal: the leader has waited for those of the accumulators, and the last ones of the stages go out in front of the accumulator's,
+  // which every epilogue warp has waited for.
+  cluster_arrive_relaxed();
   cluster_wait();
   if (warp == 1) {
     tc_fence_after_sync();

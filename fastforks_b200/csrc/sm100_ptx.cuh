@@ -339,7 +339,8 @@ __device__ __forceinline__ uint32_t cluster_cta_rank() {
 }
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
 // The same without the release: of a thread that hands over nothing but what fence.mbarrier_init or a tcgen05 fence has ordered already. The
-// release waits for the thread's own memory traffic: a barrier took some 1000 clocks with it.
+// release waits for the thread's own memory traffic: a barrier took some 1000 clocks with it. Nor does it order the thread's remote mbarrier
+// arrivals: a CTA that others signal waits for those signals itself before it goes.
 __device__ __forceinline__ void cluster_arrive_relaxed() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 // The shared::cluster address of `addr` (a shared::cta address of this CTA) in the CTA of rank `rank`.

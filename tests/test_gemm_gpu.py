@@ -139,6 +139,24 @@ def test_every_cut_of_a_product(m: int, n: int, k: int) -> None:
     check(ff.gemm(x, w, bias, scale=scale, res=res, act=ff.ACT_GELU, out=out), x, w, bias, scale, res, act=ff.ACT_GELU, what=f"[{m},{n},{k}]")
 
 
+@pytest.mark.parametrize("shapes", [
+    ((1051, 2696, 520), (1051, 2696, 72)),  # one item per pair of CTAs; more k blocks than stages, and fewer
+    ((2309, 2824, 72), (3863, 2824, 200)),  # two and three
+    ((3345, 2888, 72), (4640, 2888, 200)),  # the last ones parts of a tile, some with all columns behind n
+])  # fmt: skip
+def test_last_items_of_a_pair_of_ctas_with_the_next_kernel_behind(shapes: tuple[tuple[int, int, int], ...]) -> None:
+    """Two products in turn, the next one's CTAs taking the SMs as soon as a pair has gone: every repeat has the bits of the first."""
+    cases = [tuple(t.cuda() for t in operands(m, n, k, torch.float16, seed=m + k)) for m, n, k in shapes]
+    outs = [[torch.full((m, n), float("nan"), dtype=torch.float16, device="cuda") for _ in range(20)] for m, n, _ in shapes]
+    for i in range(20):
+        for (x, w, bias, _, res), out in zip(cases, outs, strict=True):
+            ff.gemm(x, w, bias, res=res if i % 2 else None, out=out[i])
+    for (x, w, bias, _, res), out, shape in zip(cases, outs, shapes, strict=True):
+        check(out[0], x, w, bias, what=f"{shape}")
+        check(out[1], x, w, bias, None, res, what=f"{shape} with a residual")
+        assert all(torch.equal(out[i], out[i % 2]) for i in range(20))
+
+
 def test_row_strided_views_and_leading_dims() -> None:
     """x, res and out as 2-D views with a row stride (lda, lres, ldy) and x with leading batch dims."""
     gen = torch.Generator().manual_seed(5)

@@ -310,3 +310,30 @@ def test_kernels_that_give_up_wait_for_their_products_before_they_free_tensor_me
     gives_up = lines.index("if (abort != 0)")
     assert lines.rindex("__syncthreads();", 0, gives_up) > lines.index("mbar_wait(&done")  # the flag is looked at where all warps see the same
     assert "break;" in lines[gives_up : lines.index("tmem_dealloc")]
+
+
+def test_a_pair_of_ctas_waits_for_every_signal_of_the_other_before_either_goes() -> None:
+    """An arrival on a barrier of a CTA that has gone hits whatever took its shared memory. The pair kernel's barrier at the end is relaxed
+    and orders no such arrival, so the leader waits for those that hand accumulators back: in its loop for all but the last on either
+    barrier, behind the loop for these. (Read, not run.) The phases waited for are counted here for any number of items."""
+    from fastforks_b200 import _lib
+
+    source = next(p for p in _lib.HEADERS if p.name == "gemm_sm100.cuh").read_text()
+    body = next(b for b in source.split("__global__")[1:] if "gemm_pair_kernel(" in b)
+    issuer = body[body.index("= MMA issuer") : body.index("= epilogue warps")]
+    assert "if (it >= 2) ok = __all_sync(0xffffffffu, mbar_wait(&sm.acc_empty[it & 1], ((it >> 1) - 1) & 1, abort_flag));" in issuer
+    behind = "if (ok) ok = __all_sync(0xffffffffu, lane >= min(it, 2) || mbar_wait(&sm.acc_empty[lane], ((it - 1 - lane) / 2) & 1, abort_flag));"
+    assert issuer.index("umma_commit_pair(&sm.acc_full") < issuer.index(behind) < issuer.index("umma_commit_pair(&sm.drain)")
+    for items in range(9):
+        waited = [(it & 1, (it >> 1) - 1) for it in range(2, items)] + [(lane, (items - 1 - lane) // 2) for lane in range(min(items, 2))]
+        assert sorted(waited) == sorted((it & 1, it >> 1) for it in range(items))  # every phase of both barriers, once
+
+
+def test_a_stage_is_signalled_in_front_of_the_accumulator_it_is_part_of() -> None:
+    """The signals of the last stages reach the other CTA ahead of the accumulator's, which all its epilogue warps wait for."""
+    from fastforks_b200 import _lib
+
+    source = next(p for p in _lib.HEADERS if p.name == "gemm_sm100.cuh").read_text()
+    body = next(b for b in source.split("__global__")[1:] if "gemm_pair_kernel(" in b)
+    assert body.index("umma_commit_pair(&sm.empty[st]);") < body.index("umma_commit_pair(&sm.acc_full[it & 1]);")
+    assert "mbar_wait(&sm.acc_full[it & 1], (it >> 1) & 1, abort_flag)" in body
