@@ -369,7 +369,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant
         tma_store_wait_read<0>();  // the stores of the tile before have read both buffers
         for (int i = 0; i < 2; ++i) {
           const int c = part + 2 * i;
-          if (c < pieces && inside(row0, col0 + c * 64)) {
+          if (c < pieces && inside(row0, col0 + c * 64)) {  // asked(i) below
             mbar_arrive_expect_tx(&sm.res_full[e][i], kPairChunkBytes);
             tma_load_2d(sm.stage[e][i], &tm_res, &sm.res_full[e][i], col0 + c * 64, row0);
           }
@@ -390,13 +390,18 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant
       }
       // The residual has landed long before the accumulator is finished: its waits cost nothing here, some 350 clocks each behind that.
       if (has_res) {
+        auto asked = [&](int i) { return part + 2 * i < pieces && inside(row0, col0 + (part + 2 * i) * 64); };
 #pragma unroll
         for (int i = 0; i < 2; ++i)
-          if (part + 2 * i < pieces && inside(row0, col0 + (part + 2 * i) * 64)) {
-            ok = ok && __all_sync(0xffffffffu, mbar_wait(&sm.res_full[e][i], loads[i] & 1, abort_flag)) != 0;
-            loads[i] += ok ? 1 : 0;
-          }
-        if (!ok) break;
+          if (asked(i)) ok = ok && __all_sync(0xffffffffu, mbar_wait(&sm.res_full[e][i], loads[i] & 1, abort_flag)) != 0;
+        if (!ok) {  // given up: a residual still on its way must land before the CTA goes
+          uint32_t no_abort = 0;
+          for (int i = 0; i < 2; ++i)
+            if (asked(i)) mbar_wait(&sm.res_full[e][i], loads[i] & 1, &no_abort);
+          break;
+        }
+#pragma unroll
+        for (int i = 0; i < 2; ++i) loads[i] += asked(i) ? 1 : 0;
       }
       if (!__all_sync(0xffffffffu, mbar_wait(&sm.acc_full[it & 1], (it >> 1) & 1, abort_flag))) {
         ok = false;
@@ -473,13 +478,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant
       }
     }
     if (!ok && lane == 0 && atomicExch(const_cast<uint32_t*>(abort_flag), 1u) == 0) atomicOr(p.status, kStatusGemmEpilogue);
-    if (lane == 0) {
-      tma_store_wait_read<0>();
-      if (*abort_flag != 0 && has_res) {  // a residual still on its way must land before the CTA goes
-        uint32_t no_abort = 0;
-        for (int i = 0; i < 2; ++i) mbar_wait(&sm.res_full[e][i], loads[i] & 1, &no_abort);
-      }
-    }
+    if (lane == 0) tma_store_wait_read<0>();
     __syncwarp();
   }
 

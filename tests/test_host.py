@@ -337,3 +337,22 @@ def test_a_stage_is_signalled_in_front_of_the_accumulator_it_is_part_of() -> Non
     body = next(b for b in source.split("__global__")[1:] if "gemm_pair_kernel(" in b)
     assert body.index("umma_commit_pair(&sm.empty[st]);") < body.index("umma_commit_pair(&sm.acc_full[it & 1]);")
     assert "mbar_wait(&sm.acc_full[it & 1], (it >> 1) & 1, abort_flag)" in body
+
+
+def test_a_pair_that_gives_up_waits_for_the_residuals_it_has_asked_for_and_no_others() -> None:
+    """A wait for a phase that nothing will complete runs to its limit, a second each. So the drain of residual loads lies where the wait for
+    them ran out, the only place where one can be on its way: under the condition they were asked for under, on the phase that wait was
+    for, and the count of phases moves on behind it. (Read, not run: nothing makes that wait run out on a healthy GPU.)"""
+    from fastforks_b200 import _lib
+
+    source = next(p for p in _lib.HEADERS if p.name == "gemm_sm100.cuh").read_text()
+    body = next(b for b in source.split("__global__")[1:] if "gemm_pair_kernel(" in b)
+    epilogue = body[body.index("= epilogue warps") :]
+    waits = [m.start() for m in re.finditer(r"mbar_wait\(&sm\.res_full\[e\]\[i\], loads\[i\] & 1, (&no_abort|abort_flag)\)", epilogue)]
+    assert len(waits) == 2 == epilogue.count("mbar_wait(&sm.res_full")
+    assert all(epilogue[:w].rstrip().endswith(("if (asked(i))", "if (asked(i)) ok = ok && __all_sync(0xffffffffu,")) for w in waits)
+    gives_up = epilogue.index("if (!ok) {", waits[0])
+    assert waits[0] < gives_up < waits[1] < epilogue.index("break;", gives_up) < epilogue.index("loads[i] += asked(i) ? 1 : 0;") < epilogue.index("mbar_wait(&sm.acc_full")
+    asked = "part + 2 * i < pieces && inside(row0, col0 + (part + 2 * i) * 64)"
+    assert f"auto asked = [&](int i) {{ return {asked}; }};" in epilogue
+    assert re.search(r"const int c = part \+ 2 \* i;\s+if \(c < pieces && inside\(row0, col0 \+ c \* 64\)\) \{", epilogue[: waits[0]])
