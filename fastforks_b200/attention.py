@@ -235,8 +235,8 @@ def attention(  # noqa: PLR0913
         out: Optional output view of q's shape and dtype.
         schedule: `"auto"`, `"long"` or `"short"` tile schedule; `"auto"` takes the short one for at most 256 keys whose last
             128-key tile holds at most 96 (e.g. 197 tokens). A hint for the persistent kernel: the result does not depend on it, and
-            calls without bias too small to fill the GPU (up to 512 keys) go to a kernel of their own whatever it says, as do calls of
-            up to 64 keys, and of up to 128 on few heads.
+            calls without bias too small to fill the GPU (up to 512 keys) go to a kernel of their own whatever it says, as do most
+            calls of up to 64 keys (not those of many queries without tables), and of up to 128 on few heads.
 
     Returns:
         A tensor of q's shape. Without `out` its memory is `[B, N, heads, 64]`-contiguous in both layouts, so the

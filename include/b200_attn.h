@@ -47,7 +47,8 @@ extern "C" {
  * for sequences of at most two key tiles (197 tokens: 69 keys in the second tile) and costs the long sequences a
  * little. AUTO picks SHORT for at most 256 keys whose last tile holds at most 96, else LONG; b200_attn_query
  * reports the choice. Results are identical bit for bit. Calls without bias that are too small to fill the GPU with
- * 128-row tiles go to a kernel of their own, whatever the hint, and so do calls of up to 64 keys, and of up to 128 on few heads. */
+ * 128-row tiles go to a kernel of their own, whatever the hint, and so do calls of few keys: up to 64 unless many queries per head
+ * fill the tiles (with no bias, or a dense one), and up to 128 on few heads. */
 #define B200_ATTN_SCHED_AUTO 0
 #define B200_ATTN_SCHED_LONG 1
 #define B200_ATTN_SCHED_SHORT 2

@@ -43,6 +43,25 @@ def pytest_collection_modifyitems(config: pytest.Config, items: list[pytest.Item
             item.add_marker(skip)
 
 
+def kernels_of(call) -> list[str]:  # noqa: ANN001
+    """The (mangled) names of the kernels a call launches, in order: read from a graph captured of it. Which of several kernels answers is
+    the library's choice; a test that is about one of them asserts it."""
+    import torch
+    from cuda.bindings import driver
+
+    call()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph):
+        call()
+    raw, names = graph.raw_cuda_graph(), []
+    _, _, count = driver.cuGraphGetNodes(raw, 0)
+    for node in driver.cuGraphGetNodes(raw, count)[1][:count]:
+        if driver.cuGraphNodeGetType(node)[1] == driver.CUgraphNodeType.CU_GRAPH_NODE_TYPE_KERNEL:
+            names.append(driver.cuFuncGetName(driver.cuGraphKernelNodeGetParams(node)[1].func)[1].decode())
+    return names
+
+
 def load_golden(name: str) -> dict[str, np.ndarray]:
     with np.load(GOLDEN / f"{name}.npz") as z:
         return {k: z[k] for k in z.files}

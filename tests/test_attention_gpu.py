@@ -14,7 +14,7 @@ import pytest
 import torch
 
 import fastforks_b200 as ff
-from conftest import assert_close, load_golden
+from conftest import assert_close, kernels_of, load_golden
 from oracle import attention_oracle as ao
 from oracle import c_oracle
 
@@ -800,6 +800,39 @@ def test_few_keys_in_blocks_of_64_queries(b: int, h: int, nq: int, hw: tuple[int
 def test_few_keys_in_seven_groups_of_eight(b: int, h: int, nq: int, hw: tuple[int, int], form: str, dtype: str) -> None:
     """Key counts at either end of the form that has no eighth group, and the one behind it."""
     test_few_keys_in_blocks_of_64_queries(b, h, nq, hw, form, dtype)
+
+
+# (queries, key grid, form, blocks of 64 queries per SM, in tenths, up to which the kernel for few keys answers; 0: any number)
+LINES = [
+    (256, (8, 8), "plain", 240), (256, (3, 19), "plain", 240), (256, (7, 8), "plain", 330), (256, (6, 8), "plain", 620), (256, (4, 8), "plain", 0),
+    (256, (8, 8), "dense", 240), (128, (8, 8), "dense", 240), (256, (7, 8), "dense", 0), (256, (8, 8), "rel", 0),  # full query tiles
+    (640, (8, 8), "plain", 480), (600, (7, 8), "plain", 660), (384, (8, 8), "plain", 0), (128, (8, 8), "plain", 0), (64, (8, 8), "dense", 0),
+    (256, (8, 10), "plain", 104), (128, (8, 10), "dense", 104), (256, (8, 12), "plain", 60), (256, (7, 16), "dense", 60), (100, (10, 10), "plain", 74),
+    (128, (8, 16), "plain", 40), (128, (8, 16), "dense", 20), (128, (8, 15), "dense", 40), (128, (8, 16), "rel", 65), (256, (8, 12), "rel", 86),
+]  # fmt: skip
+
+
+@pytest.mark.parametrize(("nq", "hw", "form", "tenths"), LINES)
+def test_few_keys_on_either_side_of_the_lines(nq: int, hw: tuple[int, int], form: str, tenths: int) -> None:
+    """The last number of heads the kernel for few keys answers and the first the persistent kernel does (without a line: many heads),
+    both against float32 on the same operands."""
+    per_head, sms, nk = -(-nq // 64), torch.cuda.get_device_properties(0).multi_processor_count, hw[0] * hw[1]
+    heads = tenths * sms // (10 * per_head) if tenths else 70 * sms // per_head
+    for h, kernel in ((heads, "attn_window_kernel"), (heads + 1, "attn_fwd_kernel"))[: 2 if tenths else 1]:
+        gen = torch.Generator(device="cuda").manual_seed(nq * 1000 + nk)
+        q, k, v = (torch.randn(1, n, h, 64, generator=gen, device="cuda").half() for n in (nq, nk, nk))
+        logits, kw = torch.einsum("bqhd,bkhd->bhqk", q.float(), k.float()) * 0.125, {}
+        if form == "dense":
+            kw["bias"] = ff.tile_layout(torch.randn(1, h, nq, nk, generator=gen, device="cuda").half())
+            logits += kw["bias"].float()
+        elif form == "rel":
+            kw["rel"] = tuple(torch.randn(1, h, nq, side, generator=gen, device="cuda").half() for side in hw)
+            logits += (kw["rel"][0].float()[..., :, None] + kw["rel"][1].float()[..., None, :]).reshape(1, h, nq, nk)
+        ref = torch.einsum("bhqk,bkhd->bqhd", logits.softmax(-1), v.float())
+        out = torch.full_like(q, float("nan"))
+        names = kernels_of(lambda: ff.attention(q, k, v, scale=0.125, layout="bnhd", out=out, **kw))  # noqa: B023
+        assert len(names) == 1 and kernel in names[0], (h, names)
+        assert_close(out.float().cpu().numpy(), ref.cpu().numpy(), unit_scale=True, what=f"[{h},{nq},{nk}] {form}")
 
 
 @pytest.mark.parametrize(("b", "h", "nq", "hw"), [(3, 5, 70, (57, 1)), (2, 7, 130, (64, 2)), (5, 31, 200, (60, 5)), (2, 9, 257, (63, 17)), (1, 6, 300, (120, 8)), (7, 29, 128, (100, 20)), (2, 3, 512, (72, 56)), (1, 5, 385, (64, 64)), (1, 3, 129, (96, 32))])  # fmt: skip
