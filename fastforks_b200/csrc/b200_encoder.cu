@@ -278,10 +278,13 @@ struct Forward {
   }
 
   // Activations of a large batch do not fit L2. What a kernel wrote last is still there, and one that begins with that finds it: with norms
-  // and attention going forwards through the rows, qkv, projection and fc1 go backwards, and fc2 forwards. us per forward, all forwards and
-  // so: ViT-g/14 at 16 images of 518 px 52737 and 52389, ViT-L/14 at 16 17257 and 17023, ViT-B/14 at 16 5686 and 5612, ViT-B/16 at 110 of 224 px
-  // 4567 and 4486; ViT-L/14 at 4, whose widest tensors of 34 and 45 MB fit, 4848 and 4865.
-  static constexpr int64_t kLargeQkvBytes = 64 << 20;
+  // and attention going forwards through the rows, qkv, projection and fc1 go backwards, and fc2 forwards. The line is drawn by the qkv tensor
+  // of the tokens (padded windows add up to a third to it). us for twelve blocks, all forwards and so, 518 px images, medians of five in turn:
+  // at 34 to 38 MB the same (ViT-L/14 at 4 2440 and 2443, ViT-B/14 at 6 2295 and 2300, ViT-S/14 at 12 1781 and 1801; SAM ViT-B at two images of 1024 px
+  // 2830 and 2831), at 42 to 44 hardly less (ViT-L/14 at 5 2854 and 2845, ViT-B/14 at 7 2701 and 2686), from 51 on 0.4 to 2 % less (ViT-L/14 at 6 3423
+  // and 3371, ViT-B/14 at 8 2933 and 2902, ViT-g/14 at 4 4288 and 4231; SAM at three, 57 MB, 4087 and 4044, at four 5415 and 5344; ViT-L/14 at 16, 135 MB,
+  // 8598 and 8495, ViT-B/14 at 16 5687 and 5555, ViT-g/14 at 16, 202 MB, 15955 and 15760).
+  static constexpr int64_t kLargeQkvBytes = 48 << 20;
   int block(const B200EncoderBlock& k) const {
     const int rows = static_cast<int>(l.rows), dim = a->dim;
     const bool back = l.rows * 6 * dim > kLargeQkvBytes;

@@ -87,9 +87,10 @@ def test_one_block_of_every_kind(b: int, grid: tuple[int, int], window: int, hea
     assert_close(x.float().cpu().numpy(), ref.cpu().numpy(), unit_scale=False, what=f"{b} {grid} {window} {hidden}")
 
 
-@pytest.mark.parametrize(("b", "grid", "window", "hidden", "ffn"), [(9, (40, 40), 0, 768, encoder.FFN_GELU), (9, (40, 41), 0, 776, encoder.FFN_SWIGLU), (9, (40, 41), 14, 1536, encoder.FFN_GELU_TANH)])  # fmt: skip
+@pytest.mark.parametrize(("b", "grid", "window", "hidden", "ffn"), [(7, (39, 40), 0, 768, encoder.FFN_GELU), (7, (7, 223), 0, 776, encoder.FFN_SWIGLU), (7, (40, 40), 14, 1536, encoder.FFN_GELU_TANH), (9, (40, 40), 0, 768, encoder.FFN_GELU), (9, (40, 41), 0, 776, encoder.FFN_SWIGLU), (9, (40, 41), 14, 1536, encoder.FFN_GELU_TANH)])  # fmt: skip
 def test_one_block_on_either_side_of_going_backwards(b: int, grid: tuple[int, int], window: int, hidden: int, ffn: int) -> None:
-    """A qkv tensor just below and just above 64 MiB, from which on some products take the rows from the last to the first."""
+    """A qkv tensor of the tokens just below and just above 48 MiB, from which on some products take the rows from the last to the first, the
+    same with padded windows, and larger ones."""
     test_one_block_of_every_kind(b, grid, window, 12, hidden, ffn)
 
 
