@@ -111,13 +111,13 @@ def test_tile_boundaries(n: int, dtype: str) -> None:
     assert_close(got.float().cpu().numpy(), oracle_of_packed(qkv, 0.125), unit_scale=True, what=f"n{n} {dtype}")
 
 
-@pytest.mark.parametrize("n", [1, 2, 63, 64, 65, 127, 128, 129, 130, 160, 196, 197, 225, 255, 256, 257, 383, 385, 512])
+@pytest.mark.parametrize("n", [65, 80, 96, 97, 112, 127, 128, 129, 130, 160, 196, 197, 225, 255, 256, 257, 383, 385, 512])
 @pytest.mark.parametrize("dtype", ["fp16", "bf16"])
 def test_tile_boundaries_of_the_persistent_kernel(n: int, dtype: str) -> None:
-    """The same edges (128-row query tiles, 128-key tiles, two tiles per CTA) with more heads than the kernel of small calls takes
-    (300 blocks of queries on 148 SMs), both schedules and the automatic choice with the same bits, and nothing
-    written around the output view."""
-    b, h, dt = 3, 100, DTYPES[dtype]
+    """The same edges (128-row query tiles, 128-key tiles, two tiles per CTA) with more heads than the kernels of small calls and of few
+    keys take (the latter up to 64 keys at any number of such heads, see the test of one key tile below), both schedules and the automatic
+    choice with the same bits, and nothing written around the output view."""
+    b, h, dt = 3, 100 if n > 112 else 260, DTYPES[dtype]
     gen = torch.Generator(device="cuda").manual_seed(n)
     qkv = torch.randn(b, n, 3, h, 64, generator=gen, device="cuda").to(dt)
     q, k, v = qkv.unbind(2)
@@ -132,6 +132,34 @@ def test_tile_boundaries_of_the_persistent_kernel(n: int, dtype: str) -> None:
         outs.append(out.clone())
         out.fill_(77.0)
         assert bool((big == 77.0).all())
+        assert "attn_fwd_kernel" in kernels_of(lambda: ff.attention(q, k, v, scale=0.125, layout="bnhd", out=out, schedule=schedule))[0]  # noqa: B023
+    assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
+
+
+@pytest.mark.parametrize(("b", "h", "nq", "hw"), [(64, 16, 80, (8, 10)), (64, 16, 96, (12, 8)), (6, 261, 49, (8, 12)), (5, 163, 100, (8, 10)), (3, 260, 300, (7, 10)), (10, 120, 130, (8, 16)), (9, 100, 256, (8, 8))])  # fmt: skip
+@pytest.mark.parametrize(("form", "dtype"), [("plain", "fp16"), ("plain", "bf16"), ("dense", "fp16"), ("dense", "bf16"), ("rel", "fp16"), ("rel", "bf16")])
+def test_one_key_tile_in_every_schedule_of_the_persistent_kernel(b: int, h: int, nq: int, hw: tuple[int, int], form: str, dtype: str) -> None:
+    """At most 128 keys on so many heads that the persistent kernel answers: last tiles of up to 96 keys, which the short schedule is for,
+    and fuller ones; one-tile items two by two, two-tile items, both. The three hints give the same bits; against float32."""
+    if form == "rel" and hw == (8, 8):
+        hw = (2, 31)  # tables of 33 values: more than the kernel for few keys takes
+    t, nk = DTYPES[dtype], hw[0] * hw[1]
+    gen = torch.Generator(device="cuda").manual_seed(nq * 1000 + nk)
+    q, k, v = (torch.randn(b, n, h, 64, generator=gen, device="cuda").to(t) for n in (nq, nk, nk))
+    logits, kw = torch.einsum("bqhd,bkhd->bhqk", q.float(), k.float()) * 0.125, {}
+    if form == "dense":
+        kw["bias"] = ff.tile_layout(torch.randn(1, h, nq, nk, generator=gen, device="cuda").to(t))
+        logits += kw["bias"].float()
+    elif form == "rel":
+        kw["rel"] = tuple(torch.randn(b, h, nq, side, generator=gen, device="cuda").to(t) for side in hw)
+        logits += (kw["rel"][0].float()[..., :, None] + kw["rel"][1].float()[..., None, :]).reshape(b, h, nq, nk)
+    ref = torch.einsum("bhqk,bkhd->bqhd", logits.softmax(-1), v.float())
+    outs = []
+    for schedule in ("auto", "long", "short"):
+        out = torch.full_like(q, float("nan"))
+        assert "attn_fwd_kernel" in kernels_of(lambda: ff.attention(q, k, v, scale=0.125, layout="bnhd", out=out, schedule=schedule, **kw))[0]  # noqa: B023
+        outs.append(out)
+    assert_close(outs[0].float().cpu().numpy(), ref.cpu().numpy(), unit_scale=True, what=f"[{b},{h},{nq},{nk}] {form} {dtype}")
     assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
 
 
@@ -199,8 +227,9 @@ def test_dense_bias_broadcast_and_mask(bias_dtype: torch.dtype) -> None:
 )
 @pytest.mark.parametrize("bias_dtype", [torch.float16, torch.bfloat16])
 def test_dense_bias_in_tiles(b: int, h: int, nq: int, nk: int, bias_shape: tuple[int, ...], pad: int, bias_dtype: torch.dtype) -> None:
-    """A 16-bit bias whose rows start on 16-byte boundaries reaches the kernel as 128 x 64 tiles through TMA (the
-    other layouts take the row-wise loads): every broadcast form, padded rows, -inf columns, short and long schedule."""
+    """A 16-bit bias whose rows start on 16-byte boundaries reaches the kernel as 128 x 64 tiles through TMA, or is read as it lies by the
+    kernel for few keys (77 and 64 here; the other layouts take the row-wise loads): every broadcast form, padded rows, -inf columns, short
+    and long schedule."""
     gen = torch.Generator().manual_seed(nq * 7 + nk)
     q = torch.randn(b, h, nq, 64, generator=gen).half().cuda()
     k, v = (torch.randn(b, h, nk, 64, generator=gen).half().cuda() for _ in range(2))
@@ -342,7 +371,8 @@ def test_full_size_configs_by_properties(b: int, h: int, n: int, dtype: str) -> 
                                         ((34, 34), 257), ((63, 62), 129), ((1, 120), 64), ((120, 1), 64), ((2, 64), 128), ((64, 64), 200)])  # fmt: skip
 @pytest.mark.parametrize("rel_dtype", [torch.float16, torch.bfloat16])
 def test_decomposed_bias_as_a_product(hw: tuple[int, int], nq: int, rel_dtype: torch.dtype) -> None:
-    """The decomposed bias as a second product into the logits, over several items per CTA (batch x heads > SMs / 2)."""
+    """The decomposed bias as a second product into the logits, over several items per CTA (batch x heads > SMs / 2). (Tables of q's type
+    on up to 128 keys are answered by the kernel for few keys, those of the other type by the persistent one.)"""
     kh, kw = hw
     n = kh * kw
     b, h = (3, 40) if n <= 256 else (2, 3)
@@ -370,7 +400,7 @@ def test_decomposed_bias_masks_and_other_scales() -> None:
 
 # Lists of three items and more per CTA, so that row sums, staging buffers and output tiles are handed over again and again: twins of
 # one and of four key tiles, two-tile items of one, two and three, and one-tile items behind them.
-@pytest.mark.parametrize(("b", "h", "n", "side"), [(40, 24, 60, 0), (50, 16, 97, 0), (40, 12, 250, 0), (30, 12, 384, 0), (9, 48, 390, 0), (50, 12, 196, 14)])
+@pytest.mark.parametrize(("b", "h", "n", "side"), [(40, 24, 70, 0), (50, 16, 97, 0), (40, 12, 250, 0), (30, 12, 384, 0), (9, 48, 390, 0), (50, 12, 196, 14)])
 @pytest.mark.parametrize("dtype", ["fp16", "bf16"])
 def test_many_items_per_cta(b: int, h: int, n: int, side: int, dtype: str) -> None:
     gen = torch.Generator(device="cuda").manual_seed(n)
@@ -382,6 +412,7 @@ def test_many_items_per_cta(b: int, h: int, n: int, side: int, dtype: str) -> No
         bias = (rel[0].float()[..., :, None] + rel[1].float()[..., None, :]).reshape(b, h, n, n)
     ref = ((q.float() @ k.float().mT) * 0.125 + bias).softmax(-1) @ v.float()
     got = ff.scaled_dot_product_attention(q, k, v, rel=rel, scale=0.125) if side else ff.scaled_dot_product_attention(q, k, v, scale=0.125)
+    assert "attn_fwd_kernel" in kernels_of(lambda: ff.scaled_dot_product_attention(q, k, v, rel=rel, scale=0.125))[0]
     assert ff.device_status() == 0
     assert_close(got.float().cpu().numpy(), ref.cpu().numpy(), unit_scale=True, what=f"[{b},{h},{n}] {dtype}")
 
@@ -706,7 +737,7 @@ def test_both_schedules_give_the_same_result(schedule: str, n: int) -> None:
     assert torch.equal(got, other)
 
 
-GRIDS = {9: ((3, 3), (9, 1)), 128: ((16, 8), (64, 2)), 190: ((10, 19), (2, 95)), 300: ((12, 25), (100, 3)), 640: ((20, 32), (80, 8))}
+GRIDS = {72: ((8, 9), (36, 2)), 128: ((16, 8), (64, 2)), 190: ((10, 19), (2, 95)), 300: ((12, 25), (100, 3)), 640: ((20, 32), (80, 8))}
 
 
 @pytest.mark.parametrize(("b", "h", "nq"), [(1, 2, 128), (2, 149, 49), (3, 197, 100), (3, 151, 300), (2, 222, 260), (1, 445, 300), (4, 149, 130)])
@@ -715,8 +746,11 @@ GRIDS = {9: ((3, 3), (9, 1)), 128: ((16, 8), (64, 2)), 190: ((10, 19), (2, 95)),
 def test_one_tile_remainders_of_two_heads_side_by_side(b: int, h: int, nq: int, nk: int, form: str, dtype: str) -> None:
     """Lists of one-tile items taken two by two, behind and before other kinds of items, over one to five key tiles (the
     stages of the K and V rings used once, twice, and round and round), in the forms with two and with three stages and
-    with one and two buffers of one-hot rows. Against float32 on the same 16-bit inputs, every row."""
+    with one and two buffers of one-hot rows. Against float32 on the same 16-bit inputs, every row. (Of one key tile, so many heads that
+    the kernel for few keys leaves them.)"""
     t = DTYPES[dtype]
+    if nk <= 128 and nq <= 100:
+        b *= 6 if nq < 64 else 2
     gen = torch.Generator(device="cuda").manual_seed(nq * 1000 + nk)
     q = torch.randn(b, h, nq, 64, generator=gen, device="cuda").to(t)
     k, v = (torch.randn(b, h, nk, 64, generator=gen, device="cuda").to(t) for _ in range(2))
@@ -730,6 +764,8 @@ def test_one_tile_remainders_of_two_heads_side_by_side(b: int, h: int, nq: int, 
         logits += (rel[0].float()[..., :, None] + rel[1].float()[..., None, :]).reshape(b, h, nq, nk)
     ref = torch.einsum("bhqk,bhkd->bhqd", logits.softmax(-1), v.float())
     got = ff.scaled_dot_product_attention(q, k, v, attn_mask=bias, rel=rel)
+    if b * h > 2:
+        assert "attn_fwd_kernel" in kernels_of(lambda: ff.scaled_dot_product_attention(q, k, v, attn_mask=bias, rel=rel))[0]
     assert ff.device_status() == 0
     assert_close(got.float().cpu().numpy(), ref.cpu().numpy(), unit_scale=True, what=f"[{b},{h},{nq},{nk}] {form} {dtype}")
 
