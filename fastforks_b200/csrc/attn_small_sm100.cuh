@@ -15,6 +15,7 @@
 
 #include <type_traits>
 
+#include "attn_fwd_sm100.cuh"
 #include "sm100_ptx.cuh"
 
 namespace b200 {
@@ -42,31 +43,11 @@ constexpr int small_attn_smem(int steps) {
 }
 
 template <typename T>
-__device__ __forceinline__ uint32_t small_pack2(float lo, float hi) {
-  if constexpr (std::is_same<T, __half>::value) {
-    __half2 h = __floats2half2_rn(lo, hi);
-    return *reinterpret_cast<uint32_t*>(&h);
-  } else {
-    __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
-    return *reinterpret_cast<uint32_t*>(&h);
-  }
-}
-
-__device__ __forceinline__ float small_exp2(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-
-// Rows of 128 bytes, their 16-byte chunks permuted so that eight rows of one chunk lie in different banks.
-__device__ __forceinline__ uint32_t small_chunk(uint32_t base, int row, int chunk) { return base + row * 128 + ((chunk ^ (row & 7)) << 4); }
-
-template <typename T>
 __device__ __forceinline__ void small_load(uint32_t smem, const T* rows, int64_t stride, int first, int end, int count) {
   for (int i = threadIdx.x; i < count * 8; i += kSmallThreads) {
     const int row = i >> 3, chunk = i & 7;
     const bool valid = first + row < end;
-    cp_async_16(small_chunk(smem, row, chunk), rows + (valid ? first + row : 0) * stride + chunk * 8, valid);
+    cp_async_16(swizzled_chunk(smem, row, chunk), rows + (valid ? first + row : 0) * stride + chunk * 8, valid);
   }
 }
 
@@ -104,11 +85,11 @@ __global__ void __launch_bounds__(kSmallThreads) attn_small_kernel(const SmallAt
 #pragma unroll
   for (int d = 0; d < 4; ++d) {
     uint32_t a[4];
-    ldmatrix_x4(a, small_chunk(sq, group * 16 + (lane & 15), 2 * d + (lane >> 4)));
+    ldmatrix_x4(a, swizzled_chunk(sq, group * 16 + (lane & 15), 2 * d + (lane >> 4)));
 #pragma unroll
     for (int i = 0; i < STEPS; ++i) {
       uint32_t kk[4];
-      ldmatrix_x4(kk, small_chunk(sk, key0 + i * 16 + (lane & 7) + ((lane >> 4) << 3), 2 * d + ((lane >> 3) & 1)));
+      ldmatrix_x4(kk, swizzled_chunk(sk, key0 + i * 16 + (lane & 7) + ((lane >> 4) << 3), 2 * d + ((lane >> 3) & 1)));
       mma_16816<T>(s[2 * i], a, kk[0], kk[1]);
       mma_16816<T>(s[2 * i + 1], a, kk[2], kk[3]);
     }
@@ -135,9 +116,9 @@ __global__ void __launch_bounds__(kSmallThreads) attn_small_kernel(const SmallAt
   for (int j = 0; j < 2 * STEPS; ++j) {
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
-      const float x = small_exp2(fmaf(s[j][2 * r], p.scale_log2, shift[r])), y = small_exp2(fmaf(s[j][2 * r + 1], p.scale_log2, shift[r]));
+      const float x = fast_exp2(fmaf(s[j][2 * r], p.scale_log2, shift[r])), y = fast_exp2(fmaf(s[j][2 * r + 1], p.scale_log2, shift[r]));
       sum[r] += x + y;
-      probs[j][r] = small_pack2<T>(x, y);
+      probs[j][r] = pack2<T>(x, y);
     }
   }
 #pragma unroll
@@ -160,7 +141,7 @@ __global__ void __launch_bounds__(kSmallThreads) attn_small_kernel(const SmallAt
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       uint32_t vv[4];
-      ldmatrix_x4_trans(vv, small_chunk(sv, key0 + i * 16 + (lane & 15), 2 * j + (lane >> 4)));
+      ldmatrix_x4_trans(vv, swizzled_chunk(sv, key0 + i * 16 + (lane & 15), 2 * j + (lane >> 4)));
       mma_16816<T>(acc[2 * j], a, vv[0], vv[1]);
       mma_16816<T>(acc[2 * j + 1], a, vv[2], vv[3]);
     }
@@ -184,7 +165,7 @@ __global__ void __launch_bounds__(kSmallThreads) attn_small_kernel(const SmallAt
   float out[8] = {};
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    const float weight = small_exp2(st[i].x - most);
+    const float weight = fast_exp2(st[i].x - most);
     total = fmaf(weight, st[i].y, total);
     const float4* from = reinterpret_cast<const float4*>(part + (i * kSmallRows + row) * kSmallPartStride + chunk * 8);
     const float4 lo = from[0], hi = from[1];
@@ -194,10 +175,10 @@ __global__ void __launch_bounds__(kSmallThreads) attn_small_kernel(const SmallAt
   if (row0 + row >= p.q_tokens) return;
   const float inv = 1.f / total;
   uint4 packed;
-  packed.x = small_pack2<T>(out[0] * inv, out[1] * inv);
-  packed.y = small_pack2<T>(out[2] * inv, out[3] * inv);
-  packed.z = small_pack2<T>(out[4] * inv, out[5] * inv);
-  packed.w = small_pack2<T>(out[6] * inv, out[7] * inv);
+  packed.x = pack2<T>(out[0] * inv, out[1] * inv);
+  packed.y = pack2<T>(out[2] * inv, out[3] * inv);
+  packed.z = pack2<T>(out[4] * inv, out[5] * inv);
+  packed.w = pack2<T>(out[6] * inv, out[7] * inv);
   *reinterpret_cast<uint4*>(static_cast<T*>(p.o) + b * p.o_stride[0] + (row0 + row) * p.o_stride[1] + h * p.o_stride[2] + chunk * 8) = packed;
 }
 

@@ -28,11 +28,15 @@ constexpr int kWindowMaxKeys = 128;
 constexpr int kWindowMaxRel = 32;  // values of a decomposed bias per row (rel_kh + rel_kw)
 constexpr int kWindowRows = 64;    // queries per CTA
 constexpr int kWindowThreads = 128;
-// CTAs per SM, by registers: 72 a thread hold 64 logits of two rows, 128 hold 128. us at 6 and 7: [8,192,49] / [64,192,49] with a bias
+// CTAs per SM, by registers: 72 a thread hold 64 logits of two rows but for one to four words (spilled, with a bias; without one three at 80), 128
+// hold 128. us at 6 and 7: [8,192,49] / [64,192,49] with a bias
 // 10.5 / 76.6 and 10.5 / 74.8, [8,64,64] 7.1 and 5.8, [100,12,36] with tables 8.4 and 8.0, but [64,12,64] without either 5.7 and 6.3.
 constexpr int window_ctas(int eights, int bias) { return eights > 8 ? 4 : bias == kWindowPlain ? 6 : 7; }
 // 7 x 7 windows and the 50 tokens of a 224 px image in patches of 32 need no eighth group of eight. us with it and without: [64,192,49] with a
 // bias 74.5 and 72.5, [8,192,49] 10.6 and 10.5, [64,12,50] 5.85 and 5.55. (At 64 registers and eight CTAs an SM: 77.1, 10.6, 6.5.)
+// Other counts with an odd number of groups, 17 to 24 and so on, have less from it, and six more forms for every type and bias have not been
+// taken for that. us with the last group and without, dense bias: [64,48,24] 9.1 and 8.8, [64,48,40] 12.5 and 12.2, [64,48,72] 45.3 and 45.3,
+// [8,64,104] 11.1 and 11.0, [64,48,120] 52.5 and 53.0; plain 8.0 and 7.8, 11.5 and 11.4, 37.3 and 37.2, 9.2 and 9.0, 45.4 and 45.5.
 constexpr int window_eights(int keys) { return keys > 48 && keys <= 56 ? 7 : (keys + 15) / 16 * 2; }
 
 struct WindowParams {
@@ -74,8 +78,7 @@ __device__ __forceinline__ void quad_transpose(uint32_t (&w)[4], int lane) {
   }
 }
 
-// Rows of 128 bytes (64: the one-hot operand), their 16-byte chunks permuted so that eight rows of one chunk lie in different banks.
-__device__ __forceinline__ uint32_t window_chunk(uint32_t base, int row, int chunk) { return base + row * 128 + ((chunk ^ (row & 7)) << 4); }
+// Rows of 64 bytes (the one-hot operand), permuted likewise: see swizzled_chunk.
 __device__ __forceinline__ uint32_t onehot_chunk(uint32_t base, int row, int chunk) { return base + row * 64 + ((chunk ^ ((row >> 1) & 3)) << 4); }
 
 // Loads through L2 only (the kernel in front may have written the data while this one was already on the SM), nothing where !valid.
@@ -97,7 +100,7 @@ __device__ __forceinline__ void window_load(uint32_t smem, const T* rows, int64_
 #pragma unroll
   for (int i = 0; i < ROWS * 8 / kWindowThreads; ++i) {
     const int row = (threadIdx.x >> 3) + i * (kWindowThreads / 8), chunk = threadIdx.x & 7;
-    cp_async_16(window_chunk(smem, row, chunk), rows + (row < count ? row : 0) * stride + chunk * 8, row < count);
+    cp_async_16(swizzled_chunk(smem, row, chunk), rows + (row < count ? row : 0) * stride + chunk * 8, row < count);
   }
 }
 
@@ -199,11 +202,11 @@ __global__ void __launch_bounds__(kWindowThreads, window_ctas(EIGHTS, BIAS)) att
 #pragma unroll
     for (int d = 0; d < 4; ++d) {
       uint32_t a[4];
-      ldmatrix_x4(a, window_chunk(sq, warp * 16 + (lane & 15), 2 * d + (lane >> 4)));
+      ldmatrix_x4(a, swizzled_chunk(sq, warp * 16 + (lane & 15), 2 * d + (lane >> 4)));
 #pragma unroll
       for (int i = 0; i < GROUPS; ++i) {
         uint32_t kk[4];
-        ldmatrix_x4(kk, window_chunk(sk, i * 16 + k_row, 2 * d + k_chunk));
+        ldmatrix_x4(kk, swizzled_chunk(sk, i * 16 + k_row, 2 * d + k_chunk));
         mma_16816<T>(s[2 * i], a, kk[0], kk[1]);
         if (2 * i + 1 < EIGHTS) mma_16816<T>(s[2 * i + 1], a, kk[2], kk[3]);
       }
@@ -269,7 +272,7 @@ __global__ void __launch_bounds__(kWindowThreads, window_ctas(EIGHTS, BIAS)) att
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         uint32_t vv[4];
-        ldmatrix_x4_trans(vv, window_chunk(sv, i * 16 + (lane & 15), 2 * j + (lane >> 4)));
+        ldmatrix_x4_trans(vv, swizzled_chunk(sv, i * 16 + (lane & 15), 2 * j + (lane >> 4)));
         mma_16816<T>(acc[2 * j], a, vv[0], vv[1]);
         mma_16816<T>(acc[2 * j + 1], a, vv[2], vv[3]);
       }

@@ -40,8 +40,7 @@ int64_t window_block_limit(const B200AttnArgs* a, int bias, int64_t q_blocks) {
 }  // namespace
 
 bool window_pays(const B200AttnArgs* a, const WindowCall& call, int sms) {
-  static_assert(kWindowCallMaxKeys == kWindowMaxKeys, "one limit");
-  if (a->kv_tokens > kWindowMaxKeys) return false;
+  static_assert(kWindowCallMaxKeys == kWindowMaxKeys, "the caller has looked at the key count");
   if (call.bias == kWindowCallRel && a->rel_kh + a->rel_kw > kWindowMaxRel) return false;
   const int64_t q_blocks = (static_cast<int64_t>(a->q_tokens) + kWindowRows - 1) / kWindowRows, blocks = q_blocks * a->batch * a->heads;
   const int64_t limit = window_block_limit(a, call.bias, q_blocks);

@@ -598,6 +598,8 @@ __device__ __forceinline__ void ldmatrix_x4_trans(uint32_t* r, uint32_t addr) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
 }
+// Rows of 128 bytes, their 16-byte chunks permuted so that eight rows of one chunk lie in different banks (for ldmatrix).
+__device__ __forceinline__ uint32_t swizzled_chunk(uint32_t base, int row, int chunk) { return base + row * 128 + ((chunk ^ (row & 7)) << 4); }
 // 16 bytes from global to shared memory, zeros where !valid (nothing is read then).
 __device__ __forceinline__ void cp_async_16(uint32_t smem, const void* gmem, bool valid) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem), "l"(gmem), "r"(valid ? 16 : 0) : "memory");
