@@ -273,7 +273,9 @@ int b200_rope_qk(const B200RopeArgs* args, void* stream);
  * tile (two one-tile items of different heads that are worked on side by side are listed one after the other), kind (0 whole item, 1 a part whose result goes to the workspace, 2 the part that merges the later ones) -
  * and in *later_parts how many following CTAs hold later parts of its last item.  The plan is computed by the very
  * functions the kernel runs, so tests can check on a CPU that every (query tile, key tile) of a problem is covered
- * exactly once.  `args->workspace` only matters as NULL / not NULL (with a workspace long sequences may be split).
+ * exactly once. For a call that goes to the kernel of small calls or of few keys (see the schedules above) this is the work the
+ * persistent kernel would do, which does not run then.  `args->workspace` only matters as NULL / not NULL (with a
+ * workspace long sequences may be split).
  * The reference has no counterpart: its grid is (query tiles, batch * heads), fastbb/__init__.py:130-135.
  */
 int b200_attn_plan(const B200AttnArgs* args, int32_t sms, int32_t cta, int32_t* grid, int32_t* items, int32_t max_items,
